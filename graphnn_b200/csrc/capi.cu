@@ -349,6 +349,50 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
     void* plan = ws + 3 * nd + align_up(sizeof(float) * (size_t)G * d, 256);
 
     int rc;
+    // Batches of graphs (the caller vouches for the largest one) whose embeddings fit a CTA's shared memory: the whole
+    // classifier is one kernel, with a launch before it for what every CTA would otherwise work out again, and the
+    // readout behind it.
+    //   * few graphs per CTA: the readout runs inside the kernel too, one launch in all;
+    //   * from S2V_FUSED_TABLE_NODES nodes on, the first level's product table and W in the operand layout are made
+    //     once, in front (below that the two launches cost more than they save);
+    //   * with embed_out, batches below S2V_FUSED_EMBED_NODES nodes keep one launch per level: callers of that form
+    //     observe the launch count of the per-level path.
+    //   * d = 128: batches below S2V_FUSED_TABLE_NODES nodes; larger ones go to the kernels below.
+    const bool forced = ctx->graph_tiles == 1;
+    if (ctx->graph_tiles != 0 && (d != 128 || (!forced && N < S2V_FUSED_TABLE_NODES)) && L >= 1 && N > 0 && G < (int64_t)INT32_MAX && batch->max_graph_nodes >= 1 &&
+        (forced || !embed_out || N >= S2V_FUSED_EMBED_NODES) && (batch->tags || batch->x_dense) &&
+        s2v_graph_fused_supported(ctx, d, batch->max_graph_nodes, batch->tags ? model->num_feat : 1)) {
+        if (!s2v_aligned16(model->w_n2l) || !s2v_aligned16(model->p_node_conv) || (embed_out && !s2v_aligned16(embed_out)))
+            return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "forward: weights and embed_out must be 16-byte aligned");
+        s2v_graph_fused_args a;
+        a.G = G; a.N = N; a.d = d; a.levels = L;
+        a.max_graph_nodes = batch->max_graph_nodes;
+        a.pool_average = model->pool_average;
+        a.row_ptr = batch->n2n_row_ptr; a.col_idx = batch->n2n_col_idx; a.val = batch->n2n_val; a.graph_ptr = batch->graph_ptr;
+        a.W = model->p_node_conv;
+        a.Y = y; a.embed_out = embed_out;
+        if (batch->tags) {
+            a.tags = batch->tags; a.x = model->w_n2l; a.num_tags = model->num_feat;
+        } else {
+            rc = s2v_input_proj_dense_f32(ctx, st, N, model->num_feat, d, batch->x_dense, model->w_n2l, msg, nullptr);
+            if (rc != S2V_OK) return rc;
+            a.x = msg; a.num_tags = 1;
+        }
+        const bool small = !forced && N < S2V_FUSED_TABLE_NODES;
+        if (!small) {   // (msg of a one-hot batch, ha and hb are free here)
+            if (batch->tags && ctx->first_table_on && s2v_first_table_scratch_bytes(model->num_feat + 1, d) <= nd) a.P_scratch = msg;
+            if (s2v_graph_fused_image_bytes(d) <= 2 * nd) a.image_scratch = ha;
+        }
+        const bool readout_inside = small && s2v_graph_fused_readout_ok(d, model->hidden, model->num_class);
+        if (readout_inside) {
+            a.W1 = model->h1_weight; a.W2 = model->h2_weight; a.hidden = model->hidden; a.num_class = model->num_class;
+            a.logits = logits; a.probs = probs; a.pred = pred;
+        }
+        rc = s2v_launch_graph_fused(ctx, st, a);
+        if (rc != S2V_OK || readout_inside) return rc;
+        return s2v_readout_f32(ctx, st, G, d, model->hidden, model->num_class, y, model->h1_weight, model->h2_weight, logits, probs,
+                               pred);
+    }
     // Batches of small graphs (the caller vouches for the largest one): the whole classifier up to the pooled
     // embeddings is one kernel that keeps the node embeddings of a tile of whole graphs in shared memory.
     // Measured on 20-40-node graphs, d = 128, 4 levels: one launch beats the per-level kernels by 1.9x at 16 k nodes,

@@ -172,6 +172,35 @@ int s2v_launch_level_first_table(s2v_ctx* ctx, cudaStream_t st, int64_t n, int d
                                  float* P_scratch, float* out);
 // records S2V_ERR_INVALID_ARG in the status word if any idx[i] lies outside [0, limit)
 int s2v_launch_index_check(s2v_ctx* ctx, cudaStream_t st, int64_t n, const int32_t* idx, int limit);
+// batches of whole graphs whose embeddings stay in shared memory across the levels (graph_fused.cu)
+struct s2v_graph_fused_args {
+    int64_t G = 0, N = 0;
+    int d = 0, levels = 0, max_graph_nodes = 0, pool_average = 0;
+    const int32_t* row_ptr = nullptr;
+    const int32_t* col_idx = nullptr;
+    const float* val = nullptr;
+    const int32_t* graph_ptr = nullptr;
+    const int32_t* tags = nullptr;   // one-hot tags, x = W_in [num_tags x d]; NULL: x = dense projection [N x d]
+    const float* x = nullptr;
+    int num_tags = 0;
+    const float* W = nullptr;
+    float* P_scratch = nullptr;      // (num_tags + 1) * d floats: first level as a sum of rows of ReLU(W_in) * W (tags only)
+    void* image_scratch = nullptr;   // s2v_graph_fused_image_bytes(d): W in the operand layout, converted once per batch
+    float* Y = nullptr;              // [G x d] when logits == NULL
+    float* embed_out = nullptr;
+    const float* W1 = nullptr;       // readout inside the kernel when logits != NULL
+    const float* W2 = nullptr;
+    int hidden = 0, num_class = 0;
+    float* logits = nullptr;
+    float* probs = nullptr;
+    int32_t* pred = nullptr;
+};
+constexpr int64_t S2V_FUSED_TABLE_NODES = 32768;   // batches from this many nodes on: weights and first-level table prepared by launches of their own
+constexpr int64_t S2V_FUSED_EMBED_NODES = 16384;   // batches with embed_out below this many nodes take the per-level kernels
+bool s2v_graph_fused_supported(const s2v_ctx* ctx, int d, int max_nodes, int num_tags);
+size_t s2v_graph_fused_image_bytes(int d);
+bool s2v_graph_fused_readout_ok(int d, int hidden, int num_class);
+int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_args& a);
 // whole classifier up to the pooled embeddings for batches of graphs of at most S2V_TILE_NODES nodes (d = 128, tags)
 constexpr int S2V_TILE_NODES = 128;
 constexpr int64_t S2V_TILE_AUTO_MAX_NODES = 160000;   // automatic mode: batches up to this many nodes take the tile kernel

@@ -1,0 +1,924 @@
+// The structure2vec classifier of a batch of small and medium graphs in ONE kernel: input projection, all levels,
+// pooling and (for small batches) the readout, with the node embeddings in shared memory from the first level to the
+// pooled sum.
+//
+//     H0   = ReLU(X)                               X = W_in[tag] (one-hot tags) or a dense projection made beforehand
+//     Hl+1 = ReLU((A * Hl) * W + X),  l = 0..L-1   Y[g] = sum (or mean) of HL over the nodes of graph g
+//     logits = ReLU(Y * W1) * W2, softmax, argmax
+//
+// (examples/graph_classification/src/kernel_mean_field.cpp:31-47 of the reference.)  A batch of graphs is block
+// diagonal, so a CTA that owns whole graphs never needs a row of another CTA: HBM sees the CSR, the tags and the
+// results, and the neighbour sums read shared memory at 128 bytes per clock instead of L2.
+//
+// Work split.  Every CTA owns a contiguous range of graphs that starts at an equal share of the nodes (found by a
+// search in graph_ptr, no planning launch) and walks it in tiles of whole graphs of at most `cap` nodes.  A tile is up
+// to cap/128 row blocks of 128 nodes.  Per level and row block:
+//   gather  : d/4 lanes own one node row; they add the neighbour rows in CSR order (fp32), scale the sum by a power of
+//             two taken from its own largest element, split it into an fp16 head and tail and store both as the
+//             K-major MMA operand.  The scale is per row, so a graph's results do not depend on its neighbours in the tile.
+//   product : the warp that finishes last issues tcgen05.mma, A = the 128 rows, B = W^T (head and tail, scaled by its largest element):
+//             tail*head, head*tail, head*head into one fp32 accumulator in tensor memory.  fp16 head + tail carry 22
+//             bits of every element within 2^-17 of its row's largest one and 2^-39 of that largest one below it: the
+//             TF32 head + tail pair carries the same 22 bits, at twice the operand bytes and half the MMA rate.
+//   drain   : once every row block of the level is multiplied (tensor memory holds the whole new H, so no second copy
+//             in shared memory is needed): accumulator * 2^-k + X, ReLU, back into the H rows.
+// H rows are stored in 16-byte pieces XOR-swizzled by the row's low three bits: a row is read by its lanes, and
+// written by lanes that own 32 different rows, without bank conflicts.
+//
+// Every wait is bounded and nobody leaves the sequence of barriers: after a time-out (recorded in the status word) the
+// remaining waits return at once and the kernel runs to its end.
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+#include "tcgen05.cuh"
+
+namespace
+{
+
+constexpr int GF_MAXG = 64;   // graphs per tile
+
+struct GfParams {
+    int64_t G;
+    const int32_t* row_ptr;
+    const int32_t* col_idx;
+    const float* val;
+    const int32_t* graph_ptr;
+    const int32_t* tags;      // NULL: dense input, X rows at `x`
+    const float* x;           // tags: W_in [num_tags x d]; dense: msg [N x d]
+    int num_tags;
+    const float* W;
+    const void* w_image;      // W^T as scaled fp16 head / tail in the operand layout (gf_weight_image_kernel), or NULL
+    const float* P;           // ReLU(W_in) * W, or NULL (the first level goes through the MMAs)
+    int levels;               // MMA levels
+    int pool_average;
+    float* Y;                 // [G x d], or NULL when the readout runs here
+    float* embed_out;
+    const float* W1;          // readout in this kernel when logits != NULL
+    const float* W2;
+    int hidden, num_class;
+    float* logits;
+    float* probs;
+    int32_t* pred;
+    int cap, chunk_cap;
+    uint32_t tm_cols;
+    s2v_device_status* status;
+};
+
+template <int D>
+struct GfCfg {
+    static constexpr int LPR = D / 4;                     // lanes (and 16-byte pieces) per row
+    static constexpr uint32_t ROWB = D * 4;
+    static constexpr uint32_t S_BYTES = 128 * D * 4;      // fp16 head + tail of 128 rows
+    static constexpr uint32_t W_BYTES = D * D * 4;
+    static constexpr uint32_t OFF_S = 0, OFF_W = S_BYTES, OFF_H = S_BYTES + W_BYTES;
+    // K chunks of 64 fp16 (one 128-byte swizzle row); d = 32 keeps head and tail side by side in one chunk
+    static constexpr uint32_t S_LO = D == 32 ? 64 : S_BYTES / 2, W_LO = D == 32 ? 64 : W_BYTES / 2;
+    static constexpr int SHIFT = D == 128 ? 5 : (D == 64 ? 4 : 3);
+    static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(D >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // f32 <- f16 x f16, M = 128, N = D
+};
+
+__host__ __device__ constexpr uint32_t gf_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
+
+// Byte offsets behind the H rows (one row more than cap: a row of zeros, what an unused gather slot adds).
+struct GfMap {
+    uint32_t info, roww, tags, goff, rs, bar, col, total;
+};
+template <int D>
+__host__ __device__ inline GfMap gf_map(int cap, int chunk_cap, bool has_val)
+{
+    GfMap m;
+    m.info = GfCfg<D>::OFF_H + (uint32_t)(cap + 1) * GfCfg<D>::ROWB;   // per row: first chunk of columns | chunks << 16
+    m.roww = m.info + 4u * (uint32_t)cap;                              // per row: its edge weight
+    m.tags = m.roww + (has_val ? 4u * (uint32_t)cap : 0u);
+    m.goff = m.tags + gf_up(2u * (uint32_t)(cap + 1), 16);
+    m.rs = m.goff + gf_up(4u * (GF_MAXG + 1), 16);                     // per row: exponent of its operand scale
+    m.bar = m.rs + (uint32_t)cap;
+    m.col = m.bar + 160;                                               // chunks of four 16-bit local columns
+    m.total = m.col + gf_up(8u * (uint32_t)chunk_cap, 16) + 1024;      // + slack to align the base to 1024 bytes
+    return m;
+}
+
+// element (row n, k) of a K-major fp16 operand of `rows` rows: chunk k/64, 128-byte row, 16-byte pieces XOR-swizzled
+__device__ __forceinline__ uint32_t gf_op_off(int n, int k, int rows)
+{
+    return (uint32_t)(k >> 6) * (uint32_t)(rows * 128) + (uint32_t)n * 128u + (uint32_t)((((k & 63) >> 3) ^ (n & 7)) * 16 + (k & 7) * 2);
+}
+// the tail of the same element: LO bytes behind, or (d = 32) in pieces 4..7 of the same 128-byte row
+template <int D>
+__device__ __forceinline__ uint32_t gf_op_off_lo(int n, int k, int rows, uint32_t lo)
+{
+    return D == 32 ? gf_op_off(n, k + 32, rows) : lo + gf_op_off(n, k, rows);
+}
+
+// Power-of-two scale that brings a largest magnitude into [2^14, 2^15), from its exponent e (clamped so that the scale
+// and its inverse stay normal numbers), and the inverse.
+__device__ __forceinline__ uint32_t gf_exponent(uint32_t max_bits) { return max(max_bits >> 23, 15u); }
+__device__ __forceinline__ float gf_scale(uint32_t e) { return __uint_as_float((268u - e) << 23); }
+__device__ __forceinline__ float gf_unscale(uint32_t e) { return __uint_as_float((e - 14u) << 23); }
+
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t pack2(float x, float y)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+// v < 0 ? 0 : v for values that are only added afterwards (NaN stays NaN; -0 becomes +0)
+__device__ __forceinline__ float relu_max(float v)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(v));
+    return r;
+}
+// two scaled values -> packed fp16 heads and tails (head rounded to nearest, tail = exact remainder rounded to nearest)
+__device__ __forceinline__ void split_f16(uint64_t v, uint32_t& hi, uint32_t& lo)
+{
+    const float2 f = unpack2(v);
+    const __half2 h = __floats2half2_rn(f.x, f.y);
+    const float2 hf = __half22float2(h);
+    const __half2 l = __floats2half2_rn(f.x - hf.x, f.y - hf.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        :
+        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tc_ld_cols8(uint32_t addr, uint32_t* v)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(addr)
+                 : "memory");
+}
+
+// first graph whose first node is at or behind `target` (graph_ptr ascending), found by one warp 32 probes at a time
+__device__ __forceinline__ int64_t gf_lower_graph(const int32_t* graph_ptr, int64_t G, int64_t target)
+{
+    const int lane = threadIdx.x & 31;
+    int64_t lo = 0, hi = G;   // answer in [lo, hi]
+    while (hi > lo) {
+        const int64_t step = (hi - lo + 31) / 32;
+        const int64_t at = lo + step * lane;
+        const bool below = at < hi && (int64_t)__ldg(graph_ptr + at) < target;
+        const int n = __popc(__ballot_sync(0xffffffffu, below));
+        if (n == 0) return lo;
+        lo = lo + step * (n - 1) + 1;
+        hi = lo + step - 1 < hi ? lo + step - 1 : hi;
+    }
+    return lo;
+}
+
+// W^T as the B operand: scaled fp16 head and tail.  Thread t converts pairs of consecutive k of one column n.
+// s_max is zeroed beforehand; contains a barrier, so every thread of the CTA calls it.
+template <int D, int THREADS>
+__device__ __forceinline__ void gf_convert_w(const float* __restrict__ W, unsigned char* dst, uint32_t* s_max, float& inv_w)
+{
+    constexpr int PAIRS = D * D / 2, PER = (PAIRS + THREADS - 1) / THREADS;
+    float a[PER][2];
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int p = threadIdx.x + i * THREADS;
+        const int n = p % D, k = p / D * 2;
+        a[i][0] = p < PAIRS ? __ldg(W + k * D + n) : 0.f;
+        a[i][1] = p < PAIRS ? __ldg(W + (k + 1) * D + n) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) m = fmaxf(m, fmaxf(fabsf(a[i][0]), fabsf(a[i][1])));
+    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) atomicMax(s_max, w);
+    __syncthreads();
+    const uint32_t e_w = gf_exponent(*s_max);
+    const float s = gf_scale(e_w);
+    inv_w = gf_unscale(e_w);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int p = threadIdx.x + i * THREADS;
+        if (p < PAIRS) {
+            const int n = p % D, k = p / D * 2;
+            uint32_t hi, lo;
+            split_f16(pack2(a[i][0] * s, a[i][1] * s), hi, lo);
+            *reinterpret_cast<uint32_t*>(dst + gf_op_off(n, k, D)) = hi;
+            *reinterpret_cast<uint32_t*>(dst + gf_op_off_lo<D>(n, k, D, GfCfg<D>::W_LO)) = lo;
+        }
+    }
+}
+
+// the same into global memory, once per batch: [operand image | inverse scale]
+template <int D>
+__global__ void __launch_bounds__(1024) gf_weight_image_kernel(const float* __restrict__ W, unsigned char* __restrict__ image)
+{
+    __shared__ uint32_t s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    float inv;
+    gf_convert_w<D, 1024>(W, image, &s_max, inv);
+    if (threadIdx.x == 0) *reinterpret_cast<float*>(image + GfCfg<D>::W_BYTES) = inv;
+}
+
+template <int WT>
+__device__ __forceinline__ void gf_worker_sync()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(WT) : "memory");
+}
+
+// readout of NB graphs whose pooled rows lie in shared memory: layer 1 split over threads as (hidden unit, slice of k)
+template <int D, int WT, int NB>
+__device__ __forceinline__ void gf_readout(const GfParams& p, const float* y_s, float* scratch, int nb, int64_t g_first)
+{
+    const int tid = threadIdx.x, hidden = p.hidden, C = p.num_class;
+    int slices = WT / hidden;
+    slices = slices >= 8 ? 8 : (slices >= 4 ? 4 : (slices >= 2 ? 2 : 1));
+    float* part = scratch;                                            // [slices][NB][hidden]
+    float* hid = scratch + (slices > 1 ? slices * NB * hidden : 0);   // [NB][hidden]
+    float* out_s = hid + NB * hidden;                                 // [NB][C]
+    const int items = hidden * slices, kper = D / slices;
+    for (int it = tid; it < items; it += WT) {
+        const int h = it % hidden, sl = it / hidden;
+        float acc[NB];
+#pragma unroll
+        for (int g = 0; g < NB; ++g) acc[g] = 0.f;
+        const float* w = p.W1 + (int64_t)(sl * kper) * hidden + h;
+        const float* y = y_s + sl * kper;
+        constexpr int U = NB == 1 ? 16 : 8;   // loads of W1 in flight
+        for (int k = 0; k < kper; k += U) {
+            float wv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) wv[u] = k + u < kper ? __ldg(w + (int64_t)(k + u) * hidden) : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; u += 4)
+#pragma unroll
+                for (int g = 0; g < NB; ++g) {
+                    const float4 yv = *reinterpret_cast<const float4*>(y + g * D + (k + u < kper ? k + u : 0));
+                    acc[g] = fmaf(yv.x, wv[u], acc[g]);
+                    acc[g] = fmaf(yv.y, wv[u + 1], acc[g]);
+                    acc[g] = fmaf(yv.z, wv[u + 2], acc[g]);
+                    acc[g] = fmaf(yv.w, wv[u + 3], acc[g]);
+                }
+        }
+#pragma unroll
+        for (int g = 0; g < NB; ++g) {
+            if (slices > 1) part[(sl * NB + g) * hidden + h] = acc[g];
+            else hid[g * hidden + h] = relu_ref(acc[g]);
+        }
+    }
+    gf_worker_sync<WT>();
+    if (slices > 1) {
+        for (int e = tid; e < NB * hidden; e += WT) {
+            float s = part[e];
+            for (int sl = 1; sl < slices; ++sl) s += part[sl * NB * hidden + e];
+            hid[e] = relu_ref(s);
+        }
+        gf_worker_sync<WT>();
+    }
+    const int warp = tid >> 5, lane = tid & 31;
+    for (int gc = warp; gc < nb * C; gc += WT / 32) {   // one warp per (graph, class)
+        const int g = gc / C, c = gc - g * C;
+        float acc = 0.f;
+        for (int h = lane; h < hidden; h += 32) acc = fmaf(hid[g * hidden + h], __ldg(p.W2 + (int64_t)h * C + c), acc);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) out_s[gc] = acc;
+    }
+    gf_worker_sync<WT>();
+    for (int g = tid; g < nb; g += WT) {
+        const float* l = out_s + g * C;
+        float mx = l[0];
+        int best = 0;
+        for (int c = 1; c < C; ++c)
+            if (l[c] > mx) { mx = l[c]; best = c; }
+        float s = 0.f;
+        for (int c = 0; c < C; ++c) s += expf(l[c] - mx);
+        for (int c = 0; c < C; ++c) {
+            p.logits[(g_first + g) * C + c] = l[c];
+            if (p.probs) p.probs[(g_first + g) * C + c] = expf(l[c] - mx) / s;
+        }
+        if (p.pred) p.pred[g_first + g] = best;
+    }
+}
+
+// One row's neighbour sum straight from global memory: tiles whose columns do not fit the chunk list, and rows whose
+// edges carry different weights.
+template <int D, bool HAS_VAL>
+__device__ __noinline__ ulonglong2 gf_row_from_global(const int32_t* row_ptr, const int32_t* col_idx, const float* val, s2v_device_status* status,
+                                                      const ulonglong2* H2, int node0, int nrows, int r, int sl)
+{
+    const int b = __ldg(row_ptr + node0 + r), e = __ldg(row_ptr + node0 + r + 1);
+    ulonglong2 acc = make_ulonglong2(0ull, 0ull);
+    for (int t = b; t < e; t += 4) {
+        int c[4];
+        float w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            c[u] = t + u < e ? __ldg(col_idx + t + u) - node0 : 0;
+            w[u] = HAS_VAL && t + u < e ? __ldg(val + t + u) : 1.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (t + u < e) {
+                if ((unsigned)c[u] >= (unsigned)nrows) {
+                    status->code = S2V_ERR_BAD_CSR;
+                    status->where = 5;
+                    c[u] = 0;
+                }
+                const ulonglong2 v = H2[((c[u] << GfCfg<D>::SHIFT) + (c[u] & 7)) ^ sl];
+                const uint64_t ww = pack2(w[u], w[u]);
+                acc.x = fma2(ww, v.x, acc.x);
+                acc.y = fma2(ww, v.y, acc.y);
+            }
+    }
+    return acc;
+}
+
+template <int D, int WARPS, bool HAS_VAL>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fused_kernel(const GfParams p)
+{
+    using Cfg = GfCfg<D>;
+    constexpr int WT = WARPS * 32;
+    constexpr int LPR = Cfg::LPR, GPW = 32 / LPR;   // lanes per row, row groups per warp
+    constexpr int NG = WARPS * GPW;                 // row groups
+    constexpr int RPG = 128 / NG;                   // rows of a row block per group
+    constexpr int CW = D / (WARPS / 4);             // accumulator columns a warp drains
+    constexpr int LDC = CW >= 16 ? 16 : 8;          // columns per tcgen05.ld
+    constexpr int ROUNDS = D == 128 || (D == 64 && WARPS == 8) ? 1 : (D == 32 && WARPS == 8 ? 3 : 2);   // rows per thread in the prologue
+
+    extern __shared__ unsigned char gf_smem_raw[];
+    unsigned char* smem = gf_smem_raw + ((1024u - (smem_u32(gf_smem_raw) & 1023u)) & 1023u);
+    const GfMap map = gf_map<D>(p.cap, p.chunk_cap, HAS_VAL);
+    uint32_t* const info_s = reinterpret_cast<uint32_t*>(smem + map.info);
+    float* const roww = reinterpret_cast<float*>(smem + map.roww);
+    uint16_t* const tag_s = reinterpret_cast<uint16_t*>(smem + map.tags);
+    int* const goff = reinterpret_cast<int*>(smem + map.goff);
+    uint8_t* const rs = smem + map.rs;
+    uint2* const chunks = reinterpret_cast<uint2*>(smem + map.col);
+    float4* const H4 = reinterpret_cast<float4*>(smem + Cfg::OFF_H);
+    const ulonglong2* const H2 = reinterpret_cast<const ulonglong2*>(smem + Cfg::OFF_H);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + map.bar);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + map.bar + 16);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + map.bar + 24);
+    uint32_t* s_max = reinterpret_cast<uint32_t*>(smem + map.bar + 28);
+    int* s_range = reinterpret_cast<int*>(smem + map.bar + 32);
+    uint32_t* s_arrived = reinterpret_cast<uint32_t*>(smem + map.bar + 40);
+    int* s_mixed = reinterpret_cast<int*>(smem + map.bar + 44);
+    int* s_scan = reinterpret_cast<int*>(smem + map.bar + 64);   // WARPS totals
+    const uint32_t bar_mma = smem_u32(bars);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nb_cta = gridDim.x;
+
+    if (threadIdx.x == 0) {
+        tc_mbar_init(bar_mma, 1);
+        *abort_flag = 0;
+        *s_max = 0;
+        *s_arrived = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(p.tm_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // the CTA's graphs: one each when there are no more graphs than CTAs, else an equal share of the nodes
+    if (warp == 1 || warp == 2) {
+        int64_t g;
+        const int64_t i = (int64_t)blockIdx.x + warp - 1;
+        if (p.G <= nb_cta) g = i < p.G ? i : p.G;
+        else g = i >= nb_cta ? p.G : (i == 0 ? 0 : gf_lower_graph(p.graph_ptr, p.G, (int64_t)__ldg(p.graph_ptr + p.G) * i / nb_cta));
+        if (lane == 0) s_range[warp - 1] = (int)g;
+    }
+    if (threadIdx.x < LPR) H4[p.cap * LPR + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);   // the row of zeros
+    const uint32_t zero_entry = (uint32_t)p.cap << Cfg::SHIFT;
+    if (threadIdx.x == 0) {
+        chunks[0] = make_uint2(zero_entry * 0x10001u, zero_entry * 0x10001u);                   // a chunk of zero rows
+        tag_s[p.cap] = (uint16_t)p.num_tags;                                                    // P has a row of zeros behind the last tag
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+    const int g_lo = s_range[0], g_hi = s_range[1];
+    float inv_w;
+    if (p.w_image) {
+        const uint4* src = static_cast<const uint4*>(p.w_image);
+        uint4* dst = reinterpret_cast<uint4*>(smem + Cfg::OFF_W);
+        for (int i = threadIdx.x; i < (int)(Cfg::W_BYTES / 16); i += WT) dst[i] = __ldg(src + i);
+        inv_w = __ldg(reinterpret_cast<const float*>(static_cast<const unsigned char*>(p.w_image) + Cfg::W_BYTES));
+    } else {
+        gf_convert_w<D, WT>(p.W, smem + Cfg::OFF_W, s_max, inv_w);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+
+    uint32_t job = 0;      // row blocks multiplied so far (the same count in every warp)
+    int bad_tag = 0;
+    const int q = warp & 3, jc = warp >> 2;
+    const int sub = lane / LPR, sl = lane % LPR;
+    const int grp = warp * GPW + sub;
+    const float4* __restrict__ X4 = reinterpret_cast<const float4*>(p.x);
+    for (int g0 = g_lo; g0 < g_hi;) {
+        // ---- the tile: whole graphs from g0 on, at most cap nodes and GF_MAXG graphs (every warp works it out by itself)
+        const int node0 = __ldg(p.graph_ptr + g0);
+        int g1 = g0;
+        while (g1 < g_hi && g1 - g0 < GF_MAXG) {
+            const int gi = g1 + 1 + lane;
+            const bool fits = gi <= g_hi && gi - g0 <= GF_MAXG && __ldg(p.graph_ptr + gi) - node0 <= p.cap;
+            const unsigned bal = __ballot_sync(0xffffffffu, fits);
+            const int n = bal == 0xffffffffu ? 32 : __ffs(~bal) - 1;
+            g1 += n;
+            if (n < 32) break;
+        }
+        if (g1 == g0) g1 = g0 + 1;
+        int nrows = __ldg(p.graph_ptr + g1) - node0;
+        if (nrows > p.cap) {   // a graph beyond the capacity: reported, truncated
+            nrows = p.cap;
+            p.status->code = S2V_ERR_UNSUPPORTED;
+            p.status->where = 4;
+        }
+        if (nrows < 0) nrows = 0;
+        const int ngr = g1 - g0;
+        const int mt = (nrows + 127) >> 7;
+
+        // ---- tile prologue: row structure, tags, graph offsets; then local columns in chunks of four, H0
+        int rb[ROUNDS], rn[ROUNDS];
+#pragma unroll
+        for (int k = 0; k < ROUNDS; ++k) {
+            const int r = k * WT + threadIdx.x;
+            rb[k] = rn[k] = 0;
+            if (r < nrows) {
+                rb[k] = __ldg(p.row_ptr + node0 + r);
+                rn[k] = __ldg(p.row_ptr + node0 + r + 1) - rb[k];
+                if (rn[k] < 0) rn[k] = 0;
+                if (p.tags) {
+                    const int t = __ldg(p.tags + node0 + r);
+                    bad_tag |= (unsigned)t >= (unsigned)p.num_tags ? 1 : 0;
+                    tag_s[r] = (uint16_t)((unsigned)t >= (unsigned)p.num_tags ? 0 : t);
+                }
+            }
+        }
+        for (int k = threadIdx.x; k <= ngr; k += WT) {
+            const int v = __ldg(p.graph_ptr + g0 + k) - node0;
+            goff[k] = v < 0 ? 0 : (v > nrows ? nrows : v);
+        }
+        if (HAS_VAL && threadIdx.x == 0) *s_mixed = 0;
+        int first[ROUNDS], carry = 1;   // chunk 0 is the chunk of zero rows
+#pragma unroll
+        for (int k = 0; k < ROUNDS; ++k) {
+            const int c = (rn[k] + 3) >> 2;
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (k > 0) gf_worker_sync<WT>();   // the totals of the previous round are read
+            if (lane == 31) s_scan[warp] = incl;
+            gf_worker_sync<WT>();
+            int tot = lane < WARPS ? s_scan[lane] : 0;
+            int before = lane < warp ? tot : 0;
+            tot = __reduce_add_sync(0xffffffffu, tot);
+            before = __reduce_add_sync(0xffffffffu, before);
+            first[k] = carry + before + incl - c;
+            carry += tot;
+        }
+        const bool cached = carry <= p.chunk_cap;   // uniform over the CTA
+#pragma unroll
+        for (int k = 0; k < ROUNDS; ++k) {
+            const int r = k * WT + threadIdx.x;
+            if (r < nrows) {
+                const int c = (rn[k] + 3) >> 2;
+                info_s[r] = c ? (uint32_t)first[k] | ((uint32_t)c << 16) : 0u;
+                if (cached)
+                    for (int t = 0; t < rn[k]; t += 4) {
+                        uint32_t e[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) e[u] = t + u < rn[k] ? (uint32_t)(__ldg(p.col_idx + rb[k] + t + u) - node0) : (uint32_t)p.cap;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            if (e[u] >= (uint32_t)nrows && t + u < rn[k]) {   // an edge that leaves the tile
+                                p.status->code = S2V_ERR_BAD_CSR;
+                                p.status->where = 5;
+                                e[u] = 0;
+                            }
+                            e[u] = (e[u] << Cfg::SHIFT) + (e[u] & 7u);
+                        }
+                        chunks[first[k] + (t >> 2)] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
+                    }
+                if (HAS_VAL) {
+                    const float w0 = rn[k] > 0 ? __ldg(p.val + rb[k]) : 0.f;
+                    bool mixed = false;
+                    for (int t = 1; t < rn[k]; ++t) mixed |= __ldg(p.val + rb[k] + t) != w0;
+                    roww[r] = w0;
+                    if (mixed) *s_mixed = 1;
+                }
+            }
+        }
+        if (!p.P) {
+            for (int r = grp; r < nrows; r += NG) {
+                int64_t xr = node0 + r;
+                if (p.tags) {
+                    const int t = __ldg(p.tags + xr);
+                    xr = (unsigned)t >= (unsigned)p.num_tags ? 0 : t;
+                }
+                const float4 v = __ldg(X4 + xr * LPR + sl);
+                H4[((r << Cfg::SHIFT) + (r & 7)) ^ sl] = make_float4(relu_ref(v.x), relu_ref(v.y), relu_ref(v.z), relu_ref(v.w));
+            }
+        }
+        gf_worker_sync<WT>();
+        // averaged messages give every edge of a row the same weight: the row is summed unweighted and scaled once
+        const bool listed = cached && !(HAS_VAL && *s_mixed != 0);
+        if (p.P) {   // first level: a sum of rows of P = ReLU(W_in) * W, no product
+            const float4* __restrict__ P4 = reinterpret_cast<const float4*>(p.P);
+            for (int r = grp; r < nrows; r += NG) {
+                const float4 x = __ldg(X4 + (int64_t)tag_s[r] * LPR + sl);
+                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (listed) {
+                    const uint32_t inf = info_s[r];
+                    for (uint32_t c = 0; c < (inf >> 16); ++c) {
+                        const uint2 e2 = chunks[(inf & 0xffffu) + c];
+                        const uint32_t e[4] = {e2.x & 0xffffu, e2.x >> 16, e2.y & 0xffffu, e2.y >> 16};
+                        float4 v[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) v[u] = __ldg(P4 + (int64_t)tag_s[e[u] >> Cfg::SHIFT] * LPR + sl);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
+                    }
+                    if (HAS_VAL) { const float w = roww[r]; acc.x *= w; acc.y *= w; acc.z *= w; acc.w *= w; }
+                } else {
+                    const int b = __ldg(p.row_ptr + node0 + r), e = __ldg(p.row_ptr + node0 + r + 1);
+                    for (int t = b; t < e; ++t) {
+                        int c = __ldg(p.col_idx + t) - node0;
+                        if ((unsigned)c >= (unsigned)nrows) {
+                            p.status->code = S2V_ERR_BAD_CSR;
+                            p.status->where = 5;
+                            c = 0;
+                        }
+                        const float w = HAS_VAL ? __ldg(p.val + t) : 1.f;
+                        const float4 v = __ldg(P4 + (int64_t)tag_s[c] * LPR + sl);
+                        acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
+                    }
+                }
+                H4[((r << Cfg::SHIFT) + (r & 7)) ^ sl] =
+                    make_float4(relu_max(acc.x + x.x), relu_max(acc.y + x.y), relu_max(acc.z + x.z), relu_max(acc.w + x.w));
+            }
+            gf_worker_sync<WT>();
+        }
+
+        for (int lv = 0; lv < p.levels; ++lv) {
+            // -------------------------------- gather, split, hand over --------------------------------
+            for (int m = 0; m < mt; ++m) {
+                const int rows_m = nrows - 128 * m < 128 ? nrows - 128 * m : 128;
+                uint64_t a0[RPG], a1[RPG];
+                if (listed) {
+                    // every row's first chunk is fetched before the first row is summed; further chunks in a loop whose
+                    // count is the warp's largest (a row without them reads the chunk of zero rows)
+                    uint32_t inf[RPG];
+                    uint2 ef[RPG];
+                    const uint32_t slx = (uint32_t)sl * 0x10001u;
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) inf[i] = i * NG + grp < rows_m ? info_s[128 * m + i * NG + grp] : 0u;
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) ef[i] = chunks[inf[i] & 0xffffu];
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) {
+                        a0[i] = a1[i] = 0ull;
+                        if (i * NG + warp * GPW < rows_m) {   // warp-uniform
+                            auto add4 = [&](uint2 e2) {
+                                e2.x ^= slx;
+                                e2.y ^= slx;
+                                const ulonglong2 v0 = H2[e2.x & 0xffffu], v1 = H2[e2.x >> 16], v2 = H2[e2.y & 0xffffu], v3 = H2[e2.y >> 16];
+                                a0[i] = add2(add2(add2(add2(a0[i], v0.x), v1.x), v2.x), v3.x);
+                                a1[i] = add2(add2(add2(add2(a1[i], v0.y), v1.y), v2.y), v3.y);
+                            };
+                            add4(ef[i]);
+                            const uint32_t mine = inf[i] >> 16, most = __reduce_max_sync(0xffffffffu, mine);
+                            for (uint32_t c = 1; c < most; ++c) add4(chunks[c < mine ? (inf[i] & 0xffffu) + c : 0u]);
+                            if (HAS_VAL) {
+                                const float w = i * NG + grp < rows_m ? roww[128 * m + i * NG + grp] : 0.f;
+                                a0[i] = mul2(a0[i], pack2(w, w));
+                                a1[i] = mul2(a1[i], pack2(w, w));
+                            }
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) {
+                        a0[i] = a1[i] = 0ull;
+                        if (i * NG + grp < rows_m) {
+                            const ulonglong2 v = gf_row_from_global<D, HAS_VAL>(p.row_ptr, p.col_idx, p.val, p.status, H2, node0, nrows, 128 * m + i * NG + grp, sl);
+                            a0[i] = v.x;
+                            a1[i] = v.y;
+                        }
+                    }
+                    __syncwarp();
+                }
+                // the operand buffer is free once the previous row block of this level is multiplied
+                if (m > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 40);
+                unsigned char* const s_hi = smem + Cfg::OFF_S + gf_op_off(grp, 4 * sl, 128);   // (row i*NG + grp: + i*NG*128, the same swizzle)
+                unsigned char* const s_lo = smem + Cfg::OFF_S + gf_op_off_lo<D>(grp, 4 * sl, 128, Cfg::S_LO);
+#pragma unroll
+                for (int i = 0; i < RPG; ++i) {
+                    if (i * NG + warp * GPW < rows_m) {
+                        const float2 f0 = unpack2(a0[i]), f1 = unpack2(a1[i]);
+                        uint32_t mx = __float_as_uint(fmaxf(fmaxf(fabsf(f0.x), fabsf(f0.y)), fmaxf(fabsf(f1.x), fabsf(f1.y))));
+                        if (LPR == 32) mx = __reduce_max_sync(0xffffffffu, mx);
+                        else
+#pragma unroll
+                            for (int o = LPR / 2; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                        const uint32_t ex = gf_exponent(mx);
+                        const float s = gf_scale(ex);
+                        const uint64_t ss = pack2(s, s);
+                        uint2 hi, lo;
+                        split_f16(mul2(a0[i], ss), hi.x, lo.x);
+                        split_f16(mul2(a1[i], ss), hi.y, lo.y);
+                        // (rows past the tile's last one are written too: finite, never read back)
+                        *reinterpret_cast<uint2*>(s_hi + i * NG * 128) = hi;
+                        *reinterpret_cast<uint2*>(s_lo + i * NG * 128) = lo;
+                        if (sl == 0 && i * NG + grp < rows_m) rs[128 * m + i * NG + grp] = (uint8_t)ex;
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // my stores -> visible to the tensor core
+                __syncwarp();
+                // the warp that arrives last issues the products of this row block
+                uint32_t order = 0;
+                if (lane == 0)
+                    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(order) : "r"(smem_u32(s_arrived)) : "memory");
+                order = __shfl_sync(0xffffffffu, order, 0);
+                if (order % WARPS == WARPS - 1) {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (lane == 0) {
+                        const uint32_t s_addr = smem_u32(smem + Cfg::OFF_S), w_addr = smem_u32(smem + Cfg::OFF_W);
+                        const uint32_t acc = tmem_base + (uint32_t)(m * D);
+#pragma unroll
+                        for (int pass = 0; pass < 3; ++pass) {   // tail*head, head*tail, head*head: small terms first
+                            const uint32_t a_base = s_addr + (pass == 0 ? Cfg::S_LO : 0u), b_base = w_addr + (pass == 1 ? Cfg::W_LO : 0u);
+#pragma unroll
+                            for (int ks = 0; ks < D / 16; ++ks) {
+                                const uint32_t ao = (uint32_t)(ks >> 2) * (128u * 128u) + (uint32_t)(ks & 3) * 32u;
+                                const uint32_t bo = (uint32_t)(ks >> 2) * (uint32_t)(D * 128) + (uint32_t)(ks & 3) * 32u;
+                                mma_f16_ss(acc, tc_b_desc(a_base + ao), tc_b_desc(b_base + bo), Cfg::IDESC, (pass | ks) != 0);
+                            }
+                        }
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_mma) : "memory");
+                    }
+                    __syncwarp();
+                }
+                ++job;
+            }
+            // -------------------------------- drain: H = ReLU(acc * scale + X) --------------------------------
+            // Units of LDC columns of 32 rows.  X of the next unit is on its way while one is worked on, the first unit's
+            // during the wait.  (The last product of the level completes only after every warp has finished gathering from H.)
+            constexpr int UNITS = CW / LDC;
+            float4 x[LDC / 4];
+            auto x_row = [&](int m) -> const float4* {
+                const int r = 128 * m + 32 * q + lane;
+                const int64_t xr = r < nrows ? (p.tags ? (int64_t)tag_s[r] : (int64_t)node0 + r) : 0;
+                return X4 + xr * LPR + jc * (CW / 4);
+            };
+            const float4* xp = x_row(0);
+#pragma unroll
+            for (int c = 0; c < LDC / 4; ++c) x[c] = __ldg(xp + c);
+            if (mt > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int m = 0; m < mt; ++m) {
+                if (128 * m + 32 * q >= nrows) break;   // warp-uniform
+                const int r = 128 * m + 32 * q + lane;
+                const bool have = r < nrows;
+                const float c1 = have ? gf_unscale(rs[r]) * inv_w : 0.f;
+                const uint64_t cc = pack2(c1, c1);
+                const uint32_t acc_addr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(m * D + jc * CW);
+                const uint32_t he = (uint32_t)((r << Cfg::SHIFT) + (r & 7));
+                const float4* xn = x_row(m + 1);
+#pragma unroll
+                for (int h = 0; h < UNITS; ++h) {
+                    uint32_t v[LDC];
+                    if (LDC == 16) tc_ld_cols16(acc_addr + (uint32_t)(h * LDC), v);
+                    else tc_ld_cols8(acc_addr + (uint32_t)(h * LDC), v);
+                    float4 y[LDC / 4];
+#pragma unroll
+                    for (int c = 0; c < LDC / 4; ++c) y[c] = x[c];
+                    const float4* nx = h + 1 < UNITS ? xp + (h + 1) * (LDC / 4) : xn;
+#pragma unroll
+                    for (int c = 0; c < LDC / 4; ++c) x[c] = __ldg(nx + c);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (have) {
+#pragma unroll
+                        for (int c = 0; c < LDC / 4; ++c) {
+                            const float2 lo2 = unpack2(fma2(pack2(__uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1])), cc, pack2(y[c].x, y[c].y)));
+                            const float2 hi2 = unpack2(fma2(pack2(__uint_as_float(v[4 * c + 2]), __uint_as_float(v[4 * c + 3])), cc, pack2(y[c].z, y[c].w)));
+                            H4[he ^ (uint32_t)(jc * (CW / 4) + h * (LDC / 4) + c)] = make_float4(relu_max(lo2.x), relu_max(lo2.y), relu_max(hi2.x), relu_max(hi2.y));
+                        }
+                    }
+                }
+                xp = xn;
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            gf_worker_sync<WT>();
+        }
+        // -------------------------------- node embeddings, pooling --------------------------------
+        if (p.embed_out)
+            for (int r = grp; r < nrows; r += NG)
+                reinterpret_cast<float4*>(p.embed_out)[(int64_t)(node0 + r) * LPR + sl] = H4[((r << Cfg::SHIFT) + (r & 7)) ^ sl];
+        // Graphs of up to 32 nodes are summed by one warp each; larger ones in pieces of 32 nodes (counted from the
+        // graph's first node) by different warps, the partial sums added in order.
+        float* const y_s = reinterpret_cast<float*>(smem + Cfg::OFF_S);                       // [GF_MAXG][D]
+        float4* const part4 = reinterpret_cast<float4*>(smem + Cfg::OFF_S + Cfg::S_BYTES / 2);  // [GF_MAXG][D]
+        int slot = 0;
+        auto sum_rows = [&](int nb, int ne, float wgt) -> float4 {
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int n = nb + sub; n < ne; n += GPW) {
+                const float4 v = H4[((n << Cfg::SHIFT) + (n & 7)) ^ sl];
+                acc.x = fmaf(wgt, v.x, acc.x); acc.y = fmaf(wgt, v.y, acc.y);
+                acc.z = fmaf(wgt, v.z, acc.z); acc.w = fmaf(wgt, v.w, acc.w);
+            }
+#pragma unroll
+            for (int o = 16; o >= LPR; o >>= 1) {
+                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+                acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+                acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+            }
+            return acc;
+        };
+        auto put_y = [&](int k, float4 acc) {
+            if (sub != 0) return;
+            if (p.logits) reinterpret_cast<float4*>(y_s)[k * LPR + sl] = acc;
+            else reinterpret_cast<float4*>(p.Y)[(int64_t)(g0 + k) * LPR + sl] = acc;
+        };
+        for (int k = 0; k < ngr; ++k) {
+            const int nb = goff[k], ne = goff[k + 1];
+            const float wgt = p.pool_average ? (float)(1.0 / (double)(ne - nb)) : 1.0f;
+            if (ne - nb <= 32) {
+                if (k % WARPS == warp) put_y(k, sum_rows(nb, ne, wgt));
+            } else {
+                for (int c = 0; nb + 32 * c < ne; ++c, ++slot)
+                    if ((k + c) % WARPS == warp) {
+                        const float4 acc = sum_rows(nb + 32 * c, nb + 32 * c + 32 < ne ? nb + 32 * c + 32 : ne, wgt);
+                        if (sub == 0) part4[slot * LPR + sl] = acc;
+                    }
+            }
+        }
+        gf_worker_sync<WT>();
+        if (slot > 0) {
+            slot = 0;
+            for (int k = 0; k < ngr; ++k) {
+                const int nb = goff[k], ne = goff[k + 1];
+                if (ne - nb <= 32) continue;
+                const int pieces = (ne - nb + 31) >> 5;
+                if (k % WARPS == warp) {
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int c = 0; c < pieces; ++c) {
+                        const float4 v = part4[(slot + c) * LPR + sl];
+                        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+                    }
+                    put_y(k, acc);
+                }
+                slot += pieces;
+            }
+            gf_worker_sync<WT>();
+        }
+        if (p.logits) {
+            float* scratch = reinterpret_cast<float*>(smem + Cfg::OFF_H);
+            for (int gb = 0; gb < ngr; gb += 8) {
+                const int nb = ngr - gb < 8 ? ngr - gb : 8;
+                if (nb == 1) gf_readout<D, WT, 1>(p, y_s + gb * D, scratch, nb, (int64_t)g0 + gb);
+                else gf_readout<D, WT, 8>(p, y_s + gb * D, scratch, nb, (int64_t)g0 + gb);
+                gf_worker_sync<WT>();
+            }
+        }
+        g0 = g1;
+    }
+    if (bad_tag) {
+        p.status->code = S2V_ERR_INVALID_ARG;
+        p.status->where = 3;
+    }
+    // ---- teardown: everyone is done with tensor memory before it is released
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tm_cols) : "memory");
+}
+
+template <int D, int WARPS>
+int gf_launch(s2v_ctx* ctx, cudaStream_t st, const GfParams& p, uint32_t smem, unsigned blocks)
+{
+    auto kern = p.val ? s2v_graph_fused_kernel<D, WARPS, true> : s2v_graph_fused_kernel<D, WARPS, false>;
+    S2V_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<blocks, WARPS * 32, smem, st>>>(p);
+    S2V_CHECK_LAUNCH(ctx, "s2v_graph_fused_kernel");
+    return S2V_OK;
+}
+
+}  // namespace
+
+// Whether the kernel takes a batch whose largest graph has `max_nodes` nodes: its rows, the operand buffer and W have to
+// fit the 227 KB a CTA may use (d = 128: 128 rows, d = 64: 640, d = 32: 1024), tags are kept in 16 bits.
+bool s2v_graph_fused_supported(const s2v_ctx* ctx, int d, int max_nodes, int num_tags)
+{
+    const int most = d == 128 ? 128 : (d == 64 ? 640 : (d == 32 ? 1024 : 0));
+    return max_nodes >= 1 && max_nodes <= most && num_tags < 65536 && ctx->smem_optin >= 227 * 1024;
+}
+
+size_t s2v_graph_fused_image_bytes(int d) { return sizeof(float) * (size_t)d * d + 16; }
+
+bool s2v_graph_fused_readout_ok(int d, int hidden, int num_class)
+{
+    // scratch of the readout (partial sums, hidden rows, logits of eight graphs) takes the H rows' place
+    const int slices = hidden <= 64 ? 8 : (hidden <= 128 ? 4 : (hidden <= 256 ? 2 : 1));
+    return sizeof(float) * 8 * ((size_t)hidden * (slices > 1 ? slices + 1 : 1) + num_class) <= (size_t)128 * 4 * d;
+}
+
+int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_args& a)
+{
+    if (!s2v_graph_fused_supported(ctx, a.d, a.max_graph_nodes, a.num_tags)) return S2V_ERR_UNSUPPORTED;
+    GfParams p{};
+    p.G = a.G;
+    p.row_ptr = a.row_ptr; p.col_idx = a.col_idx; p.val = a.val; p.graph_ptr = a.graph_ptr;
+    p.tags = a.tags; p.x = a.x; p.num_tags = a.num_tags;
+    p.W = a.W;
+    p.levels = a.levels;
+    p.pool_average = a.pool_average;
+    p.Y = a.Y; p.embed_out = a.embed_out;
+    p.W1 = a.W1; p.W2 = a.W2; p.hidden = a.hidden; p.num_class = a.num_class;
+    p.logits = a.logits; p.probs = a.probs; p.pred = a.pred;
+    p.status = ctx->dstatus_dev;
+    if (a.P_scratch && a.levels >= 1) {
+        const int rc = s2v_launch_first_table_product(ctx, st, a.num_tags, a.d, a.x, a.W, a.P_scratch, true);
+        if (rc != S2V_OK) return rc;
+        p.P = a.P_scratch;
+        p.levels = a.levels - 1;
+    }
+    if (a.image_scratch) {
+        unsigned char* img = static_cast<unsigned char*>(a.image_scratch);
+        if (a.d == 128) gf_weight_image_kernel<128><<<1, 1024, 0, st>>>(a.W, img);
+        else if (a.d == 64) gf_weight_image_kernel<64><<<1, 1024, 0, st>>>(a.W, img);
+        else gf_weight_image_kernel<32><<<1, 1024, 0, st>>>(a.W, img);
+        S2V_CHECK_LAUNCH(ctx, "gf_weight_image_kernel");
+        p.w_image = img;
+    }
+    // Rows per tile.  Small graphs: one row block per tile and (d <= 64) two 288-thread CTAs per SM, so that one CTA's
+    // gather runs under the other's products and drains.  Larger graphs: as many rows as the batch gives each SM, up to
+    // what fits, with 544 threads.
+    const int need = (a.max_graph_nodes + 127) / 128 * 128;
+    int warps = 16, per_sm = 1, cap = 128;
+    if (a.d == 64 && need == 128) { warps = 8; per_sm = 2; }
+    if (a.d == 64 && need > 128) {
+        const int64_t share = (a.N / ctx->sm_count + 127) / 128 * 128;
+        cap = (int)(share < 640 ? share : 640);
+        if (cap < need) cap = need;
+    }
+    if (a.d == 32) {
+        if (need <= 640) {
+            warps = 8; per_sm = 2;
+            const int64_t share = (a.N / (2 * ctx->sm_count) + 127) / 128 * 128;
+            cap = (int)(share < 640 ? share : 640);
+            if (cap < need) cap = need;
+        } else cap = 1024;
+    }
+    p.cap = cap;
+    uint32_t cols = 32;
+    while (cols < (uint32_t)(cap / 128 * a.d)) cols *= 2;
+    p.tm_cols = cols;
+    // what is left of the CTA's share of shared memory lists the columns (8 bytes per four)
+    const bool hv = a.val != nullptr;
+    auto total = [&](int n) {
+        return a.d == 128 ? gf_map<128>(cap, n, hv).total : (a.d == 64 ? gf_map<64>(cap, n, hv).total : gf_map<32>(cap, n, hv).total);
+    };
+    const uint32_t budget = per_sm == 2 ? 113 * 1024 : 227 * 1024;
+    const uint32_t left = (budget - total(0)) / 16 * 16, enough = (uint32_t)cap * 8u * 6u;   // six chunks per row are plenty
+    p.chunk_cap = (int)((left < enough ? left : enough) / 8);
+    const uint32_t smem = total(p.chunk_cap);
+    const int64_t most = (int64_t)ctx->sm_count * per_sm;
+    const unsigned blocks = (unsigned)(a.G < most ? a.G : most);
+    if (a.d == 128) return gf_launch<128, 16>(ctx, st, p, smem, blocks);
+    if (a.d == 64) return warps == 8 ? gf_launch<64, 8>(ctx, st, p, smem, blocks) : gf_launch<64, 16>(ctx, st, p, smem, blocks);
+    return warps == 8 ? gf_launch<32, 8>(ctx, st, p, smem, blocks) : gf_launch<32, 16>(ctx, st, p, smem, blocks);
+}

@@ -73,9 +73,10 @@ typedef enum s2v_option {
     S2V_OPT_LEVEL_TC = 2,            /* tcgen05 level kernel: 0 never, 1 automatic (default), 2 whenever the shape allows
                                         (default from S2V_LEVEL_TC) */
     S2V_OPT_GRAPH_TILES = 3,         /* whole-classifier tile kernel (s2v_graph_tiles_f32) inside s2v_forward_f32 for batches of
-                                        small graphs: 0 never, 1 whenever the batch allows, 2 automatic (default: batches of at
-                                        most 160,000 nodes, where one launch beats the per-level kernels by 1.1x - 1.9x; larger
-                                        batches stream better through the per-level kernels).  Default from S2V_GRAPH_TILES */
+                                        small graphs, and its counterpart for d = 32 and 64: 0 never, 1 whenever the batch
+                                        allows, 2 automatic (default; d = 128: batches of at most 160,000 nodes, where one launch
+                                        beats the per-level kernels by 1.1x - 1.9x; larger ones stream better through the
+                                        per-level kernels).  Default from S2V_GRAPH_TILES */
     S2V_OPT_RESERVED_SMS = 4,        /* the persistent kernels size their grids for (SM count - value) SMs, leaving the rest to
                                         kernels of another stream -- a communication library's, which cannot start while
                                         one-CTA-per-SM kernels hold every SM (default 0; 0 <= value < SM count) */
@@ -252,11 +253,12 @@ typedef struct s2v_batch {
     const int32_t* tags;        /* [N] one-hot node types, or NULL when x_dense is given */
     const float* x_dense;       /* [N x F] or NULL */
     int32_t max_graph_nodes;    /* node count of the largest graph of the batch, or 0 if unknown.  Device entry
-                                   points cannot read graph_ptr on the host; with 1..128 here (and d = 128, tags,
-                                   S2V_OPT_GRAPH_TILES on) s2v_forward_f32 runs the whole classifier as one tile kernel
-                                   that keeps the embeddings in shared memory.  A value that understates the truth is reported
-                                   through the status word (S2V_ERR_UNSUPPORTED) and the oversized graphs are
-                                   truncated.  s2v_infer_host_f32 computes it itself. */
+                                   points cannot read graph_ptr on the host; with a value here (and S2V_OPT_GRAPH_TILES not 0)
+                                   s2v_forward_f32 keeps whole graphs in shared memory across the levels where they fit:
+                                   up to 1024 nodes at d = 32, 640 at d = 64, 128 at d = 128.  The value promises separate
+                                   graphs: one that understates the truth (the oversized graphs are truncated) and an edge
+                                   between graphs are reported through the status word (S2V_ERR_UNSUPPORTED,
+                                   S2V_ERR_BAD_CSR).  s2v_infer_host_f32 computes it itself. */
 } s2v_batch;
 
 /* Bytes of device workspace s2v_forward_f32 needs (three [N x d] buffers + [G x d] + the tile plan). */
