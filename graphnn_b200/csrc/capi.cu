@@ -208,7 +208,7 @@ int s2v_level_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src
     S2V_ENTER(ctx);
     int rc = check_level_args(ctx, n_rows, n_src, d, row_ptr, col_idx, H, W, X, out);
     if (rc != S2V_OK || n_rows == 0) return rc;
-    return s2v_launch_level(ctx, s2v_pick_stream(ctx, stream), n_rows, n_src, d, row_ptr, false, col_idx, val, H, W, X,
+    return s2v_launch_level(ctx, s2v_pick_stream(ctx, stream), true, n_rows, n_src, d, row_ptr, false, col_idx, val, H, W, X,
                             nullptr, nullptr, 0, out);
 }
 
@@ -219,7 +219,7 @@ int s2v_level_rp64_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t 
     S2V_ENTER(ctx);
     int rc = check_level_args(ctx, n_rows, n_src, d, row_ptr, col_idx, H, W, X, out);
     if (rc != S2V_OK || n_rows == 0) return rc;
-    return s2v_launch_level(ctx, s2v_pick_stream(ctx, stream), n_rows, n_src, d, row_ptr, true, col_idx, val, H, W, X,
+    return s2v_launch_level(ctx, s2v_pick_stream(ctx, stream), true, n_rows, n_src, d, row_ptr, true, col_idx, val, H, W, X,
                             nullptr, nullptr, 0, out);
 }
 
@@ -234,7 +234,7 @@ int s2v_level_lookup_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_
     // the level kernel clamps the indices it uses; this launch finds and reports the ones outside the table
     rc = s2v_launch_index_check(ctx, s2v_pick_stream(ctx, stream), n_rows, x_index, n_table);
     if (rc != S2V_OK) return rc;
-    return s2v_launch_level(ctx, s2v_pick_stream(ctx, stream), n_rows, n_src, d, row_ptr, false, col_idx, val, H, W,
+    return s2v_launch_level(ctx, s2v_pick_stream(ctx, stream), true, n_rows, n_src, d, row_ptr, false, col_idx, val, H, W,
                             nullptr, table, x_index, n_table, out);
 }
 
@@ -265,7 +265,7 @@ int s2v_level_first_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n, int d, const
         return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "level_first: d / 4 must be a power of two up to 32; materialise H0 instead");
     rc = s2v_launch_index_check(ctx, s2v_pick_stream(ctx, stream), n, tags, n_table);
     if (rc != S2V_OK) return rc;
-    rc = s2v_launch_level_tc(ctx, s2v_pick_stream(ctx, stream), n, d, row_ptr, col_idx, val, nullptr, W, nullptr, table,
+    rc = s2v_launch_level_tc(ctx, s2v_pick_stream(ctx, stream), false, n, d, row_ptr, col_idx, val, nullptr, W, nullptr, table,
                              tags, n_table, out);
     if (rc == S2V_ERR_UNSUPPORTED) return s2v_fail(ctx, rc, "level_first: shape not supported by the tcgen05 kernel");
     return rc;
@@ -439,7 +439,7 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
     }
     if (!first_fused && onehot && L >= 1 && s2v_use_tc(ctx, d, N)) {
         float* dst = (L == 1 && embed_out) ? embed_out : ha;
-        rc = s2v_launch_level_tc(ctx, st, N, d, batch->n2n_row_ptr, batch->n2n_col_idx, batch->n2n_val, nullptr, model->p_node_conv,
+        rc = s2v_launch_level_tc(ctx, st, false, N, d, batch->n2n_row_ptr, batch->n2n_col_idx, batch->n2n_val, nullptr, model->p_node_conv,
                                  nullptr, model->w_n2l, batch->tags, model->num_feat, dst);
         if (rc == S2V_OK) first_fused = true;
         else if (rc != S2V_ERR_UNSUPPORTED) return rc;
@@ -454,18 +454,22 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
         rc = s2v_input_proj_dense_f32(ctx, st, N, model->num_feat, d, batch->x_dense, model->w_n2l, msg, ha);
     if (rc != S2V_OK) return rc;
 
+    // graphs of a few thousand nodes hold no row that is worth looking for
+    const bool long_rows = batch->max_graph_nodes <= 0 || batch->max_graph_nodes > 2048;
     float* cur = (first_fused && L == 1 && embed_out) ? embed_out : ha;
     float* nxt = hb;
     for (int lv = first_fused ? 1 : 0; lv < L; ++lv) {
         float* dst = (lv == L - 1 && embed_out) ? embed_out : nxt;
         if (onehot)
             rc = (d == 32 || d == 64 || d == 128)
-                     ? s2v_launch_level(ctx, st, N, N, d, batch->n2n_row_ptr, false, batch->n2n_col_idx, batch->n2n_val, cur,
+                     ? s2v_launch_level(ctx, st, long_rows, N, N, d, batch->n2n_row_ptr, false, batch->n2n_col_idx, batch->n2n_val, cur,
                                         model->p_node_conv, nullptr, model->w_n2l, batch->tags, model->num_feat, dst)
                      : s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "fused level kernel supports d in {32, 64, 128}");
         else
-            rc = s2v_level_f32(ctx, st, N, N, d, batch->n2n_row_ptr, batch->n2n_col_idx, batch->n2n_val, cur,
-                               model->p_node_conv, msg, dst);
+            rc = check_level_args(ctx, N, N, d, batch->n2n_row_ptr, batch->n2n_col_idx, cur, model->p_node_conv, msg, dst);
+        if (!onehot && rc == S2V_OK && N > 0)
+            rc = s2v_launch_level(ctx, st, long_rows, N, N, d, batch->n2n_row_ptr, false, batch->n2n_col_idx, batch->n2n_val, cur,
+                                  model->p_node_conv, msg, nullptr, nullptr, 0, dst);
         if (rc != S2V_OK) return rc;
         if (dst == nxt) std::swap(cur, nxt); else cur = dst;
     }

@@ -143,7 +143,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
 
 #endif  // __CUDACC__
 
-// Rows from which the d = 64 / d = 128 level goes to the tcgen05 kernel (128-row tiles, one CTA per SM).
+// Rows from which the table-lookup form of the first level is offered by the tcgen05 kernel (128-row tiles, one CTA per SM).
 constexpr int64_t S2V_TC_MIN_ROWS = 16384;
 inline bool s2v_use_tc(const s2v_ctx* ctx, int d, int64_t n_rows)
 {
@@ -152,7 +152,7 @@ inline bool s2v_use_tc(const s2v_ctx* ctx, int d, int64_t n_rows)
 }
 
 // launchers implemented in the .cu files (host side)
-int s2v_launch_level_tc(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, int d, const int32_t* row_ptr,
+int s2v_launch_level_tc(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int d, const int32_t* row_ptr,
                         const int32_t* col_idx, const float* val, const float* H, const float* W, const float* X,
                         const float* table, const int32_t* x_index, int n_table, float* out);
 int s2v_launch_wait_selftest(s2v_ctx* ctx, cudaStream_t st);
@@ -209,6 +209,7 @@ int s2v_launch_graph_tiles(s2v_ctx* ctx, cudaStream_t st, int64_t G, const int32
                            const float* val, const int32_t* graph_ptr, const int32_t* tags, int num_tags,
                            const float* W_in, const float* W, int levels, int pool_average, void* plan, float* P_scratch,
                            float* Y, float* embed_out);   // P_scratch: (num_tags + 1) * 128 floats, or NULL (first level through the MMAs)
-int s2v_launch_level(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, int64_t n_src, int d, const void* row_ptr,
+// long_rows: rows of hundreds of entries and more may occur and are summed ahead of the rest (long_rows.cuh)
+int s2v_launch_level(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int64_t n_src, int d, const void* row_ptr,
                      bool rp64, const int32_t* col_idx, const float* val, const float* H, const float* W,
                      const float* X, const float* table, const int32_t* x_index, int n_table, float* out);

@@ -29,6 +29,7 @@
 //          (add X -- streamed, or looked up in a small table --, ReLU, store) touches
 //          global memory in whole 128..512-byte rows.
 #include "common.cuh"
+#include "long_rows.cuh"
 #include "mma_tf32.cuh"
 
 namespace
@@ -95,7 +96,7 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
 
 template <int D, typename RpT, bool HAS_VAL, int XMODE /*0 none, 1 dense, 2 table lookup*/>
 __global__ void __launch_bounds__(LevelCfg<D>::WARPS * 32, LevelCfg<D>::MIN_BLOCKS)
-s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_ptr,
+s2v_level_kernel(bool long_rows, int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_ptr,
                  const int32_t* __restrict__ col_idx, const float* __restrict__ val, const float* __restrict__ H,
                  const float* __restrict__ W, const float* __restrict__ X, const int32_t* __restrict__ x_index,
                  int n_table, float* __restrict__ out, s2v_device_status* status)
@@ -122,14 +123,21 @@ s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_
 
     // ---- stage W: one bulk-async copy per CTA, completion on an mbarrier
     const uint32_t bar = smem_u32(mbar);
-    if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        mbar_expect_tx(bar, (uint32_t)(sizeof(float) * D * D));
-        for (int k = 0; k < D; ++k)  // one bulk copy per row of W, into the padded layout
+    if (warp == 0) {
+        if (lane == 0) {
+            mbar_init(bar, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            mbar_expect_tx(bar, (uint32_t)(sizeof(float) * D * D));
+        }
+        __syncwarp();
+        for (int k = lane; k < D; k += 32)  // one bulk copy per row of W, into the padded layout
             bulk_copy_g2s(smem_u32(Ws + k * W_STRIDE), W + k * D, (uint32_t)(sizeof(float) * D), bar);
     }
-    __syncthreads();  // barrier initialised before anyone polls it
+    LongLook<WARPS * 32, TILE_R, RpT> look;   // rows of hubs are looked for while W is on its way
+    look.load(n_rows, row_ptr);
+    if (__syncthreads_or(look.any(n_rows, row_ptr)) && long_rows)   // (the barrier is initialised before anyone polls it)
+        sum_long_rows<D, WARPS * 32, TILE_R, TILE_R, (int)(LevelSmem<D>::WARP_BYTES * WARPS), HAS_VAL>(smem_raw + LevelSmem<D>::W_BYTES + 16, n_rows, row_ptr,
+                                                                                                       col_idx, val, H, out);
     {
         int spins = 0;
         while (!mbar_try_wait(bar, 0)) {
@@ -149,7 +157,8 @@ s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_
     const int sub = lane / LPR, sl = lane % LPR;
     const int g = lane >> 2, tig = lane & 3;   // MMA fragment coordinates
 
-    for (int64_t tile = (int64_t)blockIdx.x * WARPS + warp; tile < num_tiles; tile += (int64_t)gridDim.x * WARPS) {
+    // (tiles go to the CTAs first and to a CTA's warps second: a small batch uses every SM)
+    for (int64_t tile = (int64_t)warp * gridDim.x + blockIdx.x; tile < num_tiles; tile += (int64_t)gridDim.x * WARPS) {
         const int64_t r0 = tile * TILE_R;
         // ---- 1. row offsets (relative to the tile's first non-zero) and the tile's indices
         int64_t rpi = r0 + lane;
@@ -176,7 +185,14 @@ s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_
         //   RPS consecutive rows as ONE stream, U loads in flight whatever the row lengths; a
         //   row's sum is flushed to the shared tile when the stream crosses its end.
         //   Otherwise: one row per lane group per pass, chunks of U neighbours.
-        if constexpr (LevelCfg<D>::FLAT) {
+        //   A tile with a long row has all its sums already (long_rows.cuh).
+        const int row_len = __shfl_down_sync(0xffffffffu, rp_rel, 1) - rp_rel;
+        if (__any_sync(0xffffffffu, lane < TILE_R && row_len > LONG_ROW) && long_rows) {
+#pragma unroll 1
+            for (int lr = sub; lr < TILE_R; lr += RPP)
+                if (r0 + lr < n_rows)
+                    *reinterpret_cast<float4*>(S + lr * S_STRIDE + sl * 4) = long_row_sum(reinterpret_cast<const float4*>(out) + (r0 + lr) * LPR + sl);
+        } else if constexpr (LevelCfg<D>::FLAT) {
             int row = sub * RPS;
             const int row_stop = row + RPS;
             int t = rp_s[row];
@@ -338,7 +354,7 @@ s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_
 }
 
 template <int D, typename RpT, bool HAS_VAL, int XMODE>
-int launch_one(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx,
+int launch_one(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx,
                const float* val, const float* H, const float* W, const float* X, const int32_t* x_index, int n_table,
                float* out)
 {
@@ -347,28 +363,30 @@ int launch_one(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const RpT* row_ptr
     const size_t smem = LevelSmem<D>::total(WARPS);
     // Opt-in shared memory size: a per-function attribute, cheap to set on every call.
     S2V_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int resident = 0;
-    S2V_CUDA_OK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, WARPS * 32, smem));
-    if (resident < 1) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "level kernel does not fit on this device");
+    static std::atomic<int> resident_of{0};   // CTAs per SM: a property of the kernel on this one architecture
+    int resident = resident_of.load(std::memory_order_relaxed);
+    if (resident == 0) {
+        S2V_CUDA_OK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, WARPS * 32, smem));
+        if (resident < 1) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "level kernel does not fit on this device");
+        resident_of.store(resident, std::memory_order_relaxed);
+    }
     const int64_t num_tiles = (n_rows + TILE_R - 1) / TILE_R;
-    int64_t blocks = (num_tiles + WARPS - 1) / WARPS;
     const int64_t persistent = (int64_t)ctx->sm_count * resident;
-    if (blocks > persistent) blocks = persistent;
-    if (blocks < 1) blocks = 1;
-    kern<<<(unsigned)blocks, WARPS * 32, smem, st>>>(n_rows, num_tiles, row_ptr, col_idx, val, H, W, X, x_index, n_table, out,
+    const int64_t blocks = num_tiles < persistent ? num_tiles : persistent;
+    kern<<<(unsigned)blocks, WARPS * 32, smem, st>>>(long_rows, n_rows, num_tiles, row_ptr, col_idx, val, H, W, X, x_index, n_table, out,
                                                       ctx->dstatus_dev);
     S2V_CHECK_LAUNCH(ctx, "s2v_level_kernel");
     return S2V_OK;
 }
 
 template <int D, typename RpT>
-int launch_d(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const RpT* rp, const int32_t* ci, const float* val,
+int launch_d(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const RpT* rp, const int32_t* ci, const float* val,
              const float* H, const float* W, const float* X, const float* table, const int32_t* x_index, int n_table,
              float* out)
 {
     const int xmode = table ? 2 : (X ? 1 : 0);
     const float* xa = table ? table : X;
-#define S2V_LVL(HV, XM) return launch_one<D, RpT, HV, XM>(ctx, st, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)
+#define S2V_LVL(HV, XM) return launch_one<D, RpT, HV, XM>(ctx, st, long_rows, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)
     if (val) {
         if (xmode == 0) S2V_LVL(true, 0);
         if (xmode == 1) S2V_LVL(true, 1);
@@ -382,22 +400,25 @@ int launch_d(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const RpT* rp, const
 
 }  // namespace
 
-int s2v_launch_level(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, int64_t n_src, int d, const void* row_ptr,
+int s2v_launch_level(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int64_t n_src, int d, const void* row_ptr,
                      bool rp64, const int32_t* col_idx, const float* val, const float* H, const float* W,
                      const float* X, const float* table, const int32_t* x_index, int n_table, float* out)
 {
     (void)n_src;
     if (n_rows == 0) return S2V_OK;
-    if (!rp64 && s2v_use_tc(ctx, d, n_rows)) {
-        const int rc = s2v_launch_level_tc(ctx, st, n_rows, d, (const int32_t*)row_ptr, col_idx, val, H, W, X, table,
+    // the sums of long rows lie in `out` for a while, so an X that shares its memory keeps the plain gather
+    if (X && X < out + n_rows * d && out < X + n_rows * d) long_rows = false;
+    // d = 64, 128: the tcgen05 kernel at every size (a single tile takes 11 us there and 18 - 30 us here)
+    if (!rp64 && (d == 64 || d == 128) && ctx->tc_mode != 0) {
+        const int rc = s2v_launch_level_tc(ctx, st, long_rows, n_rows, d, (const int32_t*)row_ptr, col_idx, val, H, W, X, table,
                                            x_index, n_table, out);
         if (rc != S2V_ERR_UNSUPPORTED) return rc;
     }
 #define S2V_D(DD)                                                                                                  \
     case DD:                                                                                                       \
-        return rp64 ? launch_d<DD, int64_t>(ctx, st, n_rows, (const int64_t*)row_ptr, col_idx, val, H, W, X, table, \
+        return rp64 ? launch_d<DD, int64_t>(ctx, st, long_rows, n_rows, (const int64_t*)row_ptr, col_idx, val, H, W, X, table, \
                                             x_index, n_table, out)                                                 \
-                    : launch_d<DD, int32_t>(ctx, st, n_rows, (const int32_t*)row_ptr, col_idx, val, H, W, X, table, \
+                    : launch_d<DD, int32_t>(ctx, st, long_rows, n_rows, (const int32_t*)row_ptr, col_idx, val, H, W, X, table, \
                                             x_index, n_table, out)
     switch (d) {
         S2V_D(32);

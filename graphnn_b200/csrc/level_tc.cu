@@ -33,6 +33,7 @@
 // is bounded: on a time-out the kernel records S2V_ERR_DEVICE_TIMEOUT, raises a CTA-wide
 // abort flag, drains, frees its tensor memory and returns.
 #include "common.cuh"
+#include "long_rows.cuh"
 #include "tcgen05.cuh"
 
 namespace
@@ -77,7 +78,8 @@ enum {
     BAR_COUNT
 };
 
-template <int D, bool HAS_VAL, int XMODE, bool HSRC_TABLE>
+// LONG: rows with many entries may occur and are summed ahead of the main loop (long_rows.cuh)
+template <int D, bool HAS_VAL, int XMODE, bool HSRC_TABLE, bool LONG>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 s2v_level_tc_kernel(int64_t n_rows, int64_t num_tiles, const int32_t* __restrict__ row_ptr,
                     const int32_t* __restrict__ col_idx, const float* __restrict__ val, const float* __restrict__ H,
@@ -120,6 +122,8 @@ s2v_level_tc_kernel(int64_t n_rows, int64_t num_tiles, const int32_t* __restrict
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    LongLook<TC_THREADS, TC_TILE, int32_t> look;
+    if (LONG) look.load(n_rows, row_ptr);
     // B[n][k] = W[k][n]; element (n, k) lives at  kb*(D*128) + n*128 + ((kk/4) ^ (n&7))*16 + (kk%4)*4,
     // kb = k/32, kk = k%32.  Each task converts 4 consecutive k of one n: one 16-byte store per matrix.
     // All loads of a thread's tasks are issued before the first conversion (one memory latency, not one per task).
@@ -127,12 +131,19 @@ s2v_level_tc_kernel(int64_t n_rows, int64_t num_tiles, const int32_t* __restrict
         constexpr int NTASK = D * D / 4;
         constexpr int PER = (NTASK + TC_THREADS - 1) / TC_THREADS;
         float wv[PER][4];
+        auto load_w = [&]() {
 #pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int e = threadIdx.x + t * TC_THREADS;
-            const int n = e % D, kq = e / D;   // k = 4*kq .. 4*kq+3
+            for (int t = 0; t < PER; ++t) {
+                const int e = threadIdx.x + t * TC_THREADS;
+                const int n = e % D, kq = e / D;   // k = 4*kq .. 4*kq+3
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) wv[t][jj] = (e < NTASK) ? __ldg(W + (int64_t)(4 * kq + jj) * D + n) : 0.f;
+                for (int jj = 0; jj < 4; ++jj) wv[t][jj] = (e < NTASK) ? __ldg(W + (int64_t)(4 * kq + jj) * D + n) : 0.f;
+            }
+        };
+        load_w();
+        if (LONG && __syncthreads_or(look.any(n_rows, row_ptr))) {
+            sum_long_rows<D, TC_THREADS, TC_TILE, TC_ROWS_PER_GW, (int)Cfg::OFF_GW, HAS_VAL>(smem, n_rows, row_ptr, col_idx, val, H, out);
+            load_w();   // (again: kept across the call they would be spilled in every launch)
         }
 #pragma unroll
         for (int t = 0; t < PER; ++t) {
@@ -254,7 +265,9 @@ s2v_level_tc_kernel(int64_t n_rows, int64_t num_tiles, const int32_t* __restrict
                 const int gs = (sub == 0) ? 0 : r_mid;                    // my group's non-zeros: [gs, gs + cnt)
                 const int cnt = ((sub == G - 1) ? r_end : r_mid) - gs;
                 const int cmax = (G == 1) ? r_end : max(r_mid, r_end - r_mid);
-                const int nseg = (cmax + WSZ - 1) / WSZ;                  // 64-non-zero segments (warp-uniform)
+                // a warp tile with a long row has all its sums already: nothing is gathered here
+                const bool summed = LONG && __any_sync(0xffffffffu, isrow && rel - relp > LONG_ROW);
+                const int nseg = summed ? 0 : (cmax + WSZ - 1) / WSZ;     // 64-non-zero segments (warp-uniform)
                 // nxtmap: 4 bits per row, the next non-empty row of the group (15: none)
                 uint32_t nxtmap = 0;
                 {
@@ -398,6 +411,14 @@ s2v_level_tc_kernel(int64_t n_rows, int64_t num_tiles, const int32_t* __restrict
                 }
 #undef TC_LOADF
 #undef TC_CONSF
+                if (summed) {
+#pragma unroll 1
+                    for (int r = r_lo; r < r_lo + RPG; ++r) {
+                        const int64_t row = ((int64_t)blockIdx.x + (int64_t)it * gridDim.x) * TC_TILE + row0 + r;
+                        if (row < n_rows)
+                            *reinterpret_cast<float4*>(slab + (size_t)r * STAGE_STRIDE + sl * 4) = long_row_sum(reinterpret_cast<const float4*>(out) + row * LPR + sl);
+                    }
+                }
                 if (HSRC_TABLE) {
                     int* nb = idx_base + ((it + 1) & 1) * IDX_BUF;
 #pragma unroll
@@ -562,10 +583,11 @@ __global__ void tc_wait_selftest_kernel(s2v_device_status* status)
 }
 
 template <int D, bool HAS_VAL, int XMODE, bool HSRC_TABLE = false>
-int tc_launch(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const int32_t* rp, const int32_t* ci, const float* val,
+int tc_launch(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const int32_t* rp, const int32_t* ci, const float* val,
               const float* H, const float* W, const float* X, const int32_t* x_index, int n_table, float* out)
 {
-    auto kern = s2v_level_tc_kernel<D, HAS_VAL, XMODE, HSRC_TABLE>;
+    auto kern = !HSRC_TABLE && long_rows ? s2v_level_tc_kernel<D, HAS_VAL, XMODE, HSRC_TABLE, !HSRC_TABLE>
+                                         : s2v_level_tc_kernel<D, HAS_VAL, XMODE, HSRC_TABLE, false>;
     constexpr size_t SMEM = TcCfg<D>::SMEM_BYTES;
     if (SMEM > ctx->smem_optin) return S2V_ERR_UNSUPPORTED;
     S2V_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
@@ -583,18 +605,18 @@ int tc_launch(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const int32_t* rp, 
 // d = 64 or 128, 32-bit row offsets.  Returns S2V_ERR_UNSUPPORTED for anything else (the caller falls back).
 // H == NULL with a table: the gather source is ReLU(table[x_index[col], :]) (square matrices only).
 template <int D>
-static int tc_dispatch(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const int32_t* row_ptr, const int32_t* col_idx,
+static int tc_dispatch(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const int32_t* row_ptr, const int32_t* col_idx,
                        const float* val, const float* H, const float* W, const float* X, const float* table,
                        const int32_t* x_index, int n_table, float* out)
 {
     if (!H) {
         if (!table || !x_index) return S2V_ERR_UNSUPPORTED;
-        return val ? tc_launch<D, true, 2, true>(ctx, st, n_rows, row_ptr, col_idx, val, nullptr, W, table, x_index, n_table, out)
-                   : tc_launch<D, false, 2, true>(ctx, st, n_rows, row_ptr, col_idx, val, nullptr, W, table, x_index, n_table, out);
+        return val ? tc_launch<D, true, 2, true>(ctx, st, false, n_rows, row_ptr, col_idx, val, nullptr, W, table, x_index, n_table, out)
+                   : tc_launch<D, false, 2, true>(ctx, st, false, n_rows, row_ptr, col_idx, val, nullptr, W, table, x_index, n_table, out);
     }
     const int xmode = table ? 2 : (X ? 1 : 0);
     const float* xa = table ? table : X;
-#define TC_GO(HV, XM) return tc_launch<D, HV, XM>(ctx, st, n_rows, row_ptr, col_idx, val, H, W, xa, x_index, n_table, out)
+#define TC_GO(HV, XM) return tc_launch<D, HV, XM>(ctx, st, long_rows, n_rows, row_ptr, col_idx, val, H, W, xa, x_index, n_table, out)
     if (val) {
         if (xmode == 0) TC_GO(true, 0);
         if (xmode == 1) TC_GO(true, 1);
@@ -606,12 +628,12 @@ static int tc_dispatch(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const int3
 #undef TC_GO
 }
 
-int s2v_launch_level_tc(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, int d, const int32_t* row_ptr,
+int s2v_launch_level_tc(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int d, const int32_t* row_ptr,
                         const int32_t* col_idx, const float* val, const float* H, const float* W, const float* X,
                         const float* table, const int32_t* x_index, int n_table, float* out)
 {
-    if (d == 128) return tc_dispatch<128>(ctx, st, n_rows, row_ptr, col_idx, val, H, W, X, table, x_index, n_table, out);
-    if (d == 64) return tc_dispatch<64>(ctx, st, n_rows, row_ptr, col_idx, val, H, W, X, table, x_index, n_table, out);
+    if (d == 128) return tc_dispatch<128>(ctx, st, long_rows, n_rows, row_ptr, col_idx, val, H, W, X, table, x_index, n_table, out);
+    if (d == 64) return tc_dispatch<64>(ctx, st, long_rows, n_rows, row_ptr, col_idx, val, H, W, X, table, x_index, n_table, out);
     return S2V_ERR_UNSUPPORTED;
 }
 

@@ -1,0 +1,232 @@
+// Long rows (hubs of a power-law graph) of the level kernels.  A level kernel gives a row to one warp, or part of one; a
+// row of 10^4 or 10^5 entries keeps that warp -- and its CTA's pipeline behind it -- busy long after everyone else is done
+// (R-MAT scale 20, d = 128: 11.3 ms, nearly all of it the longest rows).  So a CTA first looks through the offsets of the
+// rows it owns (while W is on its way) and, if there is one above LONG_ROW entries, sums such rows with all its warps,
+// together with the other rows of their groups of GROUP rows (what a warp of the main loop works on as one unit).  The sums
+// go to the rows' places in `out`, which the CTA itself overwrites with the result afterwards, so no scratch memory is
+// needed; the main loop reads such a group's sums from there instead of gathering.
+//   * Up to LONG_BIG entries a warp sums a row, in slices of up to 64 columns with 4 KB of neighbour rows on their way; a longer
+//     one, taken first, is streamed through a ring in shared memory by the whole CTA, where one warp would be bounded by latency.
+//   * Entries are added one after the other in CSR order, as everywhere else in the level: a float sum of 10^5 entries
+//     depends on its order in the fifth digit.
+#pragma once
+
+#include "common.cuh"
+
+namespace
+{
+
+constexpr int LONG_ROW = 256;      // below this a row is no longer than what the other warps of a tile work on
+constexpr int LONG_BIG = 2048;
+constexpr int LONG_LOOK = 4;       // rows per thread that are looked at ahead
+constexpr int LONG_SCAN = 8;       // rows per thread and pass of the sums
+
+template <int W> struct LongVec;
+template <> struct LongVec<2> { using T = float2; };
+template <> struct LongVec<1> { using T = float; };
+__device__ __forceinline__ void long_add(float2& a, float2 v) { a.x += v.x; a.y += v.y; }
+__device__ __forceinline__ void long_add(float& a, float v) { a += v; }
+__device__ __forceinline__ void long_fma(float2& a, float w, float2 v) { a.x = fmaf(w, v.x, a.x); a.y = fmaf(w, v.y, a.y); }
+__device__ __forceinline__ void long_fma(float& a, float w, float v) { a = fmaf(w, v, a); }
+
+// SL columns (H, out_row already point at the first of them) of one row by one warp; c: its first 32 indices, one per lane
+template <int D, int SL, bool HAS_VAL>
+__device__ __forceinline__ void long_row_by_warp(const float* __restrict__ H, const int32_t* __restrict__ col, const float* __restrict__ val, int n, int c,
+                                                 float* out_row)
+{
+    using V = typename LongVec<SL / 32>::T;
+    constexpr int U = 1024 / SL, STRIDE = D / (SL / 32);   // 4 KB in flight
+    const int lane = threadIdx.x & 31;
+    const V* __restrict__ Hv = reinterpret_cast<const V*>(H) + lane;
+    V acc{};
+    float w = HAS_VAL && lane < n ? __ldg(val + lane) : 0.f;
+    for (int t = 0; t < n; t += 32) {
+        const int cn = t + 32 + lane < n ? __ldg(col + t + 32 + lane) : 0;   // the next indices, on their way while these rows are summed
+        const float wn = HAS_VAL && t + 32 + lane < n ? __ldg(val + t + 32 + lane) : 0.f;
+#pragma unroll
+        for (int u0 = 0; u0 < 32; u0 += U) {
+            if (t + u0 >= n) break;
+            V v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int cc = __shfl_sync(0xffffffffu, c, u0 + u);
+                v[u] = V{};
+                if (t + u0 + u < n) v[u] = __ldg(Hv + (int64_t)cc * STRIDE);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {   // (what lies past the end adds zeros)
+                if (HAS_VAL) long_fma(acc, __shfl_sync(0xffffffffu, w, u0 + u), v[u]);
+                else long_add(acc, v[u]);
+            }
+        }
+        c = cn;
+        w = wn;
+    }
+    reinterpret_cast<V*>(out_row)[lane] = acc;
+}
+
+// One row by the whole CTA: the threads copy the neighbour rows through a ring of four stages (three in flight), the first D
+// threads add one column each.
+template <int D, int THREADS, int BYTES, bool HAS_VAL>
+__device__ __forceinline__ void long_row_by_cta(unsigned char* ring, const float* __restrict__ H, const int32_t* __restrict__ col,
+                                                const float* __restrict__ val, int n, float* out_row)
+{
+    constexpr int PIECES = D / 4, TURN = THREADS / PIECES, FIT = BYTES / 4 / (TURN * 4 * D), TURNS = FIT < 4 ? FIT : 4, STAGE = TURN * TURNS;
+    static_assert(TURNS >= 1, "a stage holds at least one turn");
+    const int piece = threadIdx.x % PIECES, row0 = threadIdx.x / PIECES;
+    const uint32_t ring_addr = smem_u32(ring);
+    const int stages = (n + STAGE - 1) / STAGE;
+    int c[TURNS];
+    auto fetch = [&](int s) {   // indices of stage s, a stage before they are needed
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k) {
+            const int t = s * STAGE + k * TURN + row0;
+            c[k] = row0 < TURN && t < n ? __ldg(col + t) : -1;
+        }
+    };
+    auto issue = [&](int s) {
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k)
+            if (c[k] >= 0) {
+                const float* src = H + (int64_t)c[k] * D + 4 * piece;
+                const uint32_t dst = ring_addr + (uint32_t)(((s & 3) * STAGE + k * TURN + row0) * D + 4 * piece) * 4u;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    for (int s = 0; s < 3; ++s) { issue(s); fetch(s + 1); }
+    float acc = 0.f;
+    for (int s = 0; s < stages; ++s) {
+        asm volatile("cp.async.wait_group 2;" ::: "memory");
+        __syncthreads();   // stage s has arrived, and everyone is done with the stage before it
+        issue(s + 3);
+        fetch(s + 4);
+        if (threadIdx.x < D) {
+            const float* p = reinterpret_cast<const float*>(ring) + (s & 3) * STAGE * D + threadIdx.x;
+            const int m = n - s * STAGE < STAGE ? n - s * STAGE : STAGE;
+            int r = 0;
+            for (; r + 16 <= m; r += 16) {
+                float v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) v[u] = p[(r + u) * D];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) acc = HAS_VAL ? fmaf(__ldg(val + s * STAGE + r + u), v[u], acc) : acc + v[u];
+            }
+            for (; r < m; ++r) acc = HAS_VAL ? fmaf(__ldg(val + s * STAGE + r), p[r * D], acc) : acc + p[r * D];
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (threadIdx.x < D) out_row[threadIdx.x] = acc;
+    __syncthreads();
+}
+
+// The rows of a CTA that owns the row blocks blockIdx.x, blockIdx.x + gridDim.x, ... of RB rows each, by position.
+template <int RB>
+__device__ __forceinline__ int64_t long_row_of(int j) { return ((int64_t)blockIdx.x + (int64_t)(j / RB) * gridDim.x) * RB + j % RB; }
+template <int RB>
+__device__ __forceinline__ int long_rows_owned(int64_t n_rows)
+{
+    const int64_t blocks = (n_rows + RB - 1) / RB;
+    return blocks > blockIdx.x ? (int)((blocks - 1 - blockIdx.x) / gridDim.x + 1) * RB : 0;
+}
+
+// Whether a row of this thread's share of the CTA's rows is long.  load() only issues the first loads.
+template <int THREADS, int RB, typename RpT>
+struct LongLook {
+    RpT a[LONG_LOOK], z[LONG_LOOK];
+    __device__ __forceinline__ void load(int64_t n_rows, const RpT* __restrict__ row_ptr, int j0 = 0)
+    {
+        const int owned = long_rows_owned<RB>(n_rows);
+#pragma unroll
+        for (int k = 0; k < LONG_LOOK; ++k) {
+            const int j = j0 + k * THREADS + threadIdx.x;
+            const int64_t r = long_row_of<RB>(j);
+            const bool in = j < owned && r < n_rows;
+            a[k] = in ? __ldg(row_ptr + r) : (RpT)0;
+            z[k] = in ? __ldg(row_ptr + r + 1) : (RpT)0;
+        }
+    }
+    __device__ __forceinline__ bool any(int64_t n_rows, const RpT* __restrict__ row_ptr)
+    {
+        bool found = false;
+        const int owned = long_rows_owned<RB>(n_rows);
+        for (int j0 = 0;;) {
+#pragma unroll
+            for (int k = 0; k < LONG_LOOK; ++k) found |= z[k] - a[k] > LONG_ROW;
+            j0 += THREADS * LONG_LOOK;
+            if (j0 >= owned) return found;
+            load(n_rows, row_ptr, j0);
+        }
+    }
+};
+
+// Called by all THREADS threads of the CTA; BYTES of shared memory at `smem`.  Not inlined: the main loops keep their registers.
+template <int D, int THREADS, int RB, int GROUP, int BYTES, bool HAS_VAL, typename RpT>
+__device__ __noinline__ void sum_long_rows(unsigned char* smem, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx, const float* val,
+                                           const float* H, float* out)
+{
+    constexpr int SL = D < 64 ? D : 64, SLICES = D / SL, LIST = 2 * ((THREADS * LONG_SCAN + GROUP - 1) / GROUP), RING = (16 + LIST + 127) / 128 * 128;
+    static_assert(RB % GROUP == 0 && 32 % GROUP == 0 && THREADS % 32 == 0 && RING < BYTES, "whole groups per warp; the ring behind the list");
+    int* const cnt = reinterpret_cast<int*>(smem);                  // groups listed, next slice to take
+    uint16_t* const list = reinterpret_cast<uint16_t*>(smem + 16);
+    const int lane = threadIdx.x & 31;
+    const int owned = long_rows_owned<RB>(n_rows);
+    for (int j0 = 0; j0 < owned; j0 += THREADS * LONG_SCAN) {
+        __syncthreads();
+        if (threadIdx.x == 0) cnt[0] = cnt[1] = 0;
+        __syncthreads();
+        for (int k = 0; k < LONG_SCAN; ++k) {
+            const int j = k * THREADS + threadIdx.x;
+            bool is_long = false;
+            if (j0 + j < owned) {
+                const int64_t r = long_row_of<RB>(j0 + j);
+                is_long = r < n_rows && __ldg(row_ptr + r + 1) - __ldg(row_ptr + r) > LONG_ROW;
+            }
+            const unsigned marks = __ballot_sync(0xffffffffu, is_long) >> (lane / GROUP * GROUP);
+            if (lane % GROUP == 0 && (marks & ((1u << GROUP) - 1u)) != 0) list[atomicAdd(cnt, 1)] = (uint16_t)(j / GROUP);
+        }
+        __syncthreads();
+        const int n = cnt[0];
+        for (int i = 0; i < n; ++i) {   // the longest rows
+            const int64_t r0 = long_row_of<RB>(j0 + list[i] * GROUP);
+            for (int64_t r = r0; r < r0 + GROUP && r < n_rows; ++r) {
+                const int64_t b = __ldg(row_ptr + r), len = __ldg(row_ptr + r + 1) - b;
+                if (len > LONG_BIG)
+                    long_row_by_cta<D, THREADS, BYTES - RING, HAS_VAL>(smem + RING, H, col_idx + b, HAS_VAL ? val + b : nullptr, (int)len, out + r * D);
+            }
+        }
+        while (true) {   // the others: a warp for each slice of a group
+            int i = 0;
+            if (lane == 0) i = atomicAdd(cnt + 1, 1);
+            i = __shfl_sync(0xffffffffu, i, 0);
+            if (i >= n * SLICES) break;
+            const int64_t r0 = long_row_of<RB>(j0 + list[i / SLICES] * GROUP);
+            const int c0 = i % SLICES * SL;
+            const int64_t ri = r0 + (lane <= GROUP ? lane : GROUP);
+            const RpT rp = __ldg(row_ptr + (ri < n_rows ? ri : n_rows));
+            int64_t b = __shfl_sync(0xffffffffu, rp, 0), e = __shfl_sync(0xffffffffu, rp, 1);
+            int c = b + lane < e ? __ldg(col_idx + b + lane) : 0;
+            for (int k = 0; k < GROUP; ++k) {
+                const int64_t en = __shfl_sync(0xffffffffu, rp, k + 2 <= GROUP ? k + 2 : GROUP);
+                const int cn = e + lane < en ? __ldg(col_idx + e + lane) : 0;   // the next row's first indices
+                if (r0 + k < n_rows && e - b <= LONG_BIG)
+                    long_row_by_warp<D, SL, HAS_VAL>(H + c0, col_idx + b, HAS_VAL ? val + b : nullptr, (int)(e - b), c, out + (r0 + k) * D + c0);
+                b = e;
+                e = en;
+                c = cn;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// the sum that sum_long_rows left in the row's place of `out`
+__device__ __forceinline__ float4 long_row_sum(const float4* p)
+{
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+}  // namespace
