@@ -357,9 +357,8 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
     //     once, in front (below that the two launches cost more than they save);
     //   * with embed_out, batches below S2V_FUSED_EMBED_NODES nodes keep one launch per level: callers of that form
     //     observe the launch count of the per-level path.
-    //   * d = 128: batches below S2V_FUSED_TABLE_NODES nodes; larger ones go to the kernels below.
     const bool forced = ctx->graph_tiles == 1;
-    if (ctx->graph_tiles != 0 && (d != 128 || (!forced && N < S2V_FUSED_TABLE_NODES)) && L >= 1 && N > 0 && G < (int64_t)INT32_MAX && batch->max_graph_nodes >= 1 &&
+    if (ctx->graph_tiles != 0 && L >= 1 && N > 0 && G < (int64_t)INT32_MAX && batch->max_graph_nodes >= 1 &&
         (forced || !embed_out || N >= S2V_FUSED_EMBED_NODES) && (batch->tags || batch->x_dense) &&
         s2v_graph_fused_supported(ctx, d, batch->max_graph_nodes, batch->tags ? model->num_feat : 1)) {
         if (!s2v_aligned16(model->w_n2l) || !s2v_aligned16(model->p_node_conv) || (embed_out && !s2v_aligned16(embed_out)))

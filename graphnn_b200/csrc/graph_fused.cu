@@ -35,8 +35,6 @@
 namespace
 {
 
-constexpr int GF_MAXG = 64;   // graphs per tile
-
 struct GfParams {
     int64_t G;
     const int32_t* row_ptr;
@@ -66,15 +64,23 @@ struct GfParams {
 
 template <int D>
 struct GfCfg {
+    // d = 128: the product is taken transposed, (H_new)^T = W^T * S^T, with W^T as the A operand in tensor memory and row blocks
+    // of 64: operand buffer and H rows of a 128-node tile then take 96 KB, and two CTAs fit an SM -- one gathers while the
+    // other multiplies and drains.  (With W in shared memory, one tile per SM: 16 warps in lock step, 0.70 ms on 16,384 molecules.)
+    static constexpr bool TR = D == 128;
+    static constexpr int RB = TR ? 64 : 128;              // rows per row block
+    static constexpr int MAXG = TR ? 56 : 64;             // graphs per tile
     static constexpr int LPR = D / 4;                     // lanes (and 16-byte pieces) per row
     static constexpr uint32_t ROWB = D * 4;
-    static constexpr uint32_t S_BYTES = 128 * D * 4;      // fp16 head + tail of 128 rows
+    static constexpr uint32_t S_BYTES = RB * D * 4;       // fp16 head + tail of a row block
     static constexpr uint32_t W_BYTES = D * D * 4;
-    static constexpr uint32_t OFF_S = 0, OFF_W = S_BYTES, OFF_H = S_BYTES + W_BYTES;
+    static constexpr uint32_t OFF_S = 0, OFF_W = S_BYTES, OFF_H = S_BYTES + (TR ? 0u : W_BYTES);
+    static constexpr uint32_t TM_WLO = 64, TM_ACC = 128;  // TR: tensor memory columns (W^T head at 0)
+    static constexpr uint32_t PART_OFF = MAXG * ROWB < S_BYTES / 2 ? S_BYTES / 2 : MAXG * ROWB;   // pooling: partial sums behind the pooled rows
     // K chunks of 64 fp16 (one 128-byte swizzle row); d = 32 keeps head and tail side by side in one chunk
     static constexpr uint32_t S_LO = D == 32 ? 64 : S_BYTES / 2, W_LO = D == 32 ? 64 : W_BYTES / 2;
     static constexpr int SHIFT = D == 128 ? 5 : (D == 64 ? 4 : 3);
-    static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(D >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // f32 <- f16 x f16, M = 128, N = D
+    static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)((TR ? RB : D) >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // f32 <- f16 x f16, M = 128, N = D (TR: RB)
 };
 
 __host__ __device__ constexpr uint32_t gf_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
@@ -91,8 +97,8 @@ __host__ __device__ inline GfMap gf_map(int cap, int chunk_cap, bool has_val)
     m.roww = m.info + 4u * (uint32_t)cap;                              // per row: its edge weight
     m.tags = m.roww + (has_val ? 4u * (uint32_t)cap : 0u);
     m.goff = m.tags + gf_up(2u * (uint32_t)(cap + 1), 16);
-    m.rs = m.goff + gf_up(4u * (GF_MAXG + 1), 16);                     // per row: exponent of its operand scale
-    m.bar = m.rs + (uint32_t)cap;
+    m.rs = m.goff + gf_up(4u * (GfCfg<D>::MAXG + 1), 16);              // per row: exponent of its operand scale (TR: what its products are multiplied by)
+    m.bar = m.rs + (GfCfg<D>::TR ? 4u : 1u) * (uint32_t)cap;
     m.col = m.bar + 160;                                               // chunks of four 16-bit local columns
     m.total = m.col + gf_up(8u * (uint32_t)chunk_cap, 16) + 1024;      // + slack to align the base to 1024 bytes
     return m;
@@ -173,6 +179,17 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uin
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// A (two packed fp16 per column) in tensor memory
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        :
+        : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 __device__ __forceinline__ void tc_ld_cols8(uint32_t addr, uint32_t* v)
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -232,6 +249,80 @@ __device__ __forceinline__ void gf_convert_w(const float* __restrict__ W, unsign
             *reinterpret_cast<uint32_t*>(dst + gf_op_off_lo<D>(n, k, D, GfCfg<D>::W_LO)) = lo;
         }
     }
+}
+
+// d = 128: W^T as the A operand in tensor memory: lane m = output feature, column c = the pair of input features 2c, 2c + 1.
+// Each thread holds 64 input features of one output feature: warp w of eight has lanes 32 (w % 4) .. and the half w / 4.
+__device__ __forceinline__ void gf_store_w_pairs(uint32_t tmem, const uint32_t (&hi)[32], const uint32_t (&lo)[32])
+{
+    const int warp = threadIdx.x >> 5;
+    const uint32_t at = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * (warp >> 2));
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        tc_st_cols8(at + 8 * h, hi + 8 * h);
+        tc_st_cols8(at + GfCfg<128>::TM_WLO + 8 * h, lo + 8 * h);
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// image: word (c, m) at c * 128 + m, heads first, tails behind them
+__device__ __forceinline__ void gf_load_w_t(const void* image, uint32_t tmem, float& inv_w)
+{
+    const int warp = threadIdx.x >> 5, m = 32 * (warp & 3) + (threadIdx.x & 31);
+    const uint32_t* w = static_cast<const uint32_t*>(image) + (32 * (warp >> 2)) * 128 + m;
+    uint32_t hi[32], lo[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) { hi[c] = __ldg(w + c * 128); lo[c] = __ldg(w + 64 * 128 + c * 128); }
+    inv_w = __ldg(static_cast<const float*>(image) + 128 * 128);
+    gf_store_w_pairs(tmem, hi, lo);
+}
+__device__ __forceinline__ void gf_convert_w_t(const float* __restrict__ W, uint32_t tmem, uint32_t* s_max, float& inv_w)
+{
+    const int warp = threadIdx.x >> 5, m = 32 * (warp & 3) + (threadIdx.x & 31);
+    float a[64];
+#pragma unroll
+    for (int k = 0; k < 64; ++k) a[k] = __ldg(W + (64 * (warp >> 2) + k) * 128 + m);
+    float mx = 0.f;
+#pragma unroll
+    for (int k = 0; k < 64; ++k) mx = fmaxf(mx, fabsf(a[k]));
+    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+    if ((threadIdx.x & 31) == 0) atomicMax(s_max, w);
+    __syncthreads();
+    const uint32_t e_w = gf_exponent(*s_max);
+    const float sc = gf_scale(e_w);
+    inv_w = gf_unscale(e_w);
+    uint32_t hi[32], lo[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) split_f16(pack2(a[2 * c] * sc, a[2 * c + 1] * sc), hi[c], lo[c]);
+    gf_store_w_pairs(tmem, hi, lo);
+}
+__global__ void __launch_bounds__(1024) gf_weight_image_t_kernel(const float* __restrict__ W, uint32_t* __restrict__ image)
+{
+    __shared__ uint32_t s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    float a[8][2], mx = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = threadIdx.x + i * 1024, m = e % 128, c = e / 128;
+        a[i][0] = __ldg(W + (2 * c) * 128 + m);
+        a[i][1] = __ldg(W + (2 * c + 1) * 128 + m);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fmaxf(fabsf(a[i][0]), fabsf(a[i][1])));
+    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, w);
+    __syncthreads();
+    const uint32_t e_w = gf_exponent(s_max);
+    const float sc = gf_scale(e_w);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = threadIdx.x + i * 1024;
+        uint32_t hi, lo;
+        split_f16(pack2(a[i][0] * sc, a[i][1] * sc), hi, lo);
+        image[e] = hi;
+        image[64 * 128 + e] = lo;
+    }
+    if (threadIdx.x == 0) reinterpret_cast<float*>(image)[128 * 128] = gf_unscale(e_w);
 }
 
 // the same into global memory, once per batch: [operand image | inverse scale]
@@ -367,8 +458,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     constexpr int WT = WARPS * 32;
     constexpr int LPR = Cfg::LPR, GPW = 32 / LPR;   // lanes per row, row groups per warp
     constexpr int NG = WARPS * GPW;                 // row groups
-    constexpr int RPG = 128 / NG;                   // rows of a row block per group
-    constexpr int CW = D / (WARPS / 4);             // accumulator columns a warp drains
+    constexpr int RB = Cfg::RB, RPG = RB / NG;      // rows of a row block, per group
+    constexpr int CW = D / (WARPS / 4);             // accumulator columns a warp drains (not TR)
     constexpr int LDC = CW >= 16 ? 16 : 8;          // columns per tcgen05.ld
     constexpr int ROUNDS = D == 128 || (D == 64 && WARPS == 8) ? 1 : (D == 32 && WARPS == 8 ? 3 : 2);   // rows per thread in the prologue
 
@@ -380,6 +471,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     uint16_t* const tag_s = reinterpret_cast<uint16_t*>(smem + map.tags);
     int* const goff = reinterpret_cast<int*>(smem + map.goff);
     uint8_t* const rs = smem + map.rs;
+    float* const rsf = reinterpret_cast<float*>(smem + map.rs);
     uint2* const chunks = reinterpret_cast<uint2*>(smem + map.col);
     float4* const H4 = reinterpret_cast<float4*>(smem + Cfg::OFF_H);
     const ulonglong2* const H2 = reinterpret_cast<const ulonglong2*>(smem + Cfg::OFF_H);
@@ -427,7 +519,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     const uint32_t tmem_base = *tmem_slot;
     const int g_lo = s_range[0], g_hi = s_range[1];
     float inv_w;
-    if (p.w_image) {
+    if (Cfg::TR) {
+        if (p.w_image) gf_load_w_t(p.w_image, tmem_base, inv_w);
+        else gf_convert_w_t(p.W, tmem_base, s_max, inv_w);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    } else if (p.w_image) {
         const uint4* src = static_cast<const uint4*>(p.w_image);
         uint4* dst = reinterpret_cast<uint4*>(smem + Cfg::OFF_W);
         for (int i = threadIdx.x; i < (int)(Cfg::W_BYTES / 16); i += WT) dst[i] = __ldg(src + i);
@@ -444,12 +540,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     const int grp = warp * GPW + sub;
     const float4* __restrict__ X4 = reinterpret_cast<const float4*>(p.x);
     for (int g0 = g_lo; g0 < g_hi;) {
-        // ---- the tile: whole graphs from g0 on, at most cap nodes and GF_MAXG graphs (every warp works it out by itself)
+        // ---- the tile: whole graphs from g0 on, at most cap nodes and MAXG graphs (every warp works it out by itself)
         const int node0 = __ldg(p.graph_ptr + g0);
         int g1 = g0;
-        while (g1 < g_hi && g1 - g0 < GF_MAXG) {
+        while (g1 < g_hi && g1 - g0 < Cfg::MAXG) {
             const int gi = g1 + 1 + lane;
-            const bool fits = gi <= g_hi && gi - g0 <= GF_MAXG && __ldg(p.graph_ptr + gi) - node0 <= p.cap;
+            const bool fits = gi <= g_hi && gi - g0 <= Cfg::MAXG && __ldg(p.graph_ptr + gi) - node0 <= p.cap;
             const unsigned bal = __ballot_sync(0xffffffffu, fits);
             const int n = bal == 0xffffffffu ? 32 : __ffs(~bal) - 1;
             g1 += n;
@@ -464,7 +560,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         }
         if (nrows < 0) nrows = 0;
         const int ngr = g1 - g0;
-        const int mt = (nrows + 127) >> 7;
+        const int mt = (nrows + RB - 1) / RB;
 
         // ---- tile prologue: row structure, tags, graph offsets; then local columns in chunks of four, H0
         int rb[ROUNDS], rn[ROUNDS];
@@ -483,6 +579,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 }
             }
         }
+        if (Cfg::TR && threadIdx.x >= nrows && threadIdx.x < p.cap) tag_s[threadIdx.x] = 0;   // (looked up, never used)
         for (int k = threadIdx.x; k <= ngr; k += WT) {
             const int v = __ldg(p.graph_ptr + g0 + k) - node0;
             goff[k] = v < 0 ? 0 : (v > nrows ? nrows : v);
@@ -594,7 +691,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         for (int lv = 0; lv < p.levels; ++lv) {
             // -------------------------------- gather, split, hand over --------------------------------
             for (int m = 0; m < mt; ++m) {
-                const int rows_m = nrows - 128 * m < 128 ? nrows - 128 * m : 128;
+                const int rows_m = nrows - RB * m < RB ? nrows - RB * m : RB;
                 uint64_t a0[RPG], a1[RPG];
                 if (listed) {
                     // every row's first chunk is fetched before the first row is summed; further chunks in a loop whose
@@ -603,7 +700,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                     uint2 ef[RPG];
                     const uint32_t slx = (uint32_t)sl * 0x10001u;
 #pragma unroll
-                    for (int i = 0; i < RPG; ++i) inf[i] = i * NG + grp < rows_m ? info_s[128 * m + i * NG + grp] : 0u;
+                    for (int i = 0; i < RPG; ++i) inf[i] = i * NG + grp < rows_m ? info_s[RB * m + i * NG + grp] : 0u;
 #pragma unroll
                     for (int i = 0; i < RPG; ++i) ef[i] = chunks[inf[i] & 0xffffu];
 #pragma unroll
@@ -621,7 +718,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                             const uint32_t mine = inf[i] >> 16, most = __reduce_max_sync(0xffffffffu, mine);
                             for (uint32_t c = 1; c < most; ++c) add4(chunks[c < mine ? (inf[i] & 0xffffu) + c : 0u]);
                             if (HAS_VAL) {
-                                const float w = i * NG + grp < rows_m ? roww[128 * m + i * NG + grp] : 0.f;
+                                const float w = i * NG + grp < rows_m ? roww[RB * m + i * NG + grp] : 0.f;
                                 a0[i] = mul2(a0[i], pack2(w, w));
                                 a1[i] = mul2(a1[i], pack2(w, w));
                             }
@@ -632,7 +729,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                     for (int i = 0; i < RPG; ++i) {
                         a0[i] = a1[i] = 0ull;
                         if (i * NG + grp < rows_m) {
-                            const ulonglong2 v = gf_row_from_global<D, HAS_VAL>(p.row_ptr, p.col_idx, p.val, p.status, H2, node0, nrows, 128 * m + i * NG + grp, sl);
+                            const ulonglong2 v = gf_row_from_global<D, HAS_VAL>(p.row_ptr, p.col_idx, p.val, p.status, H2, node0, nrows, RB * m + i * NG + grp, sl);
                             a0[i] = v.x;
                             a1[i] = v.y;
                         }
@@ -641,8 +738,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 }
                 // the operand buffer is free once the previous row block of this level is multiplied
                 if (m > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 40);
-                unsigned char* const s_hi = smem + Cfg::OFF_S + gf_op_off(grp, 4 * sl, 128);   // (row i*NG + grp: + i*NG*128, the same swizzle)
-                unsigned char* const s_lo = smem + Cfg::OFF_S + gf_op_off_lo<D>(grp, 4 * sl, 128, Cfg::S_LO);
+                unsigned char* const s_hi = smem + Cfg::OFF_S + gf_op_off(grp, 4 * sl, RB);   // (row i*NG + grp: + i*NG*128, the same swizzle)
+                unsigned char* const s_lo = smem + Cfg::OFF_S + gf_op_off_lo<D>(grp, 4 * sl, RB, Cfg::S_LO);
 #pragma unroll
                 for (int i = 0; i < RPG; ++i) {
                     if (i * NG + warp * GPW < rows_m) {
@@ -661,7 +758,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                         // (rows past the tile's last one are written too: finite, never read back)
                         *reinterpret_cast<uint2*>(s_hi + i * NG * 128) = hi;
                         *reinterpret_cast<uint2*>(s_lo + i * NG * 128) = lo;
-                        if (sl == 0 && i * NG + grp < rows_m) rs[128 * m + i * NG + grp] = (uint8_t)ex;
+                        if (sl == 0 && i * NG + grp < rows_m) {
+                            if (Cfg::TR) rsf[RB * m + i * NG + grp] = gf_unscale(ex) * inv_w;
+                            else rs[RB * m + i * NG + grp] = (uint8_t)ex;
+                        }
                     }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // my stores -> visible to the tensor core
@@ -675,15 +775,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (lane == 0) {
                         const uint32_t s_addr = smem_u32(smem + Cfg::OFF_S), w_addr = smem_u32(smem + Cfg::OFF_W);
-                        const uint32_t acc = tmem_base + (uint32_t)(m * D);
+                        const uint32_t acc = tmem_base + (Cfg::TR ? Cfg::TM_ACC + (uint32_t)(m * RB) : (uint32_t)(m * D));
 #pragma unroll
                         for (int pass = 0; pass < 3; ++pass) {   // tail*head, head*tail, head*head: small terms first
-                            const uint32_t a_base = s_addr + (pass == 0 ? Cfg::S_LO : 0u), b_base = w_addr + (pass == 1 ? Cfg::W_LO : 0u);
+                            const uint32_t s_base = s_addr + (pass == 0 ? Cfg::S_LO : 0u), w_base = w_addr + (pass == 1 ? Cfg::W_LO : 0u);
 #pragma unroll
                             for (int ks = 0; ks < D / 16; ++ks) {
-                                const uint32_t ao = (uint32_t)(ks >> 2) * (128u * 128u) + (uint32_t)(ks & 3) * 32u;
-                                const uint32_t bo = (uint32_t)(ks >> 2) * (uint32_t)(D * 128) + (uint32_t)(ks & 3) * 32u;
-                                mma_f16_ss(acc, tc_b_desc(a_base + ao), tc_b_desc(b_base + bo), Cfg::IDESC, (pass | ks) != 0);
+                                const uint32_t so = (uint32_t)(ks >> 2) * (uint32_t)(RB * 128) + (uint32_t)(ks & 3) * 32u;
+                                const uint32_t wo = (uint32_t)(ks >> 2) * (uint32_t)(D * 128) + (uint32_t)(ks & 3) * 32u;
+                                if (Cfg::TR) mma_f16_ts(acc, tmem_base + (pass == 1 ? Cfg::TM_WLO : 0u) + 8u * ks, tc_b_desc(s_base + so), Cfg::IDESC, (pass | ks) != 0);
+                                else mma_f16_ss(acc, tc_b_desc(s_base + so), tc_b_desc(w_base + wo), Cfg::IDESC, (pass | ks) != 0);
                             }
                         }
                         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_mma) : "memory");
@@ -695,49 +796,97 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             // -------------------------------- drain: H = ReLU(acc * scale + X) --------------------------------
             // Units of LDC columns of 32 rows.  X of the next unit is on its way while one is worked on, the first unit's
             // during the wait.  (The last product of the level completes only after every warp has finished gathering from H.)
-            constexpr int UNITS = CW / LDC;
-            float4 x[LDC / 4];
-            auto x_row = [&](int m) -> const float4* {
-                const int r = 128 * m + 32 * q + lane;
-                const int64_t xr = r < nrows ? (p.tags ? (int64_t)tag_s[r] : (int64_t)node0 + r) : 0;
-                return X4 + xr * LPR + jc * (CW / 4);
-            };
-            const float4* xp = x_row(0);
+            if constexpr (Cfg::TR) {
+                // lane = output feature f, 16 nodes at a time (their scales and tags are broadcast reads); the rows of H are
+                // written 128 bytes per instruction
+                const int f = 32 * q + lane;
+                const float* __restrict__ Xf = p.x + f;
+                const uint32_t piece = (uint32_t)(f >> 2);
+                float* const hcol = reinterpret_cast<float*>(smem + Cfg::OFF_H) + (f & 3);
+                auto load_x = [&](int r0, float (&x)[16]) {
+                    if (r0 >= nrows) return;
+                    if (p.tags) {
 #pragma unroll
-            for (int c = 0; c < LDC / 4; ++c) x[c] = __ldg(xp + c);
-            if (mt > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int m = 0; m < mt; ++m) {
-                if (128 * m + 32 * q >= nrows) break;   // warp-uniform
-                const int r = 128 * m + 32 * q + lane;
-                const bool have = r < nrows;
-                const float c1 = have ? gf_unscale(rs[r]) * inv_w : 0.f;
-                const uint64_t cc = pack2(c1, c1);
-                const uint32_t acc_addr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(m * D + jc * CW);
-                const uint32_t he = (uint32_t)((r << Cfg::SHIFT) + (r & 7));
-                const float4* xn = x_row(m + 1);
-#pragma unroll
-                for (int h = 0; h < UNITS; ++h) {
-                    uint32_t v[LDC];
-                    if (LDC == 16) tc_ld_cols16(acc_addr + (uint32_t)(h * LDC), v);
-                    else tc_ld_cols8(acc_addr + (uint32_t)(h * LDC), v);
-                    float4 y[LDC / 4];
-#pragma unroll
-                    for (int c = 0; c < LDC / 4; ++c) y[c] = x[c];
-                    const float4* nx = h + 1 < UNITS ? xp + (h + 1) * (LDC / 4) : xn;
-#pragma unroll
-                    for (int c = 0; c < LDC / 4; ++c) x[c] = __ldg(nx + c);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (have) {
-#pragma unroll
-                        for (int c = 0; c < LDC / 4; ++c) {
-                            const float2 lo2 = unpack2(fma2(pack2(__uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1])), cc, pack2(y[c].x, y[c].y)));
-                            const float2 hi2 = unpack2(fma2(pack2(__uint_as_float(v[4 * c + 2]), __uint_as_float(v[4 * c + 3])), cc, pack2(y[c].z, y[c].w)));
-                            H4[he ^ (uint32_t)(jc * (CW / 4) + h * (LDC / 4) + c)] = make_float4(relu_max(lo2.x), relu_max(lo2.y), relu_max(hi2.x), relu_max(hi2.y));
+                        for (int i = 0; i < 16; i += 4) {
+                            const uint2 t4 = *reinterpret_cast<const uint2*>(tag_s + r0 + i);
+                            x[i] = __ldg(Xf + (t4.x & 0xffffu) * 128u);
+                            x[i + 1] = __ldg(Xf + (t4.x >> 16) * 128u);
+                            x[i + 2] = __ldg(Xf + (t4.y & 0xffffu) * 128u);
+                            x[i + 3] = __ldg(Xf + (t4.y >> 16) * 128u);
                         }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) x[i] = __ldg(Xf + ((int64_t)node0 + (r0 + i < nrows ? r0 + i : nrows - 1)) * 128);
+                    }
+                };
+                float x[16];
+                load_x(32 * jc, x);
+                if (mt > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int g = 0; g < 2 * mt; ++g) {   // 16-node groups of my half of every row block
+                    const int r0 = 64 * (g >> 1) + 32 * jc + 16 * (g & 1);
+                    if (r0 >= nrows) continue;       // warp-uniform
+                    uint32_t v[16];
+                    tc_ld_cols16(tmem_base + Cfg::TM_ACC + ((uint32_t)(32 * q) << 16) + (uint32_t)r0, v);
+                    float y[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) y[i] = x[i];
+                    if (g + 1 < 2 * mt) load_x(64 * ((g + 1) >> 1) + 32 * jc + 16 * ((g + 1) & 1), x);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4) {
+                        const float4 c4 = *reinterpret_cast<const float4*>(rsf + r0 + i);
+                        const float c[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            hcol[(r0 + i + u) * 128 + ((piece ^ (uint32_t)((i + u) & 7)) * 4)] = relu_max(fmaf(__uint_as_float(v[i + u]), c[u], y[i + u]));
                     }
                 }
-                xp = xn;
+            } else {
+                constexpr int UNITS = CW / LDC;
+                float4 x[LDC / 4];
+                auto x_row = [&](int m) -> const float4* {
+                    const int r = 128 * m + 32 * q + lane;
+                    const int64_t xr = r < nrows ? (p.tags ? (int64_t)tag_s[r] : (int64_t)node0 + r) : 0;
+                    return X4 + xr * LPR + jc * (CW / 4);
+                };
+                const float4* xp = x_row(0);
+#pragma unroll
+                for (int c = 0; c < LDC / 4; ++c) x[c] = __ldg(xp + c);
+                if (mt > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int m = 0; m < mt; ++m) {
+                    if (128 * m + 32 * q >= nrows) break;   // warp-uniform
+                    const int r = 128 * m + 32 * q + lane;
+                    const bool have = r < nrows;
+                    const float c1 = have ? gf_unscale(rs[r]) * inv_w : 0.f;
+                    const uint64_t cc = pack2(c1, c1);
+                    const uint32_t acc_addr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(m * D + jc * CW);
+                    const uint32_t he = (uint32_t)((r << Cfg::SHIFT) + (r & 7));
+                    const float4* xn = x_row(m + 1);
+#pragma unroll
+                    for (int h = 0; h < UNITS; ++h) {
+                        uint32_t v[LDC];
+                        if (LDC == 16) tc_ld_cols16(acc_addr + (uint32_t)(h * LDC), v);
+                        else tc_ld_cols8(acc_addr + (uint32_t)(h * LDC), v);
+                        float4 y[LDC / 4];
+#pragma unroll
+                        for (int c = 0; c < LDC / 4; ++c) y[c] = x[c];
+                        const float4* nx = h + 1 < UNITS ? xp + (h + 1) * (LDC / 4) : xn;
+#pragma unroll
+                        for (int c = 0; c < LDC / 4; ++c) x[c] = __ldg(nx + c);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (have) {
+#pragma unroll
+                            for (int c = 0; c < LDC / 4; ++c) {
+                                const float2 lo2 = unpack2(fma2(pack2(__uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1])), cc, pack2(y[c].x, y[c].y)));
+                                const float2 hi2 = unpack2(fma2(pack2(__uint_as_float(v[4 * c + 2]), __uint_as_float(v[4 * c + 3])), cc, pack2(y[c].z, y[c].w)));
+                                H4[he ^ (uint32_t)(jc * (CW / 4) + h * (LDC / 4) + c)] = make_float4(relu_max(lo2.x), relu_max(lo2.y), relu_max(hi2.x), relu_max(hi2.y));
+                            }
+                        }
+                    }
+                    xp = xn;
+                }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             gf_worker_sync<WT>();
@@ -748,8 +897,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 reinterpret_cast<float4*>(p.embed_out)[(int64_t)(node0 + r) * LPR + sl] = H4[((r << Cfg::SHIFT) + (r & 7)) ^ sl];
         // Graphs of up to 32 nodes are summed by one warp each; larger ones in pieces of 32 nodes (counted from the
         // graph's first node) by different warps, the partial sums added in order.
-        float* const y_s = reinterpret_cast<float*>(smem + Cfg::OFF_S);                       // [GF_MAXG][D]
-        float4* const part4 = reinterpret_cast<float4*>(smem + Cfg::OFF_S + Cfg::S_BYTES / 2);  // [GF_MAXG][D]
+        float* const y_s = reinterpret_cast<float*>(smem + Cfg::OFF_S);                       // [Cfg::MAXG][D]
+        float4* const part4 = reinterpret_cast<float4*>(smem + Cfg::OFF_S + Cfg::PART_OFF);   // pieces of graphs above 32 nodes
         int slot = 0;
         auto sum_rows = [&](int nb, int ne, float wgt) -> float4 {
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -878,7 +1027,7 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     }
     if (a.image_scratch) {
         unsigned char* img = static_cast<unsigned char*>(a.image_scratch);
-        if (a.d == 128) gf_weight_image_kernel<128><<<1, 1024, 0, st>>>(a.W, img);
+        if (a.d == 128) gf_weight_image_t_kernel<<<1, 1024, 0, st>>>(a.W, reinterpret_cast<uint32_t*>(img));
         else if (a.d == 64) gf_weight_image_kernel<64><<<1, 1024, 0, st>>>(a.W, img);
         else gf_weight_image_kernel<32><<<1, 1024, 0, st>>>(a.W, img);
         S2V_CHECK_LAUNCH(ctx, "gf_weight_image_kernel");
@@ -889,6 +1038,7 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     // what fits, with 544 threads.
     const int need = (a.max_graph_nodes + 127) / 128 * 128;
     int warps = 16, per_sm = 1, cap = 128;
+    if (a.d == 128) { warps = 8; per_sm = 2; }
     if (a.d == 64 && need == 128) { warps = 8; per_sm = 2; }
     if (a.d == 64 && need > 128) {
         const int64_t share = (a.N / ctx->sm_count + 127) / 128 * 128;
@@ -906,7 +1056,7 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     p.cap = cap;
     uint32_t cols = 32;
     while (cols < (uint32_t)(cap / 128 * a.d)) cols *= 2;
-    p.tm_cols = cols;
+    p.tm_cols = a.d == 128 ? 256 : cols;   // d = 128: W^T and the accumulators of two row blocks
     // what is left of the CTA's share of shared memory lists the columns (8 bytes per four)
     const bool hv = a.val != nullptr;
     auto total = [&](int n) {
@@ -918,7 +1068,7 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     const uint32_t smem = total(p.chunk_cap);
     const int64_t most = (int64_t)ctx->sm_count * per_sm;
     const unsigned blocks = (unsigned)(a.G < most ? a.G : most);
-    if (a.d == 128) return gf_launch<128, 16>(ctx, st, p, smem, blocks);
+    if (a.d == 128) return gf_launch<128, 8>(ctx, st, p, smem, blocks);
     if (a.d == 64) return warps == 8 ? gf_launch<64, 8>(ctx, st, p, smem, blocks) : gf_launch<64, 16>(ctx, st, p, smem, blocks);
     return warps == 8 ? gf_launch<32, 8>(ctx, st, p, smem, blocks) : gf_launch<32, 16>(ctx, st, p, smem, blocks);
 }
