@@ -70,6 +70,7 @@ struct GfCfg {
     static constexpr bool TR = D == 128;
     static constexpr int RB = TR ? 64 : 128;              // rows per row block
     static constexpr int MAXG = TR ? 56 : 64;             // graphs per tile
+    static constexpr uint32_t CHUNK = TR ? 16 : 8;        // bytes of a chunk of four columns
     static constexpr int LPR = D / 4;                     // lanes (and 16-byte pieces) per row
     static constexpr uint32_t ROWB = D * 4;
     static constexpr uint32_t S_BYTES = RB * D * 4;       // fp16 head + tail of a row block
@@ -96,11 +97,11 @@ __host__ __device__ inline GfMap gf_map(int cap, int chunk_cap, bool has_val)
     m.info = GfCfg<D>::OFF_H + (uint32_t)(cap + 1) * GfCfg<D>::ROWB;   // per row: first chunk of columns | chunks << 16
     m.roww = m.info + 4u * (uint32_t)cap;                              // per row: its edge weight
     m.tags = m.roww + (has_val ? 4u * (uint32_t)cap : 0u);
-    m.goff = m.tags + gf_up(2u * (uint32_t)(cap + 1), 16);
+    m.goff = m.tags + gf_up((GfCfg<D>::TR ? 4u : 2u) * (uint32_t)(cap + 1), 16);   // TR: byte offsets of the rows' X, else tags
     m.rs = m.goff + gf_up(4u * (GfCfg<D>::MAXG + 1), 16);              // per row: exponent of its operand scale (TR: what its products are multiplied by)
     m.bar = m.rs + (GfCfg<D>::TR ? 4u : 1u) * (uint32_t)cap;
-    m.col = m.bar + 160;                                               // chunks of four 16-bit local columns
-    m.total = m.col + gf_up(8u * (uint32_t)chunk_cap, 16) + 1024;      // + slack to align the base to 1024 bytes
+    m.col = m.bar + 160;                                               // chunks of four local columns: 16-bit indices into H (TR: byte offsets)
+    m.total = m.col + gf_up(GfCfg<D>::CHUNK * (uint32_t)chunk_cap, 16) + 1024;   // + slack to align the base to 1024 bytes
     return m;
 }
 
@@ -114,6 +115,20 @@ template <int D>
 __device__ __forceinline__ uint32_t gf_op_off_lo(int n, int k, int rows, uint32_t lo)
 {
     return D == 32 ? gf_op_off(n, k + 32, rows) : lo + gf_op_off(n, k, rows);
+}
+
+// 16-byte piece `piece` of row r of H: swizzled where a warp's lanes read or write the same piece of many rows (not at d = 128,
+// where every access is a row's consecutive bytes)
+template <int D>
+__device__ __forceinline__ uint32_t gf_h(int r, int piece)
+{
+    return D == 128 ? (uint32_t)(r * 32 + piece) : (uint32_t)(((r << GfCfg<D>::SHIFT) + (r & 7)) ^ piece);
+}
+__device__ __forceinline__ ulonglong2 gf_lds(uint32_t addr)   // 16 bytes of shared memory
+{
+    ulonglong2 v;
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+    return v;
 }
 
 // Power-of-two scale that brings a largest magnitude into [2^14, 2^15), from its exponent e (clamped so that the scale
@@ -442,7 +457,7 @@ __device__ __noinline__ ulonglong2 gf_row_from_global(const int32_t* row_ptr, co
                     status->where = 5;
                     c[u] = 0;
                 }
-                const ulonglong2 v = H2[((c[u] << GfCfg<D>::SHIFT) + (c[u] & 7)) ^ sl];
+                const ulonglong2 v = H2[gf_h<D>(c[u], sl)];
                 const uint64_t ww = pack2(w[u], w[u]);
                 acc.x = fma2(ww, v.x, acc.x);
                 acc.y = fma2(ww, v.y, acc.y);
@@ -472,7 +487,9 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     int* const goff = reinterpret_cast<int*>(smem + map.goff);
     uint8_t* const rs = smem + map.rs;
     float* const rsf = reinterpret_cast<float*>(smem + map.rs);
+    uint32_t* const xo_s = reinterpret_cast<uint32_t*>(smem + map.tags);
     uint2* const chunks = reinterpret_cast<uint2*>(smem + map.col);
+    uint4* const chunks_t = reinterpret_cast<uint4*>(smem + map.col);
     float4* const H4 = reinterpret_cast<float4*>(smem + Cfg::OFF_H);
     const ulonglong2* const H2 = reinterpret_cast<const ulonglong2*>(smem + Cfg::OFF_H);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + map.bar);
@@ -510,8 +527,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     if (threadIdx.x < LPR) H4[p.cap * LPR + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);   // the row of zeros
     const uint32_t zero_entry = (uint32_t)p.cap << Cfg::SHIFT;
     if (threadIdx.x == 0) {
-        chunks[0] = make_uint2(zero_entry * 0x10001u, zero_entry * 0x10001u);                   // a chunk of zero rows
-        tag_s[p.cap] = (uint16_t)p.num_tags;                                                    // P has a row of zeros behind the last tag
+        // chunk 0: zero rows; P has a row of zeros behind the last tag
+        if (Cfg::TR) {
+            const uint32_t z = Cfg::OFF_H + (uint32_t)p.cap * Cfg::ROWB;
+            chunks_t[0] = make_uint4(z, z, z, z);
+            xo_s[p.cap] = (uint32_t)p.num_tags * Cfg::ROWB;
+        } else {
+            chunks[0] = make_uint2(zero_entry * 0x10001u, zero_entry * 0x10001u);
+            tag_s[p.cap] = (uint16_t)p.num_tags;
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -575,11 +599,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 if (p.tags) {
                     const int t = __ldg(p.tags + node0 + r);
                     bad_tag |= (unsigned)t >= (unsigned)p.num_tags ? 1 : 0;
-                    tag_s[r] = (uint16_t)((unsigned)t >= (unsigned)p.num_tags ? 0 : t);
-                }
+                    const int ok = (unsigned)t >= (unsigned)p.num_tags ? 0 : t;
+                    if (Cfg::TR) xo_s[r] = (uint32_t)ok * Cfg::ROWB;
+                    else tag_s[r] = (uint16_t)ok;
+                } else if (Cfg::TR) xo_s[r] = (uint32_t)r * Cfg::ROWB;
             }
         }
-        if (Cfg::TR && threadIdx.x >= nrows && threadIdx.x < p.cap) tag_s[threadIdx.x] = 0;   // (looked up, never used)
+        if (Cfg::TR && threadIdx.x >= nrows && threadIdx.x < p.cap) xo_s[threadIdx.x] = 0;   // (looked up, never used)
         for (int k = threadIdx.x; k <= ngr; k += WT) {
             const int v = __ldg(p.graph_ptr + g0 + k) - node0;
             goff[k] = v < 0 ? 0 : (v > nrows ? nrows : v);
@@ -624,9 +650,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                                 p.status->where = 5;
                                 e[u] = 0;
                             }
-                            e[u] = (e[u] << Cfg::SHIFT) + (e[u] & 7u);
+                            e[u] = Cfg::TR ? Cfg::OFF_H + e[u] * Cfg::ROWB : (e[u] << Cfg::SHIFT) + (e[u] & 7u);
                         }
-                        chunks[first[k] + (t >> 2)] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
+                        if (Cfg::TR) chunks_t[first[k] + (t >> 2)] = make_uint4(e[0], e[1], e[2], e[3]);
+                        else chunks[first[k] + (t >> 2)] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
                     }
                 if (HAS_VAL) {
                     const float w0 = rn[k] > 0 ? __ldg(p.val + rb[k]) : 0.f;
@@ -645,7 +672,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                     xr = (unsigned)t >= (unsigned)p.num_tags ? 0 : t;
                 }
                 const float4 v = __ldg(X4 + xr * LPR + sl);
-                H4[((r << Cfg::SHIFT) + (r & 7)) ^ sl] = make_float4(relu_ref(v.x), relu_ref(v.y), relu_ref(v.z), relu_ref(v.w));
+                H4[gf_h<D>(r, sl)] = make_float4(relu_ref(v.x), relu_ref(v.y), relu_ref(v.z), relu_ref(v.w));
             }
         }
         gf_worker_sync<WT>();
@@ -653,8 +680,50 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         const bool listed = cached && !(HAS_VAL && *s_mixed != 0);
         if (p.P) {   // first level: a sum of rows of P = ReLU(W_in) * W, no product
             const float4* __restrict__ P4 = reinterpret_cast<const float4*>(p.P);
+            if (Cfg::TR && listed) {
+                // two rows at a time, so that ten table reads are on their way together
+                const char* const Pl = reinterpret_cast<const char*>(p.P) + 16 * lane;
+                const char* const Xl = reinterpret_cast<const char*>(p.x) + 16 * lane;
+                const uint32_t xo_addr = smem_u32(xo_s) - Cfg::OFF_H / 128;   // X offset of the row at byte h of the map: at h / 128
+                auto table = [&](uint32_t h) -> ulonglong2 {
+                    uint32_t off;
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(off) : "r"(xo_addr + (h >> 7)));
+                    return __ldg(reinterpret_cast<const ulonglong2*>(Pl + off));
+                };
+                for (int r = warp; r < nrows; r += 2 * WARPS) {
+                    const int ra[2] = {r, r + WARPS < nrows ? r + WARPS : p.cap};
+                    uint32_t inf[2];
+                    ulonglong2 v[2][4], x[2];
+#pragma unroll
+                    for (int a = 0; a < 2; ++a) {
+                        inf[a] = ra[a] < nrows ? info_s[ra[a]] : 0u;
+                        const uint4 c = chunks_t[inf[a] & 0xffffu];
+                        v[a][0] = table(c.x); v[a][1] = table(c.y); v[a][2] = table(c.z); v[a][3] = table(c.w);
+                        x[a] = __ldg(reinterpret_cast<const ulonglong2*>(Xl + (ra[a] < nrows ? xo_s[ra[a]] : 0u)));
+                    }
+#pragma unroll
+                    for (int a = 0; a < 2; ++a) {
+                        uint64_t s0 = add2(add2(add2(v[a][0].x, v[a][1].x), v[a][2].x), v[a][3].x);
+                        uint64_t s1 = add2(add2(add2(v[a][0].y, v[a][1].y), v[a][2].y), v[a][3].y);
+                        for (uint32_t k = 1; k < (inf[a] >> 16); ++k) {
+                            const uint4 c = chunks_t[(inf[a] & 0xffffu) + k];
+                            const ulonglong2 w0 = table(c.x), w1 = table(c.y), w2 = table(c.z), w3 = table(c.w);
+                            s0 = add2(add2(add2(add2(s0, w0.x), w1.x), w2.x), w3.x);
+                            s1 = add2(add2(add2(add2(s1, w0.y), w1.y), w2.y), w3.y);
+                        }
+                        if (HAS_VAL) {
+                            const float w = ra[a] < nrows ? roww[ra[a]] : 0.f;
+                            s0 = mul2(s0, pack2(w, w));
+                            s1 = mul2(s1, pack2(w, w));
+                        }
+                        const float2 f0 = unpack2(add2(s0, x[a].x)), f1 = unpack2(add2(s1, x[a].y));
+                        if (ra[a] < nrows) H4[ra[a] * 32 + lane] = make_float4(relu_max(f0.x), relu_max(f0.y), relu_max(f1.x), relu_max(f1.y));
+                    }
+                }
+            } else
             for (int r = grp; r < nrows; r += NG) {
-                const float4 x = __ldg(X4 + (int64_t)tag_s[r] * LPR + sl);
+                auto x_of = [&](int c) { return Cfg::TR ? (int64_t)(xo_s[c] / 16u) : (int64_t)tag_s[c] * LPR; };
+                const float4 x = __ldg(X4 + x_of(r) + sl);
                 float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (listed) {
                     const uint32_t inf = info_s[r];
@@ -663,7 +732,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                         const uint32_t e[4] = {e2.x & 0xffffu, e2.x >> 16, e2.y & 0xffffu, e2.y >> 16};
                         float4 v[4];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) v[u] = __ldg(P4 + (int64_t)tag_s[e[u] >> Cfg::SHIFT] * LPR + sl);
+                        for (int u = 0; u < 4; ++u) v[u] = __ldg(P4 + x_of((int)(e[u] >> Cfg::SHIFT)) + sl);
 #pragma unroll
                         for (int u = 0; u < 4; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
                     }
@@ -678,11 +747,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                             c = 0;
                         }
                         const float w = HAS_VAL ? __ldg(p.val + t) : 1.f;
-                        const float4 v = __ldg(P4 + (int64_t)tag_s[c] * LPR + sl);
+                        const float4 v = __ldg(P4 + x_of(c) + sl);
                         acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
                     }
                 }
-                H4[((r << Cfg::SHIFT) + (r & 7)) ^ sl] =
+                H4[gf_h<D>(r, sl)] =
                     make_float4(relu_max(acc.x + x.x), relu_max(acc.y + x.y), relu_max(acc.z + x.z), relu_max(acc.w + x.w));
             }
             gf_worker_sync<WT>();
@@ -693,7 +762,34 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             for (int m = 0; m < mt; ++m) {
                 const int rows_m = nrows - RB * m < RB ? nrows - RB * m : RB;
                 uint64_t a0[RPG], a1[RPG];
-                if (listed) {
+                if (Cfg::TR && listed) {
+                    // (the same, a warp per row and byte offsets in the list)
+                    const uint32_t lane_addr = smem_u32(smem) + 16u * (uint32_t)lane;
+                    uint32_t inf[RPG];
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) inf[i] = i * NG + warp < rows_m ? info_s[RB * m + i * NG + warp] : 0u;
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) {
+                        a0[i] = a1[i] = 0ull;
+                        if (i * NG + warp < rows_m) {
+                            const uint4 c = chunks_t[inf[i] & 0xffffu];
+                            const ulonglong2 v0 = gf_lds(lane_addr + c.x), v1 = gf_lds(lane_addr + c.y), v2 = gf_lds(lane_addr + c.z), v3 = gf_lds(lane_addr + c.w);
+                            a0[i] = add2(add2(add2(v0.x, v1.x), v2.x), v3.x);
+                            a1[i] = add2(add2(add2(v0.y, v1.y), v2.y), v3.y);
+                            for (uint32_t k = 1; k < (inf[i] >> 16); ++k) {
+                                const uint4 d = chunks_t[(inf[i] & 0xffffu) + k];
+                                const ulonglong2 w0 = gf_lds(lane_addr + d.x), w1 = gf_lds(lane_addr + d.y), w2 = gf_lds(lane_addr + d.z), w3 = gf_lds(lane_addr + d.w);
+                                a0[i] = add2(add2(add2(add2(a0[i], w0.x), w1.x), w2.x), w3.x);
+                                a1[i] = add2(add2(add2(add2(a1[i], w0.y), w1.y), w2.y), w3.y);
+                            }
+                            if (HAS_VAL) {
+                                const float w = roww[RB * m + i * NG + warp];
+                                a0[i] = mul2(a0[i], pack2(w, w));
+                                a1[i] = mul2(a1[i], pack2(w, w));
+                            }
+                        }
+                    }
+                } else if (!Cfg::TR && listed) {
                     // every row's first chunk is fetched before the first row is summed; further chunks in a loop whose
                     // count is the warp's largest (a row without them reads the chunk of zero rows)
                     uint32_t inf[RPG];
@@ -800,47 +896,46 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 // lane = output feature f, 16 nodes at a time (their scales and tags are broadcast reads); the rows of H are
                 // written 128 bytes per instruction
                 const int f = 32 * q + lane;
-                const float* __restrict__ Xf = p.x + f;
-                const uint32_t piece = (uint32_t)(f >> 2);
-                float* const hcol = reinterpret_cast<float*>(smem + Cfg::OFF_H) + (f & 3);
+                const char* const Xf = reinterpret_cast<const char*>(p.x + f) + (p.tags ? 0 : (int64_t)node0 * Cfg::ROWB);
+                float* const hcol = reinterpret_cast<float*>(smem + Cfg::OFF_H) + f;
                 auto load_x = [&](int r0, float (&x)[16]) {
                     if (r0 >= nrows) return;
-                    if (p.tags) {
-#pragma unroll
-                        for (int i = 0; i < 16; i += 4) {
-                            const uint2 t4 = *reinterpret_cast<const uint2*>(tag_s + r0 + i);
-                            x[i] = __ldg(Xf + (t4.x & 0xffffu) * 128u);
-                            x[i + 1] = __ldg(Xf + (t4.x >> 16) * 128u);
-                            x[i + 2] = __ldg(Xf + (t4.y & 0xffffu) * 128u);
-                            x[i + 3] = __ldg(Xf + (t4.y >> 16) * 128u);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) x[i] = __ldg(Xf + ((int64_t)node0 + (r0 + i < nrows ? r0 + i : nrows - 1)) * 128);
-                    }
-                };
-                float x[16];
-                load_x(32 * jc, x);
-                if (mt > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int g = 0; g < 2 * mt; ++g) {   // 16-node groups of my half of every row block
-                    const int r0 = 64 * (g >> 1) + 32 * jc + 16 * (g & 1);
-                    if (r0 >= nrows) continue;       // warp-uniform
-                    uint32_t v[16];
-                    tc_ld_cols16(tmem_base + Cfg::TM_ACC + ((uint32_t)(32 * q) << 16) + (uint32_t)r0, v);
-                    float y[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) y[i] = x[i];
-                    if (g + 1 < 2 * mt) load_x(64 * ((g + 1) >> 1) + 32 * jc + 16 * ((g + 1) & 1), x);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int i = 0; i < 16; i += 4) {
-                        const float4 c4 = *reinterpret_cast<const float4*>(rsf + r0 + i);
-                        const float c[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            hcol[(r0 + i + u) * 128 + ((piece ^ (uint32_t)((i + u) & 7)) * 4)] = relu_max(fmaf(__uint_as_float(v[i + u]), c[u], y[i + u]));
+                        const uint4 o = *reinterpret_cast<const uint4*>(xo_s + r0 + i);
+                        x[i] = __ldg(reinterpret_cast<const float*>(Xf + o.x));
+                        x[i + 1] = __ldg(reinterpret_cast<const float*>(Xf + o.y));
+                        x[i + 2] = __ldg(reinterpret_cast<const float*>(Xf + o.z));
+                        x[i + 3] = __ldg(reinterpret_cast<const float*>(Xf + o.w));
                     }
+                };
+                float xa[16], xb[16];
+                auto finish = [&](int r0, const float (&x)[16]) {
+                    if (r0 >= nrows) return;   // warp-uniform
+                    uint32_t v[16];
+                    tc_ld_cols16(tmem_base + Cfg::TM_ACC + ((uint32_t)(32 * q) << 16) + (uint32_t)r0, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float* const h = hcol + r0 * 128;
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4) {
+                        const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(rsf + r0 + i);
+                        const float2 lo2 = unpack2(fma2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), c.x, pack2(x[i], x[i + 1])));
+                        const float2 hi2 = unpack2(fma2(pack2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), c.y, pack2(x[i + 2], x[i + 3])));
+                        h[i * 128] = relu_max(lo2.x);
+                        h[(i + 1) * 128] = relu_max(lo2.y);
+                        h[(i + 2) * 128] = relu_max(hi2.x);
+                        h[(i + 3) * 128] = relu_max(hi2.y);
+                    }
+                };
+                const int half = 32 * jc;   // my half of every row block: two groups of 16 nodes
+                load_x(half, xa);
+                if (mt > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int m = 0; m < mt; ++m) {
+                    load_x(64 * m + half + 16, xb);
+                    finish(64 * m + half, xa);
+                    if (m + 1 < mt) load_x(64 * (m + 1) + half, xa);
+                    finish(64 * m + half + 16, xb);
                 }
             } else {
                 constexpr int UNITS = CW / LDC;
@@ -894,7 +989,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         // -------------------------------- node embeddings, pooling --------------------------------
         if (p.embed_out)
             for (int r = grp; r < nrows; r += NG)
-                reinterpret_cast<float4*>(p.embed_out)[(int64_t)(node0 + r) * LPR + sl] = H4[((r << Cfg::SHIFT) + (r & 7)) ^ sl];
+                reinterpret_cast<float4*>(p.embed_out)[(int64_t)(node0 + r) * LPR + sl] = H4[gf_h<D>(r, sl)];
         // Graphs of up to 32 nodes are summed by one warp each; larger ones in pieces of 32 nodes (counted from the
         // graph's first node) by different warps, the partial sums added in order.
         float* const y_s = reinterpret_cast<float*>(smem + Cfg::OFF_S);                       // [Cfg::MAXG][D]
@@ -904,7 +999,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
             for (int n = nb + sub; n < ne; n += GPW) {
-                const float4 v = H4[((n << Cfg::SHIFT) + (n & 7)) ^ sl];
+                const float4 v = H4[gf_h<D>(n, sl)];
                 acc.x = fmaf(wgt, v.x, acc.x); acc.y = fmaf(wgt, v.y, acc.y);
                 acc.z = fmaf(wgt, v.z, acc.z); acc.w = fmaf(wgt, v.w, acc.w);
             }
@@ -1063,8 +1158,9 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
         return a.d == 128 ? gf_map<128>(cap, n, hv).total : (a.d == 64 ? gf_map<64>(cap, n, hv).total : gf_map<32>(cap, n, hv).total);
     };
     const uint32_t budget = per_sm == 2 ? 113 * 1024 : 227 * 1024;
-    const uint32_t left = (budget - total(0)) / 16 * 16, enough = (uint32_t)cap * 8u * 6u;   // six chunks per row are plenty
-    p.chunk_cap = (int)((left < enough ? left : enough) / 8);
+    const uint32_t chunk = a.d == 128 ? GfCfg<128>::CHUNK : 8u;
+    const uint32_t left = (budget - total(0)) / 16 * 16, enough = (uint32_t)cap * chunk * 6u;   // six chunks per row are plenty
+    p.chunk_cap = (int)((left < enough ? left : enough) / chunk);
     const uint32_t smem = total(p.chunk_cap);
     const int64_t most = (int64_t)ctx->sm_count * per_sm;
     const unsigned blocks = (unsigned)(a.G < most ? a.G : most);
