@@ -16,7 +16,7 @@
 //   gather  : d/4 lanes own one node row; they add the neighbour rows in CSR order (fp32), scale the sum by a power of
 //             two taken from its own largest element, split it into an fp16 head and tail and store both as the
 //             K-major MMA operand.  The scale is per row, so a graph's results do not depend on its neighbours in the tile.
-//   product : the warp that finishes last issues tcgen05.mma, A = the 128 rows, B = W^T (head and tail, scaled by its largest element):
+//   product : one warp issues tcgen05.mma, A = the 128 rows, B = W^T (head and tail, scaled by its largest element):
 //             tail*head, head*tail, head*head into one fp32 accumulator in tensor memory.  fp16 head + tail carry 22
 //             bits of every element within 2^-17 of its row's largest one and 2^-39 of that largest one below it: the
 //             TF32 head + tail pair carries the same 22 bits, at twice the operand bytes and half the MMA rate.
@@ -94,7 +94,7 @@ template <int D>
 __host__ __device__ inline GfMap gf_map(int cap, int chunk_cap, bool has_val)
 {
     GfMap m;
-    m.info = GfCfg<D>::OFF_H + (uint32_t)(cap + 1) * GfCfg<D>::ROWB;   // per row: first chunk of columns | chunks << 16
+    m.info = GfCfg<D>::OFF_H + (uint32_t)(cap + 1) * GfCfg<D>::ROWB;   // per row: first chunk of columns | entries << 16
     m.roww = m.info + 4u * (uint32_t)cap;                              // per row: its edge weight
     m.tags = m.roww + (has_val ? 4u * (uint32_t)cap : 0u);
     m.goff = m.tags + gf_up((GfCfg<D>::TR ? 4u : 2u) * (uint32_t)(cap + 1), 16);   // TR: byte offsets of the rows' X, else tags
@@ -497,16 +497,17 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + map.bar + 24);
     uint32_t* s_max = reinterpret_cast<uint32_t*>(smem + map.bar + 28);
     int* s_range = reinterpret_cast<int*>(smem + map.bar + 32);
-    uint32_t* s_arrived = reinterpret_cast<uint32_t*>(smem + map.bar + 40);
     int* s_mixed = reinterpret_cast<int*>(smem + map.bar + 44);
     int* s_scan = reinterpret_cast<int*>(smem + map.bar + 64);   // WARPS totals
-    const uint32_t bar_mma = smem_u32(bars);
+    uint32_t* s_arrived = reinterpret_cast<uint32_t*>(smem + map.bar + 40);
+    const uint32_t bar_mma = smem_u32(bars), bar_full = bar_mma + 8;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb_cta = gridDim.x;
 
     if (threadIdx.x == 0) {
         tc_mbar_init(bar_mma, 1);
+        tc_mbar_init(bar_full, WARPS);
         *abort_flag = 0;
         *s_max = 0;
         *s_arrived = 0;
@@ -637,7 +638,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             const int r = k * WT + threadIdx.x;
             if (r < nrows) {
                 const int c = (rn[k] + 3) >> 2;
-                info_s[r] = c ? (uint32_t)first[k] | ((uint32_t)c << 16) : 0u;
+                info_s[r] = c ? (uint32_t)first[k] | ((uint32_t)(rn[k] < 65535 ? rn[k] : 65535) << 16) : 0u;   // (a listed row is shorter)
                 if (cached)
                     for (int t = 0; t < rn[k]; t += 4) {
                         uint32_t e[4];
@@ -705,7 +706,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                     for (int a = 0; a < 2; ++a) {
                         uint64_t s0 = add2(add2(add2(v[a][0].x, v[a][1].x), v[a][2].x), v[a][3].x);
                         uint64_t s1 = add2(add2(add2(v[a][0].y, v[a][1].y), v[a][2].y), v[a][3].y);
-                        for (uint32_t k = 1; k < (inf[a] >> 16); ++k) {
+                        for (uint32_t k = 1; 4 * k < (inf[a] >> 16); ++k) {
                             const uint4 c = chunks_t[(inf[a] & 0xffffu) + k];
                             const ulonglong2 w0 = table(c.x), w1 = table(c.y), w2 = table(c.z), w3 = table(c.w);
                             s0 = add2(add2(add2(add2(s0, w0.x), w1.x), w2.x), w3.x);
@@ -727,7 +728,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (listed) {
                     const uint32_t inf = info_s[r];
-                    for (uint32_t c = 0; c < (inf >> 16); ++c) {
+                    for (uint32_t c = 0; c < ((inf >> 16) + 3) / 4; ++c) {
                         const uint2 e2 = chunks[(inf & 0xffffu) + c];
                         const uint32_t e[4] = {e2.x & 0xffffu, e2.x >> 16, e2.y & 0xffffu, e2.y >> 16};
                         float4 v[4];
@@ -773,14 +774,20 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                         a0[i] = a1[i] = 0ull;
                         if (i * NG + warp < rows_m) {
                             const uint4 c = chunks_t[inf[i] & 0xffffu];
-                            const ulonglong2 v0 = gf_lds(lane_addr + c.x), v1 = gf_lds(lane_addr + c.y), v2 = gf_lds(lane_addr + c.z), v3 = gf_lds(lane_addr + c.w);
-                            a0[i] = add2(add2(add2(v0.x, v1.x), v2.x), v3.x);
-                            a1[i] = add2(add2(add2(v0.y, v1.y), v2.y), v3.y);
-                            for (uint32_t k = 1; k < (inf[i] >> 16); ++k) {
-                                const uint4 d = chunks_t[(inf[i] & 0xffffu) + k];
-                                const ulonglong2 w0 = gf_lds(lane_addr + d.x), w1 = gf_lds(lane_addr + d.y), w2 = gf_lds(lane_addr + d.z), w3 = gf_lds(lane_addr + d.w);
-                                a0[i] = add2(add2(add2(add2(a0[i], w0.x), w1.x), w2.x), w3.x);
-                                a1[i] = add2(add2(add2(add2(a1[i], w0.y), w1.y), w2.y), w3.y);
+                            const ulonglong2 v0 = gf_lds(lane_addr + c.x), v1 = gf_lds(lane_addr + c.y);
+                            if (inf[i] < 0x30000u) {   // at most two neighbours: the row costs half the shared-memory reads
+                                a0[i] = add2(v0.x, v1.x);
+                                a1[i] = add2(v0.y, v1.y);
+                            } else {
+                                const ulonglong2 v2 = gf_lds(lane_addr + c.z), v3 = gf_lds(lane_addr + c.w);
+                                a0[i] = add2(add2(add2(v0.x, v1.x), v2.x), v3.x);
+                                a1[i] = add2(add2(add2(v0.y, v1.y), v2.y), v3.y);
+                                for (uint32_t k = 1; 4 * k < (inf[i] >> 16); ++k) {
+                                    const uint4 d = chunks_t[(inf[i] & 0xffffu) + k];
+                                    const ulonglong2 w0 = gf_lds(lane_addr + d.x), w1 = gf_lds(lane_addr + d.y), w2 = gf_lds(lane_addr + d.z), w3 = gf_lds(lane_addr + d.w);
+                                    a0[i] = add2(add2(add2(add2(a0[i], w0.x), w1.x), w2.x), w3.x);
+                                    a1[i] = add2(add2(add2(add2(a1[i], w0.y), w1.y), w2.y), w3.y);
+                                }
                             }
                             if (HAS_VAL) {
                                 const float w = roww[RB * m + i * NG + warp];
@@ -803,6 +810,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                     for (int i = 0; i < RPG; ++i) {
                         a0[i] = a1[i] = 0ull;
                         if (i * NG + warp * GPW < rows_m) {   // warp-uniform
+                            auto add_pair = [&](uint32_t e) {
+                                e ^= slx;
+                                const ulonglong2 v0 = H2[e & 0xffffu], v1 = H2[e >> 16];
+                                a0[i] = add2(add2(a0[i], v0.x), v1.x);
+                                a1[i] = add2(add2(a1[i], v0.y), v1.y);
+                            };
                             auto add4 = [&](uint2 e2) {
                                 e2.x ^= slx;
                                 e2.y ^= slx;
@@ -810,9 +823,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                                 a0[i] = add2(add2(add2(add2(a0[i], v0.x), v1.x), v2.x), v3.x);
                                 a1[i] = add2(add2(add2(add2(a1[i], v0.y), v1.y), v2.y), v3.y);
                             };
-                            add4(ef[i]);
                             const uint32_t mine = inf[i] >> 16, most = __reduce_max_sync(0xffffffffu, mine);
-                            for (uint32_t c = 1; c < most; ++c) add4(chunks[c < mine ? (inf[i] & 0xffffu) + c : 0u]);
+                            if (most > 2) add4(ef[i]);
+                            else add_pair(ef[i].x);
+                            uint32_t c = 1;
+                            auto next = [&]() { return chunks[4 * c < mine ? (inf[i] & 0xffffu) + c : 0u]; };
+                            for (; 4 * c + 2 < most; ++c) add4(next());
+                            if (4 * c < most) add_pair(next().x);   // one or two entries are left
                             if (HAS_VAL) {
                                 const float w = i * NG + grp < rows_m ? roww[RB * m + i * NG + grp] : 0.f;
                                 a0[i] = mul2(a0[i], pack2(w, w));
@@ -862,12 +879,20 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // my stores -> visible to the tensor core
                 __syncwarp();
-                // the warp that arrives last issues the products of this row block
-                uint32_t order = 0;
-                if (lane == 0)
-                    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(order) : "r"(smem_u32(s_arrived)) : "memory");
-                order = __shfl_sync(0xffffffffu, order, 0);
-                if (order % WARPS == WARPS - 1) {
+                bool issue;
+                if (Cfg::TR) {
+                    uint32_t order = 0;
+                    if (lane == 0)
+                        asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(order) : "r"(smem_u32(s_arrived)) : "memory");
+                    issue = __shfl_sync(0xffffffffu, order, 0) % WARPS == WARPS - 1;
+                } else {
+                    if (lane == 0) tc_mbar_arrive(bar_full);
+                    issue = (int)(job % WARPS) == warp;
+                }
+                // The products of a row block are issued by the warp that arrives last (d = 128, two CTAs: 3 % better) or by another
+                // warp each time, which waits for the others (one CTA: the counter costs 4 % there).
+                if (issue) {
+                    if (!Cfg::TR) tc_wait(bar_full, job & 1u, abort_flag, p.status, 42);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (lane == 0) {
                         const uint32_t s_addr = smem_u32(smem + Cfg::OFF_S), w_addr = smem_u32(smem + Cfg::OFF_W);
