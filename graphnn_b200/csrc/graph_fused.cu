@@ -499,7 +499,6 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     int* s_range = reinterpret_cast<int*>(smem + map.bar + 32);
     int* s_mixed = reinterpret_cast<int*>(smem + map.bar + 44);
     int* s_scan = reinterpret_cast<int*>(smem + map.bar + 64);   // WARPS totals
-    uint32_t* s_arrived = reinterpret_cast<uint32_t*>(smem + map.bar + 40);
     const uint32_t bar_mma = smem_u32(bars), bar_full = bar_mma + 8;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -510,7 +509,6 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         tc_mbar_init(bar_full, WARPS);
         *abort_flag = 0;
         *s_max = 0;
-        *s_arrived = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -879,33 +877,23 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // my stores -> visible to the tensor core
                 __syncwarp();
-                bool issue;
-                if (Cfg::TR) {
-                    uint32_t order = 0;
-                    if (lane == 0)
-                        asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(order) : "r"(smem_u32(s_arrived)) : "memory");
-                    issue = __shfl_sync(0xffffffffu, order, 0) % WARPS == WARPS - 1;
-                } else {
-                    if (lane == 0) tc_mbar_arrive(bar_full);
-                    issue = (int)(job % WARPS) == warp;
-                }
-                // The products of a row block are issued by the warp that arrives last (d = 128, two CTAs: 3 % better) or by another
-                // warp each time, which waits for the others (one CTA: the counter costs 4 % there).
-                if (issue) {
-                    if (!Cfg::TR) tc_wait(bar_full, job & 1u, abort_flag, p.status, 42);
+                if (lane == 0) tc_mbar_arrive(bar_full);
+                // one of the warps, another one for each row block, waits for all of them and issues the products
+                if ((int)(job % WARPS) == warp) {
+                    tc_wait(bar_full, job & 1u, abort_flag, p.status, 42);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (lane == 0) {
-                        const uint32_t s_addr = smem_u32(smem + Cfg::OFF_S), w_addr = smem_u32(smem + Cfg::OFF_W);
+                    if (tc_elect()) {
+                        const uint64_t s_desc = tc_b_desc(smem_u32(smem + Cfg::OFF_S)), w_desc = tc_b_desc(smem_u32(smem + Cfg::OFF_W));
                         const uint32_t acc = tmem_base + (Cfg::TR ? Cfg::TM_ACC + (uint32_t)(m * RB) : (uint32_t)(m * D));
 #pragma unroll
                         for (int pass = 0; pass < 3; ++pass) {   // tail*head, head*tail, head*head: small terms first
-                            const uint32_t s_base = s_addr + (pass == 0 ? Cfg::S_LO : 0u), w_base = w_addr + (pass == 1 ? Cfg::W_LO : 0u);
+                            const uint32_t s_off = pass == 0 ? Cfg::S_LO : 0u, w_off = pass == 1 ? Cfg::W_LO : 0u;
 #pragma unroll
                             for (int ks = 0; ks < D / 16; ++ks) {
                                 const uint32_t so = (uint32_t)(ks >> 2) * (uint32_t)(RB * 128) + (uint32_t)(ks & 3) * 32u;
                                 const uint32_t wo = (uint32_t)(ks >> 2) * (uint32_t)(D * 128) + (uint32_t)(ks & 3) * 32u;
-                                if (Cfg::TR) mma_f16_ts(acc, tmem_base + (pass == 1 ? Cfg::TM_WLO : 0u) + 8u * ks, tc_b_desc(s_base + so), Cfg::IDESC, (pass | ks) != 0);
-                                else mma_f16_ss(acc, tc_b_desc(s_base + so), tc_b_desc(w_base + wo), Cfg::IDESC, (pass | ks) != 0);
+                                if (Cfg::TR) mma_f16_ts(acc, tmem_base + (pass == 1 ? Cfg::TM_WLO : 0u) + 8u * ks, s_desc + ((s_off + so) >> 4), Cfg::IDESC, (pass | ks) != 0);
+                                else mma_f16_ss(acc, s_desc + ((s_off + so) >> 4), w_desc + ((w_off + wo) >> 4), Cfg::IDESC, (pass | ks) != 0);
                             }
                         }
                         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_mma) : "memory");

@@ -522,7 +522,7 @@ s2v_level_tc_kernel(int64_t n_rows, int64_t num_tiles, const int32_t* __restrict
             if (ok && it >= 2) ok = tc_wait(bar(BAR_DFREE0 + b), (uint32_t)(((it - 2) >> 1) & 1), abort_flag, status, 23);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
+            if (tc_elect()) {
                 const uint32_t d_tmem = TM_ACC + (uint32_t)(D * b);
                 const uint32_t bhi = smem_u32(Bhi), blo = smem_u32(Blo);
                 uint32_t accumulate = 0;

@@ -149,7 +149,7 @@ readout_tc_kernel(int64_t G, int d, int C, const float* __restrict__ Y, const fl
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (threadIdx.x == 0) {
+            if (warp == 0 && tc_elect()) {
                 const uint32_t ahi = smem_u32(smem + Cfg::OFF_AHI), alo = smem_u32(smem + Cfg::OFF_ALO);
                 const uint32_t bhi = smem_u32(smem + Cfg::OFF_BHI), blo = smem_u32(smem + Cfg::OFF_BLO);
                 uint32_t accumulate = kh > 0 ? 1u : 0u;
