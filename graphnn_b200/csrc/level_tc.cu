@@ -131,19 +131,12 @@ s2v_level_tc_kernel(int64_t n_rows, int64_t num_tiles, const int32_t* __restrict
         constexpr int NTASK = D * D / 4;
         constexpr int PER = (NTASK + TC_THREADS - 1) / TC_THREADS;
         float wv[PER][4];
-        auto load_w = [&]() {
 #pragma unroll
-            for (int t = 0; t < PER; ++t) {
-                const int e = threadIdx.x + t * TC_THREADS;
-                const int n = e % D, kq = e / D;   // k = 4*kq .. 4*kq+3
+        for (int t = 0; t < PER; ++t) {
+            const int e = threadIdx.x + t * TC_THREADS;
+            const int n = e % D, kq = e / D;   // k = 4*kq .. 4*kq+3
 #pragma unroll
-                for (int jj = 0; jj < 4; ++jj) wv[t][jj] = (e < NTASK) ? __ldg(W + (int64_t)(4 * kq + jj) * D + n) : 0.f;
-            }
-        };
-        load_w();
-        if (LONG && __syncthreads_or(look.any(n_rows, row_ptr))) {
-            sum_long_rows<D, TC_THREADS, TC_TILE, TC_ROWS_PER_GW, (int)Cfg::OFF_GW, HAS_VAL>(smem, n_rows, row_ptr, col_idx, val, H, out);
-            load_w();   // (again: kept across the call they would be spilled in every launch)
+            for (int jj = 0; jj < 4; ++jj) wv[t][jj] = (e < NTASK) ? __ldg(W + (int64_t)(4 * kq + jj) * D + n) : 0.f;
         }
 #pragma unroll
         for (int t = 0; t < PER; ++t) {
@@ -165,7 +158,10 @@ s2v_level_tc_kernel(int64_t n_rows, int64_t num_tiles, const int32_t* __restrict
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    if (!LONG) __syncthreads();
+    else if (__syncthreads_or(look.any(n_rows, row_ptr)))   // (the offsets have arrived meanwhile; buffers in the staging tile's place)
+        sum_long_rows<D, TC_THREADS, TC_TILE, TC_ROWS_PER_GW, (int)(Cfg::OFF_BAR - Cfg::OFF_STAGE), HAS_VAL>(smem + Cfg::OFF_STAGE, n_rows, row_ptr, col_idx,
+                                                                                                             val, H, out);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t TM_AHI = tmem_base + Cfg::TM_AHI, TM_ACC = tmem_base + Cfg::TM_ACC;

@@ -17,8 +17,8 @@ namespace
 {
 
 constexpr int LONG_ROW = 256;      // below this a row is no longer than what the other warps of a tile work on
-constexpr int LONG_BIG = 2048;
-constexpr int LONG_LOOK = 4;       // rows per thread that are looked at ahead
+constexpr int LONG_BIG = 2048;      // above this a row is worth the whole CTA
+constexpr int LONG_LOOK = 14;      // rows per thread that are looked at together (a million rows on 148 CTAs)
 constexpr int LONG_SCAN = 8;       // rows per thread and pass of the sums
 
 template <int W> struct LongVec;
@@ -131,29 +131,39 @@ __device__ __forceinline__ int long_rows_owned(int64_t n_rows)
     return blocks > blockIdx.x ? (int)((blocks - 1 - blockIdx.x) / gridDim.x + 1) * RB : 0;
 }
 
-// Whether a row of this thread's share of the CTA's rows is long.  load() only issues the first loads.
+// Whether a row of this thread's share of the CTA's rows is long.  load() only issues the first loads: one offset per row, the
+// next row's comes from the neighbouring lane (or, at the end of a run, from a load of its own).
 template <int THREADS, int RB, typename RpT>
 struct LongLook {
+    static constexpr int RUN = RB < 32 ? RB : 32;
+    static_assert(32 % RUN == 0 && RB % RUN == 0 && THREADS % 32 == 0, "a warp looks at whole runs of consecutive rows");
     RpT a[LONG_LOOK], z[LONG_LOOK];
     __device__ __forceinline__ void load(int64_t n_rows, const RpT* __restrict__ row_ptr, int j0 = 0)
     {
         const int owned = long_rows_owned<RB>(n_rows);
+        const bool last = threadIdx.x % RUN == RUN - 1;
 #pragma unroll
         for (int k = 0; k < LONG_LOOK; ++k) {
             const int j = j0 + k * THREADS + threadIdx.x;
             const int64_t r = long_row_of<RB>(j);
-            const bool in = j < owned && r < n_rows;
-            a[k] = in ? __ldg(row_ptr + r) : (RpT)0;
-            z[k] = in ? __ldg(row_ptr + r + 1) : (RpT)0;
+            a[k] = z[k] = 0;
+            if (j < owned) {   // (rows past the end: no entries)
+                a[k] = __ldg(row_ptr + (r < n_rows ? r : n_rows));
+                if (last) z[k] = __ldg(row_ptr + (r + 1 < n_rows ? r + 1 : n_rows));
+            }
         }
     }
     __device__ __forceinline__ bool any(int64_t n_rows, const RpT* __restrict__ row_ptr)
     {
         bool found = false;
         const int owned = long_rows_owned<RB>(n_rows);
+        const bool last = threadIdx.x % RUN == RUN - 1;
         for (int j0 = 0;;) {
 #pragma unroll
-            for (int k = 0; k < LONG_LOOK; ++k) found |= z[k] - a[k] > LONG_ROW;
+            for (int k = 0; k < LONG_LOOK; ++k) {
+                const RpT next = __shfl_down_sync(0xffffffffu, a[k], 1);
+                found |= (last ? z[k] : next) - a[k] > LONG_ROW;
+            }
             j0 += THREADS * LONG_LOOK;
             if (j0 >= owned) return found;
             load(n_rows, row_ptr, j0);
@@ -188,11 +198,13 @@ __device__ __noinline__ void sum_long_rows(unsigned char* smem, int64_t n_rows, 
         }
         __syncthreads();
         const int n = cnt[0];
+        // fewer groups than warps: the whole CTA on every long row, or most of its warps would look on
+        const int big = n * SLICES < THREADS / 32 ? LONG_ROW : LONG_BIG;
         for (int i = 0; i < n; ++i) {   // the longest rows
             const int64_t r0 = long_row_of<RB>(j0 + list[i] * GROUP);
             for (int64_t r = r0; r < r0 + GROUP && r < n_rows; ++r) {
                 const int64_t b = __ldg(row_ptr + r), len = __ldg(row_ptr + r + 1) - b;
-                if (len > LONG_BIG)
+                if (len > big)
                     long_row_by_cta<D, THREADS, BYTES - RING, HAS_VAL>(smem + RING, H, col_idx + b, HAS_VAL ? val + b : nullptr, (int)len, out + r * D);
             }
         }
@@ -210,7 +222,7 @@ __device__ __noinline__ void sum_long_rows(unsigned char* smem, int64_t n_rows, 
             for (int k = 0; k < GROUP; ++k) {
                 const int64_t en = __shfl_sync(0xffffffffu, rp, k + 2 <= GROUP ? k + 2 : GROUP);
                 const int cn = e + lane < en ? __ldg(col_idx + e + lane) : 0;   // the next row's first indices
-                if (r0 + k < n_rows && e - b <= LONG_BIG)
+                if (r0 + k < n_rows && e - b <= big)
                     long_row_by_warp<D, SL, HAS_VAL>(H + c0, col_idx + b, HAS_VAL ? val + b : nullptr, (int)(e - b), c, out + (r0 + k) * D + c0);
                 b = e;
                 e = en;

@@ -56,6 +56,46 @@ __global__ void __launch_bounds__(256) input_proj_dense_kernel(int64_t n, int F,
     }
 }
 
+// The same for the widths of the path, d = 4 * LPR: a CTA takes RPB rows at a time, their attributes come through shared
+// memory (whole lines instead of one broadcast load per row and k), and a thread owns four columns of four rows: five
+// shared reads for sixteen FMAs.  k ascending, so the sums are those of the kernel above.
+template <int LPR>
+__global__ void __launch_bounds__(256) input_proj_dense_v4_kernel(int64_t n, int F, const float* __restrict__ X, const float4* __restrict__ W_in,
+                                                                   float4* __restrict__ msg, float4* __restrict__ h0)
+{
+    constexpr int R = 4, RPP = 256 / LPR, RPB = RPP * R;
+    extern __shared__ __align__(16) float pd_sm[];
+    float4* const Ws = reinterpret_cast<float4*>(pd_sm);     // [F][LPR]
+    float* const Xs = pd_sm + 4 * F * LPR;                   // [RPB][F]
+    for (int e = threadIdx.x; e < F * LPR; e += 256) Ws[e] = __ldg(W_in + e);
+    const int sl = threadIdx.x % LPR, row = threadIdx.x / LPR;
+    for (int64_t r0 = (int64_t)blockIdx.x * RPB; r0 < n; r0 += (int64_t)gridDim.x * RPB) {
+        const int rows = (int)(n - r0 < RPB ? n - r0 : RPB);
+        __syncthreads();
+        for (int e = threadIdx.x; e < rows * F; e += 256) Xs[e] = __ldcs(X + r0 * F + e);
+        __syncthreads();
+        float4 acc[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < F; ++k) {
+            const float4 w = Ws[k * LPR + sl];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const float x = Xs[(row + i * RPP) * F + k];   // (rows past the end: whatever lies there, never stored)
+                acc[i].x = fmaf(x, w.x, acc[i].x); acc[i].y = fmaf(x, w.y, acc[i].y);
+                acc[i].z = fmaf(x, w.z, acc[i].z); acc[i].w = fmaf(x, w.w, acc[i].w);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = row + i * RPP;
+            if (r >= rows) continue;
+            if (msg) msg[(r0 + r) * LPR + sl] = acc[i];
+            if (h0) h0[(r0 + r) * LPR + sl] = make_float4(relu_ref(acc[i].x), relu_ref(acc[i].y), relu_ref(acc[i].z), relu_ref(acc[i].w));
+        }
+    }
+}
+
 // ---------------------------------------------------------------- segmented sum
 // Y[g,:] = sum_{n in [seg[g], seg[g+1])} H[n,:].  One warp per graph; d/4 lanes cover a
 // node row with float4, 32/(d/4) node rows are summed side by side and combined with
@@ -405,6 +445,17 @@ int s2v_input_proj_dense_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n, int num
     if (!X || !W_in || (!msg && !h0)) return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "input_proj: NULL pointer");
     const size_t smem = sizeof(float) * (size_t)num_feat * d;
     if (smem > 200 * 1024) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "input_proj_dense: W_in beyond 200 KB; use s2v_gemm_f32");
+    const int lpr = d / 4;
+    const size_t smem_v4 = sizeof(float) * (size_t)num_feat * ((size_t)d + (lpr > 0 ? 1024 / lpr : 0));
+    if ((d == 32 || d == 64 || d == 128) && smem_v4 <= 96 * 1024 && s2v_aligned16(W_in) && s2v_aligned16(msg) && s2v_aligned16(h0)) {
+        auto kern = d == 32 ? input_proj_dense_v4_kernel<8> : (d == 64 ? input_proj_dense_v4_kernel<16> : input_proj_dense_v4_kernel<32>);
+        const int64_t rows = 1024 / lpr;
+        S2V_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_v4));
+        kern<<<grid_cap(ctx, (n + rows - 1) / rows, 6), 256, smem_v4, s2v_pick_stream(ctx, stream)>>>(
+            n, num_feat, X, reinterpret_cast<const float4*>(W_in), reinterpret_cast<float4*>(msg), reinterpret_cast<float4*>(h0));
+        S2V_CHECK_LAUNCH(ctx, "input_proj_dense_v4_kernel");
+        return S2V_OK;
+    }
     S2V_CUDA_OK(ctx, cudaFuncSetAttribute(input_proj_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     input_proj_dense_kernel<<<grid_cap(ctx, (n + 7) / 8, 4), 256, smem, s2v_pick_stream(ctx, stream)>>>(n, num_feat, d, X,
                                                                                                           W_in, msg, h0);
