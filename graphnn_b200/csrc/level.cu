@@ -134,8 +134,8 @@ s2v_level_kernel(bool long_rows, int64_t n_rows, int64_t num_tiles, const RpT* _
             bulk_copy_g2s(smem_u32(Ws + k * W_STRIDE), W + k * D, (uint32_t)(sizeof(float) * D), bar);
     }
     LongLook<WARPS * 32, TILE_R, RpT> look;   // rows of hubs are looked for while W is on its way
-    look.load(n_rows, row_ptr);
-    if (__syncthreads_or(look.any(n_rows, row_ptr)) && long_rows)   // (the barrier is initialised before anyone polls it)
+    if (long_rows) look.load(n_rows, row_ptr);
+    if (__syncthreads_or(long_rows && look.any(n_rows, row_ptr)))   // (the barrier is initialised before anyone polls it)
         sum_long_rows<D, WARPS * 32, TILE_R, TILE_R, (int)(LevelSmem<D>::WARP_BYTES * WARPS), HAS_VAL>(smem_raw + LevelSmem<D>::W_BYTES + 16, n_rows, row_ptr,
                                                                                                        col_idx, val, H, out);
     {
@@ -372,7 +372,9 @@ int launch_one(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, co
     }
     const int64_t num_tiles = (n_rows + TILE_R - 1) / TILE_R;
     const int64_t persistent = (int64_t)ctx->sm_count * resident;
-    const int64_t blocks = num_tiles < persistent ? num_tiles : persistent;
+    int64_t blocks = (num_tiles + WARPS - 1) / WARPS;   // every SM gets a CTA before a CTA's warps all get a tile
+    if (blocks < ctx->sm_count) blocks = num_tiles < ctx->sm_count ? num_tiles : ctx->sm_count;
+    if (blocks > persistent) blocks = persistent;
     kern<<<(unsigned)blocks, WARPS * 32, smem, st>>>(long_rows, n_rows, num_tiles, row_ptr, col_idx, val, H, W, X, x_index, n_table, out,
                                                       ctx->dstatus_dev);
     S2V_CHECK_LAUNCH(ctx, "s2v_level_kernel");

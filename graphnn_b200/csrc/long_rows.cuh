@@ -18,7 +18,6 @@ namespace
 
 constexpr int LONG_ROW = 256;      // below this a row is no longer than what the other warps of a tile work on
 constexpr int LONG_BIG = 2048;      // above this a row is worth the whole CTA
-constexpr int LONG_LOOK = 14;      // rows per thread that are looked at together (a million rows on 148 CTAs)
 constexpr int LONG_SCAN = 8;       // rows per thread and pass of the sums
 
 template <int W> struct LongVec;
@@ -131,42 +130,48 @@ __device__ __forceinline__ int long_rows_owned(int64_t n_rows)
     return blocks > blockIdx.x ? (int)((blocks - 1 - blockIdx.x) / gridDim.x + 1) * RB : 0;
 }
 
-// Whether a row of this thread's share of the CTA's rows is long.  load() only issues the first loads: one offset per row, the
-// next row's comes from the neighbouring lane (or, at the end of a run, from a load of its own).
+// Whether one of the CTA's row blocks holds a long row.  Warp w looks at blocks w, w + WARPS, ... of the CTA, AHEAD of them at a
+// time; load() only issues the first loads, one offset per row.  (No division: with 64-bit ones the look took 2 us.)
 template <int THREADS, int RB, typename RpT>
 struct LongLook {
-    static constexpr int RUN = RB < 32 ? RB : 32;
-    static_assert(32 % RUN == 0 && RB % RUN == 0 && THREADS % 32 == 0, "a warp looks at whole runs of consecutive rows");
-    RpT a[LONG_LOOK], z[LONG_LOOK];
-    __device__ __forceinline__ void load(int64_t n_rows, const RpT* __restrict__ row_ptr, int j0 = 0)
+    static constexpr int WARPS = THREADS / 32, K = RB >= 32 ? RB / 32 : 1, AHEAD = RB >= 32 ? 4 : 8;
+    static_assert(RB % 32 == 0 || RB < 32, "whole warp loads, or one");
+    RpT a[AHEAD][K], end[AHEAD];
+    __device__ __forceinline__ void load(int64_t n_rows, const RpT* __restrict__ row_ptr, int t0 = 0)
     {
-        const int owned = long_rows_owned<RB>(n_rows);
-        const bool last = threadIdx.x % RUN == RUN - 1;
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-        for (int k = 0; k < LONG_LOOK; ++k) {
-            const int j = j0 + k * THREADS + threadIdx.x;
-            const int64_t r = long_row_of<RB>(j);
-            a[k] = z[k] = 0;
-            if (j < owned) {   // (rows past the end: no entries)
-                a[k] = __ldg(row_ptr + (r < n_rows ? r : n_rows));
-                if (last) z[k] = __ldg(row_ptr + (r + 1 < n_rows ? r + 1 : n_rows));
+        for (int b = 0; b < AHEAD; ++b) {
+            const int64_t r0 = ((int64_t)(t0 + b * WARPS + warp) * gridDim.x + blockIdx.x) * RB;
+            end[b] = 0;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int64_t r = r0 + 32 * k + lane;
+                a[b][k] = 0;
+                if (r0 < n_rows && (RB >= 32 || lane <= RB)) a[b][k] = __ldg(row_ptr + (r < n_rows ? r : n_rows));
             }
+            if (RB >= 32 && r0 < n_rows && lane == 31) end[b] = __ldg(row_ptr + (r0 + RB < n_rows ? r0 + RB : n_rows));
         }
     }
     __device__ __forceinline__ bool any(int64_t n_rows, const RpT* __restrict__ row_ptr)
     {
+        const int lane = threadIdx.x & 31;
         bool found = false;
-        const int owned = long_rows_owned<RB>(n_rows);
-        const bool last = threadIdx.x % RUN == RUN - 1;
-        for (int j0 = 0;;) {
+        for (int t0 = 0;;) {
 #pragma unroll
-            for (int k = 0; k < LONG_LOOK; ++k) {
-                const RpT next = __shfl_down_sync(0xffffffffu, a[k], 1);
-                found |= (last ? z[k] : next) - a[k] > LONG_ROW;
-            }
-            j0 += THREADS * LONG_LOOK;
-            if (j0 >= owned) return found;
-            load(n_rows, row_ptr, j0);
+            for (int b = 0; b < AHEAD; ++b)
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    RpT next = __shfl_down_sync(0xffffffffu, a[b][k], 1);
+                    if (RB >= 32) {
+                        const RpT wrap = k + 1 < K ? __shfl_sync(0xffffffffu, a[b][k + 1 < K ? k + 1 : 0], 0) : end[b];
+                        if (lane == 31) next = wrap;
+                    }
+                    found |= (RB >= 32 || lane < RB) && next - a[b][k] > LONG_ROW;
+                }
+            t0 += WARPS * AHEAD;
+            if (((int64_t)t0 * gridDim.x + blockIdx.x) * RB >= n_rows) return found;
+            load(n_rows, row_ptr, t0);
         }
     }
 };
