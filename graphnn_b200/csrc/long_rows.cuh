@@ -130,48 +130,41 @@ __device__ __forceinline__ int long_rows_owned(int64_t n_rows)
     return blocks > blockIdx.x ? (int)((blocks - 1 - blockIdx.x) / gridDim.x + 1) * RB : 0;
 }
 
-// Whether one of the CTA's row blocks holds a long row.  Warp w looks at blocks w, w + WARPS, ... of the CTA, AHEAD of them at a
-// time; load() only issues the first loads, one offset per row.  (No division: with 64-bit ones the look took 2 us.)
+// Whether the CTA owns a long row.  A thread takes STEP consecutive rows at a time and looks at each of them only if they have more
+// than LONG_ROW entries together.  load() issues the first loads; what they bring is looked at after the conversion of W.  The look is
+// bounded by its own instructions, fetched and run once: with a load and a shuffle per row it took 2 us of every level.
 template <int THREADS, int RB, typename RpT>
 struct LongLook {
-    static constexpr int WARPS = THREADS / 32, K = RB >= 32 ? RB / 32 : 1, AHEAD = RB >= 32 ? 4 : 8;
-    static_assert(RB % 32 == 0 || RB < 32, "whole warp loads, or one");
-    RpT a[AHEAD][K], end[AHEAD];
-    __device__ __forceinline__ void load(int64_t n_rows, const RpT* __restrict__ row_ptr, int t0 = 0)
+    static constexpr int STEP = 8, PER = RB / STEP, AHEAD = 2;
+    static_assert(RB % STEP == 0 && THREADS % PER == 0, "whole groups, whole blocks");
+    RpT a[AHEAD], z[AHEAD];
+    static __device__ __forceinline__ int64_t row_of(int j) { return ((int64_t)(j / PER) * gridDim.x + blockIdx.x) * RB + j % PER * STEP; }
+    __device__ __forceinline__ void load(int64_t n_rows, const RpT* __restrict__ row_ptr, int j0 = 0)
     {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-        for (int b = 0; b < AHEAD; ++b) {
-            const int64_t r0 = ((int64_t)(t0 + b * WARPS + warp) * gridDim.x + blockIdx.x) * RB;
-            end[b] = 0;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const int64_t r = r0 + 32 * k + lane;
-                a[b][k] = 0;
-                if (r0 < n_rows && (RB >= 32 || lane <= RB)) a[b][k] = __ldg(row_ptr + (r < n_rows ? r : n_rows));
+        for (int k = 0; k < AHEAD; ++k) {
+            const int64_t r = row_of(j0 + k * THREADS + (int)threadIdx.x);
+            a[k] = z[k] = 0;
+            if (r < n_rows) {
+                a[k] = __ldg(row_ptr + r);
+                z[k] = __ldg(row_ptr + (r + STEP < n_rows ? r + STEP : n_rows));
             }
-            if (RB >= 32 && r0 < n_rows && lane == 31) end[b] = __ldg(row_ptr + (r0 + RB < n_rows ? r0 + RB : n_rows));
         }
     }
     __device__ __forceinline__ bool any(int64_t n_rows, const RpT* __restrict__ row_ptr)
     {
-        const int lane = threadIdx.x & 31;
         bool found = false;
-        for (int t0 = 0;;) {
+        for (int j0 = 0;;) {
 #pragma unroll
-            for (int b = 0; b < AHEAD; ++b)
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    RpT next = __shfl_down_sync(0xffffffffu, a[b][k], 1);
-                    if (RB >= 32) {
-                        const RpT wrap = k + 1 < K ? __shfl_sync(0xffffffffu, a[b][k + 1 < K ? k + 1 : 0], 0) : end[b];
-                        if (lane == 31) next = wrap;
-                    }
-                    found |= (RB >= 32 || lane < RB) && next - a[b][k] > LONG_ROW;
+            for (int k = 0; k < AHEAD; ++k)
+                if (z[k] - a[k] > LONG_ROW) {
+                    const int64_t r0 = row_of(j0 + k * THREADS + (int)threadIdx.x), r1 = r0 + STEP < n_rows ? r0 + STEP : n_rows;
+#pragma unroll 1
+                    for (int64_t r = r0; r < r1; ++r) found |= __ldg(row_ptr + r + 1) - __ldg(row_ptr + r) > LONG_ROW;
                 }
-            t0 += WARPS * AHEAD;
-            if (((int64_t)t0 * gridDim.x + blockIdx.x) * RB >= n_rows) return found;
-            load(n_rows, row_ptr, t0);
+            j0 += THREADS * AHEAD;
+            if (row_of(j0) >= n_rows) return found;
+            load(n_rows, row_ptr, j0);
         }
     }
 };
