@@ -94,9 +94,9 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
                  : "memory");
 }
 
-template <int D, typename RpT, bool HAS_VAL, int XMODE /*0 none, 1 dense, 2 table lookup*/>
+template <int D, typename RpT, bool HAS_VAL, int XMODE /*0 none, 1 dense, 2 table lookup*/, bool LONG>
 __global__ void __launch_bounds__(LevelCfg<D>::WARPS * 32, LevelCfg<D>::MIN_BLOCKS)
-s2v_level_kernel(bool long_rows, int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_ptr,
+s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_ptr,
                  const int32_t* __restrict__ col_idx, const float* __restrict__ val, const float* __restrict__ H,
                  const float* __restrict__ W, const float* __restrict__ X, const int32_t* __restrict__ x_index,
                  int n_table, float* __restrict__ out, s2v_device_status* status)
@@ -133,11 +133,7 @@ s2v_level_kernel(bool long_rows, int64_t n_rows, int64_t num_tiles, const RpT* _
         for (int k = lane; k < D; k += 32)  // one bulk copy per row of W, into the padded layout
             bulk_copy_g2s(smem_u32(Ws + k * W_STRIDE), W + k * D, (uint32_t)(sizeof(float) * D), bar);
     }
-    LongLook<WARPS * 32, TILE_R, RpT> look;   // rows of hubs are looked for while W is on its way
-    if (long_rows) look.load(n_rows, row_ptr);
-    if (__syncthreads_or(long_rows && look.any(n_rows, row_ptr)))   // (the barrier is initialised before anyone polls it)
-        sum_long_rows<D, WARPS * 32, TILE_R, TILE_R, (int)(LevelSmem<D>::WARP_BYTES * WARPS), HAS_VAL>(smem_raw + LevelSmem<D>::W_BYTES + 16, n_rows, row_ptr,
-                                                                                                       col_idx, val, H, out);
+    __syncthreads();  // barrier initialised before anyone polls it
     {
         int spins = 0;
         while (!mbar_try_wait(bar, 0)) {
@@ -157,8 +153,11 @@ s2v_level_kernel(bool long_rows, int64_t n_rows, int64_t num_tiles, const RpT* _
     const int sub = lane / LPR, sl = lane % LPR;
     const int g = lane >> 2, tig = lane & 3;   // MMA fragment coordinates
 
-    // (tiles go to the CTAs first and to a CTA's warps second: a small batch uses every SM)
-    for (int64_t tile = (int64_t)warp * gridDim.x + blockIdx.x; tile < num_tiles; tile += (int64_t)gridDim.x * WARPS) {
+    // Tiles with a long row are passed over at first; if the CTA met one, all its warps sum the long rows (long_rows.cuh) and a second
+    // pass takes those tiles.  (A look through the offsets in front cost 2 of 25 us, and its registers spilled.)
+    bool found = false;
+    for (int pass = 0;; ++pass) {
+    for (int64_t tile = (int64_t)blockIdx.x * WARPS + warp; tile < num_tiles; tile += (int64_t)gridDim.x * WARPS) {
         const int64_t r0 = tile * TILE_R;
         // ---- 1. row offsets (relative to the tile's first non-zero) and the tile's indices
         int64_t rpi = r0 + lane;
@@ -167,6 +166,12 @@ s2v_level_kernel(bool long_rows, int64_t n_rows, int64_t num_tiles, const RpT* _
         const RpT base = __shfl_sync(0xffffffffu, rp_abs, 0);
         const int rp_rel = (int)(rp_abs - base);
         const int tile_nnz = __shfl_sync(0xffffffffu, rp_rel, TILE_R);
+        if (LONG) {
+            const int row_len = __shfl_down_sync(0xffffffffu, rp_rel, 1) - rp_rel;
+            const bool has_long = __any_sync(0xffffffffu, lane < TILE_R && row_len > LONG_ROW);
+            found |= has_long;
+            if (has_long != (pass == 1)) continue;
+        }
         if (lane <= TILE_R) rp_s[lane] = rp_rel;
         const bool fits = tile_nnz <= IDX_CAP;   // warp-uniform; almost always true
         if (fits) {
@@ -185,9 +190,8 @@ s2v_level_kernel(bool long_rows, int64_t n_rows, int64_t num_tiles, const RpT* _
         //   RPS consecutive rows as ONE stream, U loads in flight whatever the row lengths; a
         //   row's sum is flushed to the shared tile when the stream crosses its end.
         //   Otherwise: one row per lane group per pass, chunks of U neighbours.
-        //   A tile with a long row has all its sums already (long_rows.cuh).
-        const int row_len = __shfl_down_sync(0xffffffffu, rp_rel, 1) - rp_rel;
-        if (__any_sync(0xffffffffu, lane < TILE_R && row_len > LONG_ROW) && long_rows) {
+        //   In the second pass the sums lie in `out` already.
+        if (LONG && pass == 1) {
 #pragma unroll 1
             for (int lr = sub; lr < TILE_R; lr += RPP)
                 if (r0 + lr < n_rows)
@@ -351,15 +355,19 @@ s2v_level_kernel(bool long_rows, int64_t n_rows, int64_t num_tiles, const RpT* _
         }
         __syncwarp();  // S and idx_s are rewritten by the next tile
     }
+    if (!LONG || pass == 1 || !__syncthreads_or(found)) break;
+    sum_long_rows<D, WARPS * 32, WARPS * TILE_R, TILE_R, (int)(LevelSmem<D>::WARP_BYTES * WARPS), HAS_VAL>(smem_raw + LevelSmem<D>::W_BYTES + 16, n_rows,
+                                                                                                           row_ptr, col_idx, val, H, out);
+    }
 }
 
-template <int D, typename RpT, bool HAS_VAL, int XMODE>
-int launch_one(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx,
+template <int D, typename RpT, bool HAS_VAL, int XMODE, bool LONG>
+int launch_one(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx,
                const float* val, const float* H, const float* W, const float* X, const int32_t* x_index, int n_table,
                float* out)
 {
     constexpr int WARPS = LevelCfg<D>::WARPS;
-    auto kern = s2v_level_kernel<D, RpT, HAS_VAL, XMODE>;
+    auto kern = s2v_level_kernel<D, RpT, HAS_VAL, XMODE, LONG>;
     const size_t smem = LevelSmem<D>::total(WARPS);
     // Opt-in shared memory size: a per-function attribute, cheap to set on every call.
     S2V_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -372,10 +380,9 @@ int launch_one(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, co
     }
     const int64_t num_tiles = (n_rows + TILE_R - 1) / TILE_R;
     const int64_t persistent = (int64_t)ctx->sm_count * resident;
-    int64_t blocks = (num_tiles + WARPS - 1) / WARPS;   // every SM gets a CTA before a CTA's warps all get a tile
-    if (blocks < ctx->sm_count) blocks = num_tiles < ctx->sm_count ? num_tiles : ctx->sm_count;
+    int64_t blocks = (num_tiles + WARPS - 1) / WARPS;
     if (blocks > persistent) blocks = persistent;
-    kern<<<(unsigned)blocks, WARPS * 32, smem, st>>>(long_rows, n_rows, num_tiles, row_ptr, col_idx, val, H, W, X, x_index, n_table, out,
+    kern<<<(unsigned)blocks, WARPS * 32, smem, st>>>(n_rows, num_tiles, row_ptr, col_idx, val, H, W, X, x_index, n_table, out,
                                                       ctx->dstatus_dev);
     S2V_CHECK_LAUNCH(ctx, "s2v_level_kernel");
     return S2V_OK;
@@ -388,7 +395,9 @@ int launch_d(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, cons
 {
     const int xmode = table ? 2 : (X ? 1 : 0);
     const float* xa = table ? table : X;
-#define S2V_LVL(HV, XM) return launch_one<D, RpT, HV, XM>(ctx, st, long_rows, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)
+#define S2V_LVL(HV, XM)                                                                                                       \
+    return long_rows ? launch_one<D, RpT, HV, XM, true>(ctx, st, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)        \
+                     : launch_one<D, RpT, HV, XM, false>(ctx, st, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)
     if (val) {
         if (xmode == 0) S2V_LVL(true, 0);
         if (xmode == 1) S2V_LVL(true, 1);
