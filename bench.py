@@ -251,8 +251,6 @@ class ClassifierStep:
     device buffers, followed -- on several GPUs -- by the gather of the logits; `profile()` runs the same kernels
     composed from the library's operators so that each launch can be bracketed by CUDA events on its stream."""
 
-    TILE_AUTO_MAX_NODES = 160000     # the library's automatic mode takes the tile kernel up to this many nodes
-
     def __init__(self, torch, eng, batch, stream, gather=None, use_tiles=2):
         from graphnn_b200 import engine
         self.torch, self.eng, self.ctx, self.b, self.stream, self.gather = torch, eng, eng.ctx, batch, stream, gather
@@ -262,8 +260,7 @@ class ClassifierStep:
         G, N, d, C = batch.num_graphs, batch.num_nodes, batch.d, batch.num_class
         # use_tiles is the value of S2V_OPT_GRAPH_TILES: 0 never, 1 whenever the batch allows, 2 automatic (the library's default)
         self.mode = int(use_tiles)
-        self.tiles = (d == 128 and int(batch.nodes_per_graph.max()) <= 128 and
-                      (self.mode == 1 or (self.mode == 2 and N <= self.TILE_AUTO_MAX_NODES)))
+        self.tiles = d == 128 and int(batch.nodes_per_graph.max()) <= 128 and self.mode != 0
         self.Y = torch.empty((G, d), device=dev)
         self.logits = torch.empty((G, C), device=dev)
         self.pred = torch.empty((G,), dtype=torch.int32, device=dev)
@@ -553,16 +550,16 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         }
         if step.tiles:
             t_ms = kms["tiles"][0]
-            flops_tf32 = 3 * 2 * N * d * d * max(L - 1, 0)      # level 1 is a sum of product-table rows: no MMAs
+            flops_mma = 3 * 2 * N * d * d * max(L - 1, 0)      # level 1 is a sum of product-table rows: no MMAs
             flops_fp32 = L * (2 * E * d + 2 * N * d * d + 2 * N * d)
             hbm_bytes = 4 * (N + 1) + 4 * E + 4 * N + 4 * (G + 1) + 4 * G * d + 4 * d * d + 4 * full.num_tags * d
-            peak = peaks["bf16_tflops"] / 2
+            peak = peaks["bf16_tflops"]
             line["roofline"] = {
-                "kernel": "s2v_graph_tile_kernel (tcgen05 3xTF32; its tile-planning launch is inside the bracket)", "bound": "tensor",
-                "achieved": flops_tf32 / (t_ms * 1e-3) / 1e12, "peak": peak, "unit": "TFLOP/s",
-                "frac": flops_tf32 / (t_ms * 1e-3) / 1e12 / peak,
-                "peak_kind": f"{peaks['kind']} dense bf16 cuBLAS burst / 2: TF32 MMAs issue at half the bf16 rate",
-                "flops_model": "3 TF32 products (hi*hi, hi*lo, lo*hi) x 2*N*d*d per level x (L - 1) levels (the first level is a gather-sum over the product table)",
+                "kernel": "s2v_graph_fused_kernel (tcgen05, fp16 head + tail in three products; the launches of its product table and its W image are inside the bracket)", "bound": "tensor",
+                "achieved": flops_mma / (t_ms * 1e-3) / 1e12, "peak": peak, "unit": "TFLOP/s",
+                "frac": flops_mma / (t_ms * 1e-3) / 1e12 / peak,
+                "peak_kind": f"{peaks['kind']} dense bf16 cuBLAS burst (fp16 MMAs issue at the same rate)",
+                "flops_model": "3 fp16 products (hi*hi, hi*lo, lo*hi) x 2*N*d*d per level x (L - 1) levels (the first level is a gather-sum over the product table)",
                 "fp32_equivalent_tflops": flops_fp32 / (t_ms * 1e-3) / 1e12,
                 "ms_per_launch": t_ms, "launches": kms["tiles"][1], "traffic": None,
                 "hbm_bytes_algorithmic": hbm_bytes, "hbm_gbs": hbm_bytes / (t_ms * 1e-3) / 1e9,
@@ -625,12 +622,12 @@ def run_ours(args, rank: int, world: int, local_rank: int):
                 ctx.stream_status(stream.cuda_stream)
                 tstep.profile(10)
                 tk = tstep.kernel_ms()
-                flops_tf32 = 3 * 2 * N * d * d * max(L - 1, 0)      # level 1 is a sum of product-table rows: no MMAs
+                flops_mma = 3 * 2 * N * d * d * max(L - 1, 0)      # level 1 is a sum of product-table rows: no MMAs
                 line["tile_kernel"] = {
                     "note": "s2v_graph_tiles_f32 (S2V_OPT_GRAPH_TILES = 1): input projection + all levels + pooling in one kernel, embeddings in shared memory",
                     "value": full.num_graphs * min(args.steps, 20) / (t_ms * 1e-3), "unit": "graphs/s", "ms_per_step": t_ms / min(args.steps, 20),
-                    "kernel_ms": tk["tiles"][0], "bound": "tensor", "achieved_tflops_tf32": flops_tf32 / (tk["tiles"][0] * 1e-3) / 1e12,
-                    "peak_tflops_tf32": peaks["bf16_tflops"] / 2, "frac": flops_tf32 / (tk["tiles"][0] * 1e-3) / 1e12 / (peaks["bf16_tflops"] / 2),
+                    "kernel_ms": tk["tiles"][0], "bound": "tensor", "achieved_tflops": flops_mma / (tk["tiles"][0] * 1e-3) / 1e12,
+                    "peak_tflops": peaks["bf16_tflops"], "frac": flops_mma / (tk["tiles"][0] * 1e-3) / 1e12 / peaks["bf16_tflops"],
                     "argmax_equal_to_default_path": bool(np.array_equal(tstep.pred.cpu().numpy(), step.pred.cpu().numpy())),
                     "max_abs_logit_diff_to_default_path": float((tstep.logits - step.logits).abs().max().item())}
     # ---- several GPUs: the row-partitioned giant graph at a scale that runs in seconds
@@ -946,7 +943,7 @@ def main():
     ap.add_argument("--skip-level", action="store_true", help="leave out the 1M-node fused-level measurement")
     ap.add_argument("--tiles", type=int, default=2, choices=[0, 1, 2],
                     help="S2V_OPT_GRAPH_TILES: 0 per-level kernels only, 1 whole-classifier tile kernel whenever the batch allows, "
-                         "2 the library's default (tile kernel for batches of at most 160,000 nodes)")
+                         "2 the library's default (also whenever the batch allows)")
     ap.add_argument("--case", default=None, choices=["er_d64", "er_d64_full", "mol_d128", "prot_d64", "mol_first", "prot_first", "readout", "mol_tiles", "mol_tiles_small", "mol_paths"],
                     help="run one small launch case (for profiler captures) instead of the benchmark")
     ap.add_argument("--launches", type=int, default=3)

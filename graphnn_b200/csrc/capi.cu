@@ -271,10 +271,10 @@ int s2v_level_first_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n, int d, const
     return rc;
 }
 
-// ---------------------------------------------------------------- tile kernel for batches of small graphs
+// ---------------------------------------------------------------- batches of small graphs up to the pooled embeddings
 size_t s2v_graph_tiles_workspace_bytes(int64_t num_graphs)
 {
-    return num_graphs < 0 ? 0 : align_up(s2v_graph_tiles_plan_bytes(num_graphs), 256) + 256;
+    return num_graphs < 0 ? 0 : align_up(s2v_graph_fused_image_bytes(128), 256) + 256;   // W in the operand layout
 }
 
 int s2v_graph_tiles_f32(s2v_ctx* ctx, s2v_stream stream, int64_t num_graphs, int d, int levels, const int32_t* row_ptr,
@@ -284,7 +284,7 @@ int s2v_graph_tiles_f32(s2v_ctx* ctx, s2v_stream stream, int64_t num_graphs, int
 {
     S2V_ENTER(ctx);
     if (num_graphs < 0 || levels < 1 || num_tags <= 0) return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "graph_tiles: bad shape");
-    if (d != 128) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "graph_tiles: the tile kernel is built for d = 128");
+    if (d != 128) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "graph_tiles: built for d = 128");
     if (num_graphs == 0) return S2V_OK;
     if (num_graphs >= (int64_t)INT32_MAX) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "graph_tiles: int32 graph count only");
     if (!row_ptr || !graph_ptr || !tags || !W_in || !W || !Y) return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "graph_tiles: NULL pointer");
@@ -292,7 +292,6 @@ int s2v_graph_tiles_f32(s2v_ctx* ctx, s2v_stream stream, int64_t num_graphs, int
         return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "graph_tiles: W_in, W, Y, embed_out must be 16-byte aligned");
     if (!workspace || workspace_bytes < s2v_graph_tiles_workspace_bytes(num_graphs))
         return s2v_fail(ctx, S2V_ERR_WORKSPACE, "graph_tiles: workspace smaller than s2v_graph_tiles_workspace_bytes");
-    void* plan = reinterpret_cast<void*>(align_up(reinterpret_cast<uintptr_t>(workspace), 256));
     // the product table of the first level ((num_tags + 1) x d floats) lives in a small context-owned buffer
     float* P = nullptr;
     if (ctx->first_table_on) {
@@ -306,9 +305,18 @@ int s2v_graph_tiles_f32(s2v_ctx* ctx, s2v_stream stream, int64_t num_graphs, int
         }
         P = static_cast<float*>(ctx->first_table);
     }
-    const int rc = s2v_launch_graph_tiles(ctx, s2v_pick_stream(ctx, stream), num_graphs, row_ptr, col_idx, val, graph_ptr, tags,
-                                          num_tags, W_in, W, levels, pool_average, plan, P, Y, embed_out);
-    if (rc == S2V_ERR_UNSUPPORTED) return s2v_fail(ctx, rc, "graph_tiles: this device cannot hold the kernel's shared memory");
+    s2v_graph_fused_args a;
+    a.G = num_graphs; a.d = d; a.levels = levels;
+    a.max_graph_nodes = S2V_TILE_NODES;
+    a.pool_average = pool_average;
+    a.row_ptr = row_ptr; a.col_idx = col_idx; a.val = val; a.graph_ptr = graph_ptr;
+    a.tags = tags; a.x = W_in; a.num_tags = num_tags;
+    a.W = W;
+    a.P_scratch = P;
+    a.image_scratch = reinterpret_cast<void*>(align_up(reinterpret_cast<uintptr_t>(workspace), 256));
+    a.Y = Y; a.embed_out = embed_out;
+    const int rc = s2v_launch_graph_fused(ctx, s2v_pick_stream(ctx, stream), a);
+    if (rc == S2V_ERR_UNSUPPORTED) return s2v_fail(ctx, rc, "graph_tiles: more tags, or more shared memory, than the kernel can address here");
     return rc;
 }
 
@@ -318,7 +326,7 @@ size_t s2v_forward_workspace_bytes(int64_t num_nodes, int64_t num_graphs, int d)
     if (num_nodes < 0 || num_graphs < 0 || d <= 0) return 0;
     const size_t nd = align_up(sizeof(float) * (size_t)num_nodes * d, 256);
     const size_t gd = align_up(sizeof(float) * (size_t)num_graphs * d, 256);
-    return 3 * nd + gd + 256 + align_up(s2v_graph_tiles_plan_bytes(num_graphs), 256);
+    return 3 * nd + gd + 256;
 }
 
 int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, const s2v_batch* batch, void* workspace,
@@ -346,7 +354,6 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
     float* ha = reinterpret_cast<float*>(ws + nd);
     float* hb = reinterpret_cast<float*>(ws + 2 * nd);
     float* y = reinterpret_cast<float*>(ws + 3 * nd);
-    void* plan = ws + 3 * nd + align_up(sizeof(float) * (size_t)G * d, 256);
 
     int rc;
     // Batches of graphs (the caller vouches for the largest one) whose embeddings fit a CTA's shared memory: the whole
@@ -391,26 +398,6 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
         if (rc != S2V_OK || readout_inside) return rc;
         return s2v_readout_f32(ctx, st, G, d, model->hidden, model->num_class, y, model->h1_weight, model->h2_weight, logits, probs,
                                pred);
-    }
-    // Batches of small graphs (the caller vouches for the largest one): the whole classifier up to the pooled
-    // embeddings is one kernel that keeps the node embeddings of a tile of whole graphs in shared memory.
-    // Measured on 20-40-node graphs, d = 128, 4 levels: one launch beats the per-level kernels by 1.9x at 16 k nodes,
-    // 1.15x at 62 k, 1.09x at 123 k, and loses 5 % at 246 k and 11 % at 491 k (the per-level kernels stream better
-    // once every SM has dozens of tiles), so the automatic mode takes it up to S2V_TILE_AUTO_MAX_NODES nodes.
-    const bool want_tiles = ctx->graph_tiles == 1 || (ctx->graph_tiles == 2 && N <= S2V_TILE_AUTO_MAX_NODES);
-    if (want_tiles && d == 128 && L >= 1 && batch->tags && batch->max_graph_nodes >= 1 &&
-        batch->max_graph_nodes <= S2V_TILE_NODES && N > 0 && G < (int64_t)INT32_MAX) {
-        if (!s2v_aligned16(model->w_n2l) || !s2v_aligned16(model->p_node_conv) || (embed_out && !s2v_aligned16(embed_out)))
-            return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "forward: weights and embed_out must be 16-byte aligned");
-        // the first level's product table goes into the `msg` region of the workspace, which one-hot inputs leave unused
-        float* P = (ctx->first_table_on && s2v_first_table_scratch_bytes(model->num_feat + 1, d) <= nd) ? msg : nullptr;
-        rc = s2v_launch_graph_tiles(ctx, st, G, batch->n2n_row_ptr, batch->n2n_col_idx, batch->n2n_val, batch->graph_ptr,
-                                    batch->tags, model->num_feat, model->w_n2l, model->p_node_conv, L, model->pool_average,
-                                    plan, P, y, embed_out);
-        if (rc == S2V_OK)
-            return s2v_readout_f32(ctx, st, G, d, model->hidden, model->num_class, y, model->h1_weight, model->h2_weight,
-                                   logits, probs, pred);
-        if (rc != S2V_ERR_UNSUPPORTED) return rc;
     }
     // With one-hot tags the X term of every level is a lookup in W_in, so `msg` is
     // never materialised; a dense X needs it.

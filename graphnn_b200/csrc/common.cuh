@@ -54,7 +54,7 @@ struct s2v_ctx {
     void* first_table = nullptr;     // product table of s2v_level_first_f32 (grow-only, a few hundred KB at most)
     size_t first_table_bytes = 0;
     int tc_mode = 1;  // tcgen05 level kernel: 0 never, 1 when the batch is large enough, 2 whenever the shape allows
-    int graph_tiles = 2;    // whole-classifier tile kernel for batches of small graphs: 0 off, 1 whenever the batch allows, 2 automatic
+    int graph_tiles = 2;    // whole-classifier kernel for batches of small graphs: 0 off, 1 whenever the batch allows, 2 automatic
     int first_table_on = 1; // first level as a gather-sum over ReLU(W_in) * W (S2V_OPT_FIRST_LEVEL_TABLE)
     int validate_host = 1;  // s2v_infer_host_f32 scans its host arrays before launching
 };
@@ -201,14 +201,7 @@ bool s2v_graph_fused_supported(const s2v_ctx* ctx, int d, int max_nodes, int num
 size_t s2v_graph_fused_image_bytes(int d);
 bool s2v_graph_fused_readout_ok(int d, int hidden, int num_class);
 int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_args& a);
-// whole classifier up to the pooled embeddings for batches of graphs of at most S2V_TILE_NODES nodes (d = 128, tags)
-constexpr int S2V_TILE_NODES = 128;
-constexpr int64_t S2V_TILE_AUTO_MAX_NODES = 160000;   // automatic mode: batches up to this many nodes take the tile kernel
-size_t s2v_graph_tiles_plan_bytes(int64_t num_graphs);
-int s2v_launch_graph_tiles(s2v_ctx* ctx, cudaStream_t st, int64_t G, const int32_t* row_ptr, const int32_t* col_idx,
-                           const float* val, const int32_t* graph_ptr, const int32_t* tags, int num_tags,
-                           const float* W_in, const float* W, int levels, int pool_average, void* plan, float* P_scratch,
-                           float* Y, float* embed_out);   // P_scratch: (num_tags + 1) * 128 floats, or NULL (first level through the MMAs)
+constexpr int S2V_TILE_NODES = 128;   // s2v_graph_tiles_f32: most nodes of a graph
 // long_rows: rows of hundreds of entries and more may occur and are summed ahead of the rest (long_rows.cuh)
 int s2v_launch_level(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int64_t n_src, int d, const void* row_ptr,
                      bool rp64, const int32_t* col_idx, const float* val, const float* H, const float* W,

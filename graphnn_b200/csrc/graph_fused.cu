@@ -1101,7 +1101,8 @@ int gf_launch(s2v_ctx* ctx, cudaStream_t st, const GfParams& p, uint32_t smem, u
 bool s2v_graph_fused_supported(const s2v_ctx* ctx, int d, int max_nodes, int num_tags)
 {
     const int most = d == 128 ? 128 : (d == 64 ? 640 : (d == 32 ? 1024 : 0));
-    return max_nodes >= 1 && max_nodes <= most && num_tags < 65536 && ctx->smem_optin >= 227 * 1024;
+    const int tags = d == 128 ? 1 << 23 : 1 << 16;   // held as 32-bit byte offsets of their W_in rows, or as 16-bit tags
+    return max_nodes >= 1 && max_nodes <= most && num_tags < tags && ctx->smem_optin >= 227 * 1024;
 }
 
 size_t s2v_graph_fused_image_bytes(int d) { return sizeof(float) * (size_t)d * d + 16; }

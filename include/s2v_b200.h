@@ -72,11 +72,10 @@ typedef enum s2v_option {
                                         the environment variable S2V_VALIDATE_HOST=0 sets the default to 0) */
     S2V_OPT_LEVEL_TC = 2,            /* tcgen05 level kernel: 0 never, 1 automatic (default), 2 whenever the shape allows
                                         (default from S2V_LEVEL_TC) */
-    S2V_OPT_GRAPH_TILES = 3,         /* whole-classifier tile kernel (s2v_graph_tiles_f32) inside s2v_forward_f32 for batches of
-                                        small graphs, and its counterpart for d = 32 and 64: 0 never, 1 whenever the batch
-                                        allows, 2 automatic (default; d = 128: batches of at most 160,000 nodes, where one launch
-                                        beats the per-level kernels by 1.1x - 1.9x; larger ones stream better through the
-                                        per-level kernels).  Default from S2V_GRAPH_TILES */
+    S2V_OPT_GRAPH_TILES = 3,         /* whole-classifier kernel inside s2v_forward_f32 for batches of small and medium graphs (at most
+                                        128 nodes at d = 128, 640 at d = 64, 1024 at d = 32): 0 never, 1 whenever the batch
+                                        allows, 2 automatic (default: also whenever it allows, except that small batches with
+                                        embed_out keep one launch per level).  Default from S2V_GRAPH_TILES */
     S2V_OPT_RESERVED_SMS = 4,        /* the persistent kernels size their grids for (SM count - value) SMs, leaving the rest to
                                         kernels of another stream -- a communication library's, which cannot start while
                                         one-CTA-per-SM kernels hold every SM (default 0; 0 <= value < SM count) */
@@ -215,12 +214,12 @@ int s2v_input_proj_dense_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n, int num
 /* ---- batches of small graphs: input projection, all L levels and the pooling in ONE kernel.
  * Y[g,:] = sum (or mean) over the nodes of graph g of H_L, with H_0 = ReLU(W_in[tags]),
  * H_{l+1} = ReLU((A*H_l)*W + W_in[tags]) -- kernel_mean_field.cpp:31-44 for one-hot inputs.
- * Requires d = 128, every graph at most 128 nodes with a contiguous node range (graph_ptr, nn_common.h:63-73)
- * and no edge between graphs.  Consecutive graphs are packed into tiles of at most 128 nodes; a tile's node
- * embeddings stay in shared memory across the levels, the dense stage runs on the tcgen05 tensor cores in
- * 3xTF32, and only Y [G x d] (plus embed_out [N x d] if given) is written.  A larger graph, an edge that
- * leaves its graph's tile or a tag outside [0, num_tags) is reported through the status word, not faulted.
- * val may be NULL (all ones).  workspace: s2v_graph_tiles_workspace_bytes(G) bytes of device memory. */
+ * Requires d = 128, every graph at most 128 nodes with a contiguous node range (graph_ptr, nn_common.h:63-73),
+ * no edge between graphs and fewer than 8,388,608 tags.  Consecutive graphs are packed into tiles of at most 128 nodes; a
+ * tile's node embeddings stay in shared memory across the levels, the dense stage runs on the tcgen05 tensor cores with
+ * operands of 22 bits (fp16 head and tail, scaled per row), and only Y [G x d] (plus embed_out [N x d] if given) is
+ * written.  A larger graph, an edge that leaves its graph's tile or a tag outside [0, num_tags) is reported through the
+ * status word, not faulted.  val may be NULL (all ones).  workspace: s2v_graph_tiles_workspace_bytes(G) bytes of device memory. */
 size_t s2v_graph_tiles_workspace_bytes(int64_t num_graphs);
 int s2v_graph_tiles_f32(s2v_ctx* ctx, s2v_stream stream, int64_t num_graphs, int d, int levels, const int32_t* row_ptr,
                         const int32_t* col_idx, const float* val, const int32_t* graph_ptr, const int32_t* tags, int num_tags,
