@@ -197,6 +197,7 @@ struct s2v_graph_fused_args {
 };
 constexpr int64_t S2V_FUSED_TABLE_NODES = 32768;   // batches from this many nodes on: weights and first-level table prepared by launches of their own
 constexpr int64_t S2V_FUSED_EMBED_NODES = 16384;   // batches with embed_out below this many nodes take the per-level kernels
+constexpr int64_t S2V_FUSED_ROUND_NODES = 384;     // d = 32, larger graphs: nodes that a CTA is expected to hold at a time
 bool s2v_graph_fused_supported(const s2v_ctx* ctx, int d, int max_nodes, int num_tags);
 size_t s2v_graph_fused_image_bytes(int d);
 bool s2v_graph_fused_readout_ok(int d, int hidden, int num_class);

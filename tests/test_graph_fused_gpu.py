@@ -109,3 +109,17 @@ def test_fused_reports_a_graph_beyond_the_hint_and_an_edge_between_graphs():
     with pytest.raises(capi.S2VError) as e:
         eng.ctx.synchronize()
     assert e.value.status == -4
+
+
+@pytest.mark.parametrize("graphs", [189, 190])   # d = 32, 600 nodes each: the last batch of one round of tiles, and one beyond it
+def test_large_d32_batches(graphs):
+    b = make([600] * graphs, 6.5, 32, 5, 3, 64, 2, seed=graphs)
+    eng = engine.S2VInference(b.weights, b.levels)
+    hb = engine.build_host_batch(b)
+    db = eng.to_device(hb)
+    n0 = eng.ctx.launches
+    logits, _, _, _ = eng.forward(db)
+    eng.ctx.synchronize()
+    assert eng.ctx.launches - n0 == (4 if graphs == 189 else 6)
+    _, want = f64(b, hb.row_ptr.numpy(), hb.col_idx.numpy(), None, None, False)
+    assert_close(logits.cpu().numpy(), want, "logits", scale=max(1.0, float(np.abs(want).max())))
