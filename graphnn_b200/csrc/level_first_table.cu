@@ -20,9 +20,14 @@ namespace
 {
 
 // P[t, j] = sum_k ReLU(table[t, k]) * W[k, j], k ascending, one CTA per table row, one thread per column (strided).
-__global__ void __launch_bounds__(256) first_table_product_kernel(int n_table, int d, const float* __restrict__ table,
+// Bounded by the latency of W's loads: with d known at compile time (D = 32, 64, 128; 0: any) up to 64 of them are on their way at a
+// time (16 at a time: eight round trips to L2 at d = 128, and 2 us more of every batch that makes the table).
+template <int D>
+__global__ void __launch_bounds__(256) first_table_product_kernel(int n_table, int d_arg, const float* __restrict__ table,
                                                                   const float* __restrict__ W, float* __restrict__ P)
 {
+    constexpr int U = D == 0 ? 16 : (D < 64 ? D : 64);
+    const int d = D == 0 ? d_arg : D;
     extern __shared__ float h0[];
     const int t = blockIdx.x;
     if (t >= n_table) {   // the extra row some callers ask for: zeros (what an unused gather slot adds)
@@ -33,8 +38,19 @@ __global__ void __launch_bounds__(256) first_table_product_kernel(int n_table, i
     __syncthreads();
     for (int j = threadIdx.x; j < d; j += blockDim.x) {
         float acc = 0.f;
+        if constexpr (D != 0) {
+#pragma unroll
+            for (int k0 = 0; k0 < D; k0 += U) {
+                float w[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) w[u] = __ldg(W + (k0 + u) * D + j);
+#pragma unroll
+                for (int u = 0; u < U; ++u) acc = fmaf(h0[k0 + u], w[u], acc);
+            }
+        } else {
 #pragma unroll 16
-        for (int k = 0; k < d; ++k) acc = fmaf(h0[k], __ldg(W + (int64_t)k * d + j), acc);   // the loads of 16 steps go out together
+            for (int k = 0; k < d; ++k) acc = fmaf(h0[k], __ldg(W + (int64_t)k * d + j), acc);   // the loads of 16 steps go out together
+        }
         P[(int64_t)t * d + j] = acc;
     }
 }
@@ -191,8 +207,9 @@ size_t s2v_first_table_scratch_bytes(int n_table, int d)
 int s2v_launch_first_table_product(s2v_ctx* ctx, cudaStream_t st, int n_table, int d, const float* table, const float* W,
                                    float* P, bool extra_zero_row)
 {
-    first_table_product_kernel<<<n_table + (extra_zero_row ? 1 : 0), d < 256 ? ((d + 31) / 32) * 32 : 256, sizeof(float) * (size_t)d, st>>>(
-        n_table, d, table, W, P);
+    auto kern = d == 128 ? first_table_product_kernel<128>
+                         : (d == 64 ? first_table_product_kernel<64> : (d == 32 ? first_table_product_kernel<32> : first_table_product_kernel<0>));
+    kern<<<n_table + (extra_zero_row ? 1 : 0), d < 256 ? ((d + 31) / 32) * 32 : 256, sizeof(float) * (size_t)d, st>>>(n_table, d, table, W, P);
     S2V_CHECK_LAUNCH(ctx, "first_table_product_kernel");
     return S2V_OK;
 }
