@@ -94,7 +94,7 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
                  : "memory");
 }
 
-template <int D, typename RpT, bool HAS_VAL, int XMODE /*0 none, 1 dense, 2 table lookup*/, bool LONG>
+template <int D, typename RpT, bool HAS_VAL, int XMODE /*0 none, 1 dense, 2 table lookup*/, int LONG>
 __global__ void __launch_bounds__(LevelCfg<D>::WARPS * 32, LevelCfg<D>::MIN_BLOCKS)
 s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_ptr,
                  const int32_t* __restrict__ col_idx, const float* __restrict__ val, const float* __restrict__ H,
@@ -153,8 +153,9 @@ s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_
     const int sub = lane / LPR, sl = lane % LPR;
     const int g = lane >> 2, tig = lane & 3;   // MMA fragment coordinates
 
-    // Tiles with a long row are passed over at first; if the CTA met one, all its warps sum the long rows (long_rows.cuh) and a second
-    // pass takes those tiles.  (A look through the offsets in front cost 2 of 25 us, and its registers spilled.)
+    // Tiles with a long row are passed over at first; if there was one, a second pass takes those tiles, once their sums are made
+    // (long_rows.cuh): by this CTA, or by the kernel in front, which runs beside the first pass.  (A look through the offsets in front cost
+    // 2 of 25 us, and its registers spilled; waiting for the sums in the first pass took 559 us instead of 473 on R-MAT 2^19.)
     bool found = false;
     for (int pass = 0;; ++pass) {
     for (int64_t tile = (int64_t)blockIdx.x * WARPS + warp; tile < num_tiles; tile += (int64_t)gridDim.x * WARPS) {
@@ -166,11 +167,14 @@ s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_
         const RpT base = __shfl_sync(0xffffffffu, rp_abs, 0);
         const int rp_rel = (int)(rp_abs - base);
         const int tile_nnz = __shfl_sync(0xffffffffu, rp_rel, TILE_R);
-        if (LONG) {
+        bool summed = false;
+        if (LONG && tile_nnz > LONG_ROW) {
             const int row_len = __shfl_down_sync(0xffffffffu, rp_rel, 1) - rp_rel;
-            const bool has_long = __any_sync(0xffffffffu, lane < TILE_R && row_len > LONG_ROW);
-            found |= has_long;
-            if (has_long != (pass == 1)) continue;
+            summed = __any_sync(0xffffffffu, lane < TILE_R && row_len > LONG_ROW);
+        }
+        if (LONG) {
+            found |= summed;
+            if (summed != (pass == 1)) continue;
         }
         if (lane <= TILE_R) rp_s[lane] = rp_rel;
         const bool fits = tile_nnz <= IDX_CAP;   // warp-uniform; almost always true
@@ -355,13 +359,19 @@ s2v_level_kernel(int64_t n_rows, int64_t num_tiles, const RpT* __restrict__ row_
         }
         __syncwarp();  // S and idx_s are rewritten by the next tile
     }
-    if (!LONG || pass == 1 || !__syncthreads_or(found)) break;
-    sum_long_rows<D, WARPS * 32, WARPS * TILE_R, TILE_R, (int)(LevelSmem<D>::WARP_BYTES * WARPS), HAS_VAL>(smem_raw + LevelSmem<D>::W_BYTES + 16, n_rows,
-                                                                                                           row_ptr, col_idx, val, H, out);
+    if (!LONG || pass == 1) break;
+    if (LONG == LONG_FRONT) {
+        long_rows_wait();   // (also for whatever is launched behind this kernel)
+        if (!found) break;  // warp-uniform
+    } else {
+        if (!__syncthreads_or(found)) break;
+        sum_long_rows_call<D, WARPS * 32, WARPS * TILE_R, TILE_R, (int)(LevelSmem<D>::WARP_BYTES * WARPS), HAS_VAL>(
+            smem_raw + LevelSmem<D>::W_BYTES + 16, n_rows, row_ptr, col_idx, val, H, out);
+    }
     }
 }
 
-template <int D, typename RpT, bool HAS_VAL, int XMODE, bool LONG>
+template <int D, typename RpT, bool HAS_VAL, int XMODE, int LONG>
 int launch_one(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx,
                const float* val, const float* H, const float* W, const float* X, const int32_t* x_index, int n_table,
                float* out)
@@ -382,8 +392,13 @@ int launch_one(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const RpT* row_ptr
     const int64_t persistent = (int64_t)ctx->sm_count * resident;
     int64_t blocks = (num_tiles + WARPS - 1) / WARPS;
     if (blocks > persistent) blocks = persistent;
-    kern<<<(unsigned)blocks, WARPS * 32, smem, st>>>(n_rows, num_tiles, row_ptr, col_idx, val, H, W, X, x_index, n_table, out,
-                                                      ctx->dstatus_dev);
+    if (LONG == LONG_FRONT) {
+        const int rc = launch_long_rows<D, TILE_R, HAS_VAL>(ctx, st, n_rows, row_ptr, col_idx, val, H, out);
+        if (rc != S2V_OK) return rc;
+        S2V_CUDA_OK(ctx, launch_behind_long_rows(kern, (unsigned)blocks, WARPS * 32, smem, st, n_rows, num_tiles, row_ptr, col_idx, val, H, W, X, x_index,
+                                                 n_table, out, ctx->dstatus_dev));
+    } else
+        kern<<<(unsigned)blocks, WARPS * 32, smem, st>>>(n_rows, num_tiles, row_ptr, col_idx, val, H, W, X, x_index, n_table, out, ctx->dstatus_dev);
     S2V_CHECK_LAUNCH(ctx, "s2v_level_kernel");
     return S2V_OK;
 }
@@ -396,8 +411,9 @@ int launch_d(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, cons
     const int xmode = table ? 2 : (X ? 1 : 0);
     const float* xa = table ? table : X;
 #define S2V_LVL(HV, XM)                                                                                                       \
-    return long_rows ? launch_one<D, RpT, HV, XM, true>(ctx, st, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)        \
-                     : launch_one<D, RpT, HV, XM, false>(ctx, st, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)
+    return !long_rows                          ? launch_one<D, RpT, HV, XM, LONG_NONE>(ctx, st, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)  \
+           : n_rows >= LongCfg<D>::FRONT_ROWS ? launch_one<D, RpT, HV, XM, LONG_FRONT>(ctx, st, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out) \
+                                              : launch_one<D, RpT, HV, XM, LONG_INSIDE>(ctx, st, n_rows, rp, ci, val, H, W, xa, x_index, n_table, out)
     if (val) {
         if (xmode == 0) S2V_LVL(true, 0);
         if (xmode == 1) S2V_LVL(true, 1);

@@ -1,14 +1,18 @@
 // Long rows (hubs of a power-law graph) of the level kernels.  A level kernel gives a row to one warp, or part of one; a
 // row of 10^4 or 10^5 entries keeps that warp -- and its CTA's pipeline behind it -- busy long after everyone else is done
-// (R-MAT scale 20, d = 128: 11.3 ms, nearly all of it the longest rows).  So a CTA first looks through the offsets of the
-// rows it owns (while W is on its way) and, if there is one above LONG_ROW entries, sums such rows with all its warps,
-// together with the other rows of their groups of GROUP rows (what a warp of the main loop works on as one unit).  The sums
-// go to the rows' places in `out`, which the CTA itself overwrites with the result afterwards, so no scratch memory is
+// (R-MAT scale 20, d = 128: 11.3 ms, nearly all of it the longest rows).  So the rows above LONG_ROW entries are summed by whole
+// CTAs ahead of the rest, together with the other rows of their groups of GROUP rows (what a warp of the main loop works on as one
+// unit).  The sums go to the rows' places in `out`, which the level overwrites with the result afterwards, so no scratch memory is
 // needed; the main loop reads such a group's sums from there instead of gathering.
 //   * Up to LONG_BIG entries a warp sums a row, in slices of up to 64 columns with 4 KB of neighbour rows on their way; a longer
 //     one, taken first, is streamed through a ring in shared memory by the whole CTA, where one warp would be bounded by latency.
 //   * Entries are added one after the other in CSR order, as everywhere else in the level: a float sum of 10^5 entries
 //     depends on its order in the fifth digit.
+//   * In large levels (LongCfg::FRONT_ROWS) a kernel in front makes the sums, with the level kernel launched as its programmatic
+//     dependent.  With the look and the sums inside, the registers of the main loop cost every level 1 - 5 %, also without a long row
+//     (Erdos-Renyi, a million rows: d = 64 480 us inside, 474 in front, 473 without any of it; with edge weights 526, 473, 472;
+//     d = 32 366, 351, 349; d = 128, half a million, 601, 584, 585; R-MAT 2^20, d = 128: 4.9 ms inside, 2.9 in front).  A second
+//     launch costs up to 1 us: below, the level kernel does it for the rows it owns (30,000 rows, d = 64: 13.5 us, 14.1 in front).
 #pragma once
 
 #include "common.cuh"
@@ -19,6 +23,7 @@ namespace
 constexpr int LONG_ROW = 256;      // below this a row is no longer than what the other warps of a tile work on
 constexpr int LONG_BIG = 2048;      // above this a row is worth the whole CTA
 constexpr int LONG_SCAN = 8;       // rows per thread and pass of the sums
+enum { LONG_NONE, LONG_INSIDE, LONG_FRONT };   // where a level kernel's long rows are summed
 
 template <int W> struct LongVec;
 template <> struct LongVec<2> { using T = float2; };
@@ -104,13 +109,14 @@ __device__ __forceinline__ void long_row_by_cta(unsigned char* ring, const float
         if (threadIdx.x < D) {
             const float* p = reinterpret_cast<const float*>(ring) + (s & 3) * STAGE * D + threadIdx.x;
             const int m = n - s * STAGE < STAGE ? n - s * STAGE : STAGE;
+            constexpr int U = 16;
             int r = 0;
-            for (; r + 16 <= m; r += 16) {
-                float v[16];
+            for (; r + U <= m; r += U) {
+                float v[U];
 #pragma unroll
-                for (int u = 0; u < 16; ++u) v[u] = p[(r + u) * D];
+                for (int u = 0; u < U; ++u) v[u] = p[(r + u) * D];
 #pragma unroll
-                for (int u = 0; u < 16; ++u) acc = HAS_VAL ? fmaf(__ldg(val + s * STAGE + r + u), v[u], acc) : acc + v[u];
+                for (int u = 0; u < U; ++u) acc = HAS_VAL ? fmaf(__ldg(val + s * STAGE + r + u), v[u], acc) : acc + v[u];
             }
             for (; r < m; ++r) acc = HAS_VAL ? fmaf(__ldg(val + s * STAGE + r), p[r * D], acc) : acc + p[r * D];
         }
@@ -169,9 +175,9 @@ struct LongLook {
     }
 };
 
-// Called by all THREADS threads of the CTA; BYTES of shared memory at `smem`.  Not inlined: the main loops keep their registers.
+// Called by all THREADS threads of the CTA; BYTES of shared memory at `smem`.
 template <int D, int THREADS, int RB, int GROUP, int BYTES, bool HAS_VAL, typename RpT>
-__device__ __noinline__ void sum_long_rows(unsigned char* smem, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx, const float* val,
+__device__ __forceinline__ void sum_long_rows(unsigned char* smem, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx, const float* val,
                                            const float* H, float* out)
 {
     constexpr int SL = D < 64 ? D : 64, SLICES = D / SL, LIST = 2 * ((THREADS * LONG_SCAN + GROUP - 1) / GROUP), RING = (16 + LIST + 127) / 128 * 128;
@@ -231,7 +237,63 @@ __device__ __noinline__ void sum_long_rows(unsigned char* smem, int64_t n_rows, 
     __syncthreads();
 }
 
-// the sum that sum_long_rows left in the row's place of `out`
+// The same as a call, for the level kernels: their main loops keep their registers.
+template <int D, int THREADS, int RB, int GROUP, int BYTES, bool HAS_VAL, typename RpT>
+__device__ __noinline__ void sum_long_rows_call(unsigned char* smem, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx, const float* val,
+                                                const float* H, float* out)
+{
+    sum_long_rows<D, THREADS, RB, GROUP, BYTES, HAS_VAL>(smem, n_rows, row_ptr, col_idx, val, H, out);
+}
+
+// Shared memory: with the CTAs of the level kernel beside it an SM keeps the split of its memory into cache and shared memory, so the
+// kernel asks for no more per SM than the level kernel does (d = 64, 112 KB per CTA instead of 48: the level of a million rows 544 us
+// instead of 474; d = 128, 48 KB instead of 112: R-MAT scale 20 4.76 ms instead of 2.91).
+template <int D> struct LongCfg { static constexpr int THREADS = 512, CTAS = 2, BYTES = (D == 128 ? 112 : 48) << 10, FRONT_ROWS = 131072; };
+// (d = 32 at 131,072 rows: R-MAT 137 us inside, 141 in front; Erdos-Renyi at 180,000: 43.2 and 41.7)
+template <> struct LongCfg<32> { static constexpr int THREADS = 256, CTAS = 3, BYTES = 40 << 10, FRONT_ROWS = 160000; };
+constexpr int LONG_RB = 128;
+template <int D, int GROUP, bool HAS_VAL, typename RpT>
+__global__ void __launch_bounds__(LongCfg<D>::THREADS, LongCfg<D>::CTAS)
+long_rows_kernel(int64_t n_rows, const RpT* __restrict__ row_ptr, const int32_t* __restrict__ col_idx, const float* __restrict__ val,
+                 const float* __restrict__ H, float* __restrict__ out)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    extern __shared__ __align__(128) unsigned char long_smem[];
+    LongLook<LongCfg<D>::THREADS, LONG_RB, RpT> look;
+    look.load(n_rows, row_ptr);
+    if (__syncthreads_or(look.any(n_rows, row_ptr)))
+        sum_long_rows<D, LongCfg<D>::THREADS, LONG_RB, GROUP, LongCfg<D>::BYTES, HAS_VAL>(long_smem, n_rows, row_ptr, col_idx, val, H, out);
+}
+template <int D, int GROUP, bool HAS_VAL, typename RpT>
+int launch_long_rows(s2v_ctx* ctx, cudaStream_t st, int64_t n_rows, const RpT* row_ptr, const int32_t* col_idx, const float* val, const float* H, float* out)
+{
+    auto kern = long_rows_kernel<D, GROUP, HAS_VAL, RpT>;
+    constexpr int BYTES = LongCfg<D>::BYTES;
+    if (BYTES > (48 << 10)) S2V_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES));
+    const int64_t blocks = (n_rows + LONG_RB - 1) / LONG_RB, most = (int64_t)LongCfg<D>::CTAS * ctx->sm_count;
+    kern<<<(unsigned)(blocks < most ? blocks : most), LongCfg<D>::THREADS, BYTES, st>>>(n_rows, row_ptr, col_idx, val, H, out);
+    S2V_CHECK_LAUNCH(ctx, "long_rows_kernel");
+    return S2V_OK;
+}
+// The level kernel behind it may start while the sums are made.
+template <typename... Params, typename... Args>
+cudaError_t launch_behind_long_rows(void (*kern)(Params...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st, Args... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = blocks;
+    cfg.blockDim = threads;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+__device__ __forceinline__ void long_rows_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// the sum that long_rows_kernel left in the row's place of `out`
 __device__ __forceinline__ float4 long_row_sum(const float4* p)
 {
     float4 v;
