@@ -366,16 +366,18 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
     //     observe the launch count of the per-level path;
     //   * d = 32, graphs above one row block: a CTA holds one graph or two, and as long as the batch is one round of such
     //     tiles the kernel is ahead (100 graphs of 100 - 620 nodes 31 us against 58, 300 graphs 72 against 80); from the second
-    //     round on the level kernels are, which stream 128-byte rows (500 graphs 121 us against 170).
+    //     round on the level kernels are, which stream 128-byte rows (500 graphs 121 us against 170).  So they are where the columns
+    //     are too many to be listed in shared memory (301 graphs, 24 neighbours per node: 114 us against 132; 16: 100 against 98).
     const bool forced = ctx->graph_tiles == 1;
-    const bool rounds = d == 32 && batch->max_graph_nodes > 128 && N > (int64_t)ctx->sm_count * 2 * S2V_FUSED_ROUND_NODES;
+    const bool rounds = d == 32 && batch->max_graph_nodes > 128 &&
+                        (N > (int64_t)ctx->sm_count * 2 * S2V_FUSED_ROUND_NODES || batch->num_edges > (int64_t)ctx->sm_count * 2 * S2V_FUSED_ROUND_EDGES);
     if (ctx->graph_tiles != 0 && L >= 1 && N > 0 && G < (int64_t)INT32_MAX && batch->max_graph_nodes >= 1 &&
         (forced || !(rounds || (embed_out && N < S2V_FUSED_EMBED_NODES))) && (batch->tags || batch->x_dense) &&
         s2v_graph_fused_supported(ctx, d, batch->max_graph_nodes, batch->tags ? model->num_feat : 1)) {
         if (!s2v_aligned16(model->w_n2l) || !s2v_aligned16(model->p_node_conv) || (embed_out && !s2v_aligned16(embed_out)))
             return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "forward: weights and embed_out must be 16-byte aligned");
         s2v_graph_fused_args a;
-        a.G = G; a.N = N; a.d = d; a.levels = L;
+        a.G = G; a.N = N; a.E = batch->num_edges; a.d = d; a.levels = L;
         a.max_graph_nodes = batch->max_graph_nodes;
         a.pool_average = model->pool_average;
         a.row_ptr = batch->n2n_row_ptr; a.col_idx = batch->n2n_col_idx; a.val = batch->n2n_val; a.graph_ptr = batch->graph_ptr;

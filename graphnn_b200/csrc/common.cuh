@@ -174,7 +174,7 @@ int s2v_launch_level_first_table(s2v_ctx* ctx, cudaStream_t st, int64_t n, int d
 int s2v_launch_index_check(s2v_ctx* ctx, cudaStream_t st, int64_t n, const int32_t* idx, int limit);
 // batches of whole graphs whose embeddings stay in shared memory across the levels (graph_fused.cu)
 struct s2v_graph_fused_args {
-    int64_t G = 0, N = 0;
+    int64_t G = 0, N = 0, E = 0;     // E: 0 if unknown
     int d = 0, levels = 0, max_graph_nodes = 0, pool_average = 0;
     const int32_t* row_ptr = nullptr;
     const int32_t* col_idx = nullptr;
@@ -198,6 +198,7 @@ struct s2v_graph_fused_args {
 constexpr int64_t S2V_FUSED_TABLE_NODES = 32768;   // batches from this many nodes on: weights and first-level table prepared by launches of their own
 constexpr int64_t S2V_FUSED_EMBED_NODES = 16384;   // batches with embed_out below this many nodes take the per-level kernels
 constexpr int64_t S2V_FUSED_ROUND_NODES = 384;     // d = 32, larger graphs: nodes that a CTA is expected to hold at a time
+constexpr int64_t S2V_FUSED_ROUND_EDGES = 4500;    // ... and entries
 bool s2v_graph_fused_supported(const s2v_ctx* ctx, int d, int max_nodes, int num_tags);
 size_t s2v_graph_fused_image_bytes(int d);
 bool s2v_graph_fused_readout_ok(int d, int hidden, int num_class);

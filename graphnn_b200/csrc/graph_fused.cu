@@ -35,6 +35,9 @@
 // remaining waits return at once and the kernel runs to its end.
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 #include "tcgen05.cuh"
 
@@ -439,35 +442,125 @@ __device__ __forceinline__ void gf_readout(const GfParams& p, const float* y_s, 
     }
 }
 
-// One row's neighbour sum straight from global memory: tiles whose columns do not fit the chunk list, and rows whose
-// edges carry different weights.
-template <int D, bool HAS_VAL>
-__device__ __noinline__ ulonglong2 gf_row_from_global(const int32_t* row_ptr, const int32_t* col_idx, const float* val, s2v_device_status* status,
-                                                      const ulonglong2* H2, int node0, int nrows, int r, int sl)
+// Neighbour sums with the columns (and weights) straight from global memory: tiles whose columns do not fit the chunk list, and tiles
+// with a row whose edges carry different weights.  A row's lanes load its indices side by side, one each, the next ones on their way
+// while these are summed, and hand them round by shuffles: five instructions per neighbour and lane where the list takes four.
+// FIRST: sum of rows of P.  (Four broadcast loads, then four rows, one row at a time: 454 us instead of 270 on 1,000 graphs of 90 nodes
+// with 50 neighbours each, 122 instead of 106 on 250 proteins with unequal weights; one launch per level 270 and 97; d = 64.)
+struct GfFar {
+    uint32_t rows, xo;         // shared memory: H, X offset (d = 128) or tag of each row
+    const ulonglong2* P;
+    int node0, nrows, cap;
+    s2v_device_status* status;
+};
+// all lanes of a warp; col, val, n: the lane group's row (n = 0: none); c, w: its entry number sl, where it has one
+template <int D, bool HAS_VAL, bool FIRST>
+__device__ __noinline__ ulonglong2 gf_row_from_global(const GfFar f, const int32_t* col, const float* val, int n, int c, float w)
 {
-    const int b = __ldg(row_ptr + node0 + r), e = __ldg(row_ptr + node0 + r + 1);
+    using Cfg = GfCfg<D>;
+    constexpr int LPR = Cfg::LPR;
+    const int sl = threadIdx.x % LPR;
+    const int most = __reduce_max_sync(0xffffffffu, n);
     ulonglong2 acc = make_ulonglong2(0ull, 0ull);
-    for (int t = b; t < e; t += 4) {
-        int c[4];
-        float w[4];
+    for (int t = 0; t < most; t += LPR) {
+        const int tn = t + LPR + sl;
+        const int cn = tn < n ? __ldg(col + tn) : 0;
+        const float wn = HAS_VAL && tn < n ? __ldg(val + tn) : 0.f;
+        uint32_t e = (uint32_t)f.cap;   // past the end: the row of zeros
+        if (t + sl < n) {
+            e = (uint32_t)(c - f.node0);
+            if (e >= (uint32_t)f.nrows) {
+                f.status->code = S2V_ERR_BAD_CSR;
+                f.status->where = 5;
+                e = 0;
+            }
+        }
+        if (FIRST) {
+            if (Cfg::TR) {
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e) : "r"(f.xo + 4 * e));
+                e >>= 4;
+            } else {
+                uint16_t tag;
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(tag) : "r"(f.xo + 2 * e));
+                e = (uint32_t)tag * LPR;
+            }
+        } else e = Cfg::TR ? e * LPR : (e << Cfg::SHIFT) + (e & 7u);
+#pragma unroll
+        for (int u0 = 0; u0 < LPR; u0 += 4) {
+            if (t + u0 >= most) break;
+            ulonglong2 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t eu = __shfl_sync(0xffffffffu, e, u0 + u, LPR);
+                if (FIRST) v[u] = __ldg(f.P + eu + sl);
+                else v[u] = gf_lds(f.rows + 16u * (Cfg::TR ? eu + sl : eu ^ (uint32_t)sl));
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (HAS_VAL) {
+                    const float wu = __shfl_sync(0xffffffffu, w, u0 + u, LPR);
+                    const uint64_t ww = pack2(wu, wu);
+                    acc.x = fma2(ww, v[u].x, acc.x);
+                    acc.y = fma2(ww, v[u].y, acc.y);
+                } else {
+                    acc.x = add2(acc.x, v[u].x);
+                    acc.y = add2(acc.y, v[u].y);
+                }
+            }
+        }
+        c = cn;
+        w = wn;
+    }
+    return acc;
+}
+
+// One row's sum with a weight per entry, columns and weights from the lists in shared memory (16,384 molecules with unequal weights:
+// d = 128 577 us from global memory, 466 from the lists, 469 with one launch per level; d = 64 372, 324, 328).  chunk, weights: the row's first ones;
+// most: chunks of the warp's longest row (a row with fewer, mine, adds nothing there).
+template <int D, bool FIRST>
+__device__ __noinline__ ulonglong2 gf_row_weighted(const GfFar f, uint32_t chunk, uint32_t weights, uint32_t mine, uint32_t most)
+{
+    using Cfg = GfCfg<D>;
+    constexpr int LPR = Cfg::LPR;
+    const uint32_t sl = threadIdx.x % LPR;
+    ulonglong2 acc = make_ulonglong2(0ull, 0ull);
+    for (uint32_t c = 0; c < most; ++c) {
+        if (c >= mine) continue;
+        uint32_t e[4];
+        if (Cfg::TR) {
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(e[0]), "=r"(e[1]), "=r"(e[2]), "=r"(e[3]) : "r"(chunk + 16 * c));
+        } else {
+            uint32_t lo, hi;
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(chunk + 8 * c));
+            e[0] = lo & 0xffffu; e[1] = lo >> 16; e[2] = hi & 0xffffu; e[3] = hi >> 16;
+        }
+        const ulonglong2 w2 = gf_lds(weights + 16 * c);
+        const float2 w01 = unpack2(w2.x), w23 = unpack2(w2.y);
+        const float w[4] = {w01.x, w01.y, w23.x, w23.y};
+        ulonglong2 v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            c[u] = t + u < e ? __ldg(col_idx + t + u) - node0 : 0;
-            w[u] = HAS_VAL && t + u < e ? __ldg(val + t + u) : 1.f;
+            if (FIRST) {
+                uint32_t x;
+                if (Cfg::TR) {
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(f.xo + ((e[u] - Cfg::OFF_H) >> 7)));
+                    x >>= 4;
+                } else {
+                    uint16_t tag;
+                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(tag) : "r"(f.xo + 2 * (e[u] >> Cfg::SHIFT)));
+                    x = (uint32_t)tag * LPR;
+                }
+                v[u] = __ldg(f.P + x + sl);
+            } else {
+                v[u] = gf_lds(Cfg::TR ? f.rows - Cfg::OFF_H + e[u] + 16 * sl : f.rows + 16 * (e[u] ^ sl));
+            }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (t + u < e) {
-                if ((unsigned)c[u] >= (unsigned)nrows) {
-                    status->code = S2V_ERR_BAD_CSR;
-                    status->where = 5;
-                    c[u] = 0;
-                }
-                const ulonglong2 v = H2[gf_h<D>(c[u], sl)];
-                const uint64_t ww = pack2(w[u], w[u]);
-                acc.x = fma2(ww, v.x, acc.x);
-                acc.y = fma2(ww, v.y, acc.y);
-            }
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t ww = pack2(w[u], w[u]);
+            acc.x = fma2(ww, v[u].x, acc.x);
+            acc.y = fma2(ww, v[u].y, acc.y);
+        }
     }
     return acc;
 }
@@ -682,9 +775,39 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         }
         gf_worker_sync<WT>();
         // averaged messages give every edge of a row the same weight: the row is summed unweighted and scaled once
-        const bool listed = cached && !(HAS_VAL && *s_mixed != 0);
+        const bool mixed = HAS_VAL && *s_mixed != 0;
+        const bool listed = cached && !mixed;
+        // different weights in a row: they are listed behind the columns, where there is room
+        const uint32_t weights_at = smem_u32(smem + map.col) + gf_up(Cfg::CHUNK * (uint32_t)carry, 16);
+        const bool weighted = mixed && cached && gf_up(Cfg::CHUNK * (uint32_t)carry, 16) + 16u * (uint32_t)carry <= Cfg::CHUNK * (uint32_t)p.chunk_cap;
+        if (weighted) {
+            float4* const wl = reinterpret_cast<float4*>(smem + map.col + gf_up(Cfg::CHUNK * (uint32_t)carry, 16));
+            for (int r = threadIdx.x; r < nrows; r += WT) {
+                const int b = __ldg(p.row_ptr + node0 + r), n = __ldg(p.row_ptr + node0 + r + 1) - b;
+                float4* const to = wl + (info_s[r] & 0xffffu);
+                for (int t = 0; t < n; t += 4) {
+                    auto w = [&](int u) { return t + u < n ? __ldg(p.val + b + t + u) : 0.f; };
+                    to[t >> 2] = make_float4(w(0), w(1), w(2), w(3));
+                }
+            }
+            gf_worker_sync<WT>();
+        }
+        auto far_rows = [&]() {
+            return GfFar{smem_u32(smem + Cfg::OFF_H), smem_u32(smem + map.tags), reinterpret_cast<const ulonglong2*>(p.P), node0, nrows, p.cap, p.status};
+        };
+        auto weighted_row = [&](auto first, int r) {   // all lanes of a warp; r: the lane group's row, or beyond the last one
+            const uint32_t inf = r < nrows ? info_s[r] : 0u, mine = ((inf >> 16) + 3) / 4;
+            return gf_row_weighted<D, decltype(first)::value>(far_rows(), smem_u32(smem + map.col) + Cfg::CHUNK * (inf & 0xffffu), weights_at + 16u * (inf & 0xffffu),
+                                                              mine, __reduce_max_sync(0xffffffffu, mine));
+        };
         if (p.P) {   // first level: a sum of rows of P = ReLU(W_in) * W, no product
             const float4* __restrict__ P4 = reinterpret_cast<const float4*>(p.P);
+            auto finish_first = [&](int r, ulonglong2 v) {
+                if (r >= nrows) return;
+                const float4 x = __ldg(X4 + (Cfg::TR ? (int64_t)(xo_s[r] / 16u) : (int64_t)tag_s[r] * LPR) + sl);
+                const float2 f0 = unpack2(v.x), f1 = unpack2(v.y);
+                H4[gf_h<D>(r, sl)] = make_float4(relu_max(f0.x + x.x), relu_max(f0.y + x.y), relu_max(f1.x + x.z), relu_max(f1.y + x.w));
+            };
             if (Cfg::TR && listed) {
                 // two rows at a time, so that ten table reads are on their way together
                 const char* const Pl = reinterpret_cast<const char*>(p.P) + 16 * lane;
@@ -725,39 +848,51 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                         if (ra[a] < nrows) H4[ra[a] * 32 + lane] = make_float4(relu_max(f0.x), relu_max(f0.y), relu_max(f1.x), relu_max(f1.y));
                     }
                 }
-            } else
-            for (int r = grp; r < nrows; r += NG) {
-                auto x_of = [&](int c) { return Cfg::TR ? (int64_t)(xo_s[c] / 16u) : (int64_t)tag_s[c] * LPR; };
-                const float4 x = __ldg(X4 + x_of(r) + sl);
-                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (listed) {
+            } else if (!Cfg::TR && listed) {
+                for (int r = grp; r < nrows; r += NG) {
+                    const float4 x = __ldg(X4 + (int64_t)tag_s[r] * LPR + sl);
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
                     const uint32_t inf = info_s[r];
                     for (uint32_t c = 0; c < ((inf >> 16) + 3) / 4; ++c) {
                         const uint2 e2 = chunks[(inf & 0xffffu) + c];
                         const uint32_t e[4] = {e2.x & 0xffffu, e2.x >> 16, e2.y & 0xffffu, e2.y >> 16};
                         float4 v[4];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) v[u] = __ldg(P4 + x_of((int)(e[u] >> Cfg::SHIFT)) + sl);
+                        for (int u = 0; u < 4; ++u) v[u] = __ldg(P4 + (int64_t)tag_s[e[u] >> Cfg::SHIFT] * LPR + sl);
 #pragma unroll
                         for (int u = 0; u < 4; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
                     }
                     if (HAS_VAL) { const float w = roww[r]; acc.x *= w; acc.y *= w; acc.z *= w; acc.w *= w; }
-                } else {
-                    const int b = __ldg(p.row_ptr + node0 + r), e = __ldg(p.row_ptr + node0 + r + 1);
-                    for (int t = b; t < e; ++t) {
-                        int c = __ldg(p.col_idx + t) - node0;
-                        if ((unsigned)c >= (unsigned)nrows) {
-                            p.status->code = S2V_ERR_BAD_CSR;
-                            p.status->where = 5;
-                            c = 0;
-                        }
-                        const float w = HAS_VAL ? __ldg(p.val + t) : 1.f;
-                        const float4 v = __ldg(P4 + x_of(c) + sl);
-                        acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
-                    }
+                    H4[gf_h<D>(r, sl)] =
+                        make_float4(relu_max(acc.x + x.x), relu_max(acc.y + x.y), relu_max(acc.z + x.z), relu_max(acc.w + x.w));
                 }
-                H4[gf_h<D>(r, sl)] =
-                    make_float4(relu_max(acc.x + x.x), relu_max(acc.y + x.y), relu_max(acc.z + x.z), relu_max(acc.w + x.w));
+            } else if (HAS_VAL && weighted) {
+                for (int rw = warp * GPW; rw < nrows; rw += NG) {   // warp-uniform
+                    const int r = rw + sub;
+                    const ulonglong2 v = weighted_row(std::true_type{}, r);
+                    finish_first(r, v);
+                }
+            } else {
+                const GfFar far = far_rows();
+                auto span = [&](int r, int& b, int& n) {
+                    b = n = 0;
+                    if (r < nrows) { b = __ldg(p.row_ptr + node0 + r); n = __ldg(p.row_ptr + node0 + r + 1) - b; }
+                };
+                int b0, n0, b1, n1;   // this row's entries and the next one's
+                span(grp, b0, n0);
+                span(grp + NG, b1, n1);
+                int c0 = sl < n0 ? __ldg(p.col_idx + b0 + sl) : 0;
+                float w0 = HAS_VAL && sl < n0 ? __ldg(p.val + b0 + sl) : 0.f;
+                for (int rw = warp * GPW; rw < nrows; rw += NG) {   // warp-uniform
+                    const int r = rw + sub;
+                    int b2, n2;
+                    span(r + 2 * NG, b2, n2);
+                    const int c1 = sl < n1 ? __ldg(p.col_idx + b1 + sl) : 0;
+                    const float w1 = HAS_VAL && sl < n1 ? __ldg(p.val + b1 + sl) : 0.f;
+                    const ulonglong2 v = gf_row_from_global<D, HAS_VAL, true>(far, p.col_idx + b0, p.val + b0, n0, c0, w0);
+                    finish_first(r, v);
+                    b0 = b1; n0 = n1; b1 = b2; n1 = n2; c0 = c1; w0 = w1;
+                }
             }
             gf_worker_sync<WT>();
         }
@@ -841,17 +976,45 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                             }
                         }
                     }
-                } else {
+                } else if (HAS_VAL && weighted) {
 #pragma unroll
                     for (int i = 0; i < RPG; ++i) {
                         a0[i] = a1[i] = 0ull;
-                        if (i * NG + grp < rows_m) {
-                            const ulonglong2 v = gf_row_from_global<D, HAS_VAL>(p.row_ptr, p.col_idx, p.val, p.status, H2, node0, nrows, RB * m + i * NG + grp, sl);
+                        if (i * NG + warp * GPW < rows_m) {   // warp-uniform
+                            const ulonglong2 v = weighted_row(std::false_type{}, RB * m + i * NG + grp);
                             a0[i] = v.x;
                             a1[i] = v.y;
                         }
                     }
-                    __syncwarp();
+                } else {
+                    const GfFar far = far_rows();
+                    int rb[RPG], rn[RPG];
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) {
+                        rb[i] = rn[i] = 0;
+                        if (i * NG + grp < rows_m) {
+                            const int32_t* const rp = p.row_ptr + node0 + RB * m + i * NG + grp;
+                            rb[i] = __ldg(rp);
+                            rn[i] = __ldg(rp + 1) - rb[i];
+                        }
+                    }
+                    int c = sl < rn[0] ? __ldg(p.col_idx + rb[0] + sl) : 0;
+                    float w = HAS_VAL && sl < rn[0] ? __ldg(p.val + rb[0] + sl) : 0.f;
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) {
+                        constexpr int LAST = RPG - 1;
+                        const int j = i < LAST ? i + 1 : LAST;
+                        const int cn = i < LAST && sl < rn[j] ? __ldg(p.col_idx + rb[j] + sl) : 0;
+                        const float wn = HAS_VAL && i < LAST && sl < rn[j] ? __ldg(p.val + rb[j] + sl) : 0.f;
+                        a0[i] = a1[i] = 0ull;
+                        if (i * NG + warp * GPW < rows_m) {   // warp-uniform
+                            const ulonglong2 v = gf_row_from_global<D, HAS_VAL, false>(far, p.col_idx + rb[i], p.val + rb[i], rn[i], c, w);
+                            a0[i] = v.x;
+                            a1[i] = v.y;
+                        }
+                        c = cn;
+                        w = wn;
+                    }
                 }
                 // the operand buffer is free once the previous row block of this level is multiplied
                 if (m > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 40);
@@ -1168,18 +1331,22 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
             if (cap < need) cap = need;
         } else cap = 1024;
     }
-    p.cap = cap;
-    uint32_t cols = 32;
-    while (cols < (uint32_t)(cap / 128 * a.d)) cols *= 2;
-    p.tm_cols = a.d == 128 ? 256 : cols;   // d = 128: W^T and the accumulators of two row blocks
-    // what is left of the CTA's share of shared memory lists the columns (8 bytes per four)
+    // What is left of the CTA's share of shared memory lists the columns (four to a chunk).  Six chunks per row, or what
+    // the batch's mean asks for (1,000 graphs of 90 nodes, 30 neighbours each, d = 64: 199 us unlisted, 174).  Tiles get smaller as long as the list
+    // would not hold a full one's (d = 32, averaged messages, 16,384 molecules: tiles of 640 rows take 179 us, of 512 152).
     const bool hv = a.val != nullptr;
     auto total = [&](int n) {
         return a.d == 128 ? gf_map<128>(cap, n, hv).total : (a.d == 64 ? gf_map<64>(cap, n, hv).total : gf_map<32>(cap, n, hv).total);
     };
     const uint32_t budget = per_sm == 2 ? 113 * 1024 : 227 * 1024;
     const uint32_t chunk = a.d == 128 ? GfCfg<128>::CHUNK : 8u;
-    const uint32_t left = (budget - total(0)) / 16 * 16, enough = (uint32_t)cap * chunk * 6u;   // six chunks per row are plenty
+    const double per_row = std::min(std::max(1.1, a.N > 0 ? 0.25 * (double)a.E / (double)a.N + 0.375 : 0.), 4096.);   // chunks: rows end inside one
+    while (cap - 128 >= need && (budget - total(0)) / chunk < per_row * cap) cap -= 128;
+    p.cap = cap;
+    uint32_t cols = 32;
+    while (cols < (uint32_t)(cap / 128 * a.d)) cols *= 2;
+    p.tm_cols = a.d == 128 ? 256 : cols;   // d = 128: W^T and the accumulators of two row blocks
+    const uint32_t left = (budget - total(0)) / 16 * 16, enough = (uint32_t)(cap * std::max(6.0, 1.25 * per_row)) / 2 * 2 * chunk;   // (more would take from the cache)
     p.chunk_cap = (int)((left < enough ? left : enough) / chunk);
     const uint32_t smem = total(p.chunk_cap);
     const int64_t most = (int64_t)ctx->sm_count * per_sm;

@@ -90,6 +90,37 @@ def test_fused_forward(d, sizes, degree, opts):
     assert np.array_equal(pred.cpu().numpy(), logits.cpu().numpy().argmax(1))
 
 
+@pytest.mark.parametrize("auto", [False, True])                     # first level through the product table, and through the MMAs
+@pytest.mark.parametrize("val", [None, "row", "mixed"])
+@pytest.mark.parametrize("d,sizes,degree", [
+    (64, [640, 100, 300, 0, 1], 30.0),                               # columns straight from global memory: more of them than a row has
+    (32, [1024, 641, 3], 60.0),                                      # lanes (8, 16, 32), rows of 0, 1 and a few entries among them
+    (128, [128, 1, 100, 7, 127], 60.0),
+    (128, [33, 65, 2] * 40, 2.2), (64, [33, 65, 2] * 40, 2.2), (32, [33, 65, 2] * 40, 2.2),   # weights listed beside the columns
+    (64, [90] * 400, 12.0),                                          # several tiles per CTA, lists used again
+], ids=lambda v: None)
+def test_fused_columns_and_weights_outside_and_inside_the_list(d, sizes, degree, val, auto):
+    b = make(sizes, degree, d, 9, 3, 64, 3, seed=d + len(sizes))
+    hb = engine.build_host_batch(b)
+    eng = engine.S2VInference(b.weights, b.levels)
+    if not auto:
+        eng.ctx.set_option(eng.ctx.OPT_GRAPH_TILES, 1)
+    db = eng.to_device(hb)
+    rp, ci = hb.row_ptr.numpy(), hb.col_idx.numpy()
+    v = None
+    if val == "row":
+        v = np.repeat((1.0 / np.maximum(np.diff(rp), 1)).astype(np.float32), np.diff(rp))
+    elif val == "mixed":
+        v = (np.random.default_rng(3).random(len(ci), dtype=np.float32) - 0.3).astype(np.float32)
+    if v is not None:
+        db.val = torch.from_numpy(v).cuda()
+    logits, _, _, emb = eng.forward(db, want_embed=True)
+    eng.ctx.synchronize()
+    want_h, want = f64(b, rp, ci, v, None, False)
+    assert_close(emb.cpu().numpy(), want_h, "embeddings", scale=max(1.0, float(np.abs(want_h).max())))
+    assert_close(logits.cpu().numpy(), want, "logits", scale=max(1.0, float(np.abs(want).max())))
+
+
 def test_fused_reports_a_graph_beyond_the_hint_and_an_edge_between_graphs():
     b = make([30, 300, 25], 2.0, 64, 5, 2, 64, 2, seed=1)
     eng = engine.S2VInference(b.weights, b.levels)
