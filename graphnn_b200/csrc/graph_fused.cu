@@ -21,9 +21,10 @@
 //             two taken from its own largest element, split it into an fp16 head and tail and store both as the
 //             K-major MMA operand.  The scale is per row, so a graph's results do not depend on its neighbours in the tile.
 //   product : one warp issues tcgen05.mma, A = the 128 rows, B = W^T (head and tail, scaled by its largest element):
-//             tail*head, head*tail, head*head into one fp32 accumulator in tensor memory.  fp16 head + tail carry 22
-//             bits of every element within 2^-17 of its row's largest one and 2^-39 of that largest one below it: the
-//             TF32 head + tail pair carries the same 22 bits, at twice the operand bytes and half the MMA rate.
+//             tail*head, head*tail, head*head into one fp32 accumulator in tensor memory.  W and the sums are scaled by
+//             powers of two (GfScales, and a scale per row of sums); fp16 head + tail then carry 22 bits of every element
+//             within 2^-17 of its row's largest one and 2^-39 of that largest one below it: the TF32 head + tail pair
+//             carries the same 22 bits, at twice the operand bytes and half the MMA rate.
 //   drain   : once every row block of the level is multiplied (tensor memory holds the whole new H, so no second copy
 //             in shared memory is needed): accumulator * 2^-k + X, ReLU, back into the H rows.
 // d = 128 takes the product transposed, W^T (A operand, in tensor memory) times the row block's sums, in row blocks of 64: an
@@ -97,7 +98,7 @@ __host__ __device__ constexpr uint32_t gf_up(uint32_t v, uint32_t a) { return (v
 
 // Byte offsets behind the H rows (one row more than cap: a row of zeros, what an unused gather slot adds).
 struct GfMap {
-    uint32_t info, roww, tags, goff, rs, bar, col, total;
+    uint32_t info, roww, tags, goff, rs, bar, ws, col, total;
 };
 template <int D>
 __host__ __device__ inline GfMap gf_map(int cap, int chunk_cap, bool has_val)
@@ -109,7 +110,8 @@ __host__ __device__ inline GfMap gf_map(int cap, int chunk_cap, bool has_val)
     m.goff = m.tags + gf_up((GfCfg<D>::TR ? 4u : 2u) * (uint32_t)(cap + 1), 16);   // TR: byte offsets of the rows' X, else tags
     m.rs = m.goff + gf_up(4u * (GfCfg<D>::MAXG + 1), 16);              // per row: exponent of its operand scale (TR: what its products are multiplied by)
     m.bar = m.rs + (GfCfg<D>::TR ? 4u : 1u) * (uint32_t)cap;
-    m.col = m.bar + 160;                                               // chunks of four local columns: 16-bit indices into H (TR: byte offsets)
+    m.ws = m.bar + 160;                                                // what W was scaled by: GfScales
+    m.col = m.ws + 8u * D + 16u;                                            // chunks of four local columns: 16-bit indices into H (TR: byte offsets)
     m.total = m.col + gf_up(GfCfg<D>::CHUNK * (uint32_t)chunk_cap, 16) + 1024;   // + slack to align the base to 1024 bytes
     return m;
 }
@@ -239,40 +241,145 @@ __device__ __forceinline__ int64_t gf_lower_graph(const int32_t* graph_ptr, int6
     return lo;
 }
 
+// Scales of W, powers of two.  Where all its rows and columns are of about one size, one for all of it, which the scale of a row of
+// sums takes in.  Otherwise one on either side, W'[k][n] = W[k][n] / in[k] / out[n], so that the largest element of every column and
+// (nearly) of every row of W' is 2^14 .. 2^15; the sums are then multiplied by in[k] before they are split and the products by out[n],
+// and a result does not depend on the units its features are held in: with one scale, an output feature whose weights are 2^-24 of the
+// largest has lost half of its 22 bits.  (A column below 2^-64 of its rows is not scaled up all the way.)  Of one size: no row or column
+// (or the part of it that a warp or a thread holds) whose largest element is more than 2^EVEN below the largest of all; what is
+// lost is then 2^-31 at most.  An infinite weight calls for two scales, to which infinities and NaN don't count.
+// One scale without a look at the rows and columns: 335 us on 16,384 molecules (d = 128), 16.3 on 64 small graphs (d = 64); two always:
+// 341 and 17.8; as it is: 338 and 16.8.
+template <int D>
+struct GfScales {
+    float out[D];
+    float in[D];
+    float all;              // one scale: what the products are multiplied by (1 with scales on both sides)
+    uint32_t uneven;        // scales on both sides
+    uint32_t pad[2];
+};
+static_assert(sizeof(GfScales<64>) == 8 * 64 + 16, "its place in GfMap");
+template <int D>
+struct GfScaleWork {        // while W is converted (in the operand buffer's place)
+    float down[D];          // 1 / in
+    uint32_t row_max[D], col_max[D];
+    uint32_t most, least;   // largest element; smallest of the rows' and columns' largest ones
+    static constexpr uint32_t EVEN = 8;
+    __device__ __forceinline__ void clear()
+    {
+        if (threadIdx.x < D) row_max[threadIdx.x] = col_max[threadIdx.x] = 0u;
+        if (threadIdx.x == 0) { most = 0u; least = ~0u; }
+    }
+    // col: bits of the largest of the thread's elements, all of one column; row: the smallest of the rows' largest ones, as far as the warp sees them
+    __device__ __forceinline__ void add(uint32_t col, uint32_t row)
+    {
+        const uint32_t w = __reduce_max_sync(0xffffffffu, col), l = min(row, __reduce_min_sync(0xffffffffu, col));
+        if ((threadIdx.x & 31) == 0) {
+            atomicMax(&most, w);
+            atomicMin(&least, l);
+        }
+    }
+    // behind a barrier: whether one scale will do (its exponent stays clear of the ends of the range)
+    __device__ __forceinline__ bool even() const { return (least >> 23) + EVEN >= (most >> 23) && (most >> 23) >= 87u && (most >> 23) <= 167u; }
+    __device__ __forceinline__ float all_up() const { return pow2(268u - (most >> 23)); }
+    __device__ __forceinline__ float all_out() const { return pow2((most >> 23) - 14u); }
+    __device__ __forceinline__ static uint32_t finite_bits(float v)
+    {
+        const uint32_t b = __float_as_uint(fabsf(v));
+        return b < 0x7f800000u ? b : 0u;
+    }
+    __device__ __forceinline__ static float pow2(uint32_t biased) { return __uint_as_float(biased << 23); }
+    // behind the rows' maxima, between two barriers (exponents that keep both scales normal numbers)
+    __device__ __forceinline__ void finish_rows(GfScales<D>* s)
+    {
+        if (threadIdx.x >= D) return;
+        const uint32_t e = min(max(row_max[threadIdx.x] >> 23, 15u), 253u);
+        s->in[threadIdx.x] = pow2(e);
+        down[threadIdx.x] = pow2(254u - e);
+    }
+    // behind a barrier after the columns' maxima: what brings a column's largest element to 2^14 .. 2^15
+    __device__ __forceinline__ uint32_t col_exponent(int n) const { return max(col_max[n] >> 23, 63u); }
+    __device__ __forceinline__ float col_up(int n) const { return pow2(268u - col_exponent(n)); }
+    __device__ __forceinline__ void finish_cols(GfScales<D>* s) const
+    {
+        if (threadIdx.x < D) s->out[threadIdx.x] = pow2(col_exponent(threadIdx.x) - 14u);
+    }
+};
+
 // W^T as the B operand: scaled fp16 head and tail.  Thread t converts pairs of consecutive k of one column n.
-// s_max is zeroed beforehand; contains a barrier, so every thread of the CTA calls it.
+// `work` is cleared beforehand; contains barriers, so every thread of the CTA calls it.
 template <int D, int THREADS>
-__device__ __forceinline__ void gf_convert_w(const float* __restrict__ W, unsigned char* dst, uint32_t* s_max, float& inv_w)
+__device__ __forceinline__ bool gf_convert_w(const float* __restrict__ W, unsigned char* dst, GfScales<D>* scales, GfScaleWork<D>* work, float& all)
 {
     constexpr int PAIRS = D * D / 2, PER = (PAIRS + THREADS - 1) / THREADS;
+    static_assert(THREADS % D == 0, "a thread stays in one column, a warp in one row");
+    const int n = threadIdx.x % D;
     float a[PER][2];
-    float m = 0.f;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-        const int p = threadIdx.x + i * THREADS;
-        const int n = p % D, k = p / D * 2;
+        const int p = threadIdx.x + i * THREADS, k = p / D * 2;
         a[i][0] = p < PAIRS ? __ldg(W + k * D + n) : 0.f;
         a[i][1] = p < PAIRS ? __ldg(W + (k + 1) * D + n) : 0.f;
     }
+    {
+        float col = 0.f;
+        uint32_t row = ~0u;
 #pragma unroll
-    for (int i = 0; i < PER; ++i) m = fmaxf(m, fmaxf(fabsf(a[i][0]), fabsf(a[i][1])));
-    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-    if ((threadIdx.x & 31) == 0) atomicMax(s_max, w);
+        for (int i = 0; i < PER; ++i) col = fmaxf(col, fmaxf(fabsf(a[i][0]), fabsf(a[i][1])));
+        auto look = [&](auto first) {   // D / 32 warps hold a row; each looks at its share of the rows
+#pragma unroll
+            for (int i = decltype(first)::value; i < PER; i += D / 32)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) row = min(row, __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(a[i][h]))));
+        };
+        if (D == 32 || ((threadIdx.x >> 5) & 1) == 0) look(std::integral_constant<int, 0>{});
+        else look(std::integral_constant<int, 1>{});
+        if (threadIdx.x < PAIRS) work->add(__float_as_uint(col), row);   // (whole warps)
+    }
     __syncthreads();
-    const uint32_t e_w = gf_exponent(*s_max);
-    const float s = gf_scale(e_w);
-    inv_w = gf_unscale(e_w);
+    float up = work->all_up();
+    const bool even = work->even();
+    all = even ? work->all_out() : 1.f;
+    if (!even) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int p = threadIdx.x + i * THREADS, k = p / D * 2;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t w = __reduce_max_sync(0xffffffffu, work->finite_bits(a[i][h]));
+                if (p < PAIRS && (threadIdx.x & 31) == 0) atomicMax(work->row_max + k + h, w);
+            }
+        }
+        __syncthreads();
+        work->finish_rows(scales);
+        __syncthreads();
+        uint32_t m = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int p = threadIdx.x + i * THREADS, k = p / D * 2;
+            if (p < PAIRS) {
+                const float2 down = *reinterpret_cast<const float2*>(work->down + k);
+                a[i][0] *= down.x;
+                a[i][1] *= down.y;
+                m = max(m, max(work->finite_bits(a[i][0]), work->finite_bits(a[i][1])));
+            }
+        }
+        atomicMax(work->col_max + n, m);
+        __syncthreads();
+        work->finish_cols(scales);
+        up = work->col_up(n);
+    }
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-        const int p = threadIdx.x + i * THREADS;
+        const int p = threadIdx.x + i * THREADS, k = p / D * 2;
         if (p < PAIRS) {
-            const int n = p % D, k = p / D * 2;
             uint32_t hi, lo;
-            split_f16(pack2(a[i][0] * s, a[i][1] * s), hi, lo);
+            split_f16(pack2(a[i][0] * up, a[i][1] * up), hi, lo);
             *reinterpret_cast<uint32_t*>(dst + gf_op_off(n, k, D)) = hi;
             *reinterpret_cast<uint32_t*>(dst + gf_op_off_lo<D>(n, k, D, GfCfg<D>::W_LO)) = lo;
         }
     }
+    return !even;
 }
 
 // d = 128: W^T as the A operand in tensor memory: lane m = output feature, column c = the pair of input features 2c, 2c + 1.
@@ -289,76 +396,152 @@ __device__ __forceinline__ void gf_store_w_pairs(uint32_t tmem, const uint32_t (
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 // image: word (c, m) at c * 128 + m, heads first, tails behind them
-__device__ __forceinline__ void gf_load_w_t(const void* image, uint32_t tmem, float& inv_w)
+__device__ __forceinline__ void gf_load_w_t(const void* image, uint32_t tmem)
 {
     const int warp = threadIdx.x >> 5, m = 32 * (warp & 3) + (threadIdx.x & 31);
     const uint32_t* w = static_cast<const uint32_t*>(image) + (32 * (warp >> 2)) * 128 + m;
     uint32_t hi[32], lo[32];
 #pragma unroll
     for (int c = 0; c < 32; ++c) { hi[c] = __ldg(w + c * 128); lo[c] = __ldg(w + 64 * 128 + c * 128); }
-    inv_w = __ldg(static_cast<const float*>(image) + 128 * 128);
     gf_store_w_pairs(tmem, hi, lo);
 }
-__device__ __forceinline__ void gf_convert_w_t(const float* __restrict__ W, uint32_t tmem, uint32_t* s_max, float& inv_w)
+__device__ __forceinline__ bool gf_convert_w_t(const float* __restrict__ W, uint32_t tmem, GfScales<128>* scales, GfScaleWork<128>* work, float& all)
 {
-    const int warp = threadIdx.x >> 5, m = 32 * (warp & 3) + (threadIdx.x & 31);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = 32 * (warp & 3) + lane, k0 = 64 * (warp >> 2);
     float a[64];
 #pragma unroll
-    for (int k = 0; k < 64; ++k) a[k] = __ldg(W + (64 * (warp >> 2) + k) * 128 + m);
-    float mx = 0.f;
+    for (int k = 0; k < 64; ++k) a[k] = __ldg(W + (k0 + k) * 128 + m);
+    {
+        float col = 0.f;
+        uint32_t row = ~0u;
 #pragma unroll
-    for (int k = 0; k < 64; ++k) mx = fmaxf(mx, fabsf(a[k]));
-    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-    if ((threadIdx.x & 31) == 0) atomicMax(s_max, w);
+        for (int k = 0; k < 64; ++k) col = fmaxf(col, fabsf(a[k]));
+        auto look = [&](auto first) {   // four warps hold a row; each looks at a quarter of the rows
+#pragma unroll
+            for (int k = decltype(first)::value; k < 64; k += 4) row = min(row, __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(a[k]))));
+        };
+        switch (warp & 3) {
+            case 0: look(std::integral_constant<int, 0>{}); break;
+            case 1: look(std::integral_constant<int, 1>{}); break;
+            case 2: look(std::integral_constant<int, 2>{}); break;
+            default: look(std::integral_constant<int, 3>{});
+        }
+        work->add(__float_as_uint(col), row);
+    }
     __syncthreads();
-    const uint32_t e_w = gf_exponent(*s_max);
-    const float sc = gf_scale(e_w);
-    inv_w = gf_unscale(e_w);
+    float up = work->all_up();
+    const bool even = work->even();
+    all = even ? work->all_out() : 1.f;
+    if (!even) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t mine = 0;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+                const uint32_t w = __reduce_max_sync(0xffffffffu, work->finite_bits(a[32 * h + k]));
+                if (lane == k) mine = w;
+            }
+            atomicMax(work->row_max + k0 + 32 * h + lane, mine);
+        }
+        __syncthreads();
+        work->finish_rows(scales);
+        __syncthreads();
+        uint32_t mx = 0;
+#pragma unroll
+        for (int k = 0; k < 64; k += 4) {
+            const float4 down = *reinterpret_cast<const float4*>(work->down + k0 + k);
+            a[k] *= down.x; a[k + 1] *= down.y; a[k + 2] *= down.z; a[k + 3] *= down.w;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) mx = max(mx, work->finite_bits(a[k + u]));
+        }
+        atomicMax(work->col_max + m, mx);
+        __syncthreads();
+        work->finish_cols(scales);
+        up = work->col_up(m);
+    }
     uint32_t hi[32], lo[32];
 #pragma unroll
-    for (int c = 0; c < 32; ++c) split_f16(pack2(a[2 * c] * sc, a[2 * c + 1] * sc), hi[c], lo[c]);
+    for (int c = 0; c < 32; ++c) split_f16(pack2(a[2 * c] * up, a[2 * c + 1] * up), hi[c], lo[c]);
     gf_store_w_pairs(tmem, hi, lo);
-}
-__global__ void __launch_bounds__(1024) gf_weight_image_t_kernel(const float* __restrict__ W, uint32_t* __restrict__ image)
-{
-    __shared__ uint32_t s_max;
-    if (threadIdx.x == 0) s_max = 0;
-    __syncthreads();
-    float a[8][2], mx = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int e = threadIdx.x + i * 1024, m = e % 128, c = e / 128;
-        a[i][0] = __ldg(W + (2 * c) * 128 + m);
-        a[i][1] = __ldg(W + (2 * c + 1) * 128 + m);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fmaxf(fabsf(a[i][0]), fabsf(a[i][1])));
-    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, w);
-    __syncthreads();
-    const uint32_t e_w = gf_exponent(s_max);
-    const float sc = gf_scale(e_w);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int e = threadIdx.x + i * 1024;
-        uint32_t hi, lo;
-        split_f16(pack2(a[i][0] * sc, a[i][1] * sc), hi, lo);
-        image[e] = hi;
-        image[64 * 128 + e] = lo;
-    }
-    if (threadIdx.x == 0) reinterpret_cast<float*>(image)[128 * 128] = gf_unscale(e_w);
+    return !even;
 }
 
-// the same into global memory, once per batch: [operand image | inverse scale]
+// The same into global memory, once per batch: [operand image | scales].
 template <int D>
 __global__ void __launch_bounds__(1024) gf_weight_image_kernel(const float* __restrict__ W, unsigned char* __restrict__ image)
 {
-    __shared__ uint32_t s_max;
-    if (threadIdx.x == 0) s_max = 0;
+    __shared__ __align__(16) GfScales<D> scales;
+    __shared__ __align__(16) GfScaleWork<D> work;
+    work.clear();
     __syncthreads();
-    float inv;
-    gf_convert_w<D, 1024>(W, image, &s_max, inv);
-    if (threadIdx.x == 0) *reinterpret_cast<float*>(image + GfCfg<D>::W_BYTES) = inv;
+    float all;
+    bool uneven;
+    if constexpr (D == 128) {
+        uint32_t* const words = reinterpret_cast<uint32_t*>(image);
+        const int m = threadIdx.x % 128;
+        float a[8][2];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = threadIdx.x / 128 + 8 * i;
+            a[i][0] = __ldg(W + (2 * c) * 128 + m);
+            a[i][1] = __ldg(W + (2 * c + 1) * 128 + m);
+        }
+        float col = 0.f;
+        uint32_t row = ~0u;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                col = fmaxf(col, fabsf(a[i][h]));
+                row = min(row, __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(a[i][h]))));
+            }
+        work.add(__float_as_uint(col), row);
+        __syncthreads();
+        float up = work.all_up();
+        const bool even = work.even();
+        all = even ? work.all_out() : 1.f;
+        uneven = !even;
+        if (!even) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t w = __reduce_max_sync(0xffffffffu, work.finite_bits(a[i][h]));
+                    if ((threadIdx.x & 31) == 0) atomicMax(work.row_max + 2 * (threadIdx.x / 128 + 8 * i) + h, w);
+                }
+            __syncthreads();
+            work.finish_rows(&scales);
+            __syncthreads();
+            uint32_t mx = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float2 down = *reinterpret_cast<const float2*>(work.down + 2 * (threadIdx.x / 128 + 8 * i));
+                a[i][0] *= down.x;
+                a[i][1] *= down.y;
+                mx = max(mx, max(work.finite_bits(a[i][0]), work.finite_bits(a[i][1])));
+            }
+            atomicMax(work.col_max + m, mx);
+            __syncthreads();
+            work.finish_cols(&scales);
+            up = work.col_up(m);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int e = threadIdx.x + i * 1024;
+            uint32_t hi, lo;
+            split_f16(pack2(a[i][0] * up, a[i][1] * up), hi, lo);
+            words[e] = hi;
+            words[64 * 128 + e] = lo;
+        }
+    } else {
+        uneven = gf_convert_w<D, 1024>(W, image, &scales, &work, all);
+    }
+    if (threadIdx.x == 0) {
+        scales.all = all;
+        scales.uneven = uneven ? 1u : 0u;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < (int)(sizeof(scales) / 4); e += 1024) reinterpret_cast<float*>(image + GfCfg<D>::W_BYTES)[e] = reinterpret_cast<const float*>(&scales)[e];
 }
 
 template <int WT>
@@ -594,7 +777,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + map.bar);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + map.bar + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + map.bar + 24);
-    uint32_t* s_max = reinterpret_cast<uint32_t*>(smem + map.bar + 28);
+    GfScales<D>* const scales = reinterpret_cast<GfScales<D>*>(smem + map.ws);
+    GfScaleWork<D>* const scale_work = reinterpret_cast<GfScaleWork<D>*>(smem + Cfg::OFF_S);
     int* s_range = reinterpret_cast<int*>(smem + map.bar + 32);
     int* s_mixed = reinterpret_cast<int*>(smem + map.bar + 44);
     int* s_scan = reinterpret_cast<int*>(smem + map.bar + 64);   // WARPS totals
@@ -607,7 +791,6 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         tc_mbar_init(bar_mma, 1);
         tc_mbar_init(bar_full, WARPS);
         *abort_flag = 0;
-        *s_max = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -623,6 +806,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         if (lane == 0) s_range[warp - 1] = (int)g;
     }
     if (threadIdx.x < LPR) H4[p.cap * LPR + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);   // the row of zeros
+    scale_work->clear();
     const uint32_t zero_entry = (uint32_t)p.cap << Cfg::SHIFT;
     if (threadIdx.x == 0) {
         // chunk 0: zero rows; P has a row of zeros behind the last tag
@@ -641,18 +825,23 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     const uint32_t tmem_base = *tmem_slot;
     const int g_lo = s_range[0], g_hi = s_range[1];
     float inv_w;
-    if (Cfg::TR) {
-        if (p.w_image) gf_load_w_t(p.w_image, tmem_base, inv_w);
-        else gf_convert_w_t(p.W, tmem_base, s_max, inv_w);
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    } else if (p.w_image) {
-        const uint4* src = static_cast<const uint4*>(p.w_image);
-        uint4* dst = reinterpret_cast<uint4*>(smem + Cfg::OFF_W);
-        for (int i = threadIdx.x; i < (int)(Cfg::W_BYTES / 16); i += WT) dst[i] = __ldg(src + i);
-        inv_w = __ldg(reinterpret_cast<const float*>(static_cast<const unsigned char*>(p.w_image) + Cfg::W_BYTES));
+    bool uneven;   // scales on both sides of W, in `scales`
+    if (p.w_image) {
+        const unsigned char* const image = static_cast<const unsigned char*>(p.w_image);
+        if (Cfg::TR) gf_load_w_t(image, tmem_base);
+        else
+            for (int i = threadIdx.x; i < (int)(Cfg::W_BYTES / 16); i += WT)
+                reinterpret_cast<uint4*>(smem + Cfg::OFF_W)[i] = __ldg(reinterpret_cast<const uint4*>(image) + i);
+        if (threadIdx.x < sizeof(GfScales<D>) / 16)
+            reinterpret_cast<float4*>(scales)[threadIdx.x] = __ldg(reinterpret_cast<const float4*>(image + Cfg::W_BYTES) + threadIdx.x);
+        const GfScales<D>* const made = reinterpret_cast<const GfScales<D>*>(image + Cfg::W_BYTES);
+        inv_w = __ldg(&made->all);
+        uneven = __ldg(&made->uneven) != 0;
     } else {
-        gf_convert_w<D, WT>(p.W, smem + Cfg::OFF_W, s_max, inv_w);
+        if constexpr (Cfg::TR) uneven = gf_convert_w_t(p.W, tmem_base, scales, scale_work, inv_w);
+        else uneven = gf_convert_w<D, WT>(p.W, smem + Cfg::OFF_W, scales, scale_work, inv_w);
     }
+    if (Cfg::TR) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 
     uint32_t job = 0;      // row blocks multiplied so far (the same count in every warp)
@@ -1020,6 +1209,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 if (m > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 40);
                 unsigned char* const s_hi = smem + Cfg::OFF_S + gf_op_off(grp, 4 * sl, RB);   // (row i*NG + grp: + i*NG*128, the same swizzle)
                 unsigned char* const s_lo = smem + Cfg::OFF_S + gf_op_off_lo<D>(grp, 4 * sl, RB, Cfg::S_LO);
+                if (uneven) {
+                    const ulonglong2 in_scale = gf_lds(smem_u32(scales->in + 4 * sl));
+#pragma unroll
+                    for (int i = 0; i < RPG; ++i) {
+                        a0[i] = mul2(a0[i], in_scale.x);
+                        a1[i] = mul2(a1[i], in_scale.y);
+                    }
+                }
 #pragma unroll
                 for (int i = 0; i < RPG; ++i) {
                     if (i * NG + warp * GPW < rows_m) {
@@ -1097,6 +1294,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                     uint32_t v[16];
                     tc_ld_cols16(tmem_base + Cfg::TM_ACC + ((uint32_t)(32 * q) << 16) + (uint32_t)r0, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (uneven) {
+                        const float out_scale = scales->out[f];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * out_scale);
+                    }
                     float* const h = hcol + r0 * 128;
 #pragma unroll
                     for (int i = 0; i < 16; i += 4) {
@@ -1153,6 +1355,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
 #pragma unroll
                         for (int c = 0; c < LDC / 4; ++c) x[c] = __ldg(nx + c);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (uneven) {
+#pragma unroll
+                            for (int c = 0; c < LDC; c += 4) {
+                                const float4 o = *reinterpret_cast<const float4*>(scales->out + jc * CW + h * LDC + c);
+                                v[c] = __float_as_uint(__uint_as_float(v[c]) * o.x);
+                                v[c + 1] = __float_as_uint(__uint_as_float(v[c + 1]) * o.y);
+                                v[c + 2] = __float_as_uint(__uint_as_float(v[c + 2]) * o.z);
+                                v[c + 3] = __float_as_uint(__uint_as_float(v[c + 3]) * o.w);
+                            }
+                        }
                         if (have) {
 #pragma unroll
                             for (int c = 0; c < LDC / 4; ++c) {
@@ -1274,7 +1486,7 @@ bool s2v_graph_fused_supported(const s2v_ctx* ctx, int d, int max_nodes, int num
     return max_nodes >= 1 && max_nodes <= most && num_tags < tags && ctx->smem_optin >= 227 * 1024;
 }
 
-size_t s2v_graph_fused_image_bytes(int d) { return sizeof(float) * (size_t)d * d + 16; }
+size_t s2v_graph_fused_image_bytes(int d) { return sizeof(float) * ((size_t)d * (d + 2) + 4); }   // + GfScales
 
 bool s2v_graph_fused_readout_ok(int d, int hidden, int num_class)
 {
@@ -1305,7 +1517,7 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     }
     if (a.image_scratch) {
         unsigned char* img = static_cast<unsigned char*>(a.image_scratch);
-        if (a.d == 128) gf_weight_image_t_kernel<<<1, 1024, 0, st>>>(a.W, reinterpret_cast<uint32_t*>(img));
+        if (a.d == 128) gf_weight_image_kernel<128><<<1, 1024, 0, st>>>(a.W, img);
         else if (a.d == 64) gf_weight_image_kernel<64><<<1, 1024, 0, st>>>(a.W, img);
         else gf_weight_image_kernel<32><<<1, 1024, 0, st>>>(a.W, img);
         S2V_CHECK_LAUNCH(ctx, "gf_weight_image_kernel");
