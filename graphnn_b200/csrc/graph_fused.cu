@@ -574,15 +574,17 @@ __device__ __forceinline__ void gf_readout(const GfParams& p, const float* y_s, 
 #pragma unroll
             for (int u = 0; u < U; ++u) wv[u] = k + u < kper ? __ldg(w + (int64_t)(k + u) * hidden) : 0.f;
 #pragma unroll
-            for (int u = 0; u < U; u += 4)
+            for (int u = 0; u < U; u += 4) {
+                if (k + u >= kper) break;   // (kper is a multiple of four)
 #pragma unroll
                 for (int g = 0; g < NB; ++g) {
-                    const float4 yv = *reinterpret_cast<const float4*>(y + g * D + (k + u < kper ? k + u : 0));
+                    const float4 yv = *reinterpret_cast<const float4*>(y + g * D + k + u);
                     acc[g] = fmaf(yv.x, wv[u], acc[g]);
                     acc[g] = fmaf(yv.y, wv[u + 1], acc[g]);
                     acc[g] = fmaf(yv.z, wv[u + 2], acc[g]);
                     acc[g] = fmaf(yv.w, wv[u + 3], acc[g]);
                 }
+            }
         }
 #pragma unroll
         for (int g = 0; g < NB; ++g) {

@@ -121,6 +121,31 @@ def test_fused_columns_and_weights_outside_and_inside_the_list(d, sizes, degree,
     assert_close(logits.cpu().numpy(), want, "logits", scale=max(1.0, float(np.abs(want).max())))
 
 
+@pytest.mark.parametrize("d,hidden", [(32, 16), (32, 64), (64, 16), (64, 64), (128, 16)])
+@pytest.mark.parametrize("graphs", [1, 9])
+def test_pooled_sum_that_overflows(d, hidden, graphs):
+    """One feature of one graph sums to infinity: the logits of the readout inside the kernel are those of the readout launch."""
+    b = make([2] * graphs, 0, d, 3, 2, hidden, 3, seed=d)
+    rng = np.random.default_rng(0)
+    w_in = np.abs(b.weights["w_n2l"])
+    w_in[1, 5] = 3e38
+    w2 = np.abs(b.weights["h2_weight"])
+    w2[:, 1] *= -1
+    b.weights = dict(b.weights, w_n2l=w_in, h1_weight=np.abs(b.weights["h1_weight"]), h2_weight=w2)
+    b.tags = rng.integers(0, 1, 2 * graphs).astype(np.int32)
+    b.tags[:2] = 1
+    got = {}
+    for mode in (0, 2):
+        eng = engine.S2VInference(b.weights, b.levels)
+        eng.ctx.set_option(eng.ctx.OPT_GRAPH_TILES, mode)
+        logits, _, pred, _ = eng.forward(eng.to_device(engine.build_host_batch(b)))
+        eng.ctx.synchronize()
+        got[mode] = logits.cpu().numpy(), pred.cpu().numpy()
+    assert np.array_equal(np.isposinf(got[0][0][0]), [True, False, True]) and np.isneginf(got[0][0][0, 1])
+    np.testing.assert_allclose(got[2][0], got[0][0], rtol=1e-5, atol=1e-5)
+    assert np.array_equal(got[2][1], got[0][1])
+
+
 def test_fused_reports_a_graph_beyond_the_hint_and_an_edge_between_graphs():
     b = make([30, 300, 25], 2.0, 64, 5, 2, 64, 2, seed=1)
     eng = engine.S2VInference(b.weights, b.levels)
