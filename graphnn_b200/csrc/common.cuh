@@ -118,6 +118,14 @@ struct s2v_device_guard {
 // ---------------------------------------------------------------- device helpers
 #ifdef __CUDACC__
 
+// The shared memory a kernel may be launched with is a property of the loaded function that every thread of the process sees, so it is
+// always set to the same bound, never to what one launch needs (another thread's larger launch would fail in between).
+template <typename K>
+inline cudaError_t s2v_allow_shared(K kern, size_t bound)
+{
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bound);
+}
+
 __device__ __forceinline__ float4 ld_nc_f4(const float4* p)
 {
     return __ldg(p);

@@ -1467,11 +1467,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tm_cols) : "memory");
 }
 
+constexpr uint32_t gf_budget(int warps) { return (warps == 8 ? 113u : 227u) * 1024u; }   // shared memory of a CTA: two of eight warps share an SM
+
 template <int D, int WARPS>
 int gf_launch(s2v_ctx* ctx, cudaStream_t st, const GfParams& p, uint32_t smem, unsigned blocks)
 {
     auto kern = p.val ? s2v_graph_fused_kernel<D, WARPS, true> : s2v_graph_fused_kernel<D, WARPS, false>;
-    S2V_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    S2V_CUDA_OK(ctx, s2v_allow_shared(kern, gf_budget(WARPS)));
     kern<<<blocks, WARPS * 32, smem, st>>>(p);
     S2V_CHECK_LAUNCH(ctx, "s2v_graph_fused_kernel");
     return S2V_OK;
@@ -1552,7 +1554,7 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     auto total = [&](int n) {
         return a.d == 128 ? gf_map<128>(cap, n, hv).total : (a.d == 64 ? gf_map<64>(cap, n, hv).total : gf_map<32>(cap, n, hv).total);
     };
-    const uint32_t budget = per_sm == 2 ? 113 * 1024 : 227 * 1024;
+    const uint32_t budget = gf_budget(warps);
     const uint32_t chunk = a.d == 128 ? GfCfg<128>::CHUNK : 8u;
     const double per_row = std::min(std::max(1.1, a.N > 0 ? 0.25 * (double)a.E / (double)a.N + 0.375 : 0.), 4096.);   // chunks: rows end inside one
     while (cap - 128 >= need && (budget - total(0)) / chunk < per_row * cap) cap -= 128;

@@ -6,6 +6,8 @@
 namespace
 {
 
+constexpr size_t SMALL_SHARED = 96 * 1024, LARGE_SHARED = 200 * 1024;   // bounds on the shared memory of the kernels below
+
 // ---------------------------------------------------------------- input projection
 // One-hot node features make X * W_in a row lookup: msg[i,:] = W_in[tag[i],:],
 // h0 = ReLU(msg) (examples/graph_classification/src/kernel_mean_field.cpp:31-32 with
@@ -444,19 +446,19 @@ int s2v_input_proj_dense_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n, int num
     if (n == 0) return S2V_OK;
     if (!X || !W_in || (!msg && !h0)) return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "input_proj: NULL pointer");
     const size_t smem = sizeof(float) * (size_t)num_feat * d;
-    if (smem > 200 * 1024) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "input_proj_dense: W_in beyond 200 KB; use s2v_gemm_f32");
+    if (smem > LARGE_SHARED) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "input_proj_dense: W_in beyond 200 KB; use s2v_gemm_f32");
     const int lpr = d / 4;
     const size_t smem_v4 = sizeof(float) * (size_t)num_feat * ((size_t)d + (lpr > 0 ? 1024 / lpr : 0));
-    if ((d == 32 || d == 64 || d == 128) && smem_v4 <= 96 * 1024 && s2v_aligned16(W_in) && s2v_aligned16(msg) && s2v_aligned16(h0)) {
+    if ((d == 32 || d == 64 || d == 128) && smem_v4 <= SMALL_SHARED && s2v_aligned16(W_in) && s2v_aligned16(msg) && s2v_aligned16(h0)) {
         auto kern = d == 32 ? input_proj_dense_v4_kernel<8> : (d == 64 ? input_proj_dense_v4_kernel<16> : input_proj_dense_v4_kernel<32>);
         const int64_t rows = 1024 / lpr;
-        S2V_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_v4));
+        S2V_CUDA_OK(ctx, s2v_allow_shared(kern, SMALL_SHARED));
         kern<<<grid_cap(ctx, (n + rows - 1) / rows, 6), 256, smem_v4, s2v_pick_stream(ctx, stream)>>>(
             n, num_feat, X, reinterpret_cast<const float4*>(W_in), reinterpret_cast<float4*>(msg), reinterpret_cast<float4*>(h0));
         S2V_CHECK_LAUNCH(ctx, "input_proj_dense_v4_kernel");
         return S2V_OK;
     }
-    S2V_CUDA_OK(ctx, cudaFuncSetAttribute(input_proj_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    S2V_CUDA_OK(ctx, s2v_allow_shared(input_proj_dense_kernel, LARGE_SHARED));
     input_proj_dense_kernel<<<grid_cap(ctx, (n + 7) / 8, 4), 256, smem, s2v_pick_stream(ctx, stream)>>>(n, num_feat, d, X,
                                                                                                           W_in, msg, h0);
     S2V_CHECK_LAUNCH(ctx, "input_proj_dense_kernel");
@@ -507,30 +509,30 @@ int s2v_readout_f32(s2v_ctx* ctx, s2v_stream stream, int64_t num_graphs, int d, 
         if (rc != S2V_ERR_UNSUPPORTED) return rc;
     }
     const size_t smem4 = sizeof(float) * (size_t)TG4 * ((size_t)d + 4 + hidden + 4 + num_class);
-    if (d % 8 == 0 && (hidden == 256 || hidden == 128) && smem4 <= 96 * 1024 && s2v_aligned16(Y) && num_graphs >= 256) {
+    if (d % 8 == 0 && (hidden == 256 || hidden == 128) && smem4 <= SMALL_SHARED && s2v_aligned16(Y) && num_graphs >= 256) {
         // batches of hundreds of graphs and the two hidden sizes of the path: first layer on the tensor cores
         // four CTAs per SM (64 registers, 50 KB of shared memory each): the 512 tiles of a 16,384-graph batch run as one wave
         const unsigned grid = grid_cap(ctx, (num_graphs + TG4 - 1) / TG4, 4);
         if (hidden == 256) {
-            S2V_CUDA_OK(ctx, cudaFuncSetAttribute(readout_mma_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4));
+            S2V_CUDA_OK(ctx, s2v_allow_shared(readout_mma_kernel<8>, SMALL_SHARED));
             readout_mma_kernel<8><<<grid, 256, smem4, s2v_pick_stream(ctx, stream)>>>(num_graphs, d, num_class, Y, W1, W2, logits, probs, pred);
         } else {
-            S2V_CUDA_OK(ctx, cudaFuncSetAttribute(readout_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4));
+            S2V_CUDA_OK(ctx, s2v_allow_shared(readout_mma_kernel<4>, SMALL_SHARED));
             readout_mma_kernel<4><<<grid, 256, smem4, s2v_pick_stream(ctx, stream)>>>(num_graphs, d, num_class, Y, W1, W2, logits, probs, pred);
         }
         S2V_CHECK_LAUNCH(ctx, "readout_mma_kernel");
         return S2V_OK;
     }
-    if (d % 4 == 0 && hidden % 4 == 0 && smem4 <= 96 * 1024 && s2v_aligned16(Y) && s2v_aligned16(W1)) {
-        S2V_CUDA_OK(ctx, cudaFuncSetAttribute(readout_v4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4));
+    if (d % 4 == 0 && hidden % 4 == 0 && smem4 <= SMALL_SHARED && s2v_aligned16(Y) && s2v_aligned16(W1)) {
+        S2V_CUDA_OK(ctx, s2v_allow_shared(readout_v4_kernel, SMALL_SHARED));
         readout_v4_kernel<<<grid_cap(ctx, (num_graphs + TG4 - 1) / TG4, 2), 256, smem4, s2v_pick_stream(ctx, stream)>>>(
             num_graphs, d, hidden, num_class, Y, W1, W2, logits, probs, pred);
         S2V_CHECK_LAUNCH(ctx, "readout_v4_kernel");
         return S2V_OK;
     }
     const size_t smem = sizeof(float) * (size_t)TG * ((size_t)d + hidden + num_class);
-    if (smem > 200 * 1024) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "readout: d + hidden + classes too large for shared memory");
-    S2V_CUDA_OK(ctx, cudaFuncSetAttribute(readout_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > LARGE_SHARED) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "readout: d + hidden + classes too large for shared memory");
+    S2V_CUDA_OK(ctx, s2v_allow_shared(readout_kernel, LARGE_SHARED));
     readout_kernel<<<grid_cap(ctx, (num_graphs + TG - 1) / TG, 4), 256, smem, s2v_pick_stream(ctx, stream)>>>(
         num_graphs, d, hidden, num_class, Y, W1, W2, logits, probs, pred);
     S2V_CHECK_LAUNCH(ctx, "readout_kernel");
