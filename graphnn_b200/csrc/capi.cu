@@ -362,8 +362,6 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
     //   * few graphs per CTA: the readout runs inside the kernel too, one launch in all;
     //   * from S2V_FUSED_TABLE_NODES nodes on, the first level's product table and W in the operand layout are made
     //     once, in front (below that the two launches cost more than they save);
-    //   * with embed_out, batches below S2V_FUSED_EMBED_NODES nodes keep one launch per level: callers of that form
-    //     observe the launch count of the per-level path;
     //   * d = 32, graphs above one row block: a CTA holds one graph or two, and as long as the batch is one round of such
     //     tiles the kernel is ahead (100 graphs of 100 - 620 nodes 31 us against 58, 300 graphs 72 against 80); from the second
     //     round on the level kernels are, which stream 128-byte rows (500 graphs 121 us against 170).  So they are where the columns
@@ -372,7 +370,7 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
     const bool rounds = d == 32 && batch->max_graph_nodes > 128 &&
                         (N > (int64_t)ctx->sm_count * 2 * S2V_FUSED_ROUND_NODES || batch->num_edges > (int64_t)ctx->sm_count * 2 * S2V_FUSED_ROUND_EDGES);
     if (ctx->graph_tiles != 0 && L >= 1 && N > 0 && G < (int64_t)INT32_MAX && batch->max_graph_nodes >= 1 &&
-        (forced || !(rounds || (embed_out && N < S2V_FUSED_EMBED_NODES))) && (batch->tags || batch->x_dense) &&
+        (forced || !rounds) && (batch->tags || batch->x_dense) &&
         s2v_graph_fused_supported(ctx, d, batch->max_graph_nodes, batch->tags ? model->num_feat : 1)) {
         if (!s2v_aligned16(model->w_n2l) || !s2v_aligned16(model->p_node_conv) || (embed_out && !s2v_aligned16(embed_out)))
             return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "forward: weights and embed_out must be 16-byte aligned");

@@ -204,7 +204,6 @@ struct s2v_graph_fused_args {
     int32_t* pred = nullptr;
 };
 constexpr int64_t S2V_FUSED_TABLE_NODES = 32768;   // batches from this many nodes on: weights and first-level table prepared by launches of their own
-constexpr int64_t S2V_FUSED_EMBED_NODES = 16384;   // batches with embed_out below this many nodes take the per-level kernels
 constexpr int64_t S2V_FUSED_ROUND_NODES = 384;     // d = 32, larger graphs: nodes that a CTA is expected to hold at a time
 constexpr int64_t S2V_FUSED_ROUND_EDGES = 4500;    // ... and entries
 bool s2v_graph_fused_supported(const s2v_ctx* ctx, int d, int max_nodes, int num_tags);

@@ -10,8 +10,9 @@ from graphnn_b200 import engine, synth
 pytestmark = pytest.mark.gpu
 
 
-def run(batch, dense=False, want_embed=True):
+def run(batch, dense=False, want_embed=True, tiles=2):
     eng = engine.S2VInference(batch.weights, batch.levels)
+    eng.ctx.set_option(eng.ctx.OPT_GRAPH_TILES, tiles)
     hb = engine.build_host_batch(batch)
     db = eng.to_device(hb, batch.dense_x() if dense else None)
     logits, probs, pred, embed = eng.forward(db, want_embed=want_embed)
@@ -19,11 +20,12 @@ def run(batch, dense=False, want_embed=True):
     return eng, hb, logits.cpu().numpy(), probs.cpu().numpy(), pred.cpu().numpy(), (embed.cpu().numpy() if want_embed else None)
 
 
+@pytest.mark.parametrize("tiles", [0, 1, 2])      # per level; whole graphs in one kernel, prepared in front; the default
 @pytest.mark.parametrize("dense", [False, True])
-def test_classifier_matches_reference_golden(golden, dense):
+def test_classifier_matches_reference_golden(golden, dense, tiles):
     g = golden("mutag_like_seed0.npz")
     b = synth.mutag_like(seed=0)
-    eng, hb, logits, probs, pred, embed = run(b, dense)
+    eng, hb, logits, probs, pred, embed = run(b, dense, tiles=tiles)
     assert np.array_equal(hb.row_ptr.numpy(), g["n2n_row_ptr"])        # CSR construction: bit-exact
     assert np.array_equal(hb.col_idx.numpy(), g["n2n_col_idx"])
     assert np.array_equal(hb.graph_ptr.numpy(), g["sub_row_ptr"])      # pooling indices: bit-exact
@@ -31,29 +33,33 @@ def test_classifier_matches_reference_golden(golden, dense):
     assert_close(embed, g["last_level"], "embeddings")
     assert_close(logits, g["logits"], "logits")
     assert_close(probs, g["probs"], "probs")
-    # dense X: projection, L levels, pooling, readout; tags: product table, first level (which also range-checks the tags),
-    # L - 1 levels, pooling, readout
-    assert eng.ctx.launches == 3 + b.levels
+    # per level, dense X: projection, L levels, pooling, readout; tags: product table, first level (which also range-checks the
+    # tags), L - 1 levels, pooling, readout.  By default one launch (and the projection of a dense X).
+    assert eng.ctx.launches == {0: 3 + b.levels, 1: 4, 2: 1 + dense}[tiles]
+    _, _, logits2, probs2, pred2, _ = run(b, dense, want_embed=False, tiles=tiles)
+    assert np.array_equal(logits2, logits) and np.array_equal(probs2, probs) and np.array_equal(pred2, pred)
 
 
-def test_classifier_mixed_classes_golden(golden):
+@pytest.mark.parametrize("tiles", [0, 1, 2])
+def test_classifier_mixed_classes_golden(golden, tiles):
     g = golden("mutag_like_seed3.npz")
     b = synth.mutag_like(seed=3)
-    _, _, logits, probs, pred, _ = run(b)
+    _, _, logits, probs, pred, _ = run(b, tiles=tiles)
     assert np.array_equal(pred, g["argmax"])
     assert_close(logits, g["logits"], "logits")
     assert_close(probs, g["probs"], "probs")
 
 
+@pytest.mark.parametrize("tiles", [0, 1, 2])
 @pytest.mark.parametrize("maker", [
     lambda: synth.molecules_16k(seed=1, num_graphs=700),
     lambda: synth.proteins_4k(seed=1, num_graphs=40),
     lambda: synth.molecule_like(33, 1, 5, 4, 32, 2, 16, 3, 0.3, "uniform", seed=8),   # single-node graphs, 3 classes
 ])
-def test_classifier_matches_oracle(oracle_lib, maker):
+def test_classifier_matches_oracle(oracle_lib, maker, tiles):
     b = maker()
     o = oracle_lib.forward(b, "oracle")
-    _, hb, logits, probs, pred, embed = run(b)
+    _, hb, logits, probs, pred, embed = run(b, tiles=tiles)
     assert np.array_equal(hb.row_ptr.numpy(), o["n2n_row_ptr"])
     assert np.array_equal(hb.col_idx.numpy(), o["n2n_col_idx"])
     # the last level's values reach tens (proteins: 43): like the logits they are held to 1e-5 of their scale; fp32
