@@ -106,14 +106,17 @@ int s2v_ctx_create(int device, s2v_ctx** out)
     ctx->sm_count = ctx->sm_count_hw = prop.multiProcessorCount;
     ctx->smem_optin = prop.sharedMemPerBlockOptin;
     bool ok = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaHostAlloc((void**)&ctx->dstatus_host, sizeof(s2v_device_status), cudaHostAllocMapped) == cudaSuccess &&
+              cudaHostAlloc((void**)&ctx->dstatus_host, 3 * sizeof(s2v_device_status), cudaHostAllocMapped) == cudaSuccess &&
               cudaHostGetDevicePointer((void**)&ctx->dstatus_dev, ctx->dstatus_host, 0) == cudaSuccess;
     if (!ok) {
         s2v_ctx_destroy(ctx);
         return S2V_ERR_CUDA;
     }
-    ctx->dstatus_host->code = 0;
-    ctx->dstatus_host->where = 0;
+    for (int i = 0; i < 3; ++i) ctx->dstatus_host[i].code = ctx->dstatus_host[i].where = 0;
+    for (int i = 0; i < 2; ++i) {
+        ctx->lanes[i].edge_host = ctx->dstatus_host + 1 + i;
+        ctx->lanes[i].edge_dev = ctx->dstatus_dev + 1 + i;
+    }
     // S2V_LEVEL_TC = 0 | 1 | 2 : never / automatic / always use the tcgen05 level kernel (d = 128)
     if (const char* e = std::getenv("S2V_LEVEL_TC")) ctx->tc_mode = (e[0] == '0') ? 0 : (e[0] == '2' ? 2 : 1);
     if (const char* e = std::getenv("S2V_GRAPH_TILES")) ctx->graph_tiles = (e[0] == '0') ? 0 : ((e[0] == '1') ? 1 : 2);
@@ -329,8 +332,9 @@ size_t s2v_forward_workspace_bytes(int64_t num_nodes, int64_t num_graphs, int d)
     return 3 * nd + gd + 256;
 }
 
-int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, const s2v_batch* batch, void* workspace,
-                    size_t workspace_bytes, float* logits, float* probs, int32_t* pred, float* embed_out)
+// edge_status: where an edge between two graphs of a batch with max_graph_nodes is reported (NULL: the context's status word)
+static int forward(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, const s2v_batch* batch, void* workspace,
+                   size_t workspace_bytes, float* logits, float* probs, int32_t* pred, float* embed_out, s2v_device_status* edge_status)
 {
     S2V_ENTER(ctx);
     if (!model || !batch) return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "forward: NULL model or batch");
@@ -381,6 +385,7 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
         a.row_ptr = batch->n2n_row_ptr; a.col_idx = batch->n2n_col_idx; a.val = batch->n2n_val; a.graph_ptr = batch->graph_ptr;
         a.W = model->p_node_conv;
         a.Y = y; a.embed_out = embed_out;
+        a.edge_status = edge_status;
         if (batch->tags) {
             a.tags = batch->tags; a.x = model->w_n2l; a.num_tags = model->num_feat;
         } else {
@@ -469,6 +474,12 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
     if (rc != S2V_OK) return rc;
     return s2v_readout_f32(ctx, st, G, d, model->hidden, model->num_class, y, model->h1_weight, model->h2_weight, logits,
                            probs, pred);
+}
+
+int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, const s2v_batch* batch, void* workspace,
+                    size_t workspace_bytes, float* logits, float* probs, int32_t* pred, float* embed_out)
+{
+    return forward(ctx, stream, model, batch, workspace, workspace_bytes, logits, probs, pred, embed_out, nullptr);
 }
 
 // ---------------------------------------------------------------- host-side CSR
@@ -633,6 +644,24 @@ void hand_over(const s2v_staging& s, int64_t G, int C, float* logits, int32_t* p
     if (logits) std::memcpy(logits, s.pinned, sizeof(float) * (size_t)G * C);
     if (pred) std::memcpy(pred, static_cast<const unsigned char*>(s.pinned) + pred_at(G, C), sizeof(int32_t) * (size_t)G);
 }
+// The forward of a lane's batch and the copy of its results to the pinned buffer.
+int lane_forward(s2v_ctx* ctx, cudaStream_t st, s2v_lane& lane, const float* logits_host, const int32_t* pred_host)
+{
+    const int64_t G = lane.batch.num_graphs;
+    const int C = lane.model.num_class;
+    lane.edge_host->code = lane.edge_host->where = 0;
+    const int rc = forward(ctx, st, &lane.model, &lane.batch, lane.ws, lane.ws_bytes, reinterpret_cast<float*>(lane.dev_out), nullptr,
+                           reinterpret_cast<int32_t*>(lane.dev_out + pred_at(G, C)), nullptr, lane.edge_dev);
+    return rc == S2V_OK ? download(ctx, st, lane.staging, lane.dev_out, G, C, logits_host, pred_host) : rc;
+}
+// After the stream is done: once more with one launch per level, which don't ask for separate graphs.
+int lane_repeat(s2v_ctx* ctx, cudaStream_t st, s2v_lane& lane, const float* logits_host, const int32_t* pred_host)
+{
+    lane.batch.max_graph_nodes = 0;
+    const int rc = lane_forward(ctx, st, lane, logits_host, pred_host);
+    const int rc2 = s2v_stream_status(ctx, st);
+    return rc != S2V_OK ? rc : rc2;
+}
 }  // namespace
 
 extern "C" {
@@ -751,9 +780,25 @@ int s2v_infer_host_f32(s2v_ctx* ctx, const s2v_model* model, const s2v_batch* hb
             for (int64_t i = 0; i < N; ++i)
                 if (rp[i + 1] < rp[i]) bad_csr |= 1;
             const int32_t* ci = hb->n2n_col_idx;
-#pragma omp parallel for num_threads(T) schedule(static) reduction(| : bad_csr) if (E >= (1 << 15))
-            for (int64_t t = 0; t < E; ++t)
-                if (ci[t] < 0 || ci[t] >= N) bad_csr |= 1;
+            int crosses = 0;   // an edge between two graphs: the batch goes through the per-level kernels
+            if (!bad_csr) {
+#pragma omp parallel num_threads(T) reduction(| : bad_csr, crosses) if (E >= (1 << 15))
+                {
+                    const int64_t i0 = N * omp_get_thread_num() / omp_get_num_threads(), i1 = N * (omp_get_thread_num() + 1) / omp_get_num_threads();
+                    int64_t g = i0 < i1 ? std::upper_bound(gp, gp + G + 1, (int32_t)i0) - gp - 1 : 0;
+                    for (int64_t i = i0; i < i1;) {   // the rows of a graph, as far as they are this thread's
+                        while (gp[g + 1] <= i) ++g;
+                        const int64_t end = gp[g + 1] < i1 ? gp[g + 1] : i1;
+                        const int32_t lo = gp[g], hi = gp[g + 1];
+                        for (int64_t t = rp[i]; t < rp[end]; ++t) {
+                            if (ci[t] < 0 || ci[t] >= N) bad_csr |= 1;
+                            if (ci[t] < lo || ci[t] >= hi) crosses |= 1;
+                        }
+                        i = end;
+                    }
+                }
+            }
+            if (crosses) max_nodes = 0;
         }
         if (bad_csr) return s2v_fail(ctx, S2V_ERR_BAD_CSR, "infer_host: offsets not monotone or a column index outside [0, N)");
     }
@@ -777,7 +822,7 @@ int s2v_infer_host_f32(s2v_ctx* ctx, const s2v_model* model, const s2v_batch* hb
     const size_t o_gp = take(sizeof(int32_t) * (size_t)(G + 1));
     const size_t o_in = hb->tags ? take(sizeof(int32_t) * (size_t)N) : take(sizeof(float) * (size_t)N * F);
     const size_t o_logits = take(sizeof(float) * (size_t)G * C);
-    const size_t o_pred = take(sizeof(int32_t) * (size_t)G);
+    take(sizeof(int32_t) * (size_t)G);   // predictions, at pred_at()
     const size_t ws_bytes = s2v_forward_workspace_bytes(N, G, d);
     const size_t o_ws = take(ws_bytes);
     HostInputs in(o_logits);
@@ -795,7 +840,9 @@ int s2v_infer_host_f32(s2v_ctx* ctx, const s2v_model* model, const s2v_batch* hb
     rc = in.upload(ctx, st, dev, static_cast<unsigned char*>(stage.pinned) + out_bytes(G, C));
     if (rc != S2V_OK) return rc;
 
-    s2v_batch db = *hb;
+    s2v_lane& lane = ctx->lanes[0];
+    s2v_batch& db = lane.batch;
+    db = *hb;
     db.max_graph_nodes = max_nodes;
     db.n2n_row_ptr = reinterpret_cast<const int32_t*>(dev + o_rp);
     db.n2n_col_idx = reinterpret_cast<const int32_t*>(dev + o_ci);
@@ -803,10 +850,11 @@ int s2v_infer_host_f32(s2v_ctx* ctx, const s2v_model* model, const s2v_batch* hb
     db.graph_ptr = reinterpret_cast<const int32_t*>(dev + o_gp);
     db.tags = hb->tags ? reinterpret_cast<const int32_t*>(dev + o_in) : nullptr;
     db.x_dense = hb->tags ? nullptr : reinterpret_cast<const float*>(dev + o_in);
-    float* d_logits = reinterpret_cast<float*>(dev + o_logits);
-    int32_t* d_pred = reinterpret_cast<int32_t*>(dev + o_pred);
-    rc = s2v_forward_f32(ctx, st, model, &db, dev + o_ws, ws_bytes, d_logits, nullptr, d_pred, nullptr);
-    if (rc == S2V_OK) rc = download(ctx, st, stage, dev + o_logits, G, C, logits_host, pred_host);
+    lane.model = *model;
+    lane.ws = dev + o_ws;
+    lane.ws_bytes = ws_bytes;
+    lane.dev_out = dev + o_logits;
+    rc = lane_forward(ctx, st, lane, logits_host, pred_host);
     if (rc != S2V_OK) {
         cudaStreamSynchronize(st);   // (the next call writes into the staged inputs)
         return rc;
@@ -816,6 +864,12 @@ int s2v_infer_host_f32(s2v_ctx* ctx, const s2v_model* model, const s2v_batch* hb
     rc = s2v_ctx_synchronize(ctx);
     if (bad_tag) return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "infer_host: a node tag outside [0, num_feat)");
     if (rc != S2V_OK) return rc;
+    if (lane.edge_host->code != 0) {   // (only without the scan above: the columns are looked at before a per-level kernel reads them)
+        if (s2v_validate_csr_host(N, N, E, hb->n2n_row_ptr, hb->n2n_col_idx) != S2V_OK)
+            return s2v_fail(ctx, S2V_ERR_BAD_CSR, "infer_host: offsets not monotone or a column index outside [0, N)");
+        rc = lane_repeat(ctx, st, lane, logits_host, pred_host);
+        if (rc != S2V_OK) return rc;
+    }
     hand_over(stage, G, C, logits_host, pred_host);
     return S2V_OK;
 }
@@ -862,7 +916,7 @@ static int edges_enqueue(s2v_ctx* ctx, s2v_lane& lane, const s2v_model* model, i
     const size_t o_rp = take(sizeof(int32_t) * (size_t)(N + 1));
     const size_t o_ci = take(sizeof(int32_t) * (size_t)E);
     const size_t o_logits = take(sizeof(float) * (size_t)G * C);
-    const size_t o_pred = take(sizeof(int32_t) * (size_t)G);
+    take(sizeof(int32_t) * (size_t)G);   // predictions, at pred_at()
     const size_t sc_bytes = s2v_build_n2n_csr_scratch_bytes(N, E);
     const size_t o_sc = take(sc_bytes);
     const size_t ws_bytes = s2v_forward_workspace_bytes(N, G, d);
@@ -883,7 +937,8 @@ static int edges_enqueue(s2v_ctx* ctx, s2v_lane& lane, const s2v_model* model, i
                                0, dev + o_sc, sc_bytes, reinterpret_cast<int32_t*>(dev + o_rp), reinterpret_cast<int32_t*>(dev + o_ci),
                                nullptr);
     if (rc != S2V_OK) return rc;
-    s2v_batch db{};
+    s2v_batch& db = lane.batch;
+    db = s2v_batch{};
     db.num_graphs = G;
     db.num_nodes = N;
     db.num_edges = E;
@@ -892,11 +947,11 @@ static int edges_enqueue(s2v_ctx* ctx, s2v_lane& lane, const s2v_model* model, i
     db.graph_ptr = reinterpret_cast<const int32_t*>(dev + o_gp);
     db.tags = reinterpret_cast<const int32_t*>(dev + o_tg);
     db.max_graph_nodes = max_nodes;
-    float* d_logits = reinterpret_cast<float*>(dev + o_logits);
-    int32_t* d_pred = reinterpret_cast<int32_t*>(dev + o_pred);
-    rc = s2v_forward_f32(ctx, st, model, &db, dev + o_ws, ws_bytes, d_logits, nullptr, d_pred, nullptr);
-    if (rc != S2V_OK) return rc;
-    rc = download(ctx, st, lane.staging, dev + o_logits, G, C, logits_host, pred_host);
+    lane.model = *model;
+    lane.ws = dev + o_ws;
+    lane.ws_bytes = ws_bytes;
+    lane.dev_out = dev + o_logits;
+    rc = lane_forward(ctx, st, lane, logits_host, pred_host);
     if (rc != S2V_OK) return rc;
     lane.G = G;
     lane.C = C;
@@ -922,10 +977,14 @@ static int lane_finish(s2v_ctx* ctx, s2v_lane& lane)
 {
     if (!lane.busy) return S2V_OK;
     lane.busy = false;
-    const int rc = s2v_stream_status(ctx, lane.stream);
+    int rc = s2v_stream_status(ctx, lane.stream);
     if (lane.bad_edge) return s2v_fail(ctx, S2V_ERR_BAD_CSR, "infer_edges: graph_ptr not monotone or an edge endpoint outside [0, N)");
     if (lane.bad_tag) return s2v_fail(ctx, S2V_ERR_INVALID_ARG, "infer_edges: a node tag outside [0, num_feat)");
     if (rc != S2V_OK) return rc;
+    if (lane.G > 0 && lane.edge_host->code != 0) {   // (the device-side builder has kept the columns inside [0, N))
+        rc = lane_repeat(ctx, lane.stream, lane, lane.logits_host, lane.pred_host);
+        if (rc != S2V_OK) return rc;
+    }
     if (lane.G > 0) hand_over(lane.staging, lane.G, lane.C, lane.logits_host, lane.pred_host);
     return S2V_OK;
 }

@@ -37,6 +37,15 @@ struct s2v_lane {
     float* logits_host = nullptr;
     int32_t* pred_host = nullptr;
     int bad_edge = 0, bad_tag = 0;   // outcome of the host scan that ran beside the device work
+    // The forward of the batch, should it have to be run once more: the library says that the batch is one of separate graphs without
+    // having looked at the edges, and a kernel that finds one between two graphs reports it in the lane's own word.
+    s2v_device_status* edge_host = nullptr;   // pinned + mapped, behind the context's word
+    s2v_device_status* edge_dev = nullptr;
+    s2v_model model{};
+    s2v_batch batch{};                        // device arrays
+    unsigned char* ws = nullptr;
+    size_t ws_bytes = 0;
+    unsigned char* dev_out = nullptr;         // logits, then predictions
 };
 
 struct s2v_ctx {
@@ -202,6 +211,7 @@ struct s2v_graph_fused_args {
     float* logits = nullptr;
     float* probs = nullptr;
     int32_t* pred = nullptr;
+    s2v_device_status* edge_status = nullptr;   // where an edge between two graphs is reported; NULL: the context's status word
 };
 constexpr int64_t S2V_FUSED_TABLE_NODES = 32768;   // batches from this many nodes on: weights and first-level table prepared by launches of their own
 constexpr int64_t S2V_FUSED_ROUND_NODES = 384;     // d = 32, larger graphs: nodes that a CTA is expected to hold at a time

@@ -70,6 +70,7 @@ struct GfParams {
     int cap, chunk_cap;
     uint32_t tm_cols;
     s2v_device_status* status;
+    s2v_device_status* edge_status;   // where an edge that leaves its tile is reported
 };
 
 template <int D>
@@ -935,8 +936,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
                             if (e[u] >= (uint32_t)nrows && t + u < rn[k]) {   // an edge that leaves the tile
-                                p.status->code = S2V_ERR_BAD_CSR;
-                                p.status->where = 5;
+                                p.edge_status->code = S2V_ERR_BAD_CSR;
+                                p.edge_status->where = 5;
                                 e[u] = 0;
                             }
                             e[u] = Cfg::TR ? Cfg::OFF_H + e[u] * Cfg::ROWB : (e[u] << Cfg::SHIFT) + (e[u] & 7u);
@@ -984,7 +985,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             gf_worker_sync<WT>();
         }
         auto far_rows = [&]() {
-            return GfFar{smem_u32(smem + Cfg::OFF_H), smem_u32(smem + map.tags), reinterpret_cast<const ulonglong2*>(p.P), node0, nrows, p.cap, p.status};
+            return GfFar{smem_u32(smem + Cfg::OFF_H), smem_u32(smem + map.tags), reinterpret_cast<const ulonglong2*>(p.P), node0, nrows, p.cap, p.edge_status};
         };
         auto weighted_row = [&](auto first, int r) {   // all lanes of a warp; r: the lane group's row, or beyond the last one
             const uint32_t inf = r < nrows ? info_s[r] : 0u, mine = ((inf >> 16) + 3) / 4;
@@ -1513,6 +1514,7 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     p.W1 = a.W1; p.W2 = a.W2; p.hidden = a.hidden; p.num_class = a.num_class;
     p.logits = a.logits; p.probs = a.probs; p.pred = a.pred;
     p.status = ctx->dstatus_dev;
+    p.edge_status = a.edge_status ? a.edge_status : ctx->dstatus_dev;
     if (a.P_scratch && a.levels >= 1) {
         const int rc = s2v_launch_first_table_product(ctx, st, a.num_tags, a.d, a.x, a.W, a.P_scratch, true);
         if (rc != S2V_OK) return rc;

@@ -25,7 +25,7 @@ class HostBatch:
     col_idx: torch.Tensor    # int32 [E], pinned
     graph_ptr: torch.Tensor  # int32 [G+1], pinned
     tags: torch.Tensor       # int32 [N], pinned
-    max_graph_nodes: int = 0 # node count of the largest graph (0 = unknown)
+    max_graph_nodes: int = 0 # node count of the largest graph (0 = unknown, or an edge joins two graphs)
 
     def nbytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in (self.row_ptr, self.col_idx, self.graph_ptr, self.tags))
@@ -53,8 +53,10 @@ def build_host_batch(batch) -> HostBatch:
     """GraphBatch -> CSR arrays, through the library's host builder (bit-identical to
     Node2NodeMsgPass / SubgraphMsgPass::InitCPUWeight, src/nn/msg_pass.cpp:46-67,156-177)."""
     row_ptr, col_idx, _ = capi.build_n2n_csr_host(batch.num_nodes, batch.edge_src, batch.edge_dst, with_val=False)
+    graph = np.repeat(np.arange(batch.num_graphs), batch.nodes_per_graph)
+    separate = np.array_equal(graph[batch.edge_src], graph[batch.edge_dst])   # what max_graph_nodes promises
     return HostBatch(batch.num_graphs, batch.num_nodes, _pin(row_ptr), _pin(col_idx), _pin(batch.graph_offsets()),
-                     _pin(batch.tags.astype(np.int32)), int(batch.nodes_per_graph.max()) if batch.num_graphs else 0)
+                     _pin(batch.tags.astype(np.int32)), int(batch.nodes_per_graph.max()) if batch.num_graphs and separate else 0)
 
 
 class S2VInference:
