@@ -555,7 +555,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
             hbm_bytes = 4 * (N + 1) + 4 * E + 4 * N + 4 * (G + 1) + 4 * G * d + 4 * d * d + 4 * full.num_tags * d
             peak = peaks["bf16_tflops"]
             line["roofline"] = {
-                "kernel": "s2v_graph_fused_kernel (tcgen05, fp16 head + tail in three products; the launches of its product table and its W image are inside the bracket)", "bound": "tensor",
+                "kernel": "s2v_graph_fused_kernel (tcgen05, fp16 head + tail in three products; the launches of its product table and its W image are inside the bracket)", "bound": "shared memory, instruction issue (peak: tensor)",
                 "achieved": flops_mma / (t_ms * 1e-3) / 1e12, "peak": peak, "unit": "TFLOP/s",
                 "frac": flops_mma / (t_ms * 1e-3) / 1e12 / peak,
                 "peak_kind": f"{peaks['kind']} dense bf16 cuBLAS burst (fp16 MMAs issue at the same rate)",

@@ -365,7 +365,9 @@ static int forward(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, cons
     // readout behind it.
     //   * few graphs per CTA: the readout runs inside the kernel too, one launch in all;
     //   * from S2V_FUSED_TABLE_NODES nodes on, the first level's product table and W in the operand layout are made
-    //     once, in front (below that the two launches cost more than they save);
+    //     once, in front; below that the two launches and the readout's cost more than they save (molecules, 29,948 nodes:
+    //     d = 64 39 us in one launch, 50 prepared; d = 128 51 and 58; where the line would lie above is not measured).  The
+    //     option's value 1 asks for the prepared form at every size;
     //   * d = 32, graphs above one row block: a CTA holds one graph or two, and as long as the batch is one round of such
     //     tiles the kernel is ahead (100 graphs of 100 - 620 nodes 31 us against 58, 300 graphs 72 against 80); from the second
     //     round on the level kernels are, which stream 128-byte rows (500 graphs 121 us against 170).  So they are where the columns

@@ -62,7 +62,7 @@ struct s2v_ctx {
     s2v_lane lanes[2];
     void* first_table = nullptr;     // product table of s2v_level_first_f32 (grow-only, a few hundred KB at most)
     size_t first_table_bytes = 0;
-    int tc_mode = 1;  // tcgen05 level kernel: 0 never, 1 when the batch is large enough, 2 whenever the shape allows
+    int tc_mode = 1;  // tcgen05 kernels: 0 never, 1 automatic, 2 the first-level and readout forms earlier (S2V_OPT_LEVEL_TC)
     int graph_tiles = 2;    // whole-classifier kernel for batches of small graphs: 0 off, 1 whenever the batch allows, 2 automatic
     int first_table_on = 1; // first level as a gather-sum over ReLU(W_in) * W (S2V_OPT_FIRST_LEVEL_TABLE)
     int validate_host = 1;  // s2v_infer_host_f32 scans its host arrays before launching

@@ -1529,9 +1529,9 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
         S2V_CHECK_LAUNCH(ctx, "gf_weight_image_kernel");
         p.w_image = img;
     }
-    // Rows per tile.  Small graphs: one row block per tile and (d <= 64) two 288-thread CTAs per SM, so that one CTA's
+    // Rows per tile.  Small graphs: one row block per tile and (d <= 64) two 256-thread CTAs per SM, so that one CTA's
     // gather runs under the other's products and drains.  Larger graphs: as many rows as the batch gives each SM, up to
-    // what fits, with 544 threads.
+    // what fits, with 512 threads.
     const int need = (a.max_graph_nodes + 127) / 128 * 128;
     int warps = 16, per_sm = 1, cap = 128;
     if (a.d == 128) { warps = 8; per_sm = 2; }

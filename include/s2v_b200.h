@@ -70,12 +70,14 @@ const char* s2v_last_error(const s2v_ctx* ctx);
 typedef enum s2v_option {
     S2V_OPT_VALIDATE_HOST_INPUT = 1, /* s2v_infer_host_f32 scans its host arrays before any launch (default 1;
                                         the environment variable S2V_VALIDATE_HOST=0 sets the default to 0) */
-    S2V_OPT_LEVEL_TC = 2,            /* tcgen05 level kernel: 0 never, 1 automatic (default), 2 whenever the shape allows
-                                        (default from S2V_LEVEL_TC) */
+    S2V_OPT_LEVEL_TC = 2,            /* tcgen05 kernels: 0 never; 1 automatic (default): levels of d = 64 and 128 with 32-bit offsets at
+                                        every size, the table-lookup form of the first level from 16,384 rows on, the readout from
+                                        6,144 graphs on; 2: those two earlier (any size; 512 graphs).  Default from S2V_LEVEL_TC */
     S2V_OPT_GRAPH_TILES = 3,         /* whole-classifier kernel inside s2v_forward_f32 for batches of small and medium graphs (at most
-                                        128 nodes at d = 128, 640 at d = 64, 1024 at d = 32): 0 never, 1 whenever the batch
-                                        allows, 2 automatic (default: also whenever it allows, except that small batches with
-                                        embed_out keep one launch per level).  Default from S2V_GRAPH_TILES */
+                                        128 nodes at d = 128, 640 at d = 64, 1024 at d = 32): 0 never; 1 whenever the batch allows,
+                                        always with the weights prepared by launches of their own; 2 automatic (default): below 32,768
+                                        nodes in one launch, and at d = 32 with graphs above 128 nodes only while the batch is about
+                                        one graph per CTA and its columns fit shared memory.  Default from S2V_GRAPH_TILES */
     S2V_OPT_RESERVED_SMS = 4,        /* the persistent kernels size their grids for (SM count - value) SMs, leaving the rest to
                                         kernels of another stream -- a communication library's, which cannot start while
                                         one-CTA-per-SM kernels hold every SM (default 0; 0 <= value < SM count) */
@@ -217,7 +219,8 @@ int s2v_input_proj_dense_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n, int num
  * Requires d = 128, every graph at most 128 nodes with a contiguous node range (graph_ptr, nn_common.h:63-73),
  * no edge between graphs and fewer than 8,388,608 tags.  Consecutive graphs are packed into tiles of at most 128 nodes; a
  * tile's node embeddings stay in shared memory across the levels, the dense stage runs on the tcgen05 tensor cores with
- * operands of 22 bits (fp16 head and tail, scaled per row), and only Y [G x d] (plus embed_out [N x d] if given) is
+ * operands of 22 bits (fp16 head and tail, scaled by powers of two per row of sums and, where W is uneven, per row and
+ * column of W), and only Y [G x d] (plus embed_out [N x d] if given) is
  * written.  A larger graph, an edge that leaves its graph's tile or a tag outside [0, num_tags) is reported through the
  * status word, not faulted.  val may be NULL (all ones).  workspace: s2v_graph_tiles_workspace_bytes(G) bytes of device memory. */
 size_t s2v_graph_tiles_workspace_bytes(int64_t num_graphs);
@@ -255,12 +258,14 @@ typedef struct s2v_batch {
                                    points cannot read graph_ptr on the host; with a value here (and S2V_OPT_GRAPH_TILES not 0)
                                    s2v_forward_f32 keeps whole graphs in shared memory across the levels where they fit:
                                    up to 1024 nodes at d = 32, 640 at d = 64, 128 at d = 128.  The value promises separate
-                                   graphs: one that understates the truth (the oversized graphs are truncated) and an edge
-                                   between graphs are reported through the status word (S2V_ERR_UNSUPPORTED,
-                                   S2V_ERR_BAD_CSR).  s2v_infer_host_f32 computes it itself. */
+                                   graphs that cover every node: one that understates the truth (the oversized graphs are
+                                   truncated) is reported through the status word (S2V_ERR_UNSUPPORTED), and so is an edge
+                                   between two graphs (S2V_ERR_BAD_CSR) unless they happen to share a tile, where it is
+                                   computed as given.  The host entry points make no such demand: they find the value, and
+                                   edges between graphs, themselves. */
 } s2v_batch;
 
-/* Bytes of device workspace s2v_forward_f32 needs (three [N x d] buffers + [G x d] + the tile plan). */
+/* Bytes of device workspace s2v_forward_f32 needs (three [N x d] buffers + [G x d]). */
 size_t s2v_forward_workspace_bytes(int64_t num_nodes, int64_t num_graphs, int d);
 /* logits [G x C]; probs, pred, embed_out ([N x d], the last level) may be NULL.
  * model weights and batch arrays are device pointers. */
@@ -279,9 +284,7 @@ int s2v_forward_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, con
  * the array's address (do it at set-up, before any stream capture begins).  All calls
  * on a GPU share the array and keep its last contents; nothing needs zeroing, but
  * calls that overlap on the same GPU race and must be serialised by the caller.
- * With d = 128 the array bounds the batch to fewer than 10,900 nodes, below the 16,384 rows from which the
- * per-level tcgen05 kernel is chosen: this entry runs the warp-level (mma.sync) level kernel, or the tile
- * kernel when max_graph_nodes allows it. */
+ * With d = 128 the array bounds the batch to fewer than 10,900 nodes. */
 #define S2V_STATIC_SCRATCH_BYTES (16u << 20)
 int s2v_forward_static_f32(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, const s2v_batch* batch,
                            float* logits, float* probs, int32_t* pred, float* embed_out);
@@ -351,7 +354,8 @@ int s2v_infer_edges_host_f32(s2v_ctx* ctx, const s2v_model* model, int64_t num_g
  * reports what the scan or a kernel found, and only then writes logits_host / pred_host.  A serving loop that
  * submits batch i+1 on the other lane before it waits for batch i overlaps the PCIe transfers of one batch with
  * the kernels of the other.  The caller's arrays (inputs and outputs) must stay valid and untouched from submit to
- * wait; pinned input arrays keep the submit asynchronous.  Submitting to a lane that still holds a batch, or
+ * wait, and so must the model's weights (an edge between two graphs is found on the device, and the forward then
+ * repeated by the wait); pinned input arrays keep the submit asynchronous.  Submitting to a lane that still holds a batch, or
  * calling a synchronous host entry point (they use lane 0) while lane 0 holds one, returns S2V_ERR_INVALID_ARG;
  * waiting on an idle lane returns S2V_OK. */
 int s2v_infer_edges_host_submit(s2v_ctx* ctx, int lane, const s2v_model* model, int64_t num_graphs, int64_t num_nodes,

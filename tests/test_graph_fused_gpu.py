@@ -55,6 +55,8 @@ def f64(b, rp, ci, val, x, average):
     (32, [1024, 641, 1000, 2], 5.0, {}),                            # d = 32 with 1,024-row tiles
     (32, [640, 130, 1, 300], 3.0, {"val": "row"}),
     (64, [20] * 700, 2.2, {"dense": True, "average": True}),        # several tiles per CTA
+    (128, [1, 2, 0, 127, 128, 5, 3, 70], 2.0, {"auto": True, "dense": True}),          # dense rows at d = 128: one launch after the projection,
+    (128, [50, 77, 128, 1] * 180, 2.2, {"dense": True, "average": True}),              # and several tiles per CTA
     (64, [3] * 3000, 1.0, {"auto": True}),                          # 64 graphs end a tile; the readout inside the kernel
     (128, [30] * 900, 2.2, {"auto": True, "average": True, "val": "row"}),
 ], ids=lambda v: None)
@@ -80,7 +82,7 @@ def test_fused_forward(d, sizes, degree, opts):
     logits, probs, pred, emb = eng.forward(db, want_embed=embed)
     eng.ctx.synchronize()
     if opts.get("auto"):
-        assert eng.ctx.launches - n0 == 1              # the whole classifier in one launch
+        assert eng.ctx.launches - n0 == 1 + (x is not None)   # the whole classifier in one launch, behind a dense projection
     want_h, want = f64(b, rp, ci, val, x, opts.get("average", False))
     if embed:
         assert_close(emb.cpu().numpy(), want_h, "embeddings", scale=max(1.0, float(np.abs(want_h).max())))
@@ -88,6 +90,26 @@ def test_fused_forward(d, sizes, degree, opts):
     e = np.exp(want - want.max(1, keepdims=True))
     assert_close(probs.cpu().numpy(), e / e.sum(1, keepdims=True), "probs", scale=max(1.0, float(np.abs(want).max())))
     assert np.array_equal(pred.cpu().numpy(), logits.cpu().numpy().argmax(1))
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("sizes,degree", [([128], 6.0), ([0, 1, 0, 5, 1, 1, 0, 40, 128, 0, 3, 127, 1, 2], 2.2), ([1] * 300 + [2] * 10, 1.0),
+                                          ([100, 7, 64, 30], 99.0), ([3, 1, 6, 2] * 2000, 2.0)], ids=lambda v: None)
+def test_default_form(d, sizes, degree):
+    """The form that small batches take by default: everything in one launch, with and without the node embeddings."""
+    b = make(sizes, degree, d, 9, 4, 64, 2, seed=d + len(sizes))
+    eng = engine.S2VInference(b.weights, b.levels)
+    hb = engine.build_host_batch(b)
+    db = eng.to_device(hb)
+    n0 = eng.ctx.launches
+    logits, _, _, emb = eng.forward(db, want_embed=True)
+    again, _, _, _ = eng.forward(db)
+    eng.ctx.synchronize()
+    assert eng.ctx.launches - n0 == 2
+    want_h, want = f64(b, hb.row_ptr.numpy(), hb.col_idx.numpy(), None, None, False)
+    assert_close(emb.cpu().numpy(), want_h, "embeddings", scale=max(1.0, float(np.abs(want_h).max())))
+    assert_close(logits.cpu().numpy(), want, "logits", scale=max(1.0, float(np.abs(want).max())))
+    assert torch.equal(again, logits)
 
 
 @pytest.mark.parametrize("auto", [False, True])                     # first level through the product table, and through the MMAs

@@ -87,7 +87,7 @@ def test_tile_kernel_matches_oracle_on_molecules(oracle_lib):
     b = synth.molecules_16k(seed=1, num_graphs=700)
     o = oracle_lib.forward(b, "oracle")
     r = forward(b)
-    assert r["launches"] == 4                     # first-level product table, tile plan, tile kernel, readout
+    assert r["launches"] == 4                     # first-level product table, W in the operand layout, kernel, readout
     assert_close(r["embed"].cpu().numpy(), o["levels"][-1], "embeddings")
     assert_close(r["logits"].cpu().numpy(), o["logits"], "logits", scale=max(1.0, float(np.abs(o["logits"]).max())))
     assert_close(r["probs"].cpu().numpy(), o["probs"], "probs")
@@ -96,7 +96,7 @@ def test_tile_kernel_matches_oracle_on_molecules(oracle_lib):
     assert np.array_equal(r["pred"].cpu().numpy()[safe], o["argmax"][safe]) and safe.mean() > 0.9
     # the same kernel with its first level pushed through the MMA pipeline like the others (S2V_OPT_FIRST_LEVEL_TABLE = 0)
     q = forward(b, first_table=False)
-    assert q["launches"] == 3                     # tile plan, tile kernel, readout
+    assert q["launches"] == 3                     # W in the operand layout, kernel, readout
     assert_close(q["embed"].cpu().numpy(), o["levels"][-1], "embeddings, first level through the MMAs")
     assert_close(q["logits"].cpu().numpy(), o["logits"], "logits, first level through the MMAs", scale=max(1.0, float(np.abs(o["logits"]).max())))
     # the per-level kernels of the same library agree inside the same bar
