@@ -97,7 +97,7 @@ def test_fused_forward(d, sizes, degree, opts):
                                           ([100, 7, 64, 30], 99.0), ([3, 1, 6, 2] * 2000, 2.0)], ids=lambda v: None)
 def test_default_form(d, sizes, degree):
     """The form that small batches take by default: everything in one launch, with and without the node embeddings."""
-    b = make(sizes, degree, d, 9, 4, 64, 2, seed=d + len(sizes))
+    b = make(sizes, degree, d, 9, 4, 32 if d == 32 else 64, 2, seed=d + len(sizes))   # (hidden units whose sums fit the kernel's scratch)
     eng = engine.S2VInference(b.weights, b.levels)
     hb = engine.build_host_batch(b)
     db = eng.to_device(hb)
