@@ -143,10 +143,11 @@ __device__ __forceinline__ ulonglong2 gf_lds(uint32_t addr)   // 16 bytes of sha
     return v;
 }
 
-// Power-of-two scale that brings a largest magnitude into [2^14, 2^15), from its exponent e (clamped so that the scale
-// and its inverse stay normal numbers), and the inverse.
-__device__ __forceinline__ uint32_t gf_exponent(uint32_t max_bits) { return max(max_bits >> 23, 15u); }
-__device__ __forceinline__ float gf_scale(uint32_t e) { return __uint_as_float((268u - e) << 23); }
+// Power-of-two scale that brings a largest magnitude into [2^14, 2^15), from its exponent (clamped so that the scale and its
+// inverse stay normal numbers), and the inverse.  _field: the exponent in its place in the bits.
+__device__ __forceinline__ uint32_t gf_exponent_field(uint32_t max_bits) { return max(max_bits, 15u << 23) & 0x7f800000u; }
+__device__ __forceinline__ float gf_scale_field(uint32_t e) { return __uint_as_float((268u << 23) - e); }
+__device__ __forceinline__ float gf_unscale_field(uint32_t e) { return __uint_as_float(e - (14u << 23)); }
 __device__ __forceinline__ float gf_unscale(uint32_t e) { return __uint_as_float((e - 14u) << 23); }
 
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
@@ -775,6 +776,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     uint32_t* const xo_s = reinterpret_cast<uint32_t*>(smem + map.tags);
     uint2* const chunks = reinterpret_cast<uint2*>(smem + map.col);
     uint4* const chunks_t = reinterpret_cast<uint4*>(smem + map.col);
+    uint4* const p_chunks = reinterpret_cast<uint4*>(smem + Cfg::OFF_S);   // TR, first level
     float4* const H4 = reinterpret_cast<float4*>(smem + Cfg::OFF_H);
     const ulonglong2* const H2 = reinterpret_cast<const ulonglong2*>(smem + Cfg::OFF_H);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + map.bar);
@@ -901,6 +903,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             goff[k] = v < 0 ? 0 : (v > nrows ? nrows : v);
         }
         if (HAS_VAL && threadIdx.x == 0) *s_mixed = 0;
+        if (Cfg::TR && p.P && threadIdx.x == 0) {
+            const uint32_t z = (uint32_t)p.num_tags * Cfg::ROWB;
+            p_chunks[0] = make_uint4(z, z, z, z);
+        }
         int first[ROUNDS], carry = 1;   // chunk 0 is the chunk of zero rows
 #pragma unroll
         for (int k = 0; k < ROUNDS; ++k) {
@@ -930,7 +936,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 info_s[r] = c ? (uint32_t)first[k] | ((uint32_t)(rn[k] < 65535 ? rn[k] : 65535) << 16) : 0u;   // (a listed row is shorter)
                 if (cached)
                     for (int t = 0; t < rn[k]; t += 4) {
-                        uint32_t e[4];
+                        uint32_t e[4], xe[4];
 #pragma unroll
                         for (int u = 0; u < 4; ++u) e[u] = t + u < rn[k] ? (uint32_t)(__ldg(p.col_idx + rb[k] + t + u) - node0) : (uint32_t)p.cap;
 #pragma unroll
@@ -940,9 +946,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                                 p.edge_status->where = 5;
                                 e[u] = 0;
                             }
+                            if (Cfg::TR) xe[u] = xo_s[e[u]];
                             e[u] = Cfg::TR ? Cfg::OFF_H + e[u] * Cfg::ROWB : (e[u] << Cfg::SHIFT) + (e[u] & 7u);
                         }
-                        if (Cfg::TR) chunks_t[first[k] + (t >> 2)] = make_uint4(e[0], e[1], e[2], e[3]);
+                        if (Cfg::TR) {
+                            chunks_t[first[k] + (t >> 2)] = make_uint4(e[0], e[1], e[2], e[3]);
+                            // the first level's list: offsets of the neighbours' table rows, in the operand buffer's place
+                            if (p.P) p_chunks[first[k] + (t >> 2)] = make_uint4(xe[0], xe[1], xe[2], xe[3]);
+                        }
                         else chunks[first[k] + (t >> 2)] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
                     }
                 if (HAS_VAL) {
@@ -1001,43 +1012,51 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 H4[gf_h<D>(r, sl)] = make_float4(relu_max(f0.x + x.x), relu_max(f0.y + x.y), relu_max(f1.x + x.z), relu_max(f1.y + x.w));
             };
             if (Cfg::TR && listed) {
-                // two rows at a time, so that ten table reads are on their way together
+                // Two rows at a time, the third and fourth table row only where there is one.  The table rows' offsets are listed once per tile:
+                // with a look-up of the tag per neighbour, and four rows read always, a batch of 4,093 molecules took 46.9 us for this level alone,
+                // now 39.6.  (Four rows at a time: the registers spill, and what L1 the shared memory leaves goes to the spills: 178 us instead of 144.)
                 const char* const Pl = reinterpret_cast<const char*>(p.P) + 16 * lane;
                 const char* const Xl = reinterpret_cast<const char*>(p.x) + 16 * lane;
-                const uint32_t xo_addr = smem_u32(xo_s) - Cfg::OFF_H / 128;   // X offset of the row at byte h of the map: at h / 128
-                auto table = [&](uint32_t h) -> ulonglong2 {
-                    uint32_t off;
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(off) : "r"(xo_addr + (h >> 7)));
-                    return __ldg(reinterpret_cast<const ulonglong2*>(Pl + off));
-                };
-                for (int r = warp; r < nrows; r += 2 * WARPS) {
-                    const int ra[2] = {r, r + WARPS < nrows ? r + WARPS : p.cap};
-                    uint32_t inf[2];
-                    ulonglong2 v[2][4], x[2];
+                auto table = [&](uint32_t off) { return __ldg(reinterpret_cast<const ulonglong2*>(Pl + off)); };
+                constexpr int A = 2;
+                for (int r = warp; r < nrows; r += A * WARPS) {
+                    uint32_t inf[A];
+                    uint4 c[A];
+                    ulonglong2 v[A][2], t[A][2], x[A];
 #pragma unroll
-                    for (int a = 0; a < 2; ++a) {
-                        inf[a] = ra[a] < nrows ? info_s[ra[a]] : 0u;
-                        const uint4 c = chunks_t[inf[a] & 0xffffu];
-                        v[a][0] = table(c.x); v[a][1] = table(c.y); v[a][2] = table(c.z); v[a][3] = table(c.w);
-                        x[a] = __ldg(reinterpret_cast<const ulonglong2*>(Xl + (ra[a] < nrows ? xo_s[ra[a]] : 0u)));
+                    for (int a = 0; a < A; ++a) {
+                        const int ra = r + a * WARPS;
+                        inf[a] = ra < nrows ? info_s[ra] : 0u;
+                        c[a] = p_chunks[inf[a] & 0xffffu];
+                        x[a] = __ldg(reinterpret_cast<const ulonglong2*>(Xl + (ra < nrows ? xo_s[ra] : 0u)));
                     }
 #pragma unroll
-                    for (int a = 0; a < 2; ++a) {
-                        uint64_t s0 = add2(add2(add2(v[a][0].x, v[a][1].x), v[a][2].x), v[a][3].x);
-                        uint64_t s1 = add2(add2(add2(v[a][0].y, v[a][1].y), v[a][2].y), v[a][3].y);
-                        for (uint32_t k = 1; 4 * k < (inf[a] >> 16); ++k) {
-                            const uint4 c = chunks_t[(inf[a] & 0xffffu) + k];
-                            const ulonglong2 w0 = table(c.x), w1 = table(c.y), w2 = table(c.z), w3 = table(c.w);
-                            s0 = add2(add2(add2(add2(s0, w0.x), w1.x), w2.x), w3.x);
-                            s1 = add2(add2(add2(add2(s1, w0.y), w1.y), w2.y), w3.y);
+                    for (int a = 0; a < A; ++a) { v[a][0] = table(c[a].x); v[a][1] = table(c[a].y); }
+#pragma unroll
+                    for (int a = 0; a < A; ++a)
+                        if (inf[a] >= 0x30000u) { t[a][0] = table(c[a].z); t[a][1] = table(c[a].w); }   // three neighbours or more
+#pragma unroll
+                    for (int a = 0; a < A; ++a) {
+                        const int ra = r + a * WARPS;
+                        if (ra >= nrows) break;
+                        uint64_t s0 = add2(v[a][0].x, v[a][1].x), s1 = add2(v[a][0].y, v[a][1].y);
+                        if (inf[a] >= 0x30000u) {
+                            s0 = add2(add2(s0, t[a][0].x), t[a][1].x);
+                            s1 = add2(add2(s1, t[a][0].y), t[a][1].y);
+                            for (uint32_t k = 1; 4 * k < (inf[a] >> 16); ++k) {
+                                const uint4 d = p_chunks[(inf[a] & 0xffffu) + k];
+                                const ulonglong2 w0 = table(d.x), w1 = table(d.y), w2 = table(d.z), w3 = table(d.w);
+                                s0 = add2(add2(add2(add2(s0, w0.x), w1.x), w2.x), w3.x);
+                                s1 = add2(add2(add2(add2(s1, w0.y), w1.y), w2.y), w3.y);
+                            }
                         }
                         if (HAS_VAL) {
-                            const float w = ra[a] < nrows ? roww[ra[a]] : 0.f;
+                            const float w = roww[ra];
                             s0 = mul2(s0, pack2(w, w));
                             s1 = mul2(s1, pack2(w, w));
                         }
                         const float2 f0 = unpack2(add2(s0, x[a].x)), f1 = unpack2(add2(s1, x[a].y));
-                        if (ra[a] < nrows) H4[ra[a] * 32 + lane] = make_float4(relu_max(f0.x), relu_max(f0.y), relu_max(f1.x), relu_max(f1.y));
+                        H4[ra * 32 + lane] = make_float4(relu_max(f0.x), relu_max(f0.y), relu_max(f1.x), relu_max(f1.y));
                     }
                 }
             } else if (!Cfg::TR && listed) {
@@ -1168,79 +1187,105 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                             }
                         }
                     }
-                } else if (HAS_VAL && weighted) {
-#pragma unroll
-                    for (int i = 0; i < RPG; ++i) {
-                        a0[i] = a1[i] = 0ull;
-                        if (i * NG + warp * GPW < rows_m) {   // warp-uniform
-                            const ulonglong2 v = weighted_row(std::false_type{}, RB * m + i * NG + grp);
-                            a0[i] = v.x;
-                            a1[i] = v.y;
-                        }
-                    }
-                } else {
-                    const GfFar far = far_rows();
-                    int rb[RPG], rn[RPG];
-#pragma unroll
-                    for (int i = 0; i < RPG; ++i) {
-                        rb[i] = rn[i] = 0;
-                        if (i * NG + grp < rows_m) {
-                            const int32_t* const rp = p.row_ptr + node0 + RB * m + i * NG + grp;
-                            rb[i] = __ldg(rp);
-                            rn[i] = __ldg(rp + 1) - rb[i];
-                        }
-                    }
-                    int c = sl < rn[0] ? __ldg(p.col_idx + rb[0] + sl) : 0;
-                    float w = HAS_VAL && sl < rn[0] ? __ldg(p.val + rb[0] + sl) : 0.f;
-#pragma unroll
-                    for (int i = 0; i < RPG; ++i) {
-                        constexpr int LAST = RPG - 1;
-                        const int j = i < LAST ? i + 1 : LAST;
-                        const int cn = i < LAST && sl < rn[j] ? __ldg(p.col_idx + rb[j] + sl) : 0;
-                        const float wn = HAS_VAL && i < LAST && sl < rn[j] ? __ldg(p.val + rb[j] + sl) : 0.f;
-                        a0[i] = a1[i] = 0ull;
-                        if (i * NG + warp * GPW < rows_m) {   // warp-uniform
-                            const ulonglong2 v = gf_row_from_global<D, HAS_VAL, false>(far, p.col_idx + rb[i], p.val + rb[i], rn[i], c, w);
-                            a0[i] = v.x;
-                            a1[i] = v.y;
-                        }
-                        c = cn;
-                        w = wn;
-                    }
                 }
-                // the operand buffer is free once the previous row block of this level is multiplied
-                if (m > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 40);
                 unsigned char* const s_hi = smem + Cfg::OFF_S + gf_op_off(grp, 4 * sl, RB);   // (row i*NG + grp: + i*NG*128, the same swizzle)
                 unsigned char* const s_lo = smem + Cfg::OFF_S + gf_op_off_lo<D>(grp, 4 * sl, RB, Cfg::S_LO);
-                if (uneven) {
-                    const ulonglong2 in_scale = gf_lds(smem_u32(scales->in + 4 * sl));
-#pragma unroll
-                    for (int i = 0; i < RPG; ++i) {
-                        a0[i] = mul2(a0[i], in_scale.x);
-                        a1[i] = mul2(a1[i], in_scale.y);
+                auto largest = [](uint64_t v0, uint64_t v1) {
+                    const float2 f0 = unpack2(v0), f1 = unpack2(v1);
+                    return __float_as_uint(fmaxf(fmaxf(fabsf(f0.x), fabsf(f0.y)), fmaxf(fabsf(f1.x), fabsf(f1.y))));
+                };
+                // row i*NG + grp, mx: its largest element's bits (rows past the tile's last one are written too: finite, never read back)
+                auto put_row = [&](int i, uint64_t v0, uint64_t v1, uint32_t mx) {
+                    const uint32_t ex = gf_exponent_field(mx);
+                    const float s = gf_scale_field(ex);
+                    const uint64_t ss = pack2(s, s);
+                    uint2 hi, lo;
+                    split_f16(mul2(v0, ss), hi.x, lo.x);
+                    split_f16(mul2(v1, ss), hi.y, lo.y);
+                    *reinterpret_cast<uint2*>(s_hi + i * NG * 128) = hi;
+                    *reinterpret_cast<uint2*>(s_lo + i * NG * 128) = lo;
+                    if (sl == 0 && i * NG + grp < rows_m) {
+                        if (Cfg::TR) rsf[RB * m + i * NG + grp] = gf_unscale_field(ex) * inv_w;
+                        else rs[RB * m + i * NG + grp] = (uint8_t)(ex >> 23);
                     }
-                }
+                };
+                // the operand buffer is free once the previous row block of this level is multiplied
+                auto wait_free = [&]() {
+                    if (m > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 40);
+                };
+                if (listed) {
+                    wait_free();
+                    if (uneven) {
+                        const ulonglong2 in_scale = gf_lds(smem_u32(scales->in + 4 * sl));
 #pragma unroll
-                for (int i = 0; i < RPG; ++i) {
-                    if (i * NG + warp * GPW < rows_m) {
-                        const float2 f0 = unpack2(a0[i]), f1 = unpack2(a1[i]);
-                        uint32_t mx = __float_as_uint(fmaxf(fmaxf(fabsf(f0.x), fabsf(f0.y)), fmaxf(fabsf(f1.x), fabsf(f1.y))));
-                        if (LPR == 32) mx = __reduce_max_sync(0xffffffffu, mx);
-                        else
+                        for (int i = 0; i < RPG; ++i) {
+                            a0[i] = mul2(a0[i], in_scale.x);
+                            a1[i] = mul2(a1[i], in_scale.y);
+                        }
+                    }
+                    // Rows whose maxima are taken side by side (a row past the end: zeros): shuffles are worth it (4,096 proteins 1402 -> 1320 us, together
+                    // with the drain under the last product), the one instruction of d = 128 is not (16,384 molecules 438 us, with two rows 447).
+                    constexpr int SB = Cfg::TR ? 1 : (WARPS == 16 && RPG >= 4 ? 4 : 2);
+                    static_assert(RPG % SB == 0, "whole batches");
 #pragma unroll
-                            for (int o = LPR / 2; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-                        const uint32_t ex = gf_exponent(mx);
-                        const float s = gf_scale(ex);
-                        const uint64_t ss = pack2(s, s);
-                        uint2 hi, lo;
-                        split_f16(mul2(a0[i], ss), hi.x, lo.x);
-                        split_f16(mul2(a1[i], ss), hi.y, lo.y);
-                        // (rows past the tile's last one are written too: finite, never read back)
-                        *reinterpret_cast<uint2*>(s_hi + i * NG * 128) = hi;
-                        *reinterpret_cast<uint2*>(s_lo + i * NG * 128) = lo;
-                        if (sl == 0 && i * NG + grp < rows_m) {
-                            if (Cfg::TR) rsf[RB * m + i * NG + grp] = gf_unscale(ex) * inv_w;
-                            else rs[RB * m + i * NG + grp] = (uint8_t)ex;
+                    for (int ib = 0; ib < RPG; ib += SB) {
+                        if (ib * NG + warp * GPW >= rows_m) break;
+                        uint32_t mx[SB];
+#pragma unroll
+                        for (int i = 0; i < SB; ++i) mx[i] = largest(a0[ib + i], a1[ib + i]);
+                        if (LPR == 32) {
+#pragma unroll
+                            for (int i = 0; i < SB; ++i) mx[i] = __reduce_max_sync(0xffffffffu, mx[i]);
+                        } else {
+#pragma unroll
+                            for (int o = LPR / 2; o; o >>= 1)
+#pragma unroll
+                                for (int i = 0; i < SB; ++i) mx[i] = max(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], o));
+                        }
+#pragma unroll
+                        for (int i = 0; i < SB; ++i) put_row(ib + i, a0[ib + i], a1[ib + i], mx[i]);
+                    }
+                } else {
+                    // one row after the other (nothing is held across the calls that sum them)
+                    auto put_sum = [&](int i, ulonglong2 v) {
+                        if (i == 0) wait_free();
+                        if (uneven) {
+                            const ulonglong2 in_scale = gf_lds(smem_u32(scales->in + 4 * sl));
+                            v.x = mul2(v.x, in_scale.x);
+                            v.y = mul2(v.y, in_scale.y);
+                        }
+                        uint32_t mx = largest(v.x, v.y);
+#pragma unroll
+                        for (int o = LPR / 2; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                        put_row(i, v.x, v.y, mx);
+                    };
+                    if (warp * GPW >= rows_m) wait_free();
+                    else if (HAS_VAL && weighted) {
+#pragma unroll 1
+                        for (int i = 0; i * NG + warp * GPW < rows_m; ++i) put_sum(i, weighted_row(std::false_type{}, RB * m + i * NG + grp));
+                    } else {
+                        const GfFar far = far_rows();
+                        auto span = [&](int i, int& b, int& n) {
+                            b = n = 0;
+                            if (i * NG + grp < rows_m) {
+                                const int32_t* const rp = p.row_ptr + node0 + RB * m + i * NG + grp;
+                                b = __ldg(rp);
+                                n = __ldg(rp + 1) - b;
+                            }
+                        };
+                        int b0, n0, b1, n1;   // this row's entries and the next one's
+                        span(0, b0, n0);
+                        span(1, b1, n1);
+                        int c0 = sl < n0 ? __ldg(p.col_idx + b0 + sl) : 0;
+                        float w0 = HAS_VAL && sl < n0 ? __ldg(p.val + b0 + sl) : 0.f;
+#pragma unroll 1
+                        for (int i = 0; i * NG + warp * GPW < rows_m; ++i) {   // warp-uniform
+                            int b2, n2;
+                            span(i + 2, b2, n2);
+                            const int c1 = sl < n1 ? __ldg(p.col_idx + b1 + sl) : 0;
+                            const float w1 = HAS_VAL && sl < n1 ? __ldg(p.val + b1 + sl) : 0.f;
+                            put_sum(i, gf_row_from_global<D, HAS_VAL, false>(far, p.col_idx + b0, p.val + b0, n0, c0, w0));
+                            b0 = b1; n0 = n1; b1 = b2; n1 = n2; c0 = c1; w0 = w1;
                         }
                     }
                 }
@@ -1273,7 +1318,18 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             }
             // -------------------------------- drain: H = ReLU(acc * scale + X) --------------------------------
             // Units of LDC columns of 32 rows.  X of the next unit is on its way while one is worked on, the first unit's
-            // during the wait.  (The last product of the level completes only after every warp has finished gathering from H.)
+            // during the wait.  H may be written once every warp has handed over its last row block (bar_full): the last product runs
+            // under the drain of the row blocks before it, whose products every warp has seen complete.
+            auto wait_last = [&]() {
+                tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            };
+            auto wait_first = [&]() {
+                if (mt > 1) {
+                    tc_wait(bar_full, (job - 1) & 1u, abort_flag, p.status, 43);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                } else if (mt > 0) wait_last();
+            };
             if constexpr (Cfg::TR) {
                 // lane = output feature f, 16 nodes at a time (their scales and tags are broadcast reads); the rows of H are
                 // written 128 bytes per instruction
@@ -1316,9 +1372,9 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 };
                 const int half = 32 * jc;   // my half of every row block: two groups of 16 nodes
                 load_x(half, xa);
-                if (mt > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                wait_first();
                 for (int m = 0; m < mt; ++m) {
+                    if (m > 0 && m == mt - 1) wait_last();
                     load_x(64 * m + half + 16, xb);
                     finish(64 * m + half, xa);
                     if (m + 1 < mt) load_x(64 * (m + 1) + half, xa);
@@ -1335,10 +1391,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 const float4* xp = x_row(0);
 #pragma unroll
                 for (int c = 0; c < LDC / 4; ++c) x[c] = __ldg(xp + c);
-                if (mt > 0) tc_wait(bar_mma, (job - 1) & 1u, abort_flag, p.status, 41);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                wait_first();
                 for (int m = 0; m < mt; ++m) {
                     if (128 * m + 32 * q >= nrows) break;   // warp-uniform
+                    if (m > 0 && m == mt - 1) wait_last();
                     const int r = 128 * m + 32 * q + lane;
                     const bool have = r < nrows;
                     const float c1 = have ? gf_unscale(rs[r]) * inv_w : 0.f;
