@@ -173,6 +173,13 @@ int s2v_launch_level_tc(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n
                         const int32_t* col_idx, const float* val, const float* H, const float* W, const float* X,
                         const float* table, const int32_t* x_index, int n_table, float* out);
 int s2v_launch_wait_selftest(s2v_ctx* ctx, cudaStream_t st);
+// Large matrices, d = 32, 64, 128 (level_stream.cu).  Below, its warps' start and its two launches cost more than they save where rows are of one
+// size (6 entries a row, us, before and with it: d = 32 100,000 rows 24.6 and 27.8, 131,072 34.8 and 30.8; d = 64 65,000 26.7 and 30.2,
+// 131,072 43.3 and 42.1; d = 128 30,000 24.7 and 28.2, 131,072 86.6 and 77.9).
+constexpr int64_t S2V_STREAM_ROWS = 131072;
+int s2v_launch_level_stream(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int d, const void* row_ptr, bool rp64, const int32_t* col_idx,
+                            const float* val, const float* H, const float* W, const float* X, const float* table, const int32_t* x_index, int n_table,
+                            float* out);
 // readout (two layers + softmax / argmax) with the first layer on tcgen05 (readout_tc.cu): d in {64, 128},
 // hidden in {128, 256}, at most 8 classes, batches of at least 6,144 graphs (512 when S2V_OPT_LEVEL_TC = 2)
 bool s2v_readout_tc_supported(const s2v_ctx* ctx, int64_t G, int d, int hidden, int C);

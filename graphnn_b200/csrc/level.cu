@@ -433,6 +433,8 @@ int s2v_launch_level(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_ro
 {
     (void)n_src;
     if (n_rows == 0) return S2V_OK;
+    if (n_rows >= S2V_STREAM_ROWS && (d == 32 || d == 64 || d == 128) && ctx->tc_mode != 0)
+        return s2v_launch_level_stream(ctx, st, long_rows, n_rows, d, row_ptr, rp64, col_idx, val, H, W, X, table, x_index, n_table, out);
     // the sums of long rows lie in `out` for a while, so an X that shares its memory keeps the plain gather
     if (X && X < out + n_rows * d && out < X + n_rows * d) long_rows = false;
     // d = 64, 128: the tcgen05 kernel at every size (a single tile takes 11 us there and 18 - 30 us here)

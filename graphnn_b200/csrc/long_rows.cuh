@@ -26,8 +26,11 @@ constexpr int LONG_SCAN = 8;       // rows per thread and pass of the sums
 enum { LONG_NONE, LONG_INSIDE, LONG_FRONT };   // where a level kernel's long rows are summed
 
 template <int W> struct LongVec;
+template <> struct LongVec<4> { using T = float4; };
 template <> struct LongVec<2> { using T = float2; };
 template <> struct LongVec<1> { using T = float; };
+__device__ __forceinline__ void long_add(float4& a, float4 v) { a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w; }
+__device__ __forceinline__ void long_fma(float4& a, float w, float4 v) { a.x = fmaf(w, v.x, a.x); a.y = fmaf(w, v.y, a.y); a.z = fmaf(w, v.z, a.z); a.w = fmaf(w, v.w, a.w); }
 __device__ __forceinline__ void long_add(float2& a, float2 v) { a.x += v.x; a.y += v.y; }
 __device__ __forceinline__ void long_add(float& a, float v) { a += v; }
 __device__ __forceinline__ void long_fma(float2& a, float w, float2 v) { a.x = fmaf(w, v.x, a.x); a.y = fmaf(w, v.y, a.y); }
