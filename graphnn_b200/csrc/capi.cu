@@ -460,13 +460,13 @@ static int forward(s2v_ctx* ctx, s2v_stream stream, const s2v_model* model, cons
         if (onehot)
             rc = (d == 32 || d == 64 || d == 128)
                      ? s2v_launch_level(ctx, st, long_rows, N, N, d, batch->n2n_row_ptr, false, batch->n2n_col_idx, batch->n2n_val, cur,
-                                        model->p_node_conv, nullptr, model->w_n2l, batch->tags, model->num_feat, dst)
+                                        model->p_node_conv, nullptr, model->w_n2l, batch->tags, model->num_feat, dst, batch->num_edges)
                      : s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "fused level kernel supports d in {32, 64, 128}");
         else
             rc = check_level_args(ctx, N, N, d, batch->n2n_row_ptr, batch->n2n_col_idx, cur, model->p_node_conv, msg, dst);
         if (!onehot && rc == S2V_OK && N > 0)
             rc = s2v_launch_level(ctx, st, long_rows, N, N, d, batch->n2n_row_ptr, false, batch->n2n_col_idx, batch->n2n_val, cur,
-                                  model->p_node_conv, msg, nullptr, nullptr, 0, dst);
+                                  model->p_node_conv, msg, nullptr, nullptr, 0, dst, batch->num_edges);
         if (rc != S2V_OK) return rc;
         if (dst == nxt) std::swap(cur, nxt); else cur = dst;
     }

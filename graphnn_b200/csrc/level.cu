@@ -429,11 +429,12 @@ int launch_d(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, cons
 
 int s2v_launch_level(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int64_t n_src, int d, const void* row_ptr,
                      bool rp64, const int32_t* col_idx, const float* val, const float* H, const float* W,
-                     const float* X, const float* table, const int32_t* x_index, int n_table, float* out)
+                     const float* X, const float* table, const int32_t* x_index, int n_table, float* out, int64_t nnz)
 {
     (void)n_src;
     if (n_rows == 0) return S2V_OK;
-    if (n_rows >= S2V_STREAM_ROWS && (d == 32 || d == 64 || d == 128) && ctx->tc_mode != 0)
+    const bool sparse = d == 128 && nnz > 0 && nnz < 3 * n_rows;
+    if (n_rows >= S2V_STREAM_ROWS && (d == 32 || d == 64 || d == 128) && ctx->tc_mode != 0 && !sparse)
         return s2v_launch_level_stream(ctx, st, long_rows, n_rows, d, row_ptr, rp64, col_idx, val, H, W, X, table, x_index, n_table, out);
     // the sums of long rows lie in `out` for a while, so an X that shares its memory keeps the plain gather
     if (X && X < out + n_rows * d && out < X + n_rows * d) long_rows = false;
