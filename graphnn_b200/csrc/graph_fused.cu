@@ -570,7 +570,7 @@ __device__ __forceinline__ void gf_readout(const GfParams& p, const float* y_s, 
         for (int g = 0; g < NB; ++g) acc[g] = 0.f;
         const float* w = p.W1 + (int64_t)(sl * kper) * hidden + h;
         const float* y = y_s + sl * kper;
-        constexpr int U = NB == 1 ? 16 : 8;   // loads of W1 in flight
+        constexpr int U = NB <= 4 ? 32 : 16;   // loads of W1 in flight
         for (int k = 0; k < kper; k += U) {
             float wv[U];
 #pragma unroll
@@ -752,7 +752,10 @@ __device__ __noinline__ ulonglong2 gf_row_weighted(const GfFar f, uint32_t chunk
     return acc;
 }
 
-template <int D, int WARPS, bool HAS_VAL>
+// READOUT: logits and predictions are made here, W converted and the first level multiplied (small batches).  Otherwise the pooled rows go
+// out, and P and the image of W may have been made beforehand.  One kernel for both: 16,384 molecules 438 us and 700 of them 47 with eight loads
+// of W1 at a time in the readout, 451 and 45.5 with sixteen (the registers of the main loops spill).
+template <int D, int WARPS, bool HAS_VAL, bool READOUT>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fused_kernel(const GfParams p)
 {
     using Cfg = GfCfg<D>;
@@ -831,7 +834,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     const int g_lo = s_range[0], g_hi = s_range[1];
     float inv_w;
     bool uneven;   // scales on both sides of W, in `scales`
-    if (p.w_image) {
+    if (!READOUT && p.w_image) {
         const unsigned char* const image = static_cast<const unsigned char*>(p.w_image);
         if (Cfg::TR) gf_load_w_t(image, tmem_base);
         else
@@ -903,7 +906,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             goff[k] = v < 0 ? 0 : (v > nrows ? nrows : v);
         }
         if (HAS_VAL && threadIdx.x == 0) *s_mixed = 0;
-        if (Cfg::TR && p.P && threadIdx.x == 0) {
+        if (!READOUT && Cfg::TR && p.P && threadIdx.x == 0) {
             const uint32_t z = (uint32_t)p.num_tags * Cfg::ROWB;
             p_chunks[0] = make_uint4(z, z, z, z);
         }
@@ -946,13 +949,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                                 p.edge_status->where = 5;
                                 e[u] = 0;
                             }
-                            if (Cfg::TR) xe[u] = xo_s[e[u]];
+                            if (!READOUT && Cfg::TR) xe[u] = xo_s[e[u]];
                             e[u] = Cfg::TR ? Cfg::OFF_H + e[u] * Cfg::ROWB : (e[u] << Cfg::SHIFT) + (e[u] & 7u);
                         }
                         if (Cfg::TR) {
                             chunks_t[first[k] + (t >> 2)] = make_uint4(e[0], e[1], e[2], e[3]);
                             // the first level's list: offsets of the neighbours' table rows, in the operand buffer's place
-                            if (p.P) p_chunks[first[k] + (t >> 2)] = make_uint4(xe[0], xe[1], xe[2], xe[3]);
+                            if (!READOUT && p.P) p_chunks[first[k] + (t >> 2)] = make_uint4(xe[0], xe[1], xe[2], xe[3]);
                         }
                         else chunks[first[k] + (t >> 2)] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
                     }
@@ -965,7 +968,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                 }
             }
         }
-        if (!p.P) {
+        if (READOUT || !p.P) {
             for (int r = grp; r < nrows; r += NG) {
                 int64_t xr = node0 + r;
                 if (p.tags) {
@@ -1003,7 +1006,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             return gf_row_weighted<D, decltype(first)::value>(far_rows(), smem_u32(smem + map.col) + Cfg::CHUNK * (inf & 0xffffu), weights_at + 16u * (inf & 0xffffu),
                                                               mine, __reduce_max_sync(0xffffffffu, mine));
         };
-        if (p.P) {   // first level: a sum of rows of P = ReLU(W_in) * W, no product
+        if (!READOUT && p.P) {   // first level: a sum of rows of P = ReLU(W_in) * W, no product
             const float4* __restrict__ P4 = reinterpret_cast<const float4*>(p.P);
             auto finish_first = [&](int r, ulonglong2 v) {
                 if (r >= nrows) return;
@@ -1467,7 +1470,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
         };
         auto put_y = [&](int k, float4 acc) {
             if (sub != 0) return;
-            if (p.logits) reinterpret_cast<float4*>(y_s)[k * LPR + sl] = acc;
+            if (READOUT) reinterpret_cast<float4*>(y_s)[k * LPR + sl] = acc;
             else reinterpret_cast<float4*>(p.Y)[(int64_t)(g0 + k) * LPR + sl] = acc;
         };
         for (int k = 0; k < ngr; ++k) {
@@ -1502,11 +1505,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
             }
             gf_worker_sync<WT>();
         }
-        if (p.logits) {
+        if constexpr (READOUT) {
             float* scratch = reinterpret_cast<float*>(smem + Cfg::OFF_H);
             for (int gb = 0; gb < ngr; gb += 8) {
                 const int nb = ngr - gb < 8 ? ngr - gb : 8;
                 if (nb == 1) gf_readout<D, WT, 1>(p, y_s + gb * D, scratch, nb, (int64_t)g0 + gb);
+                else if (nb <= 4) gf_readout<D, WT, 4>(p, y_s + gb * D, scratch, nb, (int64_t)g0 + gb);
                 else gf_readout<D, WT, 8>(p, y_s + gb * D, scratch, nb, (int64_t)g0 + gb);
                 gf_worker_sync<WT>();
             }
@@ -1529,7 +1533,8 @@ constexpr uint32_t gf_budget(int warps) { return (warps == 8 ? 113u : 227u) * 10
 template <int D, int WARPS>
 int gf_launch(s2v_ctx* ctx, cudaStream_t st, const GfParams& p, uint32_t smem, unsigned blocks)
 {
-    auto kern = p.val ? s2v_graph_fused_kernel<D, WARPS, true> : s2v_graph_fused_kernel<D, WARPS, false>;
+    auto kern = p.logits ? (p.val ? s2v_graph_fused_kernel<D, WARPS, true, true> : s2v_graph_fused_kernel<D, WARPS, false, true>)
+                         : (p.val ? s2v_graph_fused_kernel<D, WARPS, true, false> : s2v_graph_fused_kernel<D, WARPS, false, false>);
     S2V_CUDA_OK(ctx, s2v_allow_shared(kern, gf_budget(WARPS)));
     kern<<<blocks, WARPS * 32, smem, st>>>(p);
     S2V_CHECK_LAUNCH(ctx, "s2v_graph_fused_kernel");
@@ -1571,13 +1576,13 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     p.logits = a.logits; p.probs = a.probs; p.pred = a.pred;
     p.status = ctx->dstatus_dev;
     p.edge_status = a.edge_status ? a.edge_status : ctx->dstatus_dev;
-    if (a.P_scratch && a.levels >= 1) {
+    if (a.P_scratch && a.levels >= 1 && !a.logits) {
         const int rc = s2v_launch_first_table_product(ctx, st, a.num_tags, a.d, a.x, a.W, a.P_scratch, true);
         if (rc != S2V_OK) return rc;
         p.P = a.P_scratch;
         p.levels = a.levels - 1;
     }
-    if (a.image_scratch) {
+    if (a.image_scratch && !a.logits) {
         unsigned char* img = static_cast<unsigned char*>(a.image_scratch);
         if (a.d == 128) gf_weight_image_kernel<128><<<1, 1024, 0, st>>>(a.W, img);
         else if (a.d == 64) gf_weight_image_kernel<64><<<1, 1024, 0, st>>>(a.W, img);
