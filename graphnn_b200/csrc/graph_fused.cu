@@ -10,9 +10,9 @@
 // diagonal, so a CTA that owns whole graphs never needs a row of another CTA: HBM sees the CSR, the tags and the
 // results, and the neighbour sums read shared memory at 128 bytes per clock instead of L2.
 //
-// Bounded by the shared-memory reads of the gather (62 % of that pipe) and instruction issue (44 %); HBM and tensor pipe are
+// Bounded by the shared-memory reads of the gather (66 % of that pipe) and instruction issue (50 %); HBM and tensor pipe are
 // idle most of the time.  Measured against one launch per level and the older kernel for d = 128: 64 small graphs, d = 64,
-// 56 -> 16 us; 700 molecules, d = 128, 82 -> 48; 4,093 220 -> 153; 16,384 645 -> 475; 4,096 proteins, d = 64, 1856 -> 1452.
+// 56 -> 16 us; 700 molecules, d = 128, 82 -> 44; 4,093 220 -> 142; 16,384 645 -> 437; 4,096 proteins, d = 64, 1856 -> 1345.
 //
 // Work split.  Every CTA owns a contiguous range of graphs that starts at an equal share of the nodes (found by a
 // search in graph_ptr, no planning launch) and walks it in tiles of whole graphs of at most `cap` nodes.  A tile is up
