@@ -55,7 +55,7 @@ METRIC = "s2v_inference_graphs_per_sec"
 NCU_TRAFFIC = {
     "level_tc_mol_d128": (259830016 + 204611328, "profiles/level_tcgen05.md (mol_d128, 16,384 graphs)"),
     "first_level_mol_d128": (8289024 + 193662464, "profiles/level_first_table.md (mol_first, 16,384 graphs; part of the output is still in L2 when the kernel ends)"),
-    "level_tc_er_d64_half": (806403584 + 119012864, "profiles/level_tcgen05.md (er_d64, n=524,288; scaled x2 for the full problem)"),
+    "level_tc_er_d64_half": (680010752 + 120546048, "profiles/level_stream.md (er_d64, n=524,288; scaled x2 for the full problem)"),
 }
 
 
