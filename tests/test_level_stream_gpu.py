@@ -83,9 +83,11 @@ def test_forms(gpu_ctx, d):
     gpu_ctx.level_lookup(rp, col, None, H, W, table, idx, out[1])
     gpu_ctx.synchronize()
     gpu_ctx.set_option(gpu_ctx.OPT_RESERVED_SMS, 20)
-    gpu_ctx.level(rp, col, None, H, W, X, out[2])
-    gpu_ctx.synchronize()
-    gpu_ctx.set_option(gpu_ctx.OPT_RESERVED_SMS, 0)
+    try:
+        gpu_ctx.level(rp, col, None, H, W, X, out[2])
+        gpu_ctx.synchronize()
+    finally:
+        gpu_ctx.set_option(gpu_ctx.OPT_RESERVED_SMS, 0)
     g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
     with torch.cuda.graph(g, stream=s):
         gpu_ctx.level(rp, col, None, H, W, X, out[3], stream=s.cuda_stream)
