@@ -493,9 +493,12 @@ s2v_level_stream_kernel(int64_t n_rows, const RpT* __restrict__ row_ptr, const i
 
 // ---------------------------------------------------------------- rows of more than `long_limit` entries, finished
 // A CTA looks through a block of rows.  Rows of more than LH_BIG entries come first, streamed through a ring in shared memory by the whole CTA,
-// one after the other; then a warp sums a row at a time, rows of more than LH_MID entries before the others.
-constexpr int LH_THREADS = 512, LH_ROWS = 1024, LH_MID = 1024, LH_BIG = 2048;   // LH_ROWS: rows looked through by a CTA, at most
-constexpr int LH_RING = 64 << 10;
+// one after the other; then a warp sums a row at a time, rows of more than LH_MID entries before the others.  Where there are fewer of those
+// than LH_FEW, the whole CTA takes the ones of more than LH_WARP entries too, or most of its warps would look on (half a million rows of one
+// entry and 500 of 524, d = 128: 303 us without, 236 with).
+constexpr int LH_THREADS = 512, LH_ROWS = 1024, LH_MID = 1024, LH_BIG = 2048, LH_WARP = 256, LH_FEW = 8;   // LH_ROWS: rows looked through by a CTA, at most
+// What leaves the level kernel's CTAs room beside one or two of these.  (d = 128 with 108 KB: R-MAT 2^20 2,130 us instead of 1,600.)
+template <int D> constexpr int LH_RING = (D == 128 ? 80 : 64) << 10;
 
 // A row's sums (shared memory) times W, by a warp: D / 32 consecutive columns a lane
 template <int D, int XMODE>
@@ -555,11 +558,14 @@ s2v_level_hub_kernel(int64_t n_rows, int rows_per_cta, const RpT* __restrict__ r
     }
     __syncthreads();
     const int num_big = cnt[2], longer = cnt[0], total = longer + cnt[1];
-    for (int i = 0; i < num_big; ++i) {
-        const int64_t r = r0 + big[i];
+    const int by_cta = num_big + (total < LH_FEW ? total : 0);
+    auto row_of = [&](int i) { return r0 + list[i < longer ? i : LH_ROWS - (i - longer)]; };
+    for (int i = 0; i < by_cta; ++i) {
+        const int64_t r = i < num_big ? r0 + big[i] : row_of(i - num_big);
         const int64_t b = __ldg(row_ptr + r), len = __ldg(row_ptr + r + 1) - b;
-        long_row_by_cta<D, LH_THREADS, LH_RING, HAS_VAL>(lh_ring, H, col_idx + b, HAS_VAL ? val + b : nullptr, (int)len, sums[i & 1]);
-        if (warp == WARPS - 1) lh_finish<D, XMODE>(sums[i & 1], W, X, x_index, n_table, out, r);   // (done before the row after next ends)
+        if (len <= LH_WARP) continue;
+        long_row_by_cta<D, LH_THREADS, LH_RING<D>, HAS_VAL>(lh_ring, H, col_idx + b, HAS_VAL ? val + b : nullptr, (int)len, sums[0]);
+        if (warp == WARPS - 1) lh_finish<D, XMODE>(sums[0], W, X, x_index, n_table, out, r);   // (done before this warp joins the next row)
     }
     __syncthreads();
     while (true) {
@@ -567,8 +573,9 @@ s2v_level_hub_kernel(int64_t n_rows, int rows_per_cta, const RpT* __restrict__ r
         if (lane == 0) i = atomicAdd(cnt + 3, 1);
         i = __shfl_sync(0xffffffffu, i, 0);
         if (i >= total) break;
-        const int64_t r = r0 + list[i < longer ? i : LH_ROWS - (i - longer)];
+        const int64_t r = row_of(i);
         const int64_t b = __ldg(row_ptr + r), len = __ldg(row_ptr + r + 1) - b;
+        if (total < LH_FEW && len > LH_WARP) continue;
         const int c = lane < len ? __ldg(col_idx + b + lane) : 0;
         long_row_by_warp<D, D, HAS_VAL>(H, col_idx + b, HAS_VAL ? val + b : nullptr, (int)len, c, sums[warp]);
         __syncwarp();
@@ -592,12 +599,12 @@ int ls_launch(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, con
     const int limit = long_rows ? LS_LONG : 0x7fffffff;
     if (long_rows) {
         auto hubs = s2v_level_hub_kernel<D, HAS_VAL, XMODE, RpT>;
-        S2V_CUDA_OK(ctx, s2v_allow_shared(hubs, LH_RING));
-        // about eight CTAs per SM or more, so that they can be dealt out as they finish
-        const int64_t share = (n_rows / (8 * (int64_t)ctx->sm_count) + 63) / 64 * 64;
+        S2V_CUDA_OK(ctx, s2v_allow_shared(hubs, LH_RING<D>));
+        // about four CTAs per SM or more, so that they can be dealt out as they finish (eight: 2 us more for every level)
+        const int64_t share = (n_rows / (4 * (int64_t)ctx->sm_count) + 63) / 64 * 64;
         const int per_cta = (int)(share < 64 ? 64 : (share > LH_ROWS ? LH_ROWS : share));
         const int64_t parts = (n_rows + per_cta - 1) / per_cta, resident = 2 * (int64_t)ctx->sm_count;
-        hubs<<<(unsigned)(all_sms || parts < resident ? parts : resident), LH_THREADS, LH_RING, st>>>(n_rows, per_cta, rp, ci, val, H, W, X, x_index, n_table,
+        hubs<<<(unsigned)(all_sms || parts < resident ? parts : resident), LH_THREADS, LH_RING<D>, st>>>(n_rows, per_cta, rp, ci, val, H, W, X, x_index, n_table,
                                                                                                    out, limit);
         S2V_CHECK_LAUNCH(ctx, "s2v_level_hub_kernel");
         S2V_CUDA_OK(ctx, launch_behind_long_rows(kern, blocks, LsCfg<D>::THREADS, LsCfg<D>::SMEM, st, n_rows, rp, ci, val, H, W, X, x_index, n_table, out, limit,

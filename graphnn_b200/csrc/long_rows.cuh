@@ -72,47 +72,52 @@ __device__ __forceinline__ void long_row_by_warp(const float* __restrict__ H, co
     reinterpret_cast<V*>(out_row)[lane] = acc;
 }
 
-// One row by the whole CTA: the threads copy the neighbour rows through a ring of four stages (three in flight), the first D
-// threads add one column each.
+// One row by the whole CTA: the threads copy the neighbour rows through a ring, TURN rows side by side, and the first D threads add one
+// column each.  A stage costs about 300 cycles (wait, barrier, copies) and 6 to 10 per row, and a row of a large H takes 1.5 us to arrive: so
+// stages of two turns where the ring has room for four of them, and up to eight stages.  (d = 128, ring of 80 KB, one row of 262,144 entries,
+// us: stages of 16 rows 4,020, of 32 2,370; with four stages of 32 rows and each stage's indices loaded one stage ahead 5,900.)
 template <int D, int THREADS, int BYTES, bool HAS_VAL>
 __device__ __forceinline__ void long_row_by_cta(unsigned char* ring, const float* __restrict__ H, const int32_t* __restrict__ col,
                                                 const float* __restrict__ val, int n, float* out_row)
 {
-    constexpr int PIECES = D / 4, TURN = THREADS / PIECES, FIT = BYTES / 4 / (TURN * 4 * D), TURNS = FIT < 4 ? FIT : 4, STAGE = TURN * TURNS;
-    static_assert(TURNS >= 1, "a stage holds at least one turn");
+    constexpr int PIECES = D / 4, TURN = THREADS / PIECES, FIT = BYTES / (TURN * 4 * D);
+    constexpr int TURNS = FIT < 8 ? 1 : (FIT / 4 < 4 ? FIT / 4 : 4), STAGE = TURN * TURNS, NS = FIT / TURNS < 8 ? FIT / TURNS : 8;   // turns and rows per stage, stages
+    static_assert(NS >= 3, "two stages on their way while one is added");
     const int piece = threadIdx.x % PIECES, row0 = threadIdx.x / PIECES;
-    const uint32_t ring_addr = smem_u32(ring);
     const int stages = (n + STAGE - 1) / STAGE;
-    int c[TURNS];
-    auto fetch = [&](int s) {   // indices of stage s, a stage before they are needed
-#pragma unroll
-        for (int k = 0; k < TURNS; ++k) {
-            const int t = s * STAGE + k * TURN + row0;
-            c[k] = row0 < TURN && t < n ? __ldg(col + t) : -1;
-        }
+    const uint32_t ring_addr = smem_u32(ring) + (uint32_t)(row0 * D + 4 * piece) * 4u;
+    // a lane has its group's index of one turn of PIECES; those of the next PIECES turns are on their way
+    auto indices = [&](int q0) {
+        const uint32_t t = (uint32_t)((q0 + piece) * TURN + row0);
+        return row0 < TURN && t < (uint32_t)n ? __ldg(col + t) : -1;
     };
-    auto issue = [&](int s) {
+    int c = indices(0), c_next = indices(PIECES), q = 0, slot = 0;
+    auto issue = [&]() {
 #pragma unroll
-        for (int k = 0; k < TURNS; ++k)
-            if (c[k] >= 0) {
-                const float* src = H + (int64_t)c[k] * D + 4 * piece;
-                const uint32_t dst = ring_addr + (uint32_t)(((s & 3) * STAGE + k * TURN + row0) * D + 4 * piece) * 4u;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+        for (int k = 0; k < TURNS; ++k, ++q) {
+            if (q > 0 && q % PIECES == 0) {
+                c = c_next;
+                c_next = indices(q + PIECES);
             }
+            const int cc = __shfl_sync(0xffffffffu, c, q % PIECES, PIECES);
+            if (cc >= 0)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_addr + (uint32_t)((slot * TURNS + k) * TURN * D) * 4u), "l"(H + (int64_t)cc * D + 4 * piece)
+                             : "memory");
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
+        slot = slot + 1 < NS ? slot + 1 : 0;
     };
-    fetch(0);
-    for (int s = 0; s < 3; ++s) { issue(s); fetch(s + 1); }
+    for (int s = 0; s < NS - 1; ++s) issue();
     float acc = 0.f;
+    int at = 0;
     for (int s = 0; s < stages; ++s) {
-        asm volatile("cp.async.wait_group 2;" ::: "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
         __syncthreads();   // stage s has arrived, and everyone is done with the stage before it
-        issue(s + 3);
-        fetch(s + 4);
+        issue();
         if (threadIdx.x < D) {
-            const float* p = reinterpret_cast<const float*>(ring) + (s & 3) * STAGE * D + threadIdx.x;
+            const float* p = reinterpret_cast<const float*>(ring) + at * STAGE * D + threadIdx.x;
             const int m = n - s * STAGE < STAGE ? n - s * STAGE : STAGE;
-            constexpr int U = 16;
+            constexpr int U = STAGE % 32 == 0 ? 32 : 16;
             int r = 0;
             for (; r + U <= m; r += U) {
                 float v[U];
@@ -123,6 +128,7 @@ __device__ __forceinline__ void long_row_by_cta(unsigned char* ring, const float
             }
             for (; r < m; ++r) acc = HAS_VAL ? fmaf(__ldg(val + s * STAGE + r), p[r * D], acc) : acc + p[r * D];
         }
+        at = at + 1 < NS ? at + 1 : 0;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (threadIdx.x < D) out_row[threadIdx.x] = acc;

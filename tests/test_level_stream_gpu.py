@@ -69,6 +69,51 @@ def test_level(gpu_ctx, d, n, weights, x, rp64):
 
 
 @pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("weights", [False, True])
+@pytest.mark.parametrize("together", [7, 8, 40])
+def test_long_rows_of_one_block(gpu_ctx, d, weights, together):
+    """Long rows next to each other: few (the whole CTA on each) and many (a warp on each), lengths around the stages of the ring."""
+    n = LEAST + 5
+    deg, rp, col, val, H, W, rng = problem(d, n, d + together, hubs=False)
+    lengths = [256, 257, 319, 320, 321, 512, 1023, 1025, 129, 16 * 32 * 32 + 1, 2048, 2049, 640, 1984, 2047]
+    deg[70000:70000 + together] = [lengths[i % len(lengths)] for i in range(together)]
+    rp = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    col = rng.integers(0, H.shape[0], int(rp[-1])).astype(np.int32)
+    val = rng.standard_normal(col.size).astype(np.float32) if weights else None
+    want, bound = reference(deg, rp, col, val, H, W, None)
+    out = torch.full((n, d), float("nan"), device="cuda")
+    gpu_ctx.level(dev(rp), dev(col), dev(val), dev(H), dev(W), None, out)
+    gpu_ctx.synchronize()
+    check(out, want, bound)
+
+
+def test_one_long_row_is_as_fast_per_byte_at_d_128(gpu_ctx):
+    """(it took 2.8 times as long as at d = 64 once; the same is 1.4)"""
+    n, long = LEAST, 200000
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    deg = torch.ones(n, dtype=torch.int64, device="cuda")
+    deg[77] = long
+    rp = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+    rp[1:] = deg.cumsum(0)
+    col = torch.randint(0, n, (int(rp[-1]),), generator=gen, device="cuda", dtype=torch.int32)
+    least = {}
+    for d in (64, 128):
+        H, W, out = torch.randn((n, d), device="cuda"), torch.randn((d, d), device="cuda"), torch.empty((n, d), device="cuda")
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(s)
+            gpu_ctx.level(rp, col, None, H, W, None, out, stream=s.cuda_stream)
+            b.record(s)
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        least[d] = min(times)
+    assert least[128] < 2.1 * least[64]
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
 def test_forms(gpu_ctx, d):
     """The same rows through a graph (twice), with SMs left to others, and with X from a table: the same bits."""
     n, tags = LEAST + 19, 5
