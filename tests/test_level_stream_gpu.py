@@ -88,8 +88,8 @@ def test_long_rows_of_one_block(gpu_ctx, d, weights, together):
 
 
 def test_one_long_row_is_as_fast_per_byte_at_d_128(gpu_ctx):
-    """(it took 2.8 times as long as at d = 64 once; the same is 1.4)"""
-    n, long = LEAST, 200000
+    """(1.84 times the time of d = 64 with stages of 32 rows and 96 rows on their way, 1.34 now; H does not fit the L2)"""
+    n, long = 4 * LEAST, 2 * LEAST
     gen = torch.Generator(device="cuda").manual_seed(1)
     deg = torch.ones(n, dtype=torch.int64, device="cuda")
     deg[77] = long
@@ -110,7 +110,7 @@ def test_one_long_row_is_as_fast_per_byte_at_d_128(gpu_ctx):
             b.synchronize()
             times.append(a.elapsed_time(b))
         least[d] = min(times)
-    assert least[128] < 2.1 * least[64]
+    assert least[128] < 1.6 * least[64], least
 
 
 @pytest.mark.parametrize("d", [32, 64, 128])
