@@ -65,6 +65,9 @@ def load_library():
         "s2v_level_f32": (i32, [vp, vp, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp]),
         "s2v_level_rp64_f32": (i32, [vp, vp, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp]),
         "s2v_level_lookup_f32": (i32, [vp, vp, i64, i64, i32, vp, vp, vp, vp, vp, vp, i32, vp, vp]),
+        "s2v_level_nnz_f32": (i32, [vp, vp, i64, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp]),
+        "s2v_level_lookup_nnz_f32": (i32, [vp, vp, i64, i64, i64, i32, vp, vp, vp, vp, vp, vp, i32, vp, vp]),
+        "s2v_level_path": (i32, [i64, i32, i64, i32, i32, i32]),
         "s2v_level_first_f32": (i32, [vp, vp, i64, i32, vp, vp, vp, vp, vp, i32, vp, vp]),
         "s2v_spmm_csr_f32": (i32, [vp, vp, i64, i64, i32, vp, vp, vp, vp, f32, f32, vp]),
         "s2v_gemm_f32": (i32, [vp, vp, i32, i32, i64, i64, i64, f32, vp, i64, vp, i64, f32, vp, i64]),
@@ -131,6 +134,11 @@ def _ptr(t):
     if isinstance(t, np.ndarray):
         return t.ctypes.data
     return t.data_ptr()
+
+
+def _count(t):
+    """Entries of a matrix, as its column indices show them (None: unknown)."""
+    return 0 if t is None else (t.size if isinstance(t, np.ndarray) else t.numel())
 
 
 def build_n2n_csr_host(num_nodes: int, edge_src: np.ndarray, edge_dst: np.ndarray, average: bool = False,
@@ -307,14 +315,16 @@ class Context:
     def level(self, row_ptr, col_idx, val, H, W, X, out, n_src=None, stream=None):
         n_rows, d = out.shape
         n_src = H.shape[0] if n_src is None else n_src
-        name = "s2v_level_rp64_f32" if row_ptr.element_size() == 8 else "s2v_level_f32"
-        self.call(name, stream, n_rows, n_src, d, _ptr(row_ptr), _ptr(col_idx), _ptr(val), _ptr(H), _ptr(W), _ptr(X),
-                  _ptr(out))
+        arrays = (d, _ptr(row_ptr), _ptr(col_idx), _ptr(val), _ptr(H), _ptr(W), _ptr(X), _ptr(out))
+        if row_ptr.element_size() == 8:
+            self.call("s2v_level_rp64_f32", stream, n_rows, n_src, *arrays)
+        else:
+            self.call("s2v_level_nnz_f32", stream, n_rows, n_src, _count(col_idx), *arrays)
         return out
 
     def level_lookup(self, row_ptr, col_idx, val, H, W, table, x_index, out, stream=None):
         n_rows, d = out.shape
-        self.call("s2v_level_lookup_f32", stream, n_rows, H.shape[0], d, _ptr(row_ptr), _ptr(col_idx), _ptr(val),
+        self.call("s2v_level_lookup_nnz_f32", stream, n_rows, H.shape[0], _count(col_idx), d, _ptr(row_ptr), _ptr(col_idx), _ptr(val),
                   _ptr(H), _ptr(W), _ptr(table), table.shape[0], _ptr(x_index), _ptr(out))
         return out
 

@@ -208,11 +208,17 @@ int s2v_level_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src
                   const int32_t* col_idx, const float* val, const float* H, const float* W, const float* X,
                   float* out)
 {
+    return s2v_level_nnz_f32(ctx, stream, n_rows, n_src, 0, d, row_ptr, col_idx, val, H, W, X, out);
+}
+
+int s2v_level_nnz_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src, int64_t nnz, int d, const int32_t* row_ptr,
+                      const int32_t* col_idx, const float* val, const float* H, const float* W, const float* X, float* out)
+{
     S2V_ENTER(ctx);
     int rc = check_level_args(ctx, n_rows, n_src, d, row_ptr, col_idx, H, W, X, out);
     if (rc != S2V_OK || n_rows == 0) return rc;
     return s2v_launch_level(ctx, s2v_pick_stream(ctx, stream), true, n_rows, n_src, d, row_ptr, false, col_idx, val, H, W, X,
-                            nullptr, nullptr, 0, out);
+                            nullptr, nullptr, 0, out, nnz);
 }
 
 int s2v_level_rp64_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src, int d, const int64_t* row_ptr,
@@ -230,6 +236,13 @@ int s2v_level_lookup_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_
                          const int32_t* row_ptr, const int32_t* col_idx, const float* val, const float* H,
                          const float* W, const float* table, int n_table, const int32_t* x_index, float* out)
 {
+    return s2v_level_lookup_nnz_f32(ctx, stream, n_rows, n_src, 0, d, row_ptr, col_idx, val, H, W, table, n_table, x_index, out);
+}
+
+int s2v_level_lookup_nnz_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src, int64_t nnz, int d,
+                             const int32_t* row_ptr, const int32_t* col_idx, const float* val, const float* H,
+                             const float* W, const float* table, int n_table, const int32_t* x_index, float* out)
+{
     S2V_ENTER(ctx);
     int rc = check_level_args(ctx, n_rows, n_src, d, row_ptr, col_idx, H, W, table, out);
     if (rc != S2V_OK || n_rows == 0) return rc;
@@ -238,7 +251,7 @@ int s2v_level_lookup_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_
     rc = s2v_launch_index_check(ctx, s2v_pick_stream(ctx, stream), n_rows, x_index, n_table);
     if (rc != S2V_OK) return rc;
     return s2v_launch_level(ctx, s2v_pick_stream(ctx, stream), true, n_rows, n_src, d, row_ptr, false, col_idx, val, H, W,
-                            nullptr, table, x_index, n_table, out);
+                            nullptr, table, x_index, n_table, out, nnz);
 }
 
 int s2v_level_first_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n, int d, const int32_t* row_ptr, const int32_t* col_idx,

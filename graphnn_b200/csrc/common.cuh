@@ -175,8 +175,7 @@ int s2v_launch_level_tc(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n
 int s2v_launch_wait_selftest(s2v_ctx* ctx, cudaStream_t st);
 // Large matrices, d = 32, 64, 128 (level_stream.cu).  Below, its warps' start and its two launches cost more than they save where rows are of one
 // size (6 entries a row, us, before and with it: d = 32 100,000 rows 24.6 and 27.8, 131,072 47 and 33; d = 64 65,000 26.7 and 30.2, 131,072
-// 48.7 and 47.2; d = 128 30,000 24.7 and 28.2, 131,072 89.6 and 85.8).  At d = 128 rows of two entries, half a million of them, take 203 us
-// without it and 224 with it, of eight 582 and 420: where a matrix is known to have fewer than three a row it stays with level_tc.cu.
+// 48.7 and 47.2; d = 128 30,000 24.7 and 28.2, 131,072 89.6 and 85.8).
 constexpr int64_t S2V_STREAM_ROWS = 131072;
 int s2v_launch_level_stream(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int d, const void* row_ptr, bool rp64, const int32_t* col_idx,
                             const float* val, const float* H, const float* W, const float* X, const float* table, const int32_t* x_index, int n_table,

@@ -427,19 +427,35 @@ int launch_d(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, cons
 
 }  // namespace
 
+// Which kernel a level takes.  level_tc.cu below S2V_STREAM_ROWS rows: a single tile takes 11 us there and 18 - 30 us here.  Above, level_stream.cu,
+// but for matrices with few entries a row at d = 128: a unit of level_stream.cu is two rows, whose cost is the same with two entries and
+// with eight.  Time of level_tc.cu over that of level_stream.cu, no hubs, with X / without / X from a table / edge weights:
+//     entries a row       1                    2                    3                    4                    6
+//     131,072 rows   .84 .74 .81 .82      .93 .84 .90 .90      .98 .91 .96 .97      1.02  .94 1.00  .99   1.06  .98 1.02 1.02
+//     524,288        .83 .65 .75 .79      .94 .79 .85 .90     1.03 .95 .99 1.04     1.19 1.09 1.13 1.11   1.33 1.26 1.29 1.31
+// Hence 3 entries with X and 3.5 without.  (Long rows turn it: half a million rows of one entry and 2,000 of 131, 347 us there and 255; but a caller with so few
+// entries has hardly any.)  At d = 64 rows of one entry take .83 to .91, of two .90 to 1.01, of three .96 to 1.10, and with hubs up to 3.2:
+// level_stream.cu throughout.
+extern "C" int s2v_level_path(int64_t n_rows, int d, int64_t nnz, int offsets64, int dense_x, int level_tc)
+{
+    if (level_tc == 0 || (d != 32 && d != 64 && d != 128)) return S2V_LEVEL_PATH_MMA;
+    const bool sparse = d == 128 && !offsets64 && nnz > 0 && 2 * nnz < (dense_x ? 6 : 7) * n_rows;
+    if (n_rows >= S2V_STREAM_ROWS && !sparse) return S2V_LEVEL_PATH_STREAM;
+    return !offsets64 && d != 32 ? S2V_LEVEL_PATH_TC : S2V_LEVEL_PATH_MMA;
+}
+
 int s2v_launch_level(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int64_t n_src, int d, const void* row_ptr,
                      bool rp64, const int32_t* col_idx, const float* val, const float* H, const float* W,
                      const float* X, const float* table, const int32_t* x_index, int n_table, float* out, int64_t nnz)
 {
     (void)n_src;
     if (n_rows == 0) return S2V_OK;
-    const bool sparse = d == 128 && nnz > 0 && nnz < 3 * n_rows;
-    if (n_rows >= S2V_STREAM_ROWS && (d == 32 || d == 64 || d == 128) && ctx->tc_mode != 0 && !sparse)
+    const int path = s2v_level_path(n_rows, d, nnz, rp64, X != nullptr, ctx->tc_mode);
+    if (path == S2V_LEVEL_PATH_STREAM)
         return s2v_launch_level_stream(ctx, st, long_rows, n_rows, d, row_ptr, rp64, col_idx, val, H, W, X, table, x_index, n_table, out);
     // the sums of long rows lie in `out` for a while, so an X that shares its memory keeps the plain gather
     if (X && X < out + n_rows * d && out < X + n_rows * d) long_rows = false;
-    // d = 64, 128: the tcgen05 kernel at every size (a single tile takes 11 us there and 18 - 30 us here)
-    if (!rp64 && (d == 64 || d == 128) && ctx->tc_mode != 0) {
+    if (path == S2V_LEVEL_PATH_TC) {
         const int rc = s2v_launch_level_tc(ctx, st, long_rows, n_rows, d, (const int32_t*)row_ptr, col_idx, val, H, W, X, table,
                                            x_index, n_table, out);
         if (rc != S2V_ERR_UNSUPPORTED) return rc;

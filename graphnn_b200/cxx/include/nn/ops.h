@@ -429,8 +429,8 @@ public:
         ASSERT(A.cols() == H.rows() && H.cols() == W.rows() && W.rows() == W.cols(), "shape mismatch in S2VLevel");
         auto& out = detail::dense<mode, Dtype>(outputs[0]);
         out.Reshape({A.rows(), W.cols()});
-        S2V_ASSERT_OK(s2v_level_f32(GpuHandle::ctx(), nullptr, (int64_t)A.rows(), (int64_t)A.cols(), (int)W.cols(), A.data->row_ptr,
-                                    A.data->col_idx, A.data->val, H.data->ptr, W.data->ptr, X, out.data->ptr));
+        S2V_ASSERT_OK(s2v_level_nnz_f32(GpuHandle::ctx(), nullptr, (int64_t)A.rows(), (int64_t)A.cols(), (int64_t)A.data->nnz, (int)W.cols(),
+                                        A.data->row_ptr, A.data->col_idx, A.data->val, H.data->ptr, W.data->ptr, X, out.data->ptr));
     }
 };
 

@@ -116,6 +116,10 @@ int s2v_level_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src
 int s2v_level_rp64_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src, int d,
                        const int64_t* row_ptr, const int32_t* col_idx, const float* val, const float* H,
                        const float* W, const float* X, float* out);
+/* s2v_level_f32 for a caller who knows the number of entries, row_ptr[n_rows] (<= 0: unknown, as s2v_level_f32 assumes).  It is only used to
+ * choose the kernel: from 131,072 rows on at d = 128, fewer than 3 entries a row (3.5 without X) make another one the faster by up to a third. */
+int s2v_level_nnz_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src, int64_t nnz, int d, const int32_t* row_ptr,
+                      const int32_t* col_idx, const float* val, const float* H, const float* W, const float* X, float* out);
 /* Level whose X term is a table lookup: X[i,:] = table[x_index[i],:]; this is
  * X = onehot(tags) * W_in without materialising the product (the reference's
  * node_input * w_n2l, kernel_mean_field.cpp:31, with the one-hot X GetBatch builds,
@@ -125,6 +129,18 @@ int s2v_level_rp64_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t 
 int s2v_level_lookup_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src, int d,
                          const int32_t* row_ptr, const int32_t* col_idx, const float* val, const float* H,
                          const float* W, const float* table, int n_table, const int32_t* x_index, float* out);
+/* The same with the number of entries, as s2v_level_nnz_f32. */
+int s2v_level_lookup_nnz_f32(s2v_ctx* ctx, s2v_stream stream, int64_t n_rows, int64_t n_src, int64_t nnz, int d,
+                             const int32_t* row_ptr, const int32_t* col_idx, const float* val, const float* H,
+                             const float* W, const float* table, int n_table, const int32_t* x_index, float* out);
+/* Diagnostic: which kernel a level of this size takes (offsets64: 64-bit row offsets; dense_x: X is given,
+ * and not from a table; level_tc: the value of S2V_OPT_LEVEL_TC). */
+typedef enum s2v_level_path_kind {
+    S2V_LEVEL_PATH_MMA = 0,    /* warp-level matrix instructions: every form */
+    S2V_LEVEL_PATH_TC = 1,     /* tcgen05, d = 64 and 128, 32-bit offsets */
+    S2V_LEVEL_PATH_STREAM = 2  /* tcgen05, large matrices */
+} s2v_level_path_kind;
+int s2v_level_path(int64_t n_rows, int d, int64_t nnz, int offsets64, int dense_x, int level_tc);
 
 /* First level of the classifier with one-hot inputs, without materialising H0:
  * out = ReLU((A * ReLU(table[tags,:])) * W + table[tags,:]), A square [n x n]; i.e. MatMul(data, w_n2l),

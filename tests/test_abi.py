@@ -129,3 +129,38 @@ def test_edge_level_builders_on_a_large_batch_and_bad_input(lib, oracle_lib):
     assert m["n2e"][1].tolist() == [0, 1, 2, 0]
     with pytest.raises(capi.S2VError):
         capi.build_edge_csrs_host(3, np.array([0, 5], np.int32), np.array([1, 2], np.int32))
+
+
+def test_level_path(lib):
+    """The kernel that a level takes, over sizes, widths, entry counts, offsets and the option: large matrices the streaming kernel, but for
+    32-bit offsets, d = 128 and a known count below 3 a row (3.5 without a dense X); 64-bit offsets and d = 32 never level_tc.cu; option 0 neither."""
+    MMA, TC, STREAM = 0, 1, 2
+    limit = 131072
+    for d in (16, 32, 64, 128, 256):
+        for rp64 in (0, 1):
+            for tc in (0, 1, 2):
+                for n in (1, 127, limit - 1, limit, limit + 1, 1 << 22, 1 << 33):
+                    for nnz in (-1, 0, 1, n, 3 * n - 1, 3 * n, (7 * n - 1) // 2, (7 * n + 1) // 2, 4 * n, 100 * n):
+                        for x in (0, 1):
+                            known_sparse = d == 128 and not rp64 and nnz > 0 and nnz < (3 if x else 3.5) * n
+                            want = (MMA if tc == 0 or d not in (32, 64, 128) else STREAM if n >= limit and not known_sparse
+                                    else TC if not rp64 and d != 32 else MMA)
+                            assert lib.s2v_level_path(n, d, nnz, rp64, x, tc) == want, (n, d, nnz, rp64, x, tc)
+
+
+def test_levels_pass_their_entry_count():
+    """Context.level and level_lookup tell the library how many entries there are; 64-bit offsets have no use for it."""
+    import torch
+    ctx, calls = object.__new__(capi.Context), []
+    ctx.call = lambda name, stream, *args: calls.append((name, args))
+    col, H, out = torch.zeros(10, dtype=torch.int32), torch.zeros(7, 32), torch.zeros(4, 32)
+    W, X, idx = torch.zeros(32, 32), torch.zeros(4, 32), torch.zeros(4, dtype=torch.int32)
+    try:
+        for dtype in (torch.int32, torch.int64):
+            ctx.level(torch.zeros(5, dtype=dtype), col, None, H, W, X, out)
+        ctx.level_lookup(torch.zeros(5, dtype=torch.int32), col, None, H, W, X, idx, out)
+        ctx.level(torch.zeros(5, dtype=torch.int32), None, None, H, W, X, out)
+    finally:
+        ctx.h = None   # (nothing to close)
+    assert [(n, a[:4]) for n, a in calls] == [("s2v_level_nnz_f32", (4, 7, 10, 32)), ("s2v_level_rp64_f32", (4, 7, 32, calls[1][1][3])),
+                                              ("s2v_level_lookup_nnz_f32", (4, 7, 10, 32)), ("s2v_level_nnz_f32", (4, 7, 0, 32))]

@@ -22,6 +22,31 @@ def sparse_rows(n, seed, hubs):
     return deg, rp, rng.integers(0, n, int(rp[-1])).astype(np.int32), rng
 
 
+@pytest.mark.parametrize("x", [False, True])
+@pytest.mark.parametrize("weights", [False, True])
+def test_level(gpu_ctx, x, weights):
+    """One level with the count known (level_tc.cu), and as the entry without it takes it (level_stream.cu)."""
+    d, n = 128, LEAST + 50
+    deg, rp, col, rng = sparse_rows(n, 11, True)
+    val = rng.standard_normal(col.size).astype(np.float32) if weights else None
+    H, W = rng.standard_normal((n, d), dtype=np.float32), rng.standard_normal((d, d), dtype=np.float32) * 0.1
+    X = rng.standard_normal((n, d), dtype=np.float32) if x else None
+    A = sp.csr_matrix((np.ones(col.size) if val is None else val.astype(np.float64), col, rp), (n, n))
+    want = np.maximum(A @ H.astype(np.float64) @ W.astype(np.float64) + (0 if X is None else X), 0)
+    rows = np.maximum(np.abs(want).max(1, keepdims=True), 1)   # hub sums are held to 1e-5 of their row's scale
+    args = [None if a is None else torch.from_numpy(a).cuda() for a in (rp, col, val, H, W, X)]
+    ptr = lambda t: None if t is None else t.data_ptr()
+    for known in (True, False):
+        out = torch.full((n, d), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        if known:
+            gpu_ctx.level(*args, out)
+        else:
+            gpu_ctx.call("s2v_level_f32", None, n, n, d, *map(ptr, args), ptr(out))
+        gpu_ctx.synchronize()
+        np.testing.assert_allclose(out.cpu().numpy() / rows, want / rows, rtol=1e-5, atol=1e-5)
+
+
 @pytest.mark.parametrize("hubs", [False, True])
 @pytest.mark.parametrize("weights", [False, True])
 def test_forward(hubs, weights):
