@@ -38,13 +38,17 @@ namespace
 
 constexpr int LS_RING = 16;                   // tiles that are known at a time
 constexpr int LS_LONG = 128;                  // longer rows are left to the kernel in front
-template <int D>
+// ONE: one CTA per SM at every d, for grids that are to leave SMs free (CTAs go to every SM before one gets two).  24 gather warps with eight loads a lane at
+// 64 registers, the most that AHEAD allows.  A million rows, 8 entries each, with one and with 20 SMs left, us: d = 64 404 and 443 (one CTA of the two 638 and 726,
+// 16 warps 493 and 552; level_tc.cu 482 and 501), d = 32 218 and 242 (341 and 388); R-MAT 2^20, d = 64, 908 and 945 (963 and 1,097; 1,812 and 4,602).
+// R-MAT 2^17 with one SM left loses (d = 64 137 -> 161): there is no room beside a CTA of the kernel in front.
+template <int D, bool ONE = false>
 struct LsCfg {
     static constexpr int SUB = 128 / D, LPR = D / 4;      // lane groups of a warp, lanes per group
-    static constexpr int CTAS = D == 128 ? 1 : 2;         // per SM: tensor memory has 512 columns, W^T takes 2 d of them
-    static constexpr int GW = D == 128 ? 15 : 19, EW = D == 128 ? 8 : 4, MW = GW + EW, THREADS = (MW + 1) * 32;   // gather and epilogue warps, number of the MMA warp
+    static constexpr int CTAS = D == 128 || ONE ? 1 : 2;  // per SM: tensor memory has 512 columns, W^T takes 2 d of them
+    static constexpr int GW = D == 128 ? 15 : (ONE ? 24 : 19), EW = D == 128 ? 8 : 4, MW = GW + EW, THREADS = (MW + 1) * 32;   // gather and epilogue warps, number of the MMA warp
     static constexpr int R = D == 128 ? 2 : 1;            // rows per lane group and unit
-    static constexpr int U = D == 128 ? 8 : 4;            // neighbours whose rows are on their way together
+    static constexpr int U = D == 128 || ONE ? 8 : 4;     // neighbours whose rows are on their way together
     static constexpr int HELD = D == 128 ? 3 : 2;         // units a gather warp has taken and not stored
     static constexpr int TN = 16, STAGES = 4, ROWS = TN * R * SUB, WROWS = TN * R;   // units per tile, tiles of operands, rows per tile and epilogue warp
     static constexpr int ACC = D == 32 ? 2 : 4;           // accumulators
@@ -120,13 +124,13 @@ __device__ __forceinline__ int ls_answer(uint32_t resp)
     return x;
 }
 
-template <int D, bool HAS_VAL, int XMODE /*0 none, 1 dense, 2 table lookup*/, typename RpT>
-__global__ void __launch_bounds__(LsCfg<D>::THREADS, LsCfg<D>::CTAS)
+template <int D, bool HAS_VAL, int XMODE /*0 none, 1 dense, 2 table lookup*/, typename RpT, bool ONE>
+__global__ void __launch_bounds__(LsCfg<D, ONE>::THREADS, LsCfg<D, ONE>::CTAS)
 s2v_level_stream_kernel(int64_t n_rows, const RpT* __restrict__ row_ptr, const int32_t* __restrict__ col_idx, const float* __restrict__ val,
                         const float* __restrict__ H, const float* __restrict__ W, const float* X, const int32_t* __restrict__ x_index, int n_table,
                         float* out, int long_limit, int num_tiles, s2v_device_status* status)
 {
-    using Cfg = LsCfg<D>;
+    using Cfg = LsCfg<D, ONE>;
     constexpr int SUB = Cfg::SUB, LPR = Cfg::LPR, TN = Cfg::TN, ROWS = Cfg::ROWS, STAGES = Cfg::STAGES, ACC = Cfg::ACC, U = Cfg::U, WROWS = Cfg::WROWS;
     extern __shared__ unsigned char ls_smem_raw[];
     unsigned char* const smem = ls_smem_raw + ((1024u - (smem_u32(ls_smem_raw) & 1023u)) & 1023u);
@@ -585,17 +589,18 @@ s2v_level_hub_kernel(int64_t n_rows, int rows_per_cta, const RpT* __restrict__ r
     }
 }
 
-template <int D, bool HAS_VAL, int XMODE, typename RpT>
-int ls_launch(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const RpT* rp, const int32_t* ci, const float* val, const float* H,
-              const float* W, const float* X, const int32_t* x_index, int n_table, float* out)
+// ONE: some SMs are left to others (S2V_OPT_RESERVED_SMS); the kernel in front does not keep off them, but ends early
+template <int D, bool HAS_VAL, int XMODE, typename RpT, bool ONE>
+int ls_launch_on(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const RpT* rp, const int32_t* ci, const float* val, const float* H,
+                 const float* W, const float* X, const int32_t* x_index, int n_table, float* out)
 {
-    auto kern = s2v_level_stream_kernel<D, HAS_VAL, XMODE, RpT>;
-    S2V_CUDA_OK(ctx, s2v_allow_shared(kern, LsCfg<D>::SMEM));
-    constexpr int64_t ROWS = LsCfg<D>::ROWS;
+    using Cfg = LsCfg<D, ONE && D != 128>;
+    auto kern = s2v_level_stream_kernel<D, HAS_VAL, XMODE, RpT, ONE && D != 128>;
+    S2V_CUDA_OK(ctx, s2v_allow_shared(kern, Cfg::SMEM));
+    constexpr int64_t ROWS = Cfg::ROWS;
     const int64_t tiles = (n_rows + ROWS - 1) / ROWS;
     if (tiles >= (int64_t)INT32_MAX) return s2v_fail(ctx, S2V_ERR_UNSUPPORTED, "level: too many rows");
-    const bool all_sms = ctx->sm_count == ctx->sm_count_hw;   // (S2V_OPT_RESERVED_SMS)
-    const unsigned blocks = (unsigned)(all_sms || tiles < ctx->sm_count ? tiles : ctx->sm_count);
+    const unsigned blocks = (unsigned)(!ONE || tiles < ctx->sm_count ? tiles : ctx->sm_count);
     const int limit = long_rows ? LS_LONG : 0x7fffffff;
     if (long_rows) {
         auto hubs = s2v_level_hub_kernel<D, HAS_VAL, XMODE, RpT>;
@@ -604,15 +609,24 @@ int ls_launch(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, con
         const int64_t share = (n_rows / (4 * (int64_t)ctx->sm_count) + 63) / 64 * 64;
         const int per_cta = (int)(share < 64 ? 64 : (share > LH_ROWS ? LH_ROWS : share));
         const int64_t parts = (n_rows + per_cta - 1) / per_cta, resident = 2 * (int64_t)ctx->sm_count;
-        hubs<<<(unsigned)(all_sms || parts < resident ? parts : resident), LH_THREADS, LH_RING<D>, st>>>(n_rows, per_cta, rp, ci, val, H, W, X, x_index, n_table,
-                                                                                                   out, limit);
+        hubs<<<(unsigned)(!ONE || parts < resident ? parts : resident), LH_THREADS, LH_RING<D>, st>>>(n_rows, per_cta, rp, ci, val, H, W, X, x_index, n_table,
+                                                                                                    out, limit);
         S2V_CHECK_LAUNCH(ctx, "s2v_level_hub_kernel");
-        S2V_CUDA_OK(ctx, launch_behind_long_rows(kern, blocks, LsCfg<D>::THREADS, LsCfg<D>::SMEM, st, n_rows, rp, ci, val, H, W, X, x_index, n_table, out, limit,
+        S2V_CUDA_OK(ctx, launch_behind_long_rows(kern, blocks, Cfg::THREADS, Cfg::SMEM, st, n_rows, rp, ci, val, H, W, X, x_index, n_table, out, limit,
                                                  (int)tiles, ctx->dstatus_dev));
     } else
-        kern<<<blocks, LsCfg<D>::THREADS, LsCfg<D>::SMEM, st>>>(n_rows, rp, ci, val, H, W, X, x_index, n_table, out, limit, (int)tiles, ctx->dstatus_dev);
+        kern<<<blocks, Cfg::THREADS, Cfg::SMEM, st>>>(n_rows, rp, ci, val, H, W, X, x_index, n_table, out, limit, (int)tiles, ctx->dstatus_dev);
     S2V_CHECK_LAUNCH(ctx, "s2v_level_stream_kernel");
     return S2V_OK;
+}
+
+template <int D, bool HAS_VAL, int XMODE, typename RpT>
+int ls_launch(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const RpT* rp, const int32_t* ci, const float* val, const float* H,
+              const float* W, const float* X, const int32_t* x_index, int n_table, float* out)
+{
+    return ctx->sm_count == ctx->sm_count_hw
+               ? ls_launch_on<D, HAS_VAL, XMODE, RpT, false>(ctx, st, long_rows, n_rows, rp, ci, val, H, W, X, x_index, n_table, out)
+               : ls_launch_on<D, HAS_VAL, XMODE, RpT, true>(ctx, st, long_rows, n_rows, rp, ci, val, H, W, X, x_index, n_table, out);
 }
 
 template <int D, typename RpT>

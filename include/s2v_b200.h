@@ -80,7 +80,9 @@ typedef enum s2v_option {
                                         one graph per CTA and its columns fit shared memory.  Default from S2V_GRAPH_TILES */
     S2V_OPT_RESERVED_SMS = 4,        /* the persistent kernels size their grids for (SM count - value) SMs, leaving the rest to
                                         kernels of another stream -- a communication library's, which cannot start while
-                                        one-CTA-per-SM kernels hold every SM (default 0; 0 <= value < SM count) */
+                                        one-CTA-per-SM kernels hold every SM (default 0; 0 <= value < SM count).  The kernel that
+                                        sums or finishes long rows in front of a large level does not keep off them: it takes a
+                                        few us where no row is long, and up to the time of its longest rows */
     S2V_OPT_FIRST_LEVEL_TABLE = 5    /* first level from one-hot tags as a gather-sum over the product table ReLU(W_in) * W
                                         (see s2v_level_first_f32): 1 (default) whenever d allows, 0 never (the level kernels'
                                         own table-lookup form is used instead) */
