@@ -74,14 +74,14 @@ __device__ __forceinline__ void long_row_by_warp(const float* __restrict__ H, co
 
 // One row by the whole CTA: the threads copy the neighbour rows through a ring, TURN rows side by side, and the first D threads add one
 // column each.  A stage costs about 300 cycles (wait, barrier, copies) and 6 to 10 per row, and a row of a large H takes 1.5 us to arrive: so
-// stages of two turns where the ring has room for four of them, and up to eight stages.  (d = 128, ring of 80 KB, one row of 262,144 entries,
-// us: stages of 16 rows 4,020, of 32 2,370; with four stages of 32 rows and each stage's indices loaded one stage ahead 5,900.)
+// stages of two turns where the ring has room for four of them (four, not three, where there is room for more), and up to eight stages.  (d = 128, ring of 80 KB, one row of 262,144 entries,
+// us: stages of 16 rows 4,020, of 32 2,370; ring of 110 KB, stages of 48 rows 2,820, of 32 2,460; with four stages of 32 rows and each stage's indices loaded one stage ahead 5,900.)
 template <int D, int THREADS, int BYTES, bool HAS_VAL>
 __device__ __forceinline__ void long_row_by_cta(unsigned char* ring, const float* __restrict__ H, const int32_t* __restrict__ col,
                                                 const float* __restrict__ val, int n, float* out_row)
 {
     constexpr int PIECES = D / 4, TURN = THREADS / PIECES, FIT = BYTES / (TURN * 4 * D);
-    constexpr int TURNS = FIT < 8 ? 1 : (FIT / 4 < 4 ? FIT / 4 : 4), STAGE = TURN * TURNS, NS = FIT / TURNS < 8 ? FIT / TURNS : 8;   // turns and rows per stage, stages
+    constexpr int TURNS = FIT < 8 ? 1 : (FIT < 16 ? 2 : 4), STAGE = TURN * TURNS, NS = FIT / TURNS < 8 ? FIT / TURNS : 8;   // turns and rows per stage, stages
     static_assert(NS >= 3, "two stages on their way while one is added");
     const int piece = threadIdx.x % PIECES, row0 = threadIdx.x / PIECES;
     const int stages = (n + STAGE - 1) / STAGE;
