@@ -779,7 +779,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
     uint32_t* const xo_s = reinterpret_cast<uint32_t*>(smem + map.tags);
     uint2* const chunks = reinterpret_cast<uint2*>(smem + map.col);
     uint4* const chunks_t = reinterpret_cast<uint4*>(smem + map.col);
-    uint4* const p_chunks = reinterpret_cast<uint4*>(smem + Cfg::OFF_S);   // TR, first level
+    uint4* const p_chunks = reinterpret_cast<uint4*>(smem + Cfg::OFF_S);   // TR, first level: as long as `chunks_t`, which the launch keeps within S_BYTES
     float4* const H4 = reinterpret_cast<float4*>(smem + Cfg::OFF_H);
     const ulonglong2* const H2 = reinterpret_cast<const ulonglong2*>(smem + Cfg::OFF_H);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + map.bar);
@@ -1627,6 +1627,8 @@ int s2v_launch_graph_fused(s2v_ctx* ctx, cudaStream_t st, const s2v_graph_fused_
     p.tm_cols = a.d == 128 ? 256 : cols;   // d = 128: W^T and the accumulators of two row blocks
     const uint32_t left = (budget - total(0)) / 16 * 16, enough = (uint32_t)(cap * std::max(6.0, 1.25 * per_row)) / 2 * 2 * chunk;   // (more would take from the cache)
     p.chunk_cap = (int)((left < enough ? left : enough) / chunk);
+    // the first level's list at d = 128 (p_chunks) has a chunk for each of these in the operand buffer, right in front of H
+    static_assert((gf_budget(8) - GfCfg<128>::OFF_H - 128 * GfCfg<128>::ROWB) / GfCfg<128>::CHUNK <= GfCfg<128>::S_BYTES / GfCfg<128>::CHUNK, "cap = 128, two CTAs per SM");
     const uint32_t smem = total(p.chunk_cap);
     const int64_t most = (int64_t)ctx->sm_count * per_sm;
     const unsigned blocks = (unsigned)(a.G < most ? a.G : most);
