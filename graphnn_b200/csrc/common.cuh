@@ -173,9 +173,15 @@ int s2v_launch_level_tc(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n
                         const int32_t* col_idx, const float* val, const float* H, const float* W, const float* X,
                         const float* table, const int32_t* x_index, int n_table, float* out);
 int s2v_launch_wait_selftest(s2v_ctx* ctx, cudaStream_t st);
-// Large matrices, d = 32, 64, 128 (level_stream.cu).  Below, its warps' start and its two launches cost more than they save where rows are of one
-// size (6 entries a row, us, before and with it: d = 32 100,000 rows 24.6 and 27.8, 131,072 47 and 33; d = 64 65,000 26.7 and 30.2, 131,072
-// 48.7 and 47.2; d = 128 30,000 24.7 and 28.2, 131,072 89.6 and 85.8).
+// Large matrices, d = 32, 64, 128 (level_stream.cu).  Its warps' start and its second launch cost 3 to 10 us, which rows of one size pay back from 30,000 to
+// 130,000 rows on; 131,072 is the safe end of that at every d.  Median us of the kernel without it and of it, other buffers for each call and the L2
+// flushed, uniform rows of 2 and of 6 entries, dense X:
+//                     d = 32                  d = 64                  d = 128
+//      30,000    20.5 19.5  22.5 21.5    18.4 25.6  20.5 29.5    26.7 26.7  32.8 35.8     (d = 128, 2 entries: level_tc.cu both times)
+//     100,000    32.8 29.7  38.9 33.8    34.8 35.8  45.1 42.0    55.3 55.3  78.0 70.7
+//     131,072    43.0 29.7  51.2 35.8    39.9 42.0  52.2 48.1    62.5 62.5  95.2 89.1
+//     200,000    52.3 33.8  66.6 41.0    54.3 54.3  76.8 66.6    91.1 91.1   155  134
+// R-MAT, 16 x 2 entries a row, gains at each of 2^13 to 2^17 rows: d = 64 92 -> 36 at 2^13, 305 -> 101 at 2^16; d = 128 106 -> 53, 341 -> 156.
 constexpr int64_t S2V_STREAM_ROWS = 131072;
 int s2v_launch_level_stream(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, int d, const void* row_ptr, bool rp64, const int32_t* col_idx,
                             const float* val, const float* H, const float* W, const float* X, const float* table, const int32_t* x_index, int n_table,

@@ -10,7 +10,7 @@
 // diagonal, so a CTA that owns whole graphs never needs a row of another CTA: HBM sees the CSR, the tags and the
 // results, and the neighbour sums read shared memory at 128 bytes per clock instead of L2.
 //
-// Bounded by the shared-memory reads of the gather (66 % of that pipe) and instruction issue (50 %); HBM and tensor pipe are
+// Bounded by the shared-memory reads of the gather (63 % of that pipe) and instruction issue (47 %); HBM and tensor pipe are
 // idle most of the time.  Measured against one launch per level and the older kernel for d = 128: 64 small graphs, d = 64,
 // 56 -> 16 us; 700 molecules, d = 128, 82 -> 44; 4,093 220 -> 142; 16,384 645 -> 437; 4,096 proteins, d = 64, 1856 -> 1345.
 //
@@ -1227,7 +1227,9 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) s2v_graph_fuse
                         }
                     }
                     // Rows whose maxima are taken side by side (a row past the end: zeros): shuffles are worth it (4,096 proteins 1402 -> 1320 us, together
-                    // with the drain under the last product), the one instruction of d = 128 is not (16,384 molecules 438 us, with two rows 447).
+                    // with the drain under the last product; one row at a time as everything else is now: 2,000 proteins, 16 warps, 703 us instead of 683; two rows at eight
+                    // warps, 8,000 molecules at d = 64 192.4 -> 189.3, 16,000 at d = 32 183.8 -> 181.4), the one instruction of d = 128 is not (16,384 molecules 438 us,
+                    // with two rows 447).
                     constexpr int SB = Cfg::TR ? 1 : (WARPS == 16 && RPG >= 4 ? 4 : 2);
                     static_assert(RPG % SB == 0, "whole batches");
 #pragma unroll

@@ -434,8 +434,9 @@ int launch_d(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, cons
 //     131,072 rows   .84 .74 .81 .82      .93 .84 .90 .90      .98 .91 .96 .97      1.02  .94 1.00  .99   1.06  .98 1.02 1.02
 //     524,288        .83 .65 .75 .79      .94 .79 .85 .90     1.03 .95 .99 1.04     1.19 1.09 1.13 1.11   1.33 1.26 1.29 1.31
 // Hence 3 entries with X and 3.5 without.  (Long rows turn it: half a million rows of one entry and 2,000 of 131, 347 us there and 255; but a caller with so few
-// entries has hardly any.)  At d = 64 rows of one entry take .83 to .91, of two .90 to 1.01, of three .96 to 1.10, and with hubs up to 3.2:
-// level_stream.cu throughout.
+// entries has hardly any.)  At d = 64 level_stream.cu throughout: the same line would lie at two entries (us there and here, with X: 131,072 rows of one entry 31.0
+// and 37.0, of two 35.6 and 38.8, of three 39.5 and 39.3; a million 185 and 207, 216 and 213, 251 and 240; without X 176 and 222 of one, 206 and 211 of
+// two), but with hubs the other kernel takes up to 3.2 times as long, more than a caller with few entries would gain.
 extern "C" int s2v_level_path(int64_t n_rows, int d, int64_t nnz, int offsets64, int dense_x, int level_tc)
 {
     if (level_tc == 0 || (d != 32 && d != 64 && d != 128)) return S2V_LEVEL_PATH_MMA;

@@ -5,24 +5,27 @@
 // The sum is a gather of random rows of H, and what bounds it is how many bytes an SM keeps on their way: a kernel that only sums, with 2,048
 // threads per SM, takes 333 us for a million rows with 8.4 million entries (d = 64, X read and out written), where level_tc.cu, whose warps
 // gather, convert and store by turns, took 473.  So some warps do nothing but gather, and others take the sums through the tensor core and
-// out.  Measured against the kernels it replaced from S2V_STREAM_ROWS rows on (us, other buffers each time; Erdos-Renyi, 8 entries a row):
-// d = 32, a million rows, 354 -> 191; d = 64, a million, 474 -> 367, with edge weights 491 -> 420; d = 128, half a million, 582 -> 412;
-// 2 entries a row: d = 64 216 -> 215, d = 128 203 -> 227; R-MAT with 2^20 rows, d = 128, 2,910 -> 1,710.
+// out.  Measured against the kernels it replaced from S2V_STREAM_ROWS rows on (us; other buffers each time and the L2 flushed; Erdos-Renyi, 8 entries a
+// row, dense X): d = 32, a million rows, 361 -> 200; d = 64, a million, 483 -> 376; d = 128, half a million, 591 -> 416; R-MAT with 2^20 rows, d = 64,
+// 1,830 -> 640, with 2^19, d = 128, 937 -> 580.  Rows of 2 entries: d = 64, a million, 216 -> 213 (of one 185 -> 207); d = 128: s2v_level_path.
 //
 // A tile is 16 units; a unit is what a warp sums at a time: a row for each group of d/4 lanes, two rows at d = 128.
 //
 //   gather warps  : take units one by one (a counter in shared memory).  Four 16-byte loads a lane go out together (d = 128: eight), and the
 //                   next unit's indices and row offsets are on their way meanwhile.  Entries are added in CSR order.  A sum is split into a
 //                   TF32 head and tail and stored as a row of the K-major B operand of its tile (four tiles in shared memory).  d = 32, 64:
-//                   2 x 19 warps per SM at 40 registers (d = 64: one CTA of 15 warps, eight loads each: 404 us with the same buffers each
-//                   time, 367 so).  d = 128: tensor memory holds W^T once, so one CTA per SM, 15 warps at 80 registers, with the unit
+//                   2 x 19 warps per SM at 40 registers (d = 64, a million rows, the same buffers each time: one CTA of 15 warps with eight
+//                   loads each 404 us, this 367).  Instances with edge weights and those of d = 128 spill 4 to 16 bytes.
+//                   d = 128: tensor memory holds W^T once, so one CTA per SM, 15 warps at 80 registers, with the unit
 //                   behind the next one begun too.
 //   MMA warp      : out^T = W^T * sum^T: W^T (A operand, head and tail; 128 / d copies below each other) stays in tensor memory, 3 * d/8
 //                   tcgen05.mma of 128 x ROWS x 8 per tile (lo*hi, hi*lo, hi*hi) into one of several accumulators.  It also asks for the
 //                   next tiles: the grid has a CTA per tile, and a running CTA takes over tiles whose CTAs have not started
 //                   (clusterlaunchcontrol), so that an SM that starts late or has longer rows does fewer of them.
 //   epilogue warps: an accumulator lane is an output column (the copies: of other rows), so X is read and out written 128 bytes per
-//                   instruction, both past the L2's other contents, which is left to H.
+//                   instruction, both past the L2's other contents, which is left to H (three levels in a row, where out is the next one's H:
+//                   d = 64, 400,000 rows, 8 entries, 381 us, with ordinary stores 384; d = 32 206 and 209; d = 128 946 and 929; 131,072 and 200,000 rows
+//                   0 to 1 % in its favour).
 //
 // Rows of more than LS_LONG entries would hold up their tile.  A kernel in front finishes them (sum, product, X, ReLU); this kernel, its
 // programmatic dependent, does not wait for it before its own end and leaves those rows out.
@@ -93,7 +96,7 @@ __device__ __forceinline__ void ls_ld_cols8(uint32_t addr, uint32_t* v)
 }
 // 16 bytes of a row.  (Volatile: the loads of a step stay together.  Under a condition, which the additions share, the compiler made one
 // branch of both, and every load waited for the addition before it: d = 64, a million rows, 596 us instead of 404.  Lanes past the end of
-// their row load its last entry again, or row 0; as one load for zeros, or at row 0 always, 378 and 382 us instead of 367.)
+// their row load its last entry again, or row 0; as one load for zeros, or at row 0 always, 378 and 382 us instead of 367, the same buffers each time.)
 __device__ __forceinline__ ulonglong2 ls_row(const ulonglong2* p)
 {
     ulonglong2 v;

@@ -8,8 +8,9 @@
 //     one, taken first, is streamed through a ring in shared memory by the whole CTA, where one warp would be bounded by latency.
 //   * Entries are added one after the other in CSR order, as everywhere else in the level: a float sum of 10^5 entries
 //     depends on its order in the fifth digit.
-//   * In large levels (LongCfg::FRONT_ROWS; level_stream.cu finishes such rows its own way) a kernel in front makes the sums, with the level
-//     kernel launched as its programmatic dependent.  With the look and the sums inside, the registers of the main loop cost every level 1 - 5 %, also without a long row
+//   * In large levels (LongCfg::FRONT_ROWS) a kernel in front makes the sums, with the level kernel launched as its programmatic dependent: in level_tc.cu
+//     for sparse matrices at d = 128, in level.cu where tcgen05 is switched off (level_stream.cu finishes such rows its own way).  The figures are of a time
+//     when these two took every large level.  With the look and the sums inside, the registers of the main loop cost every level 1 - 5 %, also without a long row
 //     (Erdos-Renyi, a million rows: d = 64 480 us inside, 474 in front, 473 without any of it; with edge weights 526, 473, 472;
 //     d = 32 366, 351, 349; d = 128, half a million, 601, 584, 585; R-MAT 2^20, d = 128: 4.9 ms inside, 2.9 in front).  A second
 //     launch costs up to 1 us: below, the level kernel does it for the rows it owns (30,000 rows, d = 64: 13.5 us, 14.1 in front).

@@ -71,7 +71,7 @@ typedef enum s2v_option {
     S2V_OPT_VALIDATE_HOST_INPUT = 1, /* s2v_infer_host_f32 scans its host arrays before any launch (default 1;
                                         the environment variable S2V_VALIDATE_HOST=0 sets the default to 0) */
     S2V_OPT_LEVEL_TC = 2,            /* tcgen05 kernels: 0 never; 1 automatic (default): levels of d = 64 and 128 with 32-bit offsets at
-                                        every size, the table-lookup form of the first level from 16,384 rows on, the readout from
+                                        every size, those of d = 32 and with 64-bit offsets from 131,072 rows on, the table-lookup form of the first level from 16,384 rows on, the readout from
                                         6,144 graphs on; 2: those two earlier (any size; 512 graphs).  Default from S2V_LEVEL_TC */
     S2V_OPT_GRAPH_TILES = 3,         /* whole-classifier kernel inside s2v_forward_f32 for batches of small and medium graphs (at most
                                         128 nodes at d = 128, 640 at d = 64, 1024 at d = 32): 0 never; 1 whenever the batch allows,
