@@ -592,7 +592,7 @@ s2v_level_hub_kernel(int64_t n_rows, int rows_per_cta, const RpT* __restrict__ r
     }
 }
 
-// ONE: some SMs are left to others (S2V_OPT_RESERVED_SMS); the kernel in front does not keep off them, but ends early
+// ONE: some SMs are left to others (S2V_OPT_RESERVED_SMS); the kernel in front does not keep off them
 template <int D, bool HAS_VAL, int XMODE, typename RpT, bool ONE>
 int ls_launch_on(s2v_ctx* ctx, cudaStream_t st, bool long_rows, int64_t n_rows, const RpT* rp, const int32_t* ci, const float* val, const float* H,
                  const float* W, const float* X, const int32_t* x_index, int n_table, float* out)
