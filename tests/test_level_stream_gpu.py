@@ -88,7 +88,8 @@ def test_long_rows_of_one_block(gpu_ctx, d, weights, together):
 
 
 def test_one_long_row_is_as_fast_per_byte_at_d_128(gpu_ctx):
-    """(1.84 times the time of d = 64 with stages of 32 rows and 96 rows on their way, 1.34 now; H does not fit the L2)"""
+    """(1.84 times the time of d = 64 with stages of 32 rows and 96 rows on their way; 1.41 now, through the kernel in front of level_tc.cu, which
+    a matrix with so few entries a row takes at d = 128, 1.34 through level_stream.cu; H does not fit the L2)"""
     n, long = 4 * LEAST, 2 * LEAST
     gen = torch.Generator(device="cuda").manual_seed(1)
     deg = torch.ones(n, dtype=torch.int64, device="cuda")
